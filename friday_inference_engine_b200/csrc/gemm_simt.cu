@@ -1,14 +1,23 @@
 // out[m][n] = sum_k a[m][k] * w[n][k]  (+ bias[n]) (+ residual[m][n])
 //
-// CUDA-core matrix product with fp32 multiply-adds in the order of k: the true
-// 32-bit path of the model (no tensor cores, no reduced-precision mode), and the
-// fallback of the bf16 path for sizes that the tensor-core kernel refuses.  Both
-// operands are row-major with k innermost, which is how activations [rows][k] and
-// projection weights [out][in] are stored, so nothing is transposed.  Any m, n, k.
+// CUDA-core matrix product with fp32 multiply-adds: the true 32-bit path of the model
+// (no tensor cores, no reduced-precision mode), and the fallback of the bf16 path for
+// sizes that the tensor-core kernel refuses.  Both operands are row-major with k
+// innermost, which is how activations [rows][k] and projection weights [out][in] are
+// stored, so nothing is transposed.  Any m, n, k.  Three kernels:
+//
+//   gemm_f32_kernel    fp32 operands in 16-byte pieces, more than FEW_ROWS rows: tiles
+//                      in registers, k in two interleaved sums (fma.rn.f32x2), k split
+//                      over the CTAs of a cluster where there are few tiles;
+//   few_rows_kernel    the same operands, up to FEW_ROWS rows: a warp per few columns,
+//                      its lanes along k;
+//   gemm_simt_kernel   everything else (mixed storage, unaligned rows).
 //
 // The reference's counterpart is its int8 tensor-core GEMM with the same epilogue
 // (bias, then residual, in place allowed): prefill_kernels.cu:156-171, 173-327.
 #include "common.cuh"
+
+#include <atomic>
 
 FR_EXPORT const char* gemm_simt_last_error() { return fr_error_text; }
 
@@ -87,6 +96,268 @@ int launch(const void* a, const void* w, void* out, FrVec bias, const void* resi
     return FR_OK;
 }
 
+
+// ------------------------------------------------------------------ fp32 operands in 16-byte pieces
+typedef unsigned long long Pair;                            // two floats: the sums over k = 0, 2, ... and 1, 3, ...
+__device__ __forceinline__ void fma_pair(Pair& acc, Pair x, Pair y) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(x), "l"(y)); }
+__device__ __forceinline__ float pair_sum(Pair v) { return __uint_as_float((uint32_t)v) + __uint_as_float((uint32_t)(v >> 32)); }
+
+struct F32Args {
+    const float* a;
+    const float* w;
+    float* out;
+    FrVec bias;
+    const float* residual;
+    int m, n, k, lda, ldw, ldo;
+    int splits, kb_per;          // CTAs of the cluster that share a tile's k, k blocks of each
+};
+
+__device__ __forceinline__ void finish(const F32Args& p, int gm, int gn, float v) {
+    if (gm >= p.m || gn >= p.n) return;
+    if (p.bias.p != nullptr) v += p.bias.at(gn);
+    const size_t at = (size_t)gm * p.ldo + gn;
+    if (p.residual != nullptr) v += p.residual[at];
+    p.out[at] = v;
+}
+
+constexpr int F32_BK = 32, F32_LD = F32_BK + 4, F32_STAGES = 3;   // LD: eight consecutive rows' 16-byte pieces lie in different banks
+template <int TM, int TN>
+constexpr int f32_smem() { return F32_STAGES * (8 * TM + 16 * TN) * F32_LD * 4; }
+
+// 128 threads, 8 TM x 16 TN outputs, TM x TN per thread: a warp has 4 rows x 8 columns of threads, whose rows and columns lie
+// 4 and 8 apart.  Both operands keep their k-innermost layout in shared memory, so that a 16-byte read gives two operand pairs
+// of the packed multiply-add as they are; the two halves of an accumulator are added at the end.  Bound by the rate of the
+// multiply-adds: per 4 k a warp issues 2 TM TN of them (two cycles each) and TM + TN shared-memory reads.
+template <int TM, int TN>
+__global__ void __launch_bounds__(128, 2)
+gemm_f32_kernel(const F32Args p) {
+    constexpr int BM = 8 * TM, BN = 16 * TN, STAGE = (BM + BN) * F32_LD;
+    extern __shared__ __align__(16) float sm[];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tile = blockIdx.x / p.splits, split = blockIdx.x - tile * p.splits;
+    const int m0 = blockIdx.y * BM, n0 = tile * BN;
+    const int kb0 = split * p.kb_per, kb1 = min((p.k + F32_BK - 1) / F32_BK, kb0 + p.kb_per);
+    // neighbouring lanes share a column, so that both operands of a half-warp take one pass through the banks
+    const int row0 = (warp >> 1) * 4 * TM + (lane >> 4) * 2 + (lane & 1), col0 = (warp & 1) * 8 * TN + ((lane >> 1) & 7);
+    fr_pdl_wait();
+    fr_pdl_launch();
+    auto fill = [&](int kb, int stage) {
+        float* base = sm + stage * STAGE;
+#pragma unroll
+        for (int i = 0; i < (BM + BN + 15) / 16; ++i) {
+            const int idx = tid + i * 128, r = idx >> 3, c = (idx & 7) * 4;
+            if ((BM + BN) % 16 != 0 && r >= BM + BN) break;
+            const int gk = kb * F32_BK + c;
+            const bool of_a = r < BM;
+            const int g = of_a ? m0 + r : n0 + r - BM;
+            const bool there = gk < p.k && g < (of_a ? p.m : p.n);
+            const float* src = there ? (of_a ? p.a + (size_t)g * p.lda + gk : p.w + (size_t)g * p.ldw + gk) : p.w;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(base + r * F32_LD + c)),
+                         "l"(src), "r"(there ? 16 : 0)
+                         : "memory");
+        }
+    };
+    Pair acc[TM][TN];
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = 0ull;
+#pragma unroll
+    for (int s = 0; s < F32_STAGES - 1; ++s) {
+        if (kb0 + s < kb1) fill(kb0 + s, s);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    int stage = 0;
+    for (int kb = kb0; kb < kb1; ++kb) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(F32_STAGES - 2) : "memory");
+        __syncthreads();                                     // this block is here, and everyone is done with the one before
+        const int refill = stage == 0 ? F32_STAGES - 1 : stage - 1;
+        if (kb + F32_STAGES - 1 < kb1) fill(kb + F32_STAGES - 1, refill);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const float* as = sm + stage * STAGE + row0 * F32_LD;
+        const float* ws = sm + stage * STAGE + (BM + col0) * F32_LD;
+#pragma unroll
+        for (int kk = 0; kk < F32_BK; kk += 4) {
+            ulonglong2 x[TM];
+#pragma unroll
+            for (int i = 0; i < TM; ++i) x[i] = *(const ulonglong2*)(as + i * 4 * F32_LD + kk);
+#pragma unroll
+            for (int j = 0; j < TN; ++j) {
+                const ulonglong2 y = *(const ulonglong2*)(ws + j * 8 * F32_LD + kk);
+#pragma unroll
+                for (int i = 0; i < TM; ++i) fma_pair(acc[i][j], x[i].x, y.x);
+#pragma unroll
+                for (int i = 0; i < TM; ++i) fma_pair(acc[i][j], x[i].y, y.y);
+            }
+        }
+        if (++stage == F32_STAGES) stage = 0;
+    }
+    if (p.splits == 1) {
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) finish(p, m0 + row0 + 4 * i, n0 + col0 + 8 * j, pair_sum(acc[i][j]));
+        return;
+    }
+    // the tile's parts lie in the shared memory of the cluster's CTAs; each finishes a share of it, adding them in order of k
+    static_assert(BM * BN <= F32_STAGES * STAGE, "the partial tile takes the ring's place");
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) sm[(row0 + 4 * i) * BN + col0 + 8 * j] = pair_sum(acc[i][j]);
+    fr_cluster_sync();
+    for (int idx = (split * 128 + tid) * 4; idx < BM * BN; idx += p.splits * 512) {
+        float4 v = fr_cluster_load4(sm + idx, 0);
+        for (int s = 1; s < p.splits; ++s) {
+            const float4 o = fr_cluster_load4(sm + idx, s);
+            v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
+        }
+        const int gm = m0 + idx / BN, gn = n0 + idx % BN;
+        finish(p, gm, gn, v.x);
+        finish(p, gm, gn + 1, v.y);
+        finish(p, gm, gn + 2, v.z);
+        finish(p, gm, gn + 3, v.w);
+    }
+    fr_cluster_sync();                                       // nobody leaves while its shared memory is being read
+}
+
+// Bound by reading the weights once (or by the launch, for small ones).  Up to MR rows per block: a warp has NC columns, its lanes take 16-byte pieces of k in turn, every weight is read once per
+// block of rows; the MR * NC sums are then added over the lanes so that lane l ends with the l-th.
+// Four columns per warp where there are enough of them to keep the SMs' loads in flight: a piece of x is then read once for
+// four weights (4 x 37888 x 3584: 108 us, 5.0 TB/s, against 129 with one column; 2 x 5000 x 3584 22 us either way).  Against
+// the general kernel: 694 and 338 us.  At 9 to 16 rows the weights are read twice, the second time from L2: up to 8,191
+// columns that beats the tiles (12 x 3584 x 3584: 30 us against 38, 16 x 4608 x 3584: 35 against 44), above it does not
+// (12 x 37888 x 3584: 212 us on tiles, the fastest form).
+constexpr int FEW_ROWS = 16, FEW_ROWS_WIDE = 8;
+template <int MR, int NC>
+__global__ void __launch_bounds__(128)
+few_rows_kernel(const F32Args p) {
+    constexpr int V = MR * NC;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n0 = (blockIdx.x * 4 + warp) * NC, m0 = blockIdx.y * MR;
+    fr_pdl_wait();
+    fr_pdl_launch();
+    if (n0 >= p.n) return;
+    Pair acc[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) acc[v] = 0ull;
+    const ulonglong2* w[NC];
+    const ulonglong2* x[MR];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) w[c] = (const ulonglong2*)(p.w + (size_t)min(n0 + c, p.n - 1) * p.ldw);
+#pragma unroll
+    for (int r = 0; r < MR; ++r) x[r] = (const ulonglong2*)(p.a + (size_t)min(m0 + r, p.m - 1) * p.lda);
+#pragma unroll 2
+    for (int q = lane; q < p.k / 4; q += 32) {
+        ulonglong2 y[NC];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) y[c] = __ldg(w[c] + q);
+#pragma unroll
+        for (int r = 0; r < MR; ++r) {
+            const ulonglong2 z = x[r][q];
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                fma_pair(acc[r * NC + c], z.x, y[c].x);
+                fma_pair(acc[r * NC + c], z.y, y[c].y);
+            }
+        }
+    }
+    float s[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) s[v] = pair_sum(acc[v]);
+    // halve the values and double the lanes behind each: the half that a lane keeps is chosen by one of its bits
+    int at = 0;
+#pragma unroll
+    for (int half = V / 2, bit = 16; bit > 0; bit >>= 1) {
+        if (half > 0) {
+            const bool upper = (lane & bit) != 0;
+#pragma unroll
+            for (int v = 0; v < V / 2; ++v)
+                if (v < half) {
+                    const float give = upper ? s[v] : s[v + half], keep = upper ? s[v + half] : s[v];
+                    s[v] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+                }
+            if (upper) at += half;
+            half >>= 1;
+        } else {
+            s[0] += __shfl_xor_sync(0xffffffffu, s[0], bit);
+        }
+    }
+    constexpr int SPARE = 32 / V;                            // lanes with the same value
+    if (lane % SPARE == 0) finish(p, m0 + at / NC, n0 + at % NC, s[0]);
+}
+
+template <int MR, int NC>
+int launch_few(const F32Args& p, cudaStream_t stream) {
+    FR_CUDA(fr_launch(few_rows_kernel<MR, NC>, dim3((p.n + 4 * NC - 1) / (4 * NC), (p.m + MR - 1) / MR), dim3(128), 0, stream, p));
+    FR_CHECK_LAUNCH("gemm_simt (few rows)");
+    return FR_OK;
+}
+
+template <int TM, int TN>
+int launch_f32(const F32Args& p, cudaStream_t stream) {
+    static std::atomic<unsigned long long> configured{0};    // devices (as bits) on which the limit has been raised
+    int device = 0;
+    FR_CUDA(cudaGetDevice(&device));
+    if (device < 0 || device >= 64) FR_REFUSE("gemm_simt: device %d is outside the table of 64", device);
+    if (!(configured.load(std::memory_order_acquire) & (1ull << device))) {
+        FR_CUDA(cudaFuncSetAttribute(gemm_f32_kernel<TM, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, f32_smem<TM, TN>()));
+        configured.fetch_or(1ull << device, std::memory_order_release);
+    }
+    const dim3 grid((p.n + 16 * TN - 1) / (16 * TN) * p.splits, (p.m + 8 * TM - 1) / (8 * TM));
+    FR_CUDA(fr_launch_cluster(gemm_f32_kernel<TM, TN>, grid, dim3(128), f32_smem<TM, TN>(), stream, (unsigned)p.splits, p));
+    FR_CHECK_LAUNCH("gemm_simt (fp32)");
+    return FR_OK;
+}
+
+// Tile and split of k: the choice whose busiest SM has the least to do (a lone CTA leaves a third of the multiply-add rate).
+// Measured on B200, this kernel against the general one below: 333 x 37888 x 3584 1,902 us (47.6 TFLOP/s; two thirds of the
+// rate at 1.88 GHz, whatever the tile and with plain multiply-adds too) against 3,998, 333 x 3584 x 18944 1,070 (7 x 8, four
+// splits) against 2,923, 64 x 3584 x 3584 57 against 338, 40 x 3584 x 18944 164 against 3,133.
+struct F32Plan {
+    int tm, tn, splits;
+};
+F32Plan f32_plan(int m, int n, int k, int sms) {
+    F32Plan best{8, 8, 1};
+    double best_cost = 1e300;
+    const int kb = (k + F32_BK - 1) / F32_BK;
+    for (int tn = 8; tn >= 4; tn -= 4)
+        for (int tm = 8; tm >= 4; --tm) {
+            const long long tiles = (long long)((m + 8 * tm - 1) / (8 * tm)) * ((n + 16 * tn - 1) / (16 * tn));
+            for (int s = 1; s <= 8; ++s) {
+                if (s > 1 && kb < 4 * s) break;
+                if (s > 2 && s != 4 && tiles * s > sms) continue;      // several waves of clusters of other sizes leave places empty
+                const int per = (kb + s - 1) / s;
+                const long long load = (tiles * s + sms - 1) / sms;
+                const double block = tm * tn + 8.0;           // a k block's multiply-adds and what goes with them
+                const double cost = (load == 1 ? 1.5 : (double)load) * (per * block + 4 * 64.0 + (s > 1 ? 4 * 64.0 : 0.0));
+                if (cost < best_cost) { best_cost = cost; best = F32Plan{tm, tn, s}; }
+            }
+        }
+    return best;
+}
+
+int run_f32(F32Args p, cudaStream_t stream) {
+    if (p.m <= (p.n < 8192 ? FEW_ROWS : FEW_ROWS_WIDE)) {
+        const bool wide = p.n >= 2368;
+        if (p.m == 1) return wide ? launch_few<1, 4>(p, stream) : launch_few<1, 1>(p, stream);
+        if (p.m == 2) return wide ? launch_few<2, 4>(p, stream) : launch_few<2, 1>(p, stream);
+        if (p.m <= 4) return wide ? launch_few<4, 4>(p, stream) : launch_few<4, 1>(p, stream);
+        return wide ? launch_few<8, 4>(p, stream) : launch_few<8, 1>(p, stream);
+    }
+    const int sms = fr_sm_count();
+    const F32Plan plan = f32_plan(p.m, p.n, p.k, sms > 0 ? sms : 148);
+    const int kb = (p.k + F32_BK - 1) / F32_BK;
+    p.splits = plan.splits;
+    p.kb_per = (kb + p.splits - 1) / p.splits;
+#define FR_TILE(TM, TN) if (plan.tm == TM && plan.tn == TN) return launch_f32<TM, TN>(p, stream)
+    FR_TILE(8, 8); FR_TILE(7, 8); FR_TILE(6, 8); FR_TILE(5, 8); FR_TILE(4, 8);
+    FR_TILE(8, 4); FR_TILE(7, 4); FR_TILE(6, 4); FR_TILE(5, 4); FR_TILE(4, 4);
+#undef FR_TILE
+    FR_REFUSE("gemm_simt: no tile of %d x %d", plan.tm, plan.tn);
+}
+
 }  // namespace
 
 // a: [m][k] (row stride lda), w: [n][k] (row stride ldw), out and residual: [m][n]
@@ -99,6 +370,10 @@ FR_EXPORT int gemm_simt(const void* a, int a_dtype, const void* w, int w_dtype, 
     if (k <= 0) FR_REFUSE("gemm_simt: k = %d", k);
     FrVec bv{bias, bias_dtype};
     typedef __nv_bfloat16 bf16;
+    // rows in 16-byte pieces (and no grid beyond the launch limits): the fp32 kernels
+    if (a_dtype == FR_F32 && w_dtype == FR_F32 && out_dtype == FR_F32 && !((k | lda | ldw) & 3) && !(((uintptr_t)a | (uintptr_t)w) & 15) &&
+        m <= 65535 * 32)
+        return run_f32(F32Args{(const float*)a, (const float*)w, (float*)out, bv, (const float*)residual, m, n, k, lda, ldw, ldo, 1, 0}, stream);
     const int key = a_dtype * 4 + w_dtype * 2 + out_dtype;
     switch (key) {
         case 0: return launch<float, float, float>(a, w, out, bv, residual, m, n, k, lda, ldw, ldo, stream);

@@ -1,0 +1,40 @@
+"""Matrix products at the edges of their kernels' ranges: rows around the tiles' heights, columns around their widths, k around
+the blocks, unaligned rows, strided operands; against 64-bit sums."""
+import pytest
+import torch
+
+from friday_inference_engine_b200 import ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def rnd(shape, seed, scale=1.0):
+    return (torch.randn(shape, generator=torch.Generator().manual_seed(seed)) * scale).to(DEV)
+
+
+# up to 8 / 16 rows a warp per columns, then tiles of 32 to 64 rows; one column and four per warp meet at 2,368 columns,
+# narrow and wide results at 8,192; k = 4 (one 16-byte piece), around 32 and 128, long enough for every split
+@pytest.mark.parametrize("m", [1, 2, 3, 5, 8, 9, 16, 17, 33, 57, 129, 333])
+@pytest.mark.parametrize("n,k", [(1, 4), (65, 36), (129, 128), (2371, 260), (8195, 100), (3584, 4100)])
+def test_float32_product(m, n, k):
+    a, w, bias, res = rnd((m, k), 1), rnd((n, k), 2, 0.05), rnd((n,), 3), rnd((m, n), 4)
+    want = a.double() @ w.double().T + bias.double() + res.double()
+    # any order of k + 2 roundings of a sum errs by at most (k + 2) units of the sum of the terms' sizes
+    bound = (k + 2) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T + bias.double().abs() + res.double().abs())
+    out = res.clone()
+    ops.backend()._linear_simt(a, w, bias, out, out)
+    assert bool(((out.double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("m", [3, 12, 40])
+@pytest.mark.parametrize("shift", [0, 1, 4])
+def test_float32_product_strided_operands(m, shift):
+    """Rows with a stride of their own; a start off the 16-byte boundary takes the general kernel."""
+    n, k = 70, 64
+    big_a, big_w = rnd((m, k + 8), 5), rnd((n, k + 12), 6)
+    a, w = big_a[:, shift:shift + k], big_w[:, shift:shift + k]
+    out = torch.empty((m, n), device=DEV)
+    ops.backend()._linear_simt(a, w, None, None, out)
+    bound = (k + 2) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
+    assert bool(((out.double() - a.double() @ w.double().T).abs() <= bound).all())
