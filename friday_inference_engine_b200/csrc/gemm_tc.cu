@@ -87,6 +87,7 @@ struct GemmParams {
     int act;            // 1 to 3: the product's columns are (gate, up) pairs and out, half as wide, gets the gated unit fr_gated(act, ...);
                         // ACT_RELU_SQUARED: max(x, 0)^2 of every column
     int tiles_p, tiles_q, splits, kb_total, kb_per;
+    int group_p;        // pairs of SMs: row tiles that go together (gemm_tc_pair.cuh)
     // Work decomposition.  The first dp_tiles tiles are cut into `splits` equal k ranges each and dealt out round
     // robin (splits = 1: whole tiles).  The remaining sk_tiles tiles ("stream-k"): their k blocks, laid end to end,
     // are cut into one contiguous run of sk_units per CTA, so that a last, partial wave of tiles keeps every SM busy.
@@ -1176,6 +1177,7 @@ FR_EXPORT int gemm_tc_fused(const void* x, const void* w, void* out, int out_dty
         p.tiles_p = (m + 2 * TILE_P - 1) / (2 * TILE_P);
         const int pair_tiles = p.tiles_p * p.tiles_q;
         p.dp_tiles = pair_tiles;
+        p.group_p = pair_group(p.tiles_p, p.tiles_q, sm_count / 2);
         CUtensorMap mp, mq;
         int rc = make_map(&mp, x, m, k, lda, TILE_P);
         if (rc) return rc;

@@ -53,6 +53,29 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
                  : "memory");
 }
 
+// Row tiles of a group.  Every group reads all weights again, so wide outputs want groups as high as L2 keeps their rows
+// (17971 x 37888 x 3584, TFLOP/s at 4 / 8 / 12 / 16 / 24 row tiles: 1,304 / 1,353 / 1,373 / 1,372 / 1,364; 4096 rows: 1,310 /
+// 1,344 / 1,345 / 1,379 with all 16 in one).  Where the columns are so few that a handful of row tiles keeps every pair busy,
+// higher groups only spread the rows that are in use (17971 x 3584 x 18944: 1,308 / 1,305 / 1,284 / 1,287 / 1,222, x 4608 x
+// 3584: 1,347 / 1,326 / 1,315 / 1,316 / 1,304).  The groups are made alike.
+inline int pair_group(int tiles_p, int tiles_q, int pairs) {
+    int high = 16;
+    if (2 * tiles_q < pairs) high = (pairs + tiles_q - 1) / tiles_q < 4 ? 4 : (pairs + tiles_q - 1) / tiles_q;
+    const int groups = (tiles_p + high - 1) / high;
+    return (tiles_p + groups - 1) / groups;
+}
+
+// Where a tile lies.  Row tiles go in groups of p.group_p: a group's row tiles run fastest, then its columns, then the next
+// group, so that the 74 tiles that are computed at a time find each other's operands in L2.  With all row tiles in one group
+// a prompt batch of 17,971 rows read its activations (130 MB at k = 3584, as much as L2 holds) again for every column tile:
+// 17971 x 37888 x 3584 ran at 1,106 TFLOP/s under the power cap, 1,372 with groups of 16 (cuBLAS: 1,386).
+__device__ __forceinline__ void pair_tile(const GemmParams& p, int tile, int& p_blk, int& q_blk) {
+    const int group = tile / (p.group_p * p.tiles_q), first = group * p.group_p;
+    const int high = min(p.group_p, p.tiles_p - first), at = tile - first * p.tiles_q;
+    q_blk = at / high;
+    p_blk = first + at - q_blk * high;
+}
+
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_q, const GemmParams p) {
     constexpr int STAGES = PAIR_STAGES, STAGE_BYTES = PAIR_STAGE_BYTES, BN = PAIR_BN;
@@ -109,8 +132,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
                 __device__ void open(const GemmParams& pp) {
                     live = work.next(item);
                     if (!live) return;
-                    q_blk = item.tile / pp.tiles_p;
-                    p_blk = item.tile - q_blk * pp.tiles_p;
+                    pair_tile(pp, item.tile, p_blk, q_blk);
                     kb = item.kb0;
                 }
                 __device__ void step(const GemmParams& pp) {
@@ -190,7 +212,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
         Work work(p, pair, pairs);
         Item item;
         for (; ok && work.next(item); ++it) {
-            const int q_blk = item.tile / p.tiles_p, p_blk = 2 * (item.tile - q_blk * p.tiles_p) + (int)rank;
+            int p_blk, q_blk;
+            pair_tile(p, item.tile, p_blk, q_blk);
+            p_blk = 2 * p_blk + (int)rank;
             const int a = it & 1;
             const uint32_t acc_phase = (it >> 1) & 1;
             const int gi = p_blk * TILE_P + i_local;

@@ -38,3 +38,15 @@ def test_float32_product_strided_operands(m, shift):
     ops.backend()._linear_simt(a, w, None, None, out)
     bound = (k + 2) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
     assert bool(((out.double() - a.double() @ w.double().T).abs() <= bound).all())
+
+
+# pairs of SMs take the row tiles in groups: one group, two alike (17 and 33 row tiles of 256, wide), unequal ones, columns so
+# few that a group has many row tiles, a last row tile of one row
+@pytest.mark.parametrize("m,n,k", [(257, 512, 64), (4097, 9488, 64), (8449, 9600, 72), (3300, 272, 136), (5121, 4608, 64), (2561, 1040, 200)])
+def test_row_groups_on_pairs(m, n, k):
+    a, w, res = (rnd(s, i, c).bfloat16() for i, (s, c) in enumerate((((m, k), 1.0), ((n, k), 0.1), ((m, n), 1.0))))
+    out = ops.linear(a, w, None, res)
+    want = a.double() @ w.double().T + res.double()
+    size = a.double().abs() @ w.double().abs().T + res.double().abs()
+    # the product of two bf16 numbers is exact in 32 bits; k + 1 sums that may cut instead of round, then bf16's rounding
+    assert bool(((out.double() - want).abs() <= (k + 1) * 2.0 ** -23 * size + 2.0 ** -8 * want.abs()).all())
