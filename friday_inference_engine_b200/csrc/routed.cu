@@ -11,13 +11,15 @@
 //   gate_up          for every (row, choice): act = silu(Wg_e h) * (Wu_e h) (or the clipped unit), expert e's rows read where they lie
 //   down_combine     out[row] = residual[row] + sum over choices of weight * (Wd_e act)
 //
-// gate_up and down_combine read only the chosen experts' weights, once per (row, choice): the form for one-token
-// steps, where those bytes are the cost.  With many rows the dense form (all experts through the tensor-core
+// gate_up and down_combine read only the chosen experts' weights, up to 16 rows of bf16 once for all pairs that chose an
+// expert, else once per (row, choice): the form for one-token steps, where those bytes are the cost.  With many rows the dense form (all experts through the tensor-core
 // product, scale_by_route, one down product) does more arithmetic but runs on the tensor cores.
 //
 // Router logits, the choice and the weights are fp32.  Gate and up weights are stored row by row in turn
 // (gate 0, up 0, gate 1, ...), expert after expert: [experts * 2 * inner][width]; down: [width][experts * inner].
 #include <math.h>
+
+#include <atomic>
 
 #include "common.cuh"
 
@@ -184,163 +186,203 @@ gate_up_kernel(const T* __restrict__ h, const int* __restrict__ ids, const T* __
     }
 }
 
-// Few rows: a block owns one expert and a tile of `inner`; it gathers the rows that chose the expert (at most MAX_SHARE,
-// staged in shared memory in their own dtype) and reads every weight row once for all of them, 16 bytes per lane.
-constexpr int MAX_SHARE = 16;
+// Few rows: the weights of the experts that were chosen stream through once for all the (row, choice) pairs that chose them.
+// A unit is two weight rows of one expert: a channel's gate and up rows, or two columns of the down matrix.  The units of all
+// chosen experts, one expert after another, are dealt out over the warps of two blocks per SM.  A warp keeps the next
+// RING - 1 pieces of its units on their way into shared memory (every lane reads back what it copied itself, so nothing is
+// synchronised between threads) and takes its lanes' share of the pairs' activations from L1.  Bound by reading the weights: at
+// width 2048, inner 2048, 8 experts, 16 pairs on a B200 the gate/up and down products of a decoding step take 35 to 39 and 21 to 27
+// us for some 117 and 59 MB (63 to 73 and 44 to 51 us when a block of one expert staged the rows first and then read its weights
+// in a few rounds).
+constexpr int SHARE = 16;                      // pairs of one expert that are finished together; more take the expert again
+constexpr int RING = 4, PIECE = 512;           // pieces of a warp's ring; elements of a weight row in one piece
+constexpr int MAX_FEW = 16;                    // rows of a call that runs here
+constexpr int MAX_FEW_PAIRS = MAX_FEW * 32;
+constexpr int STREAM_WARPS = 8;
+constexpr int STREAM_SMEM = STREAM_WARPS * RING * 2 * PIECE * 2;
 
-template <typename T>
-__global__ void __launch_bounds__(256)
-gate_up_by_expert_kernel(const T* __restrict__ h, const int* __restrict__ ids, const T* __restrict__ w_gate_up, T* __restrict__ act,
-                         int rows, int top, int width, int inner, int per_block, int kind, float limit, float slope) {
-    extern __shared__ __align__(16) unsigned char raw[];
-    T* hs = (T*)raw;                           // [MAX_SHARE][width]
-    __shared__ int pairs[MAX_SHARE];
-    __shared__ int n_pairs;
-    constexpr int PER = 16 / sizeof(T);
-    fr_pdl_wait();
-    fr_pdl_launch();
-    const int e = blockIdx.x;
-    // the pairs that chose this expert, in order: the ids are read side by side, then one thread lists the matches
-    __shared__ int chosen[MAX_SHARE * 32];
-    for (int pr = threadIdx.x; pr < rows * top; pr += blockDim.x) chosen[pr] = ids[pr];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int n = 0;
-        for (int pr = 0; pr < rows * top && n < MAX_SHARE; ++pr)
-            if (chosen[pr] == e) pairs[n++] = pr;
-        n_pairs = n;
-    }
-    __syncthreads();
-    const int n = n_pairs;
-    if (n == 0) return;
-    for (int idx = threadIdx.x; idx < n * (width / PER); idx += blockDim.x) {
-        const int r = idx / (width / PER), c = idx % (width / PER);
-        ((uint4*)(hs + (size_t)r * width))[c] = ((const uint4*)(h + (size_t)(pairs[r] / top) * width))[c];
-    }
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int f0 = blockIdx.y * per_block;
-    const T* w = w_gate_up + (size_t)e * 2 * inner * width;
-    for (int f = f0 + warp; f < min(f0 + per_block, inner); f += 8) {
-        const uint4* g4 = (const uint4*)(w + (size_t)(2 * f) * width);
-        const uint4* u4 = (const uint4*)(w + (size_t)(2 * f + 1) * width);
-        float sg[MAX_SHARE], su[MAX_SHARE];
+template <int N>
+struct Number {
+    static constexpr int value = N;
+};
+
+typedef unsigned long long Two;                // two floats
+__device__ __forceinline__ Two two_of(uint32_t bf16_pair) {
+    return (Two)(bf16_pair << 16) | ((Two)(bf16_pair & 0xffff0000u) << 32);
+}
+__device__ __forceinline__ void fma_two(Two& acc, Two x, Two y) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(x), "l"(y)); }
+__device__ __forceinline__ float sum_two(Two v) { return __uint_as_float((uint32_t)v) + __uint_as_float((uint32_t)(v >> 32)); }
+
+struct StreamArgs {
+    const bf16* x;            // activations: row pair / x_share for pair
+    const int* ids;           // [pairs]
+    const bf16* w;            // row 0 of expert 0
+    void* out;                // gate_up: bf16 [pairs][units]; down: fp32 [pairs][width]
+    long long w_expert;       // elements from one expert's first weight row to the next's
+    long long ld;             // elements from weight row to weight row
+    int x_share, pairs, experts, k, units, width, kind;
+    float limit, slope;
+};
+
+// One piece of a unit: its lanes' products with `n` (at most NB) pairs' activations into acc[2 r], acc[2 r + 1].
+template <int NB>
+__device__ __forceinline__ void stream_piece(const uint4* slot, const bf16* x, int ldx, const int* rows, int n, int q0, int q_end, int lane, Two* acc) {
 #pragma unroll
-        for (int r = 0; r < MAX_SHARE; ++r) sg[r] = su[r] = 0.f;
-        for (int c0 = lane; c0 < width / PER; c0 += 32 * 4) {
-            uint4 gv[4], uv[4];                   // four pieces of each row in flight
+    for (int i = 0; i < PIECE / 256; ++i) {
+        const int q = q0 + lane + 32 * i;
+        if (q >= q_end) break;
+        const uint4 g = slot[lane + 32 * i], u = slot[PIECE / 8 + lane + 32 * i];
+        const Two gw[4] = {two_of(g.x), two_of(g.y), two_of(g.z), two_of(g.w)}, uw[4] = {two_of(u.x), two_of(u.y), two_of(u.z), two_of(u.w)};
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int c = c0 + 32 * k;
-                if (c < width / PER) {
-                    gv[k] = __ldg(g4 + c);
-                    uv[k] = __ldg(u4 + c);
-                }
-            }
+        for (int r = 0; r < NB; ++r) {
+            if (NB > 4 && r >= n) break;
+            const uint4 xv = ((const uint4*)(x + (size_t)rows[NB > 4 ? r : min(r, n - 1)] * ldx))[q];
+            const Two xw[4] = {two_of(xv.x), two_of(xv.y), two_of(xv.z), two_of(xv.w)};
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int c = c0 + 32 * k;
-                if (c >= width / PER) break;
-                float gf[PER], uf[PER];
-#pragma unroll
-                for (int i = 0; i < PER; ++i) {
-                    gf[i] = fr_load((const T*)&gv[k] + i);
-                    uf[i] = fr_load((const T*)&uv[k] + i);
-                }
-#pragma unroll
-                for (int r = 0; r < MAX_SHARE; ++r) {
-                    if (r < n) {
-                        const uint4 hv = ((const uint4*)(hs + (size_t)r * width))[c];
-#pragma unroll
-                        for (int i = 0; i < PER; ++i) {
-                            const float x = fr_load((const T*)&hv + i);
-                            sg[r] = fmaf(x, gf[i], sg[r]);
-                            su[r] = fmaf(x, uf[i], su[r]);
-                        }
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < MAX_SHARE; ++r) {
-            if (r < n) {
-                const float a = fr_warp_sum(sg[r]), b = fr_warp_sum(su[r]);
-                if (lane == 0) fr_store(act + (size_t)pairs[r] * inner + f, fr_gated(kind, a, b, limit, slope));
+            for (int j = 0; j < 4; ++j) {
+                fma_two(acc[2 * r], xw[j], gw[j]);
+                fma_two(acc[2 * r + 1], xw[j], uw[j]);
             }
         }
     }
 }
 
-// The same for the down product: a block owns one expert and a tile of output columns, stages the activations of the
-// (row, choice) pairs that chose the expert, reads every weight row once for all of them and leaves each pair's part
-// [pairs][width] in fp32; combine_kernel then adds the parts to the residual in the order of the choices, so the sum
-// does not depend on which block finished first.
-template <typename T>
-__global__ void __launch_bounds__(256)
-down_by_expert_kernel(const T* __restrict__ act, const int* __restrict__ ids, const T* __restrict__ w_down, int ld_down,
-                      float* __restrict__ part, int rows, int top, int width, int inner, int per_block) {
+// The sums over the lanes of 2 NB values; lane (v * 16 / NB) ends with value v.
+template <int NB>
+__device__ __forceinline__ float lane_sums(const Two* acc, int lane) {
+    float s[2 * NB];
+#pragma unroll
+    for (int v = 0; v < 2 * NB; ++v) s[v] = sum_two(acc[v]);
+    int half = NB;
+#pragma unroll
+    for (int bit = 16; bit > 0; bit >>= 1) {
+        if (half > 0) {
+            const bool upper = (lane & bit) != 0;
+#pragma unroll
+            for (int v = 0; v < NB; ++v)
+                if (v < half) {
+                    const float give = upper ? s[v] : s[v + half], keep = upper ? s[v + half] : s[v];
+                    s[v] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+                }
+            half >>= 1;
+        } else {
+            s[0] += __shfl_xor_sync(0xffffffffu, s[0], bit);
+        }
+    }
+    return s[0];
+}
+
+template <int NB, bool DOWN>
+__device__ __forceinline__ void stream_store(const StreamArgs& p, const Two* acc, const int* pairs, int n, int unit, int lane) {
+    const float v = lane_sums<NB>(acc, lane);
+    constexpr int EACH = 16 / NB;                        // lanes that hold the same value
+    const float up = __shfl_down_sync(0xffffffffu, v, EACH);
+    const int value = lane / EACH, r = value >> 1;
+    if (lane % EACH != 0 || r >= n) return;
+    if (DOWN) {
+        const int c = 2 * unit + (value & 1);
+        if (c < p.width) ((float*)p.out)[(size_t)pairs[r] * p.width + c] = v;
+    } else if ((value & 1) == 0) {
+        fr_store((bf16*)p.out + (size_t)pairs[r] * p.units + unit, fr_gated(p.kind, v, up, p.limit, p.slope));
+    }
+}
+
+template <bool DOWN>
+__global__ void __launch_bounds__(32 * STREAM_WARPS, 2)
+expert_stream_kernel(const StreamArgs p) {
     extern __shared__ __align__(16) unsigned char raw[];
-    T* as = (T*)raw;                           // [MAX_SHARE][inner]
-    __shared__ int pairs[MAX_SHARE];
-    __shared__ int n_pairs;
-    constexpr int PER = 16 / sizeof(T);
+    __shared__ int count[256], group_expert[256 + MAX_FEW_PAIRS / SHARE], group_at[256 + MAX_FEW_PAIRS / SHARE], group_n[256 + MAX_FEW_PAIRS / SHARE];
+    __shared__ int pair_of[MAX_FEW_PAIRS], row_of[MAX_FEW_PAIRS], id_of[MAX_FEW_PAIRS], place_of[MAX_FEW_PAIRS], n_groups;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int e = threadIdx.x; e < p.experts; e += blockDim.x) count[e] = 0;
     fr_pdl_wait();
     fr_pdl_launch();
-    const int e = blockIdx.x;
-    // the pairs that chose this expert, in order: the ids are read side by side, then one thread lists the matches
-    __shared__ int chosen[MAX_SHARE * 32];
-    for (int pr = threadIdx.x; pr < rows * top; pr += blockDim.x) chosen[pr] = ids[pr];
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int n = 0;
-        for (int pr = 0; pr < rows * top && n < MAX_SHARE; ++pr)
-            if (chosen[pr] == e) pairs[n++] = pr;
-        n_pairs = n;
+    // the pairs of every expert in groups of at most SHARE (which of an expert's places a pair gets depends on scheduling; no
+    // result does, since every pair's sums are its own)
+    for (int i = threadIdx.x; i < p.pairs; i += blockDim.x) {
+        const int e = p.ids[i];
+        id_of[i] = e;
+        if (e >= 0 && e < p.experts) place_of[i] = atomicAdd(&count[e], 1);
     }
     __syncthreads();
-    const int n = n_pairs;
-    if (n == 0) return;
-    for (int idx = threadIdx.x; idx < n * (inner / PER); idx += blockDim.x) {
-        const int r = idx / (inner / PER), c = idx % (inner / PER);
-        ((uint4*)(as + (size_t)r * inner))[c] = ((const uint4*)(act + (size_t)pairs[r] * inner))[c];
+    if (warp == 0) {
+        int pairs_before = 0, groups_before = 0;
+        for (int e0 = 0; e0 < p.experts; e0 += 32) {
+            const int e = e0 + lane, n = e < p.experts ? count[e] : 0, groups = (n + SHARE - 1) / SHARE;
+            int pn = n, gn = groups;                     // sums over the lanes up to this one
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int a = __shfl_up_sync(0xffffffffu, pn, o), b = __shfl_up_sync(0xffffffffu, gn, o);
+                if (lane >= o) { pn += a; gn += b; }
+            }
+            const int at = pairs_before + pn - n, g0 = groups_before + gn - groups;
+            for (int g = 0; g < groups; ++g) {
+                group_expert[g0 + g] = e;
+                group_at[g0 + g] = at + g * SHARE;
+                group_n[g0 + g] = min(SHARE, n - g * SHARE);
+            }
+            if (e < p.experts) count[e] = at;
+            pairs_before += __shfl_sync(0xffffffffu, pn, 31);
+            groups_before += __shfl_sync(0xffffffffu, gn, 31);
+        }
+        if (lane == 0) n_groups = groups_before;
     }
     __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int c0 = blockIdx.y * per_block;
-    for (int col = c0 + warp; col < min(c0 + per_block, width); col += 8) {
-        const uint4* w4 = (const uint4*)(w_down + (size_t)col * ld_down + (size_t)e * inner);
-        float acc[MAX_SHARE];
+    for (int i = threadIdx.x; i < p.pairs; i += blockDim.x) {
+        const int e = id_of[i];
+        if (e < 0 || e >= p.experts) continue;
+        pair_of[count[e] + place_of[i]] = i;
+        row_of[count[e] + place_of[i]] = i / p.x_share;
+    }
+    __syncthreads();
+    const int total = n_groups * p.units, step = gridDim.x * STREAM_WARPS;
+    const int pieces = (p.k + PIECE - 1) / PIECE, q_end = p.k / 8;
+    uint4* ring = (uint4*)raw + warp * (RING * 2 * PIECE / 8);
+    // the next piece to fetch: piece `fetch_piece` of item `fetch`; an item is (group, unit)
+    int fetch = blockIdx.x * STREAM_WARPS + warp, fetch_piece = 0, fetch_slot = 0;
+    auto fetch_next = [&]() {
+        if (fetch < total) {
+            const int g = fetch / p.units, unit = fetch - g * p.units;
+            const bf16* w0 = p.w + (size_t)group_expert[g] * p.w_expert + (size_t)(2 * unit) * p.ld;
+            const bf16* w1 = DOWN && 2 * unit + 1 >= p.width ? w0 : w0 + p.ld;
+            uint4* slot = ring + fetch_slot * (2 * PIECE / 8);
 #pragma unroll
-        for (int r = 0; r < MAX_SHARE; ++r) acc[r] = 0.f;
-        for (int f0 = lane; f0 < inner / PER; f0 += 32 * 4) {
-            uint4 wv[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (f0 + 32 * k < inner / PER) wv[k] = __ldg(w4 + f0 + 32 * k);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int f = f0 + 32 * k;
-                if (f >= inner / PER) break;
-                float wf[PER];
-#pragma unroll
-                for (int i = 0; i < PER; ++i) wf[i] = fr_load((const T*)&wv[k] + i);
-#pragma unroll
-                for (int r = 0; r < MAX_SHARE; ++r) {
-                    if (r < n) {
-                        const uint4 av = ((const uint4*)(as + (size_t)r * inner))[f];
-#pragma unroll
-                        for (int i = 0; i < PER; ++i) acc[r] = fmaf(fr_load((const T*)&av + i), wf[i], acc[r]);
-                    }
+            for (int i = 0; i < PIECE / 256; ++i) {
+                const int q = fetch_piece * (PIECE / 8) + lane + 32 * i;
+                if (q < q_end) {
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(slot + lane + 32 * i)), "l"((const uint4*)w0 + q) : "memory");
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(slot + PIECE / 8 + lane + 32 * i)), "l"((const uint4*)w1 + q) : "memory");
                 }
             }
+            if (++fetch_piece == pieces) { fetch_piece = 0; fetch += step; }
+            if (++fetch_slot == RING) fetch_slot = 0;
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
 #pragma unroll
-        for (int r = 0; r < MAX_SHARE; ++r) {
-            if (r < n) {
-                const float v = fr_warp_sum(acc[r]);
-                if (lane == 0) part[(size_t)pairs[r] * width + col] = v;
-            }
+    for (int i = 0; i < RING - 1; ++i) fetch_next();
+    int slot = 0;
+    auto unit_of = [&](auto nb, int g, int unit, int n) {
+        constexpr int NB = decltype(nb)::value;
+        Two acc[2 * NB];
+#pragma unroll
+        for (int v = 0; v < 2 * NB; ++v) acc[v] = 0ull;
+        for (int piece = 0; piece < pieces; ++piece) {
+            fetch_next();                                // into the slot that was read last
+            asm volatile("cp.async.wait_group %0;" ::"n"(RING - 1) : "memory");
+            stream_piece<NB>(ring + slot * (2 * PIECE / 8), p.x, p.k, row_of + group_at[g], n, piece * (PIECE / 8), q_end, lane, acc);
+            if (++slot == RING) slot = 0;
         }
+        stream_store<NB, DOWN>(p, acc, pair_of + group_at[g], n, unit, lane);
+    };
+    for (int item = blockIdx.x * STREAM_WARPS + warp; item < total; item += step) {
+        const int g = item / p.units, unit = item - g * p.units, n = group_n[g];
+        if (n == 1) unit_of(Number<1>{}, g, unit, n);
+        else if (n == 2) unit_of(Number<2>{}, g, unit, n);
+        else if (n <= 4) unit_of(Number<4>{}, g, unit, n);
+        else if (n <= 8) unit_of(Number<8>{}, g, unit, n);
+        else unit_of(Number<16>{}, g, unit, n);
     }
 }
 
@@ -480,16 +522,26 @@ down_combine_kernel(const T* __restrict__ act, const int* __restrict__ ids, cons
     }
 }
 
-// Channels (of the inner size, or of the width) that a block of the by-expert kernels owns; FRIDAY_EXPERT_TILE overrides
-// (a multiple of 8, for measurements: 8 to 64 differ by less than a tenth).
-inline int expert_tile() {
-    static int v = 0;
-    if (v == 0) {
-        const char* e = getenv("FRIDAY_EXPERT_TILE");
-        const int t = e ? atoi(e) : 0;
-        v = (t >= 8 && t <= 256 && t % 8 == 0) ? t : 16;
+// Whether the kernel above takes a call: few rows, weight rows of k elements, ld apart, in 16-byte pieces.
+inline bool few_pairs_stream(int rows, int top, int experts, int k, int ld) {
+    return rows <= MAX_FEW && top <= 32 && experts > 0 && experts <= 256 && k % 8 == 0 && ld % 8 == 0;
+}
+
+template <bool DOWN>
+int launch_stream(const StreamArgs& p, cudaStream_t stream) {
+    static std::atomic<unsigned long long> configured{0};          // devices (as bits) on which the limit has been raised
+    int device = 0;
+    FR_CUDA(cudaGetDevice(&device));
+    if (device < 0 || device >= 64) FR_REFUSE("experts: device %d is outside the table of 64", device);
+    if (!(configured.load(std::memory_order_acquire) & (1ull << device))) {
+        FR_CUDA(cudaFuncSetAttribute(expert_stream_kernel<DOWN>, cudaFuncAttributeMaxDynamicSharedMemorySize, STREAM_SMEM));
+        configured.fetch_or(1ull << device, std::memory_order_release);
     }
-    return v;
+    const int sms = fr_sm_count() > 0 ? fr_sm_count() : 148;
+    const long long most = ((long long)p.pairs * p.units + STREAM_WARPS - 1) / STREAM_WARPS;      // blocks that can find a unit
+    FR_CUDA(fr_launch(expert_stream_kernel<DOWN>, dim3((unsigned)(most < 2 * sms ? most : 2 * sms)), dim3(32 * STREAM_WARPS), STREAM_SMEM, stream, p));
+    FR_CHECK_LAUNCH("experts (streamed)");
+    return FR_OK;
 }
 
 }  // namespace
@@ -529,19 +581,9 @@ FR_EXPORT int routed_gate_up(const void* h, const int* ids, const void* w_gate_u
     const int per_block = inner < 64 ? inner : 64;
     const dim3 grid(rows * top, (inner + per_block - 1) / per_block);
     if (grid.y > 65535) FR_REFUSE("gate_up: inner size %d", inner);
-    // few rows: one block per (expert, tile) reads the weights once for all rows that chose the expert
-    const size_t esize = dtype == FR_F32 ? 4 : 2;
-    const size_t share = (size_t)(rows < MAX_SHARE ? rows : MAX_SHARE) * width * esize;     // rows that can choose one expert
-    if (dtype == FR_BF16 && rows <= MAX_SHARE && experts > 0 && width % (16 / esize) == 0 && share <= 160 * 1024 &&
-        ((((uintptr_t)h) | ((uintptr_t)w_gate_up)) & 15) == 0) {
-        const int eper = expert_tile();          // inner channels per block: enough blocks to fill the device
-        const dim3 eg(experts, (inner + eper - 1) / eper);
-        if (share > 48 * 1024) FR_CUDA(cudaFuncSetAttribute(gate_up_by_expert_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)share));
-        FR_CUDA(fr_launch(gate_up_by_expert_kernel<bf16>, eg, dim3(256), share, stream, (const bf16*)h, ids, (const bf16*)w_gate_up,
-                          (bf16*)act, rows, top, width, inner, eper, kind, limit, slope));
-        FR_CHECK_LAUNCH("gate_up (by expert)");
-        return FR_OK;
-    }
+    if (dtype == FR_BF16 && few_pairs_stream(rows, top, experts, width, width) && ((((uintptr_t)h) | ((uintptr_t)w_gate_up)) & 15) == 0)
+        return launch_stream<false>(StreamArgs{(const bf16*)h, ids, (const bf16*)w_gate_up, act, 2ll * inner * width, width, top, rows * top, experts, width,
+                                               inner, width, kind, limit, slope}, stream);
     if (dtype == FR_F32) {
         if (smem > 48 * 1024) FR_CUDA(cudaFuncSetAttribute(gate_up_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         FR_CUDA(fr_launch(gate_up_kernel<float>, grid, dim3(256), smem, stream, (const float*)h, ids, (const float*)w_gate_up,
@@ -559,9 +601,7 @@ FR_EXPORT int routed_gate_up(const void* h, const int* ids, const void* w_gate_u
 
 // Floats of scratch that routed_down_combine wants for these sizes (0: none).
 FR_EXPORT long long routed_down_scratch_floats(int rows, int top, int width, int inner, int dtype) {
-    const size_t share = (size_t)(rows < MAX_SHARE ? rows : MAX_SHARE) * inner * 2;
-    if (dtype == FR_BF16 && rows <= MAX_SHARE && inner % 8 == 0 && share <= 160 * 1024) return (long long)rows * top * width;
-    return 0;
+    return dtype == FR_BF16 && few_pairs_stream(rows, top, 1, inner, inner) ? (long long)rows * top * width : 0;
 }
 
 // residual and out [rows][width] in res_dtype (fp32 for a 32-bit residual stream); residual may be null.
@@ -569,14 +609,10 @@ FR_EXPORT int routed_down_combine(const void* act, const int* ids, const float* 
                                   const void* residual, void* out, int res_dtype, int rows, int top, int experts, int width, int inner,
                                   float* scratch, int dtype, cudaStream_t stream) {
     if (rows <= 0) return FR_OK;
-    if (scratch != nullptr && routed_down_scratch_floats(rows, top, width, inner, dtype) > 0 && experts > 0 && ld_down % 8 == 0 &&
-        ((((uintptr_t)act) | ((uintptr_t)w_down)) & 15) == 0 && rows <= 65535) {
-        const size_t share = (size_t)(rows < MAX_SHARE ? rows : MAX_SHARE) * inner * 2;
-        const int per = expert_tile();
-        if (share > 48 * 1024) FR_CUDA(cudaFuncSetAttribute(down_by_expert_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)share));
-        FR_CUDA(fr_launch(down_by_expert_kernel<bf16>, dim3(experts, (width + per - 1) / per), dim3(256), share, stream, (const bf16*)act, ids,
-                          (const bf16*)w_down, ld_down, scratch, rows, top, width, inner, per));
-        FR_CHECK_LAUNCH("down (by expert)");
+    if (scratch != nullptr && dtype == FR_BF16 && few_pairs_stream(rows, top, experts, inner, ld_down) && ((((uintptr_t)act) | ((uintptr_t)w_down)) & 15) == 0) {
+        const int rc = launch_stream<true>(StreamArgs{(const bf16*)act, ids, (const bf16*)w_down, scratch, inner, ld_down, 1, rows * top, experts, inner,
+                                                      (width + 1) / 2, width, 1, 0.f, 0.f}, stream);
+        if (rc) return rc;
         const dim3 cg((width + 255) / 256, rows);
         if (res_dtype == FR_F32 && combine_by_four(scratch, residual, out, width))
             FR_CUDA(fr_launch(combine_four_kernel, dim3((width + 1023) / 1024, cg.y), dim3(256), 0, stream, (const float*)scratch, ids, weights,
