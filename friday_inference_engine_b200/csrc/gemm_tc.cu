@@ -52,6 +52,7 @@
 
 #include "common.cuh"
 #include <atomic>
+#include <string.h>
 #include <mutex>
 #include <unordered_map>
 #include "tc_common.cuh"
@@ -88,6 +89,8 @@ struct GemmParams {
                         // ACT_RELU_SQUARED: max(x, 0)^2 of every column
     int tiles_p, tiles_q, splits, kb_total, kb_per;
     int group_p;        // pairs of SMs: row tiles that go together (gemm_tc_pair.cuh)
+    const int* group_rows;      // rows in groups with weights of their own: [groups + 1], where they begin (null: one group)
+    int groups;
     // Work decomposition.  The first dp_tiles tiles are cut into `splits` equal k ranges each and dealt out round
     // robin (splits = 1: whole tiles).  The remaining sk_tiles tiles ("stream-k"): their k blocks, laid end to end,
     // are cut into one contiguous run of sk_units per CTA, so that a last, partial wave of tiles keeps every SM busy.
@@ -885,6 +888,22 @@ int encode_map(CUtensorMap* map, const void* base, int rows, int k, int ld, int 
     return FR_OK;
 }
 
+// The same for groups of matrices: [groups][rows][k], `group` elements from matrix to matrix; what lies beyond a matrix's rows
+// or its k reads as zero, also where the next matrix begins there.
+int encode_group_map(CUtensorMap* map, const void* base, int groups, long long group, int rows, int k, int ld, int box_rows) {
+    EncodeTiled enc = encode_fn();
+    if (enc == nullptr) FR_REFUSE("gemm_tc: the driver does not offer cuTensorMapEncodeTiled");
+    cuuint64_t dims[3] = {(cuuint64_t)k, (cuuint64_t)rows, (cuuint64_t)groups};
+    cuuint64_t strides[2] = {(cuuint64_t)ld * 2, (cuuint64_t)group * 2};
+    cuuint32_t box[3] = {(cuuint32_t)TILE_K, (cuuint32_t)box_rows, 1};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) FR_REFUSE("gemm_tc: cuTensorMapEncodeTiled failed with %d (%d matrices %lld apart, rows %d, k %d, ld %d)", (int)r, groups, group, rows, k, ld);
+    return FR_OK;
+}
+
 // FRIDAY_STREAM_K=1 cuts a partial last wave of tiles along k over all SMs.  Off by default: measured at
 // 2048 x 3584 x 3584 (224 tiles on 148 SMs) the merge of 128 x 256 partial tiles through global memory costs more
 // (117 us) than the idle SMs of the last wave (59 us).
@@ -970,6 +989,18 @@ int launch(const CUtensorMap& mp, const CUtensorMap& mq, const GemmParams& p, in
 
 }  // namespace
 
+// Width of the tiles of many rows: the one whose waves of `units` tiles cost least.
+static int tile_width(long long tiles_p, int q_rows, long long units, int narrowest) {
+    long long best = -1;
+    int bn = 256;
+    for (int cand = 256; cand >= narrowest; cand -= 16) {
+        const long long tiles = tiles_p * ((q_rows + cand - 1) / cand);
+        const long long cost = ((tiles + units - 1) / units) * (cand + 16);
+        if (best < 0 || cost < best) { best = cost; bn = cand; }
+    }
+    return bn;
+}
+
 // What the launcher would choose for a shape: fills plan[0..3] = {swapped, BN, splits, scratch floats needed}
 // and plan[4] = counters needed.  bn / splits / swap < 0 let the heuristics decide.
 FR_EXPORT int gemm_tc_plan(int m, int n, int k, int sm_count, int swap, int bn, int splits, long long* plan) {
@@ -994,15 +1025,9 @@ FR_EXPORT int gemm_tc_plan(int m, int n, int k, int sm_count, int swap, int bn, 
             const bool pair = pair_shape(m, n, swap, sm_count);
             const long long tiles_p = pair ? (p_rows + 2 * TILE_P - 1) / (2 * TILE_P) : (p_rows + TILE_P - 1) / TILE_P;
             const long long units = pair ? sm_count / 2 : sm_count;
-            long long best = -1;
             // (pairs of SMs also take narrower tiles; they pay where k is short and the wider tiles leave pairs idle:
             // 256 x 4608 x 3584 runs 36 tiles of 128 in 19.7 us and 72 of 64 in 17.6 us; long k is split instead)
-            const int narrowest = pair && kb_total < 128 ? 64 : 128;
-            for (int cand = 256; cand >= narrowest; cand -= 16) {
-                const long long tiles = tiles_p * ((q_rows + cand - 1) / cand);
-                const long long cost = ((tiles + units - 1) / units) * (cand + 16);
-                if (best < 0 || cost < best) { best = cost; bn = cand; }
-            }
+            bn = tile_width(tiles_p, q_rows, units, pair && kb_total < 128 ? 64 : 128);
         } else if (!skinny) bn = q_rows > 64 ? 128 : 64;
         else if (kb_total >= 128 && q_rows < 8192 && 2 * ((q_rows + 63) / 64) <= sm_count) bn = 64;   // long k, cut in two (96 x 3584 x 18944: 42.7 us; 128-wide tiles in four splits: 47.1 us)
         else if (q_rows >= 8192 || kb_total >= 128) bn = 128;
@@ -1188,11 +1213,11 @@ FR_EXPORT int gemm_tc_fused(const void* x, const void* w, void* out, int out_dty
         rc = current_device_bit(&bit);
         if (rc) return rc;
         if (!(configured.load(std::memory_order_acquire) & bit)) {
-            FR_CUDA(cudaFuncSetAttribute(gemm_tc_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM_BYTES));
+            FR_CUDA(cudaFuncSetAttribute(gemm_tc_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM_BYTES));
             configured.fetch_or(bit, std::memory_order_release);
         }
         const int pairs = pair_tiles < sm_count / 2 ? pair_tiles : sm_count / 2;
-        FR_CUDA(fr_launch_cluster(gemm_tc_pair_kernel, dim3(2 * pairs), dim3(THREADS), PAIR_SMEM_BYTES, stream, 2u, mp, mq, p));
+        FR_CUDA(fr_launch_cluster(gemm_tc_pair_kernel<false>, dim3(2 * pairs), dim3(THREADS), PAIR_SMEM_BYTES, stream, 2u, mp, mq, p));
         FR_CHECK_LAUNCH("gemm_tc (pairs)");
         return FR_OK;
     }
@@ -1212,6 +1237,56 @@ FR_EXPORT int gemm_tc_fused(const void* x, const void* w, void* out, int out_dty
         case 128: return launch<128, 6>(mp, mq, p, grid, stream);
         default: return launch<256, 4>(mp, mq, p, grid, stream);       // any width from 144 to 256
     }
+}
+
+// Rows in groups, each times weights of its own (experts' products): rows offsets[g] .. offsets[g + 1] - 1 of x and out (device
+// memory, ascending from 0; an earlier kernel of the stream may have written it) times the n x k matrix that starts w_group
+// elements after the one before, row stride ldw.  One launch of the kernel above over the tiles of all groups: a launch per
+// group left most pairs idle (eight experts of some 512 rows, 2048 x 4096 and 2048 x 2048, bf16: 16 launches, 315 us in all
+// on a B200; two of this kernel 154).
+// row_tiles: how many tiles of 256 rows the groups have in all, as far as the caller knows (for the width of the tiles).
+// act as in gemm_tc_act; rows beyond the last group are left as they are.
+FR_EXPORT int gemm_tc_grouped(const void* x, const void* w, long long w_group, void* out, int out_dtype, const int* offsets, int groups, int rows,
+                              int n, int k, int lda, int ldw, int ldo, int row_tiles, int act, float act_limit, float act_slope, int* status, int sm_count,
+                              cudaStream_t stream) {
+    if (rows <= 0 || n <= 0 || groups <= 0) return FR_OK;
+    if (act < 0 || act > ACT_RELU_SQUARED || (act && ((n % 2 && act != ACT_RELU_SQUARED) || out_dtype != FR_BF16)))
+        FR_REFUSE("gemm_tc_grouped: an activation (%d) needs bf16 output, a gated one an even n", act);
+    if (act == 3 && !(act_limit > 0.f)) FR_REFUSE("gemm_tc_grouped: the clipped gated unit needs its limit");
+    if (k <= 0 || k % 8 || lda % 8 || ldw % 8 || w_group % 8 || w_group <= 0 || (((uintptr_t)x | (uintptr_t)w) & 15))
+        FR_REFUSE("gemm_tc_grouped: k = %d, the strides (%d, %d, %lld) and the operands' starts must keep to 16 bytes", k, lda, ldw, w_group);
+    if (groups > MAX_GROUPS || sm_count < 2 || status == nullptr || offsets == nullptr)
+        FR_REFUSE("gemm_tc_grouped: %d groups (at most %d) need their offsets, a status word and two SMs", groups, MAX_GROUPS);
+    GemmParams p;
+    memset(&p, 0, sizeof p);
+    p.f.act_limit = act_limit; p.f.act_slope = act_slope;
+    p.out = out; p.status = status;
+    p.p_rows = rows; p.q_rows = n; p.ldo = ldo; p.out_dtype = out_dtype;
+    p.act = act;
+    p.bn = tile_width(row_tiles > 0 ? row_tiles : 1, n, sm_count / 2, 128);
+    p.tiles_q = (n + p.bn - 1) / p.bn;
+    p.splits = 1; p.kb_total = p.kb_per = (k + TILE_K - 1) / TILE_K;
+    p.group_rows = offsets;
+    p.groups = groups;
+    CUtensorMap mp, mq;
+    int rc = make_map(&mp, x, rows, k, lda, TILE_P);
+    if (rc) return rc;
+    rc = encode_group_map(&mq, w, groups, w_group, n, k, ldw, p.bn / 2);
+    if (rc) return rc;
+    static std::atomic<unsigned long long> configured{0};
+    unsigned long long bit = 0;
+    rc = current_device_bit(&bit);
+    if (rc) return rc;
+    if (!(configured.load(std::memory_order_acquire) & bit)) {
+        FR_CUDA(cudaFuncSetAttribute(gemm_tc_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM_BYTES));
+        configured.fetch_or(bit, std::memory_order_release);
+    }
+    // no more tiles than this, whatever the groups' sizes
+    const long long most = ((long long)rows / (2 * TILE_P) + (rows < groups ? rows : groups)) * p.tiles_q;
+    const int pairs = most < sm_count / 2 ? (int)most : sm_count / 2;
+    FR_CUDA(fr_launch_cluster(gemm_tc_pair_kernel<true>, dim3(2 * pairs), dim3(THREADS), PAIR_SMEM_BYTES, stream, 2u, mp, mq, p));
+    FR_CHECK_LAUNCH("gemm_tc (groups)");
+    return FR_OK;
 }
 
 // ------------------------------------------------------------------ the entry point that allocates nothing

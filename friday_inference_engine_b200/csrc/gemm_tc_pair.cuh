@@ -76,8 +76,53 @@ __device__ __forceinline__ void pair_tile(const GemmParams& p, int tile, int& p_
     p_blk = first + at - q_blk * high;
 }
 
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+        ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
+        : "memory");
+}
+
+// The tiles of one pair, in the order in which all three roles walk them.  GROUPED: the rows are groups (rows off[g] to
+// off[g + 1] - 1), each with weights of its own; a group's row tiles start at its first row, and its tiles lie together.
+template <bool GROUPED>
+struct PairWalk {
+    const GemmParams& p;
+    const int* off;
+    int tile, step, group, base;               // base: the group's first tile
+    int row0, row_end, q_blk;                  // the tile's first row, where its rows end, its column tile
+    __device__ PairWalk(const GemmParams& p_, const int* off_, int pair, int pairs)
+        : p(p_), off(off_), tile(pair - pairs), step(pairs), group(0), base(0), row0(0), row_end(p_.p_rows), q_blk(0) {}
+    __device__ bool next() {
+        tile += step;
+        if constexpr (GROUPED) {
+            int high = 0;
+            for (;; ++group) {
+                if (group >= p.groups) return false;
+                high = (off[group + 1] - off[group] + 2 * TILE_P - 1) / (2 * TILE_P);
+                if (tile < base + high * p.tiles_q) break;
+                base += high * p.tiles_q;
+            }
+            const int at = tile - base;
+            q_blk = at / high;
+            row0 = off[group] + (at - q_blk * high) * (2 * TILE_P);
+            row_end = off[group + 1];
+        } else {
+            if (tile >= p.dp_tiles) return false;
+            int p_blk;
+            pair_tile(p, tile, p_blk, q_blk);
+            row0 = p_blk * (2 * TILE_P);
+        }
+        return true;
+    }
+};
+
+constexpr int MAX_GROUPS = 256;
+
+template <bool GROUPED>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_q, const GemmParams p) {
+    __shared__ int s_off[GROUPED ? MAX_GROUPS + 1 : 1];
     constexpr int STAGES = PAIR_STAGES, STAGE_BYTES = PAIR_STAGE_BYTES, BN = PAIR_BN;
     constexpr int TMEM_COLS = 2 * BN;
     const int bn = p.bn, half = bn >> 1;
@@ -112,6 +157,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
+    if constexpr (GROUPED) {                               // where the groups lie is the predecessor's result
+        fr_pdl_wait();
+        for (int g = threadIdx.x; g <= p.groups; g += THREADS) s_off[g] = p.group_rows[g];
+    }
     tc_fence_before();
     __syncthreads();
     fr_cluster_sync();                                     // the other CTA's barriers are ready before anything reaches them
@@ -124,47 +173,46 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
             asm volatile("prefetch.tensormap [%0];" ::"l"(&map_p) : "memory");
             asm volatile("prefetch.tensormap [%0];" ::"l"(&map_q) : "memory");
             struct Walk {                                  // the k blocks this pair will load, in order
-                Work work;
-                Item item;
-                int kb, p_blk, q_blk;
+                PairWalk<GROUPED> tiles;
+                int kb;
                 bool live;
-                __device__ Walk(const GemmParams& pp, int cta, int grid) : work(pp, cta, grid), live(true) { open(pp); }
-                __device__ void open(const GemmParams& pp) {
-                    live = work.next(item);
-                    if (!live) return;
-                    pair_tile(pp, item.tile, p_blk, q_blk);
-                    kb = item.kb0;
+                __device__ Walk(const GemmParams& pp, const int* off, int cta, int grid) : tiles(pp, off, cta, grid), kb(0) { live = tiles.next(); }
+                __device__ void step() {
+                    if (++kb >= tiles.p.kb_total) {
+                        kb = 0;
+                        live = tiles.next();
+                    }
                 }
-                __device__ void step(const GemmParams& pp) {
-                    if (++kb >= item.kb1) open(pp);
-                }
+            };
+            auto load_weights = [&](const Walk& at, uint32_t dst, uint32_t bar) {
+                const int row = at.tiles.q_blk * bn + (int)rank * half;
+                if constexpr (GROUPED) tma_load_3d_pair(dst, &map_q, at.kb * TILE_K, row, at.tiles.group, bar);
+                else tma_load_2d_pair(dst, &map_q, at.kb * TILE_K, row, bar);
             };
             // The weights do not depend on the kernel before this one; the activations do.  Fill the ring with
             // weight slices first, then wait for the predecessor, then add the activation slices.
             const uint32_t stage_tx = 2u * (P_BYTES + (uint32_t)half * TILE_K * 2);      // both CTAs' bytes of a stage
-            Walk head(p, pair, pairs);
-            Walk ahead(p, pair, pairs);
+            Walk head(p, s_off, pair, pairs);
+            Walk ahead(p, s_off, pair, pairs);
             int early = 0;
-            for (; early < STAGES && ahead.live; ++early, ahead.step(p)) {
+            for (; early < STAGES && ahead.live; ++early, ahead.step()) {
                 if (rank == 0) mbar_expect_tx(full0 + 8 * early, stage_tx);
-                tma_load_2d_pair(smem_u32(smem + early * STAGE_BYTES) + P_BYTES, &map_q, ahead.kb * TILE_K,
-                                 ahead.q_blk * bn + (int)rank * half, first_full0 + 8 * early);
+                load_weights(ahead, smem_u32(smem + early * STAGE_BYTES) + P_BYTES, first_full0 + 8 * early);
             }
             fr_pdl_wait();
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
-            for (; head.live && ok; head.step(p)) {
+            for (; head.live && ok; head.step()) {
                 const uint32_t dst = smem_u32(smem + stage * STAGE_BYTES);
                 if (early > 0) {
                     --early;                                 // the weight slice of this stage is already on its way
                 } else {
                     if (!(ok = mbar_wait(empty0 + 8 * stage, phase ^ 1, p.status, 1))) break;
                     if (rank == 0) mbar_expect_tx(full0 + 8 * stage, stage_tx);
-                    tma_load_2d_pair(dst + P_BYTES, &map_q, head.kb * TILE_K, head.q_blk * bn + (int)rank * half,
-                                     first_full0 + 8 * stage);
+                    load_weights(head, dst + P_BYTES, first_full0 + 8 * stage);
                 }
-                tma_load_2d_pair(dst, &map_p, head.kb * TILE_K, (2 * head.p_blk + (int)rank) * TILE_P, first_full0 + 8 * stage);
+                tma_load_2d_pair(dst, &map_p, head.kb * TILE_K, head.tiles.row0 + (int)rank * TILE_P, first_full0 + 8 * stage);
                 if (++stage == STAGES) { stage = 0; phase ^= 1; }
             }
         }
@@ -176,22 +224,21 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
             uint32_t phase = 0;
             bool ok = true;
             int it = 0;
-            Work work(p, pair, pairs);
-            Item item;
-            for (; ok && work.next(item); ++it) {
+            PairWalk<GROUPED> tiles(p, s_off, pair, pairs);
+            for (; ok && tiles.next(); ++it) {
                 const int a = it & 1;
                 const uint32_t acc_phase = (it >> 1) & 1;
                 if (!(ok = mbar_wait(acce0 + 8 * a, acc_phase ^ 1, p.status, 2))) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + a * BN;
-                for (int kb = item.kb0; kb < item.kb1; ++kb) {
+                for (int kb = 0; kb < p.kb_total; ++kb) {
                     if (!(ok = mbar_wait(full0 + 8 * stage, phase, p.status, 3))) break;
                     tc_fence_after();
                     const uint32_t pa = smem_u32(smem + stage * STAGE_BYTES);
                     const uint64_t da = smem_desc(pa), db = smem_desc(pa + P_BYTES);
 #pragma unroll
                     for (int k = 0; k < TILE_K / UMMA_K; ++k)
-                        tc_mma_pair(d_tmem, da + 2 * k, db + 2 * k, idesc, (kb > item.kb0 || k > 0) ? 1u : 0u);
+                        tc_mma_pair(d_tmem, da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
                     tc_commit_pair(empty0 + 8 * stage);   // the stage is free in both CTAs once these products are done
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
                 }
@@ -207,24 +254,20 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
         int it = 0;
         const GemmFusion& f = p.f;
         const bool norm_rows = f.norm_out != nullptr;
-        int scale_blk = -1;
+        int scale_row = -1;
         float row_scale = 1.f;
-        Work work(p, pair, pairs);
-        Item item;
-        for (; ok && work.next(item); ++it) {
-            int p_blk, q_blk;
-            pair_tile(p, item.tile, p_blk, q_blk);
-            p_blk = 2 * p_blk + (int)rank;
+        PairWalk<GROUPED> tiles(p, s_off, pair, pairs);
+        for (; ok && tiles.next(); ++it) {
+            const int q_blk = tiles.q_blk, gi = tiles.row0 + (int)rank * TILE_P + i_local;
             const int a = it & 1;
             const uint32_t acc_phase = (it >> 1) & 1;
-            const int gi = p_blk * TILE_P + i_local;
-            if (f.in_ssq != nullptr && p_blk != scale_blk) {
+            if (f.in_ssq != nullptr && gi != scale_row) {
                 // the deferred norm of the input: the factor of this thread's row
                 float ss = 0.f;
                 if (gi < p.p_rows)
                     for (int t = 0; t < f.in_parts; ++t) ss += __ldcg(f.in_ssq + (size_t)t * p.p_rows + gi);
                 row_scale = 1.0f / sqrtf(ss / f.in_width + f.in_eps);
-                scale_blk = p_blk;
+                scale_row = gi;
             }
             float ss_row = 0.f;                            // with a norm begun: this row's sum of squares over the tile
             if (norm_rows) {
@@ -252,7 +295,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
                     for (int j = 0; j < 16; ++j) v[j] *= row_scale;
                 const int gj0 = q_blk * bn + c * 16;
                 if (norm_rows) finish16_begin_norm(p, s_gw + c * 16, gi, gj0, v, ss_row);
-                else finish16(p, gi, gj0, v);
+                else if (!GROUPED || gi < tiles.row_end) finish16(p, gi, gj0, v);
             }
             tc_fence_before();
             __syncwarp();

@@ -470,6 +470,7 @@ __global__ void __launch_bounds__(1024) sort_pairs_kernel(const int* __restrict_
     }
     __syncthreads();
     for (int e = threadIdx.x; e <= experts; e += blockDim.x) offsets[e] = off[e];
+    for (int place = off[experts] + threadIdx.x; place < n_pairs; place += blockDim.x) row_at[place] = 0;      // places of no pair: a row that exists
     for (int p = threadIdx.x; p < n_pairs; p += blockDim.x) {
         const int e = ids[p];
         if (e >= 0 && e < experts) {

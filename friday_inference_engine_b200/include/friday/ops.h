@@ -332,12 +332,11 @@ public:
     Tensor expert_gate_up(const Tensor& h, const Routing& r, const Tensor& w_gate_up, int top, int inner, int act = 1, float limit = 0.f,
                           float slope = 1.f);
     Tensor expert_down_combine(const Tensor& act, const Routing& r, const Tensor& w_down, const Tensor& residual, int top, int inner);
-    // Many rows: the rows are gathered expert by expert and every expert with rows runs its two products on the tensor
-    // cores over its own rows only.  The host reads the experts' row counts (one small copy and a wait per call) unless it knows
-    // them already (`counts`: a number of choices per expert), so this is for prompts, never inside a captured step.  w_gate_up [experts * 2 * inner, width] (gate and up row by row in
-    // turn), w_down [width, experts * inner].
+    // Many rows: the rows are gathered expert by expert and every expert runs its two products on the tensor cores over its
+    // own rows only, all experts in one launch per product.  row_tiles: how many tiles of 256 rows that makes, as far as the
+    // caller knows.  bf16.  w_gate_up [experts * 2 * inner, width] (gate and up row by row in turn), w_down [width, experts * inner].
     Tensor experts_grouped(const Tensor& h, const Routing& r, const Tensor& w_gate_up, const Tensor& w_down, const Tensor& residual,
-                           int top, int inner, int act = 1, float limit = 0.f, float slope = 1.f, const std::vector<int>* counts = nullptr);
+                           int top, int inner, int act = 1, float limit = 0.f, float slope = 1.f, int row_tiles = 0);
 
     // ---- matrix products: x [rows, k] @ weight [n, k]^T (+ bias [n]) (+ residual [rows, n])
     Tensor linear(const Rows& x, const Tensor& weight, const Tensor* bias = nullptr, const Tensor* residual = nullptr,

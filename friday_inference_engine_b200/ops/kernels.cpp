@@ -96,7 +96,8 @@ FAMILY(Rowwise, rowwise, "rowwise",
        resolve(h, fam, "rowwise_scale_rows", t.scale_rows); resolve(h, fam, "rowwise_finish_logits", t.finish_logits);
        resolve(h, fam, "rowwise_random_normal", t.random_normal);)
 FAMILY(GemmSimt, gemm_simt, "gemm_simt", resolve(h, fam, "gemm_simt", t.gemm);)
-FAMILY(GemmTc, gemm_tc, "gemm_tc", resolve(h, fam, "gemm_tc_fused", t.fused); resolve(h, fam, "gemm_tc_plan", t.plan);)
+FAMILY(GemmTc, gemm_tc, "gemm_tc", resolve(h, fam, "gemm_tc_fused", t.fused); resolve(h, fam, "gemm_tc_plan", t.plan);
+       resolve(h, fam, "gemm_tc_grouped", t.grouped);)
 FAMILY(AttentionSimt, attention_simt, "attention_simt", resolve(h, fam, "attention_simt", t.run);
        resolve(h, fam, "attention_simt_masked", t.masked);)
 FAMILY(AttentionWindow, attention_window, "attention_window", resolve(h, fam, "attention_window_fits", t.fits);

@@ -41,6 +41,8 @@ struct GemmTc {
     int (*fused)(const void*, const void*, void*, int, const void*, int, const void*, int, int, int, int, int, int, float*,
                  long long, int*, int, int*, int, int, int, int, int, const GemmFusion*, cudaStream_t);
     int (*plan)(int, int, int, int, int, int, int, long long*);
+    int (*grouped)(const void*, const void*, long long, void*, int, const int*, int, int, int, int, int, int, int, int, int, float, float, int*, int,
+                   cudaStream_t);
 };
 struct AttentionSimt {
     last_error_fn last_error;

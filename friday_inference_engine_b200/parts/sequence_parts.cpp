@@ -497,22 +497,24 @@ public:
         }
         const bool tensor_cores = x.dtype == DType::BF16 && x.rows() > 32 && tensor("w_gate_up").dtype == DType::BF16 &&
                                   x.cols() % 8 == 0 && inner_ % 8 == 0;
-        // Arithmetic of the dense form against the grouped one, in units of a product's multiply-adds: all experts for
-        // every row, or the chosen ones plus what two launches per expert and the host's wait cost (measured on a B200:
-        // grouping broke even at width 2,048 with 8 experts of inner size 2,048, 2 chosen, 2,048 rows, and won a fifth
-        // of the prompt's time at width 4,096; a launch counts as 25 G multiply-adds, the wait as 100 G).  Grouping
-        // needs the host, so a one-token step (which may be captured in a graph) never groups.  Where the host knows the counts
-        // without looking (a table of token ids) there is no wait and the queue stays full: a launch counts as 17 G (the two forms
-        // were within a fiftieth of each other at width 2,048, 3.56 and 3.63 ms a prompt).
-        const double per_row = 3.0 * (double)inner_ * (double)x.cols();
-        const double dense_work = (double)x.rows() * experts_ * per_row;
+        // The dense form (all experts for every row) against the grouped one, in tiles of 256 rows of a product.  As far as 256 rows
+        // both read every expert's weights once, and the dense form needs no sorting; from there the grouped form has fewer tiles
+        // (a prompt of 2,048 rows, width and
+        // inner size 2048, 8 experts, 2 chosen: 3,006 us a pass of seven layers, 3,560 in the dense form).  Without a table only the device knows how the
+        // rows fall, half a tile per expert is left over on average.  Grouping is for prompts: a one-token step never groups.
         const std::vector<int> counts = choices_per_expert(ctx);          // empty: only the device knows
-        const double grouped_work = (double)x.rows() * top_ * per_row + (counts.empty() ? 2.0 * experts_ * 25e9 + 100e9 : 2.0 * experts_ * 17e9) / 2.0;
+        const int64_t pairs = x.rows() * top_, some = std::min<int64_t>(experts_, pairs);
+        int64_t grouped_tiles = std::max(some, pairs / 256 + some / 2);
+        if (!counts.empty()) {
+            grouped_tiles = 0;
+            for (int n : counts) grouped_tiles += (n + 255) / 256;
+        }
+        const int64_t dense_tiles = (x.rows() + 255) / 256 * experts_;
         // FRIDAY_EXPERTS=grouped|dense|pairs forces a form where it can run (for comparisons and tests)
         const char* force = getenv("FRIDAY_EXPERTS");
         const std::string forced = force ? force : "";
-        const bool may_group = tensor_cores && !ctx.decode && ctx.rows == (int)x.rows() && ctx.n_seqs > 0;
-        const bool grouped = may_group && (forced == "grouped" || (forced.empty() && grouped_work < dense_work));
+        const bool may_group = tensor_cores && tensor("w_down").dtype == DType::BF16 && !ctx.decode && ctx.rows == (int)x.rows() && ctx.n_seqs > 0;
+        const bool grouped = may_group && (forced == "grouped" || (forced.empty() && grouped_tiles < dense_tiles && x.rows() > 256));
         const bool dense = tensor_cores && !grouped && (forced == "dense" || (forced.empty() && experts_ <= 16 * top_));
         Ops::Routing r = tabled_ ? ops.route_table(ctx.tokens, x.rows(), tensor("table"), experts_, dense)
                         : sigmoid_ ? ops.route_scored(logits, top_, choice_bias_.empty() ? nullptr : &tensor(choice_bias_), groups_, keep_,
@@ -539,7 +541,7 @@ public:
             residual = with_shared(residual_in);
         }
         if (grouped)
-            return PartOut(ops.experts_grouped(x, r, tensor("w_gate_up"), tensor("w_down"), residual, top_, inner_, act_, limit_, slope_, counts.empty() ? nullptr : &counts));
+            return PartOut(ops.experts_grouped(x, r, tensor("w_gate_up"), tensor("w_down"), residual, top_, inner_, act_, limit_, slope_, (int)grouped_tiles));
         if (dense) {
             Tensor act = ops.linear_swiglu(Rows(x), tensor("w_gate_up"), act_, limit_, slope_);
             ops.scale_by_route(act, r.dense, experts_, inner_);

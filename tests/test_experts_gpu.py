@@ -1,4 +1,5 @@
-"""The experts' products alone: the streamed form for few rows at the edges of its pieces and groups, against 64-bit sums."""
+"""The experts' products alone: the streamed form for few rows and the grouped form for many, at the edges of their pieces,
+tiles and groups, against 64-bit sums."""
 from ctypes import c_float, c_int, c_longlong, c_void_p
 
 import pytest
@@ -64,3 +65,47 @@ def test_streamed_experts(rows, top, experts, spread, width, inner):
             total[pair // top] += weights.flatten()[pair].double() * (w @ act[pair].double())
             size[pair // top] += weights.flatten()[pair].double() * (w.abs() @ act[pair].double().abs())
     assert bool(((out.double() - total).abs() <= (inner + 2 * top + 2) * 2.0 ** -24 * size).all())
+
+
+# groups: none, one row, around 256 rows, several tiles, rows beyond the last group; columns and k around the tiles; matrices
+# side by side (the next one's numbers lie where this one's k ends) and one after another
+@pytest.mark.parametrize("sizes", [[0, 1, 256, 257, 0], [700], [3] * 40, [255, 512, 0, 130]])
+@pytest.mark.parametrize("n,k,act", [(16, 8, 0), (272, 72, 0), (4096, 200, 1), (520, 64, 3)])
+@pytest.mark.parametrize("side_by_side", [False, True])
+def test_grouped_product(sizes, n, k, act, side_by_side):
+    g = lib.family("gemm_tc")
+    g.declare("gemm_tc_grouped", [P, P, L, P, I, P, I, I, I, I, I, I, I, I, I, F, F, P, I, P])
+    groups, used = len(sizes), sum(sizes)
+    rows = used + 5
+    x = rnd((rows, k), 7)
+    if side_by_side:
+        w = rnd((n, groups * k), 8, 0.3)
+        parts, ldw, step = [w[:, e * k:(e + 1) * k] for e in range(groups)], groups * k, k
+    else:
+        w = rnd((groups * n, k), 8, 0.3)
+        parts, ldw, step = [w[e * n:(e + 1) * n] for e in range(groups)], k, n * k
+    offsets = torch.tensor([sum(sizes[:e]) for e in range(groups + 1)], dtype=torch.int32, device=DEV)
+    out = torch.full((rows, n // 2 if act else n), 7.0, dtype=torch.bfloat16 if act else torch.float32, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    if side_by_side and not act:
+        parts[0].fill_(float("nan"))           # reaches no other group's sums
+    g.call("gemm_tc_grouped", ptr(x), ptr(w), step, ptr(out), 1 if act else 0, ptr(offsets), groups, rows, n, k, k, ldw, out.shape[1],
+           sum((s + 255) // 256 for s in sizes), act, 2.0, 1.702, ptr(status), sms, stream())
+    assert int(status) == 0
+    assert bool((out[used:] == 7.0).all())
+    at = 0
+    for e, size in enumerate(sizes):
+        a, b = x[at:at + size].double(), parts[e].double()
+        got, z, mag = out[at:at + size].double(), a @ b.T, a.abs() @ b.abs().T
+        at += size
+        if side_by_side and not act and e == 0:
+            assert bool(torch.isnan(got).all())
+        elif act:
+            gate, up = z[:, 0::2], z[:, 1::2]
+            want = silu(gate) * up if act == 1 else gate.clamp(max=2.0) * torch.sigmoid(1.702 * gate.clamp(max=2.0)) * (up.clamp(-2.0, 2.0) + 1.0)
+            # bf16's rounding, and the sums' errors (k 2^-23 of the terms' size) times what the unit makes of them
+            slack = k * 2.0 ** -23 * (mag[:, 0::2] * (up.abs() + 1.0) * 2.0 + mag[:, 1::2] * (gate.abs() + 1.0))
+            assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + slack + 1e-6).all())
+        else:
+            assert bool(((got - z).abs() <= k * 2.0 ** -23 * mag).all())
