@@ -820,6 +820,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
 }  // namespace
 
 #include "gemm_tc_pair.cuh"
+#include "gemm_tc_skinny.cuh"
 
 namespace {
 
@@ -1001,6 +1002,21 @@ static int tile_width(long long tiles_p, int q_rows, long long units, int narrow
     return bn;
 }
 
+// Whether the launcher, left to itself, takes the kernel of few rows and a small matrix.  Measured in captured chains on B200
+// (us a product, tcgen05 against this one): 8 rows: 64 x 2048 8.0 / 2.1, 2048 x 2048 6.5 / 3.4, 4608 x 3584 9.9 / 7.0,
+// 12288 x 2048 12.2 / 11.1, 3584 x 18944 27.5 / 27.4, 32768 x 2048 24.8 / 25.6.  16 rows: 64 x 2048 8.2 / 2.4, 4096 x 2048
+// 8.2 / 6.7, 2048 x 6144 9.3 / 7.7, 7168 x 2048 11.0 / 11.8, 3584 x 3584 9.3 / 11.0.
+static bool skinny_shape(int m, int n, int k, int sm_count) {
+    const long long size = (long long)n * k;
+    if (m <= 8) return size <= (32ll << 20);
+    return m <= 16 && (size <= (8ll << 20) || (size <= (16ll << 20) && n <= SKINNY_N * sm_count));
+}
+// Nothing but the activation's constants.
+static bool nothing_fused(const GemmFusion& f) {
+    return f.in_ssq == nullptr && f.norm_out == nullptr && f.norm_w == nullptr && f.out_ssq == nullptr && f.row_pos == nullptr && f.row_seq == nullptr &&
+           f.denom == nullptr && f.k_pool == nullptr && f.trace == nullptr;
+}
+
 // What the launcher would choose for a shape: fills plan[0..3] = {swapped, BN, splits, scratch floats needed}
 // and plan[4] = counters needed.  bn / splits / swap < 0 let the heuristics decide.
 FR_EXPORT int gemm_tc_plan(int m, int n, int k, int sm_count, int swap, int bn, int splits, long long* plan) {
@@ -1108,6 +1124,18 @@ FR_EXPORT int gemm_tc_fused(const void* x, const void* w, void* out, int out_dty
         FR_REFUSE("gemm_tc: k = %d and the row strides (%d, %d) must be multiples of 8 (16-byte rows for TMA)", k, lda, ldw);
     if (((uintptr_t)x & 15) || ((uintptr_t)w & 15)) FR_REFUSE("gemm_tc: operands must be 16-byte aligned");
     if (status == nullptr) FR_REFUSE("gemm_tc: a status word is needed");
+    // (bf16 results of a multiple of 128 columns may be a product that another path fuses with a norm or a rotation: both give
+    // the same bits, so both stay on one kernel unless the caller says that there is no other path)
+    const bool same_bits = swap != GEMM_TC_ANY_KERNEL && out_dtype == FR_BF16 && act == 0 && n % TILE_P == 0;
+    if (swap < 0 && bn < 0 && splits < 0 && !same_bits && skinny_shape(m, n, k, sm_count) && (fusion == nullptr || nothing_fused(*fusion))) {
+        SkinnyParams p{};
+        if (fusion != nullptr) p.f = *fusion;
+        p.x = (const __nv_bfloat16*)x; p.w = (const __nv_bfloat16*)w; p.out = out; p.bias = bias; p.residual = residual;
+        p.m = m; p.n = n; p.k = k; p.lda = lda; p.ldw = ldw; p.ldo = ldo; p.out_dtype = out_dtype; p.bias_dtype = bias_dtype; p.act = act;
+        // sixteen warps where k is long and there is at most a block per SM (2048 x 6144: 6.8 us against 8.5; 3584 x 3584: 7.6 against 6.5)
+        if (k <= 8 * SKINNY_K || n > SKINNY_N * sm_count) return m <= 8 ? launch_skinny<8, 1>(p, stream) : launch_skinny<8, 2>(p, stream);
+        return m <= 8 ? launch_skinny<16, 1>(p, stream) : launch_skinny<16, 2>(p, stream);
+    }
     long long plan[5];
     const bool splits_free = splits < 0;
     gemm_tc_plan(m, n, k, sm_count, swap, bn, splits, plan);

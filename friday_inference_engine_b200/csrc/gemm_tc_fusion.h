@@ -38,3 +38,6 @@ struct GemmFusion {
     // (5) Constants of the activation: limit and slope of the clipped gated unit.
     float act_limit, act_slope;
 };
+
+// For `swap`: the launcher chooses, also a kernel whose sums differ in order from the fused forms' (a product that has none).
+#define GEMM_TC_ANY_KERNEL (-2)

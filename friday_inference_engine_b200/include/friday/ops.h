@@ -341,6 +341,10 @@ public:
     // ---- matrix products: x [rows, k] @ weight [n, k]^T (+ bias [n]) (+ residual [rows, n])
     Tensor linear(const Rows& x, const Tensor& weight, const Tensor* bias = nullptr, const Tensor* residual = nullptr,
                   int out_dtype = -1, Tensor* out = nullptr);
+    // The same for a product that has no fused form to agree with bit by bit (linear_norm, qkv_rope_write): few rows may run on
+    // the kernel for small matrices.  (linear takes that kernel only where no fused form exists: fp32 results, columns that are
+    // no multiple of 128.)
+    Tensor linear_alone(const Rows& x, const Tensor& weight, const Tensor* bias = nullptr);
     // linear(...) and the RMSNorm of its result.  For bf16 rows whose sizes allow it the norm is begun in the
     // product's epilogue and the second result is deferred; otherwise the norm's kernel runs.
     std::pair<Tensor, Rows> linear_norm(const Rows& x, const Tensor& weight, const Tensor& norm_weight, float eps,

@@ -1189,6 +1189,14 @@ Tensor Ops::linear(const Rows& x, const Tensor& weight, const Tensor* bias, cons
     return linear_simt(xin, weight, bias, residual, o);
 }
 
+Tensor Ops::linear_alone(const Rows& x, const Tensor& weight, const Tensor* bias) {
+    if (x.deferred) return linear(x, weight, bias);
+    check_product(x.t, weight);
+    Tensor o = alloc(x.t.dtype, x.t.rows(), weight.rows());
+    if (!tensor_core_ok(x.t, weight, o, nullptr)) return linear_simt(x.t, weight, bias, nullptr, o);
+    return linear_tc(x.t, weight, bias, nullptr, o, GEMM_TC_ANY_KERNEL, -1, -1, 0, nullptr);
+}
+
 Tensor Ops::materialize(const Rows& h) {
     return h.deferred ? rmsnorm(h.source, h.weight, h.eps) : h.t;
 }

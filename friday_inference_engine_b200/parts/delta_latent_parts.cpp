@@ -106,12 +106,12 @@ public:
     PartOut forward(Ops& ops, const Rows& h, const Tensor& residual, const StepContext& ctx, const CacheView& view, Norm*) override {
         const int64_t qk = (int64_t)qk_heads_ * dk_, hv = (int64_t)heads_ * dv_;
         Tensor x = ops.materialize(h);
-        Tensor in = ops.linear(Rows(x), tensor("w_in"));
+        Tensor in = ops.linear_alone(Rows(x), tensor("w_in"));
         Tensor rec = ops.linear(Rows(x), tensor("w_rec"), nullptr, nullptr, (int)DType::F32);
         Tensor b_raw = columns(rec, 0, heads_), a_raw, gate;
-        if (per_channel_) a_raw = ops.linear(Rows(ops.linear(Rows(x), tensor("a1"))), tensor("a2"), nullptr, nullptr, (int)DType::F32);
+        if (per_channel_) a_raw = ops.linear(Rows(ops.linear_alone(Rows(x), tensor("a1"))), tensor("a2"), nullptr, nullptr, (int)DType::F32);
         else a_raw = columns(rec, heads_, heads_);
-        if (low_rank_gate_) gate = ops.linear(Rows(ops.linear(Rows(x), tensor("g1"))), tensor("g2"));
+        if (low_rank_gate_) gate = ops.linear_alone(Rows(ops.linear_alone(Rows(x), tensor("g1"))), tensor("g2"));
         else gate = columns(in, 2 * qk + hv, hv);
         Ops::DeltaSpec sp;
         sp.heads = heads_;
@@ -179,7 +179,7 @@ public:
         if (rot_ == 0) throw ConfigError("latent_attention without a rotated part is not built");
         const int64_t qd = (int64_t)heads_ * (dim_ + rot_), kvd = (int64_t)rank_ + rot_;
         Tensor x = ops.materialize(h);
-        Tensor in = ops.linear(Rows(x), tensor("w_in"));
+        Tensor in = ops.linear_alone(Rows(x), tensor("w_in"));
         Ops::LatentSpec sp;
         sp.heads = heads_;
         sp.dim = dim_;

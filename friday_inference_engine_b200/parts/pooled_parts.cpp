@@ -183,7 +183,7 @@ public:
             const Tensor& b = tensor("b_in");
             bias_flat = Tensor::make(b.data, b.dtype, {b.numel()});
         }
-        Tensor in = ops.linear(h, tensor("w_in"), bias_ ? &bias_flat : nullptr);
+        Tensor in = ops.linear_alone(h, tensor("w_in"), bias_ ? &bias_flat : nullptr);
         Ops::PooledSpec sp;
         sp.heads = heads_;
         sp.kv_heads = kv_heads_;
@@ -273,10 +273,10 @@ public:
     PartOut forward(Ops& ops, const Rows& h, const Tensor& residual, const StepContext& ctx, const CacheView& view, Norm*) override {
         const int64_t hd = (int64_t)heads_ * dim_;
         Tensor x = ops.materialize(h);
-        Tensor in = ops.linear(Rows(x), tensor("w_in"));
+        Tensor in = ops.linear_alone(Rows(x), tensor("w_in"));
         // what enters the recurrence stays 32-bit: the removal's and the decay's raw projections
         Tensor a_raw = ops.linear(Rows(x), tensor("a"), nullptr, nullptr, (int)DType::F32);
-        Tensor lw = ops.linear(Rows(x), tensor("w1"));
+        Tensor lw = ops.linear_alone(Rows(x), tensor("w1"));
         ops.tanh_rows(lw);
         Tensor z = ops.linear(Rows(lw), tensor("w2"), nullptr, nullptr, (int)DType::F32);
         Ops::GeneralDeltaSpec sp;

@@ -89,9 +89,9 @@ public:
     PartOut forward(Ops& ops, const Rows& h, const Tensor& residual, const StepContext& ctx, const CacheView& view, Norm*) override {
         const int64_t hk = (int64_t)heads_ * dk_, hv = (int64_t)heads_ * dv_;
         Tensor x = ops.materialize(h);
-        Tensor in = ops.linear(Rows(x), tensor("w_in"));
+        Tensor in = ops.linear_alone(Rows(x), tensor("w_in"));
         Tensor q = columns(in, 0, hk), k = columns(in, hk, hk), v = columns(in, 2 * hk, hv), g = columns(in, 2 * hk + hv, hv);
-        Tensor z = ops.linear(Rows(ops.linear(Rows(x), tensor("a1"))), tensor("a2"), nullptr, nullptr, (int)DType::F32);
+        Tensor z = ops.linear(Rows(ops.linear_alone(Rows(x), tensor("a1"))), tensor("a2"), nullptr, nullptr, (int)DType::F32);
         Ops::ScanSpec sp;
         sp.heads = heads_;
         sp.dk = dk_;
@@ -148,7 +148,7 @@ public:
 
     PartOut forward(Ops& ops, const Rows& h, const Tensor& residual, const StepContext& ctx, const CacheView& view, Norm*) override {
         const int64_t hk = (int64_t)heads_ * dk_, hv = (int64_t)heads_ * dv_;
-        Tensor in = ops.linear(h, tensor("w_in"));
+        Tensor in = ops.linear_alone(h, tensor("w_in"));
         Ops::DecaySpec sp;
         sp.heads = heads_;
         sp.dk = dk_;
@@ -207,11 +207,11 @@ public:
         Tensor x = ops.materialize(h);
         const int64_t rows = x.rows();
         Tensor mixes = ops.shift_mix(x, {tensor("mu.r"), tensor("mu.k"), tensor("mu.v"), tensor("mu.g"), tensor("mu.w")}, view, ctx);
-        Tensor r = ops.linear(Rows(mixes.row_slice(0, rows)), tensor("r"));
-        Tensor k = ops.linear(Rows(mixes.row_slice(rows, rows)), tensor("k"));
-        Tensor v = ops.linear(Rows(mixes.row_slice(2 * rows, rows)), tensor("v"));
-        Tensor g = ops.linear(Rows(mixes.row_slice(3 * rows, rows)), tensor("g"));
-        Tensor lw = ops.linear(Rows(mixes.row_slice(4 * rows, rows)), tensor("w1"));
+        Tensor r = ops.linear_alone(Rows(mixes.row_slice(0, rows)), tensor("r"));
+        Tensor k = ops.linear_alone(Rows(mixes.row_slice(rows, rows)), tensor("k"));
+        Tensor v = ops.linear_alone(Rows(mixes.row_slice(2 * rows, rows)), tensor("v"));
+        Tensor g = ops.linear_alone(Rows(mixes.row_slice(3 * rows, rows)), tensor("g"));
+        Tensor lw = ops.linear_alone(Rows(mixes.row_slice(4 * rows, rows)), tensor("w1"));
         ops.tanh_rows(lw);
         Tensor z = ops.linear(Rows(lw), tensor("w2"), nullptr, nullptr, (int)DType::F32);
         const Tensor& u = tensor("u");

@@ -50,3 +50,32 @@ def test_row_groups_on_pairs(m, n, k):
     size = a.double().abs() @ w.double().abs().T + res.double().abs()
     # the product of two bf16 numbers is exact in 32 bits; k + 1 sums that may cut instead of round, then bf16's rounding
     assert bool(((out.double() - want).abs() <= (k + 1) * 2.0 ** -23 * size + 2.0 ** -8 * want.abs()).all())
+
+
+# few rows and a small matrix: around 8 and 16 rows, columns around the blocks of 16, k around a warp's 32 and 256 and a block's
+# 2,048 (one turn, several, sixteen warps), every epilogue; beyond these sizes the other kernel
+@pytest.mark.parametrize("m", [1, 7, 8, 9, 16, 17])
+@pytest.mark.parametrize("n,k", [(16, 8), (30, 264), (64, 2048), (2058, 72), (250, 2056), (96, 6152), (4096, 2304), (6000, 2048)])
+def test_few_rows_small_matrix(m, n, k):
+    big = rnd((m, k + 8), 1).bfloat16()
+    a, w = big[:, :k], rnd((n, k), 2, k ** -0.5).bfloat16()
+    bias, res32, res16 = rnd((n,), 3), rnd((m, n), 4), rnd((m, n), 5).bfloat16()
+    z, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    slack = (k + 3) * 2.0 ** -23
+    out = res32.clone()
+    ops.backend()._linear_tc(a, w, bias, out, out)
+    assert bool(((out.double() - (z + bias.double() + res32.double())).abs() <= slack * (size + bias.abs() + res32.abs())).all())
+    out = torch.empty_like(res16)
+    ops.backend()._linear_tc(a, w, None, res16, out, swap=-2)
+    want = z + res16.double()
+    assert bool(((out.double() - want).abs() <= slack * (size + res16.abs()) + 2.0 ** -8 * want.abs()).all())
+    half = torch.empty((m, n // 2), dtype=torch.bfloat16, device=DEV)
+    ops.backend()._linear_tc(a, w, None, None, half, act=1)
+    gate, up = z[:, 0::2], z[:, 1::2]
+    want = gate * torch.sigmoid(gate) * up
+    wide = 2 * slack * (size[:, 0::2] * (up.abs() + 1.0) + size[:, 1::2] * (gate.abs() + 1.0))
+    assert bool(((half.double() - want).abs() <= wide + 2.0 ** -8 * want.abs() + 1e-6).all())
+    squared = torch.empty((m, n), dtype=torch.bfloat16, device=DEV)
+    ops.backend()._linear_tc(a, w, None, None, squared, act=4)
+    want = z.clamp(min=0.0) ** 2
+    assert bool(((squared.double() - want).abs() <= 3 * slack * size * (z.abs() + 1.0) + 2.0 ** -8 * want + 1e-6).all())
