@@ -150,6 +150,97 @@ layernorm_cast_kernel(const TI* __restrict__ x, FrVec w, FrVec b, TO* __restrict
     }
 }
 
+// Both norms for rows of whole groups of four numbers: what a thread has of the row, the weights and the bias is fetched at
+// once, before the first sum.  A decoding step has one block per row and nothing beside it, so the chain of waits is the cost
+// (8 rows of 2,048 in
+// a decoding step: 11 us with the kernels above, 2.3 to 3.4 with this one).
+__device__ __forceinline__ void four_of(const float* p, int i, float (&v)[4]) {
+    const float4 a = *(const float4*)(p + i);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+}
+__device__ __forceinline__ void four_of(const bf16* p, int i, float (&v)[4]) { FrVec{p, FR_BF16}.four(i, v); }
+__device__ __forceinline__ void put_four(float* p, const float (&v)[4]) { *(float4*)p = make_float4(v[0], v[1], v[2], v[3]); }
+__device__ __forceinline__ void put_four(bf16* p, const float (&v)[4]) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+    *(uint2*)p = make_uint2(*(const uint32_t*)&a, *(const uint32_t*)&b);
+}
+
+// CENTRED: the layer norm above; else the norm around zero.  NV groups of four per thread.
+template <typename TI, typename TO, int NV, bool CENTRED>
+__global__ void __launch_bounds__(256)
+row_norm_kernel(const TI* __restrict__ x, FrVec w, FrVec b, float offset, TO* __restrict__ y, int width, float eps) {
+    __shared__ float sums[8], squares[8];
+    fr_pdl_wait();
+    fr_pdl_launch();
+    const TI* xr = x + (size_t)blockIdx.x * width;
+    TO* yr = y + (size_t)blockIdx.x * width;
+    float v[NV][4], wv[NV][4], bv[NV][4];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        const int i = 4 * (threadIdx.x + k * 256);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[k][e] = wv[k][e] = bv[k][e] = 0.f;
+        if (i < width) {
+            four_of(xr, i, v[k]);
+            w.four(i, wv[k]);
+            if (CENTRED && b.p != nullptr) b.four(i, bv[k]);
+        }
+    }
+    auto over_block = [&](float s, float* partial) {
+        s = fr_warp_sum(s);
+        if ((threadIdx.x & 31) == 0) partial[threadIdx.x >> 5] = s;
+        __syncthreads();
+        float total = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) total += partial[i];
+        return total;
+    };
+    float mean = 0.f;
+    if (CENTRED) {
+        float sum = 0.f;
+#pragma unroll
+        for (int k = 0; k < NV; ++k) sum += (v[k][0] + v[k][1]) + (v[k][2] + v[k][3]);
+        mean = over_block(sum, sums) / (float)width;
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+        if (4 * (int)(threadIdx.x + k * 256) < width)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                v[k][e] -= mean;
+                ss = fmaf(v[k][e], v[k][e], ss);
+            }
+    const float inv = 1.0f / sqrtf(over_block(ss, squares) / (float)width + eps);
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        const int i = 4 * (threadIdx.x + k * 256);
+        if (i >= width) break;
+        float o[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[e] = CENTRED ? v[k][e] * inv * wv[k][e] + bv[k][e] : v[k][e] * inv * (offset + wv[k][e]);
+        put_four(yr + i, o);
+    }
+}
+
+// Rows of up to 4,096 numbers that begin on 16 bytes (8 for bf16): groups of four per thread, 0 where the row is another.
+inline int row_norm_groups(const void* x, int in_dtype, const void* y, int out_dtype, int width) {
+    const uintptr_t in = in_dtype == FR_BF16 ? 7 : 15, out = out_dtype == FR_BF16 ? 7 : 15;
+    if (width % 4 || width > 4096 || width < 4 || ((uintptr_t)x & in) || ((uintptr_t)y & out)) return 0;
+    return (width + 1023) / 1024;
+}
+
+template <typename TI, typename TO, bool CENTRED>
+int launch_row_norm(int groups, const void* x, FrVec w, FrVec b, float offset, void* y, int n_rows, int width, float eps, cudaStream_t stream) {
+    const TI* xt = (const TI*)x;
+    TO* yt = (TO*)y;
+    if (groups == 1) FR_CUDA(fr_launch(row_norm_kernel<TI, TO, 1, CENTRED>, dim3(n_rows), dim3(256), 0, stream, xt, w, b, offset, yt, width, eps));
+    else if (groups == 2) FR_CUDA(fr_launch(row_norm_kernel<TI, TO, 2, CENTRED>, dim3(n_rows), dim3(256), 0, stream, xt, w, b, offset, yt, width, eps));
+    else FR_CUDA(fr_launch(row_norm_kernel<TI, TO, 4, CENTRED>, dim3(n_rows), dim3(256), 0, stream, xt, w, b, offset, yt, width, eps));
+    FR_CHECK_LAUNCH("row norm");
+    return FR_OK;
+}
+
 // out[r] = table[tokens[r]] * scale as 32-bit rows (ids outside the table leave zeros)
 template <typename TW>
 __global__ void embed_rows_kernel(const int* __restrict__ tokens, const TW* __restrict__ table, float* __restrict__ out, int width,
@@ -287,6 +378,12 @@ FR_EXPORT int residual_norm_cast(const void* x, int in_dtype, const void* w, int
                                  int n_rows, int width, float eps, cudaStream_t stream) {
     if (n_rows <= 0) return FR_OK;
     FrVec wv{w, w_dtype};
+    const FrVec none{nullptr, FR_F32};
+    if (const int groups = row_norm_groups(x, in_dtype, y, out_dtype, width)) {
+        if (in_dtype == FR_F32 && out_dtype == FR_F32) return launch_row_norm<float, float, false>(groups, x, wv, none, offset, y, n_rows, width, eps, stream);
+        if (in_dtype == FR_F32 && out_dtype == FR_BF16) return launch_row_norm<float, bf16, false>(groups, x, wv, none, offset, y, n_rows, width, eps, stream);
+        if (in_dtype == FR_BF16 && out_dtype == FR_BF16) return launch_row_norm<bf16, bf16, false>(groups, x, wv, none, offset, y, n_rows, width, eps, stream);
+    }
     const int key = in_dtype * 2 + out_dtype;
     switch (key) {
         case 0: FR_CUDA(fr_launch(norm_cast_kernel<float, float>, dim3(n_rows), dim3(256), 0, stream, (const float*)x, wv, offset, (float*)y, width, eps)); break;
@@ -400,6 +497,11 @@ FR_EXPORT int residual_layernorm_cast(const void* x, int in_dtype, const void* w
                                       int n_rows, int width, float eps, cudaStream_t stream) {
     if (n_rows <= 0) return FR_OK;
     FrVec wv{w, w_dtype}, bv{b, w_dtype};
+    if (const int groups = row_norm_groups(x, in_dtype, y, out_dtype, width)) {
+        if (in_dtype == FR_F32 && out_dtype == FR_F32) return launch_row_norm<float, float, true>(groups, x, wv, bv, 0.f, y, n_rows, width, eps, stream);
+        if (in_dtype == FR_F32 && out_dtype == FR_BF16) return launch_row_norm<float, bf16, true>(groups, x, wv, bv, 0.f, y, n_rows, width, eps, stream);
+        if (in_dtype == FR_BF16 && out_dtype == FR_BF16) return launch_row_norm<bf16, bf16, true>(groups, x, wv, bv, 0.f, y, n_rows, width, eps, stream);
+    }
     const int key = in_dtype * 2 + out_dtype;
     switch (key) {
         case 0: FR_CUDA(fr_launch(layernorm_cast_kernel<float, float>, dim3(n_rows), dim3(256), 0, stream, (const float*)x, wv, bv, (float*)y, width, eps)); break;
