@@ -1245,7 +1245,7 @@ FR_EXPORT int gemm_tc_fused(const void* x, const void* w, void* out, int out_dty
             configured.fetch_or(bit, std::memory_order_release);
         }
         const int pairs = pair_tiles < sm_count / 2 ? pair_tiles : sm_count / 2;
-        FR_CUDA(fr_launch_cluster(gemm_tc_pair_kernel<false>, dim3(2 * pairs), dim3(THREADS), PAIR_SMEM_BYTES, stream, 2u, mp, mq, p));
+        FR_CUDA(fr_launch_cluster(gemm_tc_pair_kernel<false>, dim3(2 * pairs), dim3(PAIR_THREADS), PAIR_SMEM_BYTES, stream, 2u, mp, mq, p));
         FR_CHECK_LAUNCH("gemm_tc (pairs)");
         return FR_OK;
     }
@@ -1312,7 +1312,7 @@ FR_EXPORT int gemm_tc_grouped(const void* x, const void* w, long long w_group, v
     // no more tiles than this, whatever the groups' sizes
     const long long most = ((long long)rows / (2 * TILE_P) + (rows < groups ? rows : groups)) * p.tiles_q;
     const int pairs = most < sm_count / 2 ? (int)most : sm_count / 2;
-    FR_CUDA(fr_launch_cluster(gemm_tc_pair_kernel<true>, dim3(2 * pairs), dim3(THREADS), PAIR_SMEM_BYTES, stream, 2u, mp, mq, p));
+    FR_CUDA(fr_launch_cluster(gemm_tc_pair_kernel<true>, dim3(2 * pairs), dim3(PAIR_THREADS), PAIR_SMEM_BYTES, stream, 2u, mp, mq, p));
     FR_CHECK_LAUNCH("gemm_tc (groups)");
     return FR_OK;
 }

@@ -11,7 +11,7 @@
 //   * the first CTA's MMA thread waits for full[s], issues the instructions, and commits to empty[s] of BOTH CTAs
 //     (a multicast commit), after a tile's last k block to acc_full[a] of both;
 //   * both CTAs' epilogue warps read their own 128 lanes of the accumulator and arrive on the FIRST CTA's
-//     acc_empty[a] (eight arrivals).
+//     acc_empty[a] (sixteen arrivals).
 // Every wait is bounded as in gemm_tc.cu.  Neither CTA leaves before the other (a cluster barrier before tensor
 // memory is freed): a CTA's shared memory and barriers are written from outside until the pair is done.
 #pragma once
@@ -22,7 +22,11 @@ constexpr int PAIR_BN = 256;                          // widest tile; p.bn may b
 constexpr int PAIR_STAGES = 6;
 constexpr int PAIR_Q_BYTES = (PAIR_BN / 2) * TILE_K * 2;
 constexpr int PAIR_STAGE_BYTES = P_BYTES + PAIR_Q_BYTES;
-constexpr int PAIR_SMEM_BYTES = PAIR_STAGES * PAIR_STAGE_BYTES + 1024 + (2 * PAIR_STAGES + 4) * 8 + 64 + PAIR_BN * 4;
+constexpr int PAIR_SMEM_BYTES = PAIR_STAGES * PAIR_STAGE_BYTES + 1024 + (2 * PAIR_STAGES + 4) * 8 + 64 + PAIR_BN * 4 + TILE_P * 4;
+// Eight warps finish a tile, two to each quarter of the accumulator's lanes, which take its groups of 16 columns in turn: with
+// one per quarter a gated tile's epilogue was longer than its products where k is short (2048 x 12288 x 2048: 107 us with one, 70 with two; eight experts
+// of some 512 rows, x 4096 x 2048: 113 and 70 to 76; prompts of the 7B shape 4 to 9 % less).
+constexpr int PAIR_FINISHERS = 256, PAIR_THREADS = 64 + PAIR_FINISHERS;
 
 __device__ __forceinline__ uint32_t cluster_addr(uint32_t local, uint32_t rank) {
     uint32_t remote;
@@ -120,7 +124,7 @@ struct PairWalk {
 constexpr int MAX_GROUPS = 256;
 
 template <bool GROUPED>
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __launch_bounds__(PAIR_THREADS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_q, const GemmParams p) {
     __shared__ int s_off[GROUPED ? MAX_GROUPS + 1 : 1];
     constexpr int STAGES = PAIR_STAGES, STAGE_BYTES = PAIR_STAGE_BYTES, BN = PAIR_BN;
@@ -131,7 +135,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
     uint64_t* bars = (uint64_t*)(smem + STAGES * STAGE_BYTES);
     // bars: full[STAGES], empty[STAGES], acc_full[2], acc_empty[2]
     uint32_t* tmem_slot = (uint32_t*)(bars + 2 * STAGES + 4);
+    volatile int* s_gave_up = (volatile int*)(tmem_slot + 1);               // a finisher of this CTA has stopped waiting
     float* s_gw = (float*)((uint8_t*)(bars + 2 * STAGES + 4) + 64);         // [BN] norm weights of the tile's columns
+    float* s_ss = s_gw + BN;                                                // [128] sums of squares that a row's other warp found
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = fr_cluster_rank();                                 // 0: the CTA that issues the instructions
     const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
@@ -140,13 +146,14 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
     const uint32_t first_full0 = cluster_addr(full0, 0), first_acce0 = cluster_addr(acce0, 0);
 
     if (threadIdx.x == 0) {
+        *s_gave_up = 0;
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(full0 + 8 * s, 1);
             mbar_init(empty0 + 8 * s, 1);
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(accf0 + 8 * a, 1);
-            mbar_init(acce0 + 8 * a, 8);                   // the epilogue warps of both CTAs
+            mbar_init(acce0 + 8 * a, 2 * PAIR_FINISHERS / 32);      // the epilogue warps of both CTAs
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -159,7 +166,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
     }
     if constexpr (GROUPED) {                               // where the groups lie is the predecessor's result
         fr_pdl_wait();
-        for (int g = threadIdx.x; g <= p.groups; g += THREADS) s_off[g] = p.group_rows[g];
+        for (int g = threadIdx.x; g <= p.groups; g += PAIR_THREADS) s_off[g] = p.group_rows[g];
     }
     tc_fence_before();
     __syncthreads();
@@ -248,7 +255,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
     } else {
         const int quarter = warp & 3;                      // TMEM lanes this warp may read: 32*quarter ..
         const int i_local = quarter * 32 + lane;
-        const int et = threadIdx.x - 64;                   // 0..127 among the epilogue threads
+        const int et = threadIdx.x - 64;                   // 0..255 among the epilogue threads
+        const int share = et >> 7;                         // which of the quarter's two warps
         fr_pdl_wait();
         bool ok = true;
         int it = 0;
@@ -271,19 +279,25 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
             }
             float ss_row = 0.f;                            // with a norm begun: this row's sum of squares over the tile
             if (norm_rows) {
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                for (int i = et; i < bn; i += 128) {
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+                for (int i = et; i < bn; i += PAIR_FINISHERS) {
                     const int col = q_blk * bn + i;
                     s_gw[i] = col >= p.q_rows ? 0.f : f.norm_w_dtype == FR_F32 ? ((const float*)f.norm_w)[col]
                                                                                : __bfloat162float(((const __nv_bfloat16*)f.norm_w)[col]);
                 }
-                asm volatile("bar.sync 1, 128;" ::: "memory");
+                asm volatile("bar.sync 1, 256;" ::: "memory");
             }
-            if (!(ok = mbar_wait(accf0 + 8 * a, acc_phase, p.status, 4))) break;
+            ok = mbar_wait(accf0 + 8 * a, acc_phase, p.status, 4);
+            if (norm_rows) {                               // these warps meet again below: they go on, or leave, together
+                if (!ok) *s_gave_up = 1;
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+                ok = *s_gave_up == 0;
+            }
+            if (!ok) break;
             tc_fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + a * BN;
 #pragma unroll 1
-            for (int c = 0; c < bn / 16; ++c) {
+            for (int c = share; c < bn / 16; c += 2) {
                 uint32_t r[16];
                 tc_ld16(taddr + c * 16, r);
                 tc_ld_wait();
@@ -300,7 +314,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(first_acce0 + 8 * a);     // the accumulator may be overwritten
-            if (norm_rows && gi < p.p_rows) f.out_ssq[(size_t)q_blk * p.p_rows + gi] = ss_row;
+            if (norm_rows) {                               // a row's two shares, the columns' even groups first
+                if (share == 1) s_ss[i_local] = ss_row;
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+                if (share == 0 && gi < p.p_rows) f.out_ssq[(size_t)q_blk * p.p_rows + gi] = ss_row + s_ss[i_local];
+            }
         }
     }
     tc_fence_before();
