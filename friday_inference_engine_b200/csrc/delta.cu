@@ -472,6 +472,205 @@ FR_EXPORT int delta_scan(const float* qkv, const void* a_raw, int ld_a, const vo
     FR_REFUSE("delta scan: unknown dtype %d", raw_dtype);
 }
 
+// ------------------------------------------------------------------ a step of one token per sequence
+// What the three kernels above and the heads' gated norm do for one token, in one: a block per (sequence, head) keeps the
+// head's matrix in registers (16 bytes of a row per thread and turn) while the convolution, the unit norms, the decay, the
+// correction along the key, the read-out, the norm over the head and the gate pass through shared memory.  Heads that share a
+// query and key head form a cluster: its first block moves their history on once all have read it.
+//
+// Bound by the matrices' bytes (8 sequences, 16 heads of 128 x 128: 16.8 MB, 2.6 us) and a chain of five barriers
+// (10.1 us; conv_prepare, scan and head_norm_gate took 25 us in a decoding
+// step, 36 with a decay per channel).
+namespace {
+
+struct StepArgs {
+    ConvArgs c;               // x, taps, state, geometry (out unused)
+    const float* a_raw;       // [rows][ld_a]
+    const float* b_raw;       // [rows][ld_b]
+    FrVec a_log, dt_bias, norm;
+    const void* gate;         // [rows][ld_gate] in x's dtype
+    void* y;                  // [rows][heads * dv] in x's dtype
+    long long s_off;
+    int ld_a, ld_b, ld_gate, heads, dv, gate_act;
+    float eps, out_scale;
+};
+
+constexpr int STEP_ROWS = 16;      // rows of the matrix per thread
+constexpr int STEP_CHANNELS = 256; // key or value channels of a head at most
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
+
+template <typename T, bool PER_CHANNEL>
+__global__ void __launch_bounds__(256) delta_step_kernel(const StepArgs p) {
+    __shared__ float sq[STEP_CHANNELS], sk[STEP_CHANNELS], sv[STEP_CHANNELS], sg[STEP_CHANNELS], su[STEP_CHANNELS], wsum[8];
+    __shared__ __align__(16) float part[2][1024];
+    const ConvArgs& c = p.c;
+    const int head = blockIdx.x, seq = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int share = p.heads / c.qk_heads, group = head / share, dk = c.dk, dv = p.dv;
+    const int qk = c.qk_heads * dk, channels = 2 * qk + c.v_channels, keep = c.taps - 1;
+    fr_pdl_wait();
+    fr_pdl_launch();
+    const int row = c.seq_start[seq];
+    if (c.seq_qlen[seq] <= 0 || c.row_seq[row] < 0) return;                 // (the whole cluster: its blocks have one sequence)
+    float* hist = c.state + (size_t)c.seq_slots[seq] * c.state_stride;
+    float4* S = (float4*)(hist + p.s_off + (size_t)head * dk * dv);
+    // this thread's part of the matrix: columns 4 c4 .. 4 c4 + 3 of rows rg, rg + groups, ...
+    const int across = dv >> 2, groups = 256 / across, c4 = tid % across, rg = tid / across;
+    float4 s[STEP_ROWS];
+#pragma unroll
+    for (int j = 0; j < STEP_ROWS; ++j) {
+        const int i = rg + j * groups;
+        s[j] = rg < groups && i < dk ? S[(size_t)i * across + c4] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const T* x = (const T*)c.x + (size_t)row * c.ld;
+    auto place = [&](int n, int& src, int& channel) {                       // the n-th of this head's q, k, v channels
+        const int which = n < dk ? 0 : n < 2 * dk ? 1 : 2, d = n - which * dk;
+        src = which == 0 ? c.q_off + group * dk + d : which == 1 ? c.k_off + group * dk + d : c.v_off + head * dv + d;
+        channel = which == 0 ? group * dk + d : which == 1 ? qk + group * dk + d : 2 * qk + head * dv + d;
+        return which;
+    };
+    const FrVec taps{c.taps_w, c.w_dtype};
+    for (int n = tid; n < 2 * dk + dv; n += 256) {
+        int src, channel;
+        const int which = place(n, src, channel);
+        const float now = fr_load(x + src);
+        float past[MAX_TAPS], acc = 0.f;
+#pragma unroll
+        for (int j = 0; j < MAX_TAPS; ++j)
+            if (j < keep) past[j] = hist[(size_t)j * channels + channel];
+#pragma unroll
+        for (int j = 0; j < MAX_TAPS; ++j)
+            if (j < keep) acc = fmaf(taps.at(channel * c.taps + j), past[j], acc);
+        acc = fmaf(taps.at(channel * c.taps + keep), now, acc);
+        const float v = silu_f(acc);
+        if (which == 0) sq[n] = v;
+        else if (which == 1) sk[n - dk] = v;
+        else {
+            sv[n - 2 * dk] = v;
+#pragma unroll
+            for (int j = 0; j < MAX_TAPS; ++j)                              // a value channel's history is this block's own
+                if (j < keep) hist[(size_t)j * channels + channel] = j + 1 < keep ? past[(j + 1) % MAX_TAPS] : now;
+        }
+    }
+    const float rate = expf(p.a_log.at(head));
+    if (PER_CHANNEL)
+        for (int i = tid; i < dk; i += 256) sg[i] = expf(-rate * softplus_f(p.a_raw[(size_t)row * p.ld_a + head * dk + i] + p.dt_bias.at(head * dk + i)));
+    const float decay = PER_CHANNEL ? 1.f : expf(-rate * softplus_f(p.a_raw[(size_t)row * p.ld_a + head] + p.dt_bias.at(head)));
+    const float beta = 1.0f / (1.0f + expf(-p.b_raw[(size_t)row * p.ld_b + head]));
+    float gate = 0.f, weight = 0.f;
+    if (tid < dv) {
+        gate = fr_load((const T*)p.gate + (size_t)row * p.ld_gate + head * dv + tid);
+        weight = p.norm.at(tid);
+    }
+    __syncthreads();
+    cluster_arrive();                                                       // this block has read its history
+    float qq = 0.f, kk = 0.f;                                               // every warp for itself
+    for (int i = lane; i < dk; i += 32) {
+        qq = fmaf(sq[i], sq[i], qq);
+        kk = fmaf(sk[i], sk[i], kk);
+    }
+    const float inv_q = c.q_scale / sqrtf(fr_warp_sum(qq) + c.unit_eps), inv_k = 1.0f / sqrtf(fr_warp_sum(kk) + c.unit_eps);
+    float4 r = make_float4(0.f, 0.f, 0.f, 0.f), o = r;
+#pragma unroll
+    for (int j = 0; j < STEP_ROWS; ++j) {
+        const int i = rg + j * groups;
+        if (i < dk) {
+            const float g = PER_CHANNEL ? sg[i] : decay, k = sk[i] * inv_k;
+            s[j].x *= g; s[j].y *= g; s[j].z *= g; s[j].w *= g;
+            r.x = fmaf(k, s[j].x, r.x); r.y = fmaf(k, s[j].y, r.y); r.z = fmaf(k, s[j].z, r.z); r.w = fmaf(k, s[j].w, r.w);
+        }
+    }
+    if (rg < groups) ((float4*)part[0])[rg * across + c4] = r;
+    __syncthreads();
+    if (tid < dv) {
+        float sum = 0.f;
+        for (int g = 0; g < groups; ++g) sum += part[0][g * dv + tid];
+        su[tid] = beta * (sv[tid] - sum);
+    }
+    __syncthreads();
+    if (rg < groups) {
+        const float4 u = make_float4(su[4 * c4], su[4 * c4 + 1], su[4 * c4 + 2], su[4 * c4 + 3]);
+#pragma unroll
+        for (int j = 0; j < STEP_ROWS; ++j) {
+            const int i = rg + j * groups;
+            if (i < dk) {
+                const float k = sk[i] * inv_k, q = sq[i] * inv_q;
+                s[j].x = fmaf(k, u.x, s[j].x); s[j].y = fmaf(k, u.y, s[j].y); s[j].z = fmaf(k, u.z, s[j].z); s[j].w = fmaf(k, u.w, s[j].w);
+                o.x = fmaf(q, s[j].x, o.x); o.y = fmaf(q, s[j].y, o.y); o.z = fmaf(q, s[j].z, o.z); o.w = fmaf(q, s[j].w, o.w);
+                S[(size_t)i * across + c4] = s[j];
+            }
+        }
+        ((float4*)part[1])[rg * across + c4] = o;
+    }
+    __syncthreads();
+    float v = 0.f;
+    if (tid < dv)
+        for (int g = 0; g < groups; ++g) v += part[1][g * dv + tid];
+    const float ss = fr_warp_sum(v * v);
+    if (lane == 0) wsum[warp] = ss;
+    __syncthreads();
+    float total = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) total += wsum[w];
+    if (tid < dv) {
+        const float inv = p.out_scale / sqrtf(total / (float)dv + p.eps), sig = 1.0f / (1.0f + expf(-gate));
+        fr_store((T*)p.y + (size_t)row * p.heads * dv + head * dv + tid, v * inv * weight * (p.gate_act == 1 ? sig : gate * sig));
+    }
+    cluster_wait();
+    if (head % share == 0) {                                                // all blocks of the query and key head have read its history
+        for (int n = tid; n < 2 * dk; n += 256) {
+            int src, channel;
+            place(n, src, channel);
+            float next[MAX_TAPS];
+#pragma unroll
+            for (int j = 0; j < MAX_TAPS; ++j)
+                if (j < keep) next[j] = j + 1 < keep ? hist[(size_t)(j + 1) * channels + channel] : fr_load(x + src);
+#pragma unroll
+            for (int j = 0; j < MAX_TAPS; ++j)
+                if (j < keep) hist[(size_t)j * channels + channel] = next[j];
+        }
+    }
+}
+
+}  // namespace
+
+// Whether delta_step takes these sizes: a thread holds its part of the matrix, heads on one query and key head fit a cluster.
+FR_EXPORT int delta_step_supports(int heads, int qk_heads, int dk, int dv, int taps, long long state_stride) {
+    if (heads <= 0 || qk_heads <= 0 || heads % qk_heads || heads / qk_heads > 8 || dk <= 0 || dk > STEP_CHANNELS || dv < 4 || dv > STEP_CHANNELS || dv % 4) return 0;
+    if (taps < 1 || taps > MAX_TAPS || state_stride % 4) return 0;
+    const long long s_off = (long long)(taps - 1) * (2ll * qk_heads * dk + (long long)heads * dv);
+    const int groups = 256 / (dv / 4);
+    return s_off % 4 == 0 && (dk + groups - 1) / groups <= STEP_ROWS ? 1 : 0;
+}
+
+// One token of every sequence (conv_prepare, scan and head_norm_gate in one; arguments as there, raw decays and betas fp32).
+FR_EXPORT int delta_step(const void* x, int ld, int q_off, int k_off, int v_off, const void* taps_w, int w_dtype, const float* a_raw, int ld_a,
+                         const float* b_raw, int ld_b, const void* a_log, const void* dt_bias, int vec_dtype, const void* gate, int ld_gate,
+                         int gate_act, const void* norm, int norm_dtype, float eps, float out_scale, void* y, float* state, long long state_stride,
+                         const int* row_seq, const int* seq_start, const int* seq_qlen, const int* seq_slots, int n_seqs, int heads, int qk_heads,
+                         int dk, int dv, int taps, float q_scale, float unit_eps, int per_channel, int dtype, cudaStream_t stream) {
+    if (n_seqs <= 0) return FR_OK;
+    if (!delta_step_supports(heads, qk_heads, dk, dv, taps, state_stride) || ((uintptr_t)state & 15) || n_seqs > 65535)
+        FR_REFUSE("delta step: %d heads of %d x %d on %d query/key heads, %d taps, or a state off 16 bytes", heads, dk, dv, qk_heads, taps);
+    StepArgs p;
+    const int rc = fill_conv(p.c, x, ld, q_off, k_off, v_off, taps_w, w_dtype, nullptr, state, state_stride, row_seq, seq_start, seq_qlen, seq_slots,
+                             n_seqs, qk_heads, dk, heads * dv, taps, q_scale, unit_eps);
+    if (rc != FR_OK) return rc;
+    p.a_raw = a_raw; p.b_raw = b_raw; p.ld_a = ld_a; p.ld_b = ld_b; p.a_log = FrVec{a_log, vec_dtype}; p.dt_bias = FrVec{dt_bias, vec_dtype};
+    p.norm = FrVec{norm, norm_dtype}; p.gate = gate; p.ld_gate = ld_gate; p.gate_act = gate_act; p.y = y; p.eps = eps; p.out_scale = out_scale;
+    p.s_off = (long long)(taps - 1) * (2ll * qk_heads * dk + (long long)heads * dv); p.heads = heads; p.dv = dv;
+    const dim3 grid(heads, n_seqs);
+    const unsigned share = (unsigned)(heads / qk_heads);
+    if (dtype == FR_F32 && per_channel) FR_CUDA(fr_launch_cluster(delta_step_kernel<float, true>, grid, dim3(256), 0, stream, share, p));
+    else if (dtype == FR_F32) FR_CUDA(fr_launch_cluster(delta_step_kernel<float, false>, grid, dim3(256), 0, stream, share, p));
+    else if (dtype == FR_BF16 && per_channel) FR_CUDA(fr_launch_cluster(delta_step_kernel<bf16, true>, grid, dim3(256), 0, stream, share, p));
+    else if (dtype == FR_BF16) FR_CUDA(fr_launch_cluster(delta_step_kernel<bf16, false>, grid, dim3(256), 0, stream, share, p));
+    else FR_REFUSE("delta step: unknown dtype %d", dtype);
+    FR_CHECK_LAUNCH("delta step");
+    return FR_OK;
+}
+
 // ------------------------------------------------------------------ the generalized delta rule
 // A decay per head and key channel and a removal along the unit key, both reading the old state:
 //

@@ -212,6 +212,12 @@ public:
     // dt_bias [heads (* dk)]: beta = sigmoid(b_raw), decay = exp(-exp(a_log) * softplus(a_raw + dt_bias)); out [rows, heads * dv] fp32
     Tensor delta_scan(const Tensor& qkv, const Tensor& a_raw, const Tensor& b_raw, const Tensor& a_log, const Tensor& dt_bias,
                       const DeltaSpec& spec, const CacheView& view, const StepContext& ctx);
+    // conv_silu_unit, delta_scan and head_norm_gate (a weight shared by the heads) in one kernel, for steps of one token per
+    // sequence whose sizes it takes and whose gate is in the projection's dtype; a_raw and b_raw fp32
+    bool delta_step_ok(const Tensor& proj, const Tensor& a_raw, const Tensor& gate, const DeltaSpec& spec, const CacheView& view, const StepContext& ctx) const;
+    Tensor delta_step(const Tensor& proj, const Tensor& taps, const Tensor& a_raw, const Tensor& b_raw, const Tensor& a_log, const Tensor& dt_bias,
+                      const Tensor& gate, const Tensor& norm, float eps, float out_scale, bool gate_sigmoid, const DeltaSpec& spec,
+                      const CacheView& view, const StepContext& ctx);
 
     // The generalized delta rule: S <- diag(w) S - (a u)(u^T S) + k v^T with both terms reading the old state, o = S^T r;
     // u = k / sqrt(sum k^2 + unit_eps) per head, w = exp(-rate * sigmoid(z + z_bias)), a = sigmoid(a_raw + a_bias).

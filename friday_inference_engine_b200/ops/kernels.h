@@ -130,6 +130,10 @@ struct Delta {
                            int, float, float, int, cudaStream_t);
     int (*general_scan)(const float*, const void*, int, int, float*, float*, long long, long long, const int*, const int*, const int*, int,
                         int, int, int, int, cudaStream_t);
+    int (*step_supports)(int, int, int, int, int, long long);
+    int (*step)(const void*, int, int, int, int, const void*, int, const float*, int, const float*, int, const void*, const void*, int, const void*, int,
+                int, const void*, int, float, float, void*, float*, long long, const int*, const int*, const int*, const int*, int, int, int, int, int, int,
+                float, float, int, int, cudaStream_t);
 };
 struct AttentionPooled {
     last_error_fn last_error;

@@ -833,6 +833,32 @@ Tensor Ops::delta_scan(const Tensor& qkv, const Tensor& a_raw, const Tensor& b_r
     return out;
 }
 
+bool Ops::delta_step_ok(const Tensor& proj, const Tensor& a_raw, const Tensor& gate, const DeltaSpec& s, const CacheView& view, const StepContext& ctx) const {
+    return ctx.decode && a_raw.dtype == DType::F32 && gate.dtype == proj.dtype && view.kind == CacheRequest::State && view.state.defined() &&
+           view.state.dtype == DType::F32 && aligned16(view.state.data) && ctx.n_seqs <= 65535 &&
+           kernels::delta().step_supports(s.heads, s.qk_heads, s.dk, s.dv, s.taps, view.state.numel() / view.state.shape[0]) != 0;
+}
+
+Tensor Ops::delta_step(const Tensor& proj, const Tensor& taps, const Tensor& a_raw, const Tensor& b_raw, const Tensor& a_log, const Tensor& dt_bias,
+                       const Tensor& gate, const Tensor& norm, float eps, float out_scale, bool gate_sigmoid, const DeltaSpec& s, const CacheView& view,
+                       const StepContext& ctx) {
+    const int64_t channels = 2 * (int64_t)s.qk_heads * s.dk + (int64_t)s.heads * s.dv;
+    const long long stride = view.state.numel() / view.state.shape[0];
+    if (!delta_step_ok(proj, a_raw, gate, s, view, ctx) || b_raw.dtype != DType::F32 || a_log.numel() != s.heads || a_log.dtype != dt_bias.dtype ||
+        dt_bias.numel() != (s.per_channel ? (int64_t)s.heads * s.dk : (int64_t)s.heads) || norm.numel() != s.dv || taps.numel() != channels * s.taps ||
+        (int64_t)(s.taps - 1) * channels + (int64_t)s.heads * s.dk * s.dv > stride)
+        throw KernelError("delta_step: one token per sequence, fp32 decays and betas, taps, rates, biases and norm of the heads' sizes, a state that holds them");
+    Tensor y = alloc(proj.dtype, proj.rows(), (int64_t)s.heads * s.dv);
+    const auto& k = kernels::delta();
+    Timed t(*this, Attention);
+    call(launches_, k, k.step(proj.data, (int)proj.ld, (int)s.q_off, (int)s.k_off, (int)s.v_off, taps.data, code(taps.dtype), (const float*)a_raw.data,
+                              (int)a_raw.ld, (const float*)b_raw.data, (int)b_raw.ld, a_log.data, dt_bias.data, code(a_log.dtype), gate.data, (int)gate.ld,
+                              gate_sigmoid ? 1 : 0, norm.data, code(norm.dtype), eps, out_scale, y.data, (float*)view.state.data, stride, ctx.row_seq,
+                              ctx.seq_start, ctx.seq_qlen, view.seq_slots, ctx.n_seqs, s.heads, s.qk_heads, s.dk, s.dv, s.taps, s.q_scale, s.unit_eps,
+                              s.per_channel ? 1 : 0, code(proj.dtype), stream_), "delta_step");
+    return y;
+}
+
 // ------------------------------------------------------------------ attention over a cached latent
 void Ops::rotate_pairs(Tensor& x, const StepContext& ctx, const float* freq, float mult, int heads, int64_t head_stride, int64_t first,
                        int dims) {

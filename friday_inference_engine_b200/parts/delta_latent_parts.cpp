@@ -125,6 +125,11 @@ public:
         sp.q_off = 0;
         sp.k_off = qk;
         sp.v_off = 2 * qk;
+        if (ops.delta_step_ok(in, a_raw, gate, sp, view, ctx)) {
+            Tensor one = ops.delta_step(in, tensor("taps"), a_raw, b_raw, tensor("A_log"), tensor("dt_bias"), gate, tensor("norm"), eps_, out_scale,
+                                        low_rank_gate_, sp, view, ctx);
+            return PartOut(ops.linear_residual(Rows(one), tensor("o"), nullptr, residual));
+        }
         Tensor qkv = ops.conv_silu_unit(in, tensor("taps"), sp, view, ctx);
         Tensor o = ops.delta_scan(qkv, a_raw, b_raw, tensor("A_log"), tensor("dt_bias"), sp, view, ctx);
         Tensor y = ops.head_norm_gate(o, gate, tensor("norm"), false, heads_, dv_, eps_, out_scale, x.dtype, ctx, low_rank_gate_);
