@@ -477,19 +477,19 @@ __global__ void key_concat_kernel(const T* __restrict__ kn, const T* __restrict_
     }
 }
 
-// Row r of scores [rows][ld] (fp32, unscaled) belongs to position pos0 + r and sees keys 0 .. pos0 + r.  Its softmax
+// scores [heads][rows][ld] (fp32, unscaled), heads head0, head0 + 1, ...  Row r belongs to position pos0 + r and sees keys 0 .. pos0 + r.  Its softmax
 // (scores times scale, the sink in the denominator) is written as two bf16 numbers per weight, p = hi + lo, so that the
 // product with the values keeps the weights' 32-bit precision in effect; keys out of sight get zeros.
-__global__ void __launch_bounds__(256) softmax_split_kernel(const float* __restrict__ s, int ld, int n_pad, int pos0, float scale,
-                                                            const void* sink, int sink_dtype, int head, bf16* __restrict__ hi,
+__global__ void __launch_bounds__(256) softmax_split_kernel(const float* __restrict__ s, int ld, int rows, int n_pad, int pos0, float scale,
+                                                            const void* sink, int sink_dtype, int head0, bf16* __restrict__ hi,
                                                             bf16* __restrict__ lo, int ld_p) {
     __shared__ float red[8];
     __shared__ float bc;
     fr_pdl_wait();
     fr_pdl_launch();
-    const int row = blockIdx.x;
-    const int n = min(pos0 + row + 1, n_pad);
-    const float* sr = s + (size_t)row * ld;
+    const size_t row = blockIdx.x;
+    const int head = head0 + (int)(row / rows), n = min(pos0 + (int)(row % rows) + 1, n_pad);
+    const float* sr = s + row * ld;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float m = -INFINITY;
     for (int j = threadIdx.x; j < n; j += blockDim.x) m = fmaxf(m, sr[j] * scale);
@@ -518,8 +518,8 @@ __global__ void __launch_bounds__(256) softmax_split_kernel(const float* __restr
     }
     __syncthreads();
     const float inv = bc;
-    bf16* h = hi + (size_t)row * ld_p;
-    bf16* o = lo + (size_t)row * ld_p;
+    bf16* h = hi + row * ld_p;
+    bf16* o = lo + row * ld_p;
     for (int j = threadIdx.x; j < n_pad; j += blockDim.x) {
         const float p = j < n ? expf(sr[j] * scale - m) * inv : 0.f;
         const bf16 ph = __float2bfloat16_rn(p);
@@ -528,7 +528,7 @@ __global__ void __launch_bounds__(256) softmax_split_kernel(const float* __restr
     }
 }
 
-// out[row][h * vd + n] = x[row][h * vd + n] * sigmoid(gate[row][gate_off + h]) (gate null: 1), fp32 -> T
+// out[row][h * vd + n] = x[h][row][n] * sigmoid(gate[row][gate_off + h]) (gate null: 1), fp32 [heads][rows][vd] -> T [rows][heads * vd]
 template <typename T>
 __global__ void gate_cast_kernel(const float* __restrict__ x, const T* __restrict__ gate, int ld_gate, int gate_off, int heads, int vd,
                                  T* __restrict__ out) {
@@ -536,7 +536,7 @@ __global__ void gate_cast_kernel(const float* __restrict__ x, const T* __restric
     fr_pdl_launch();
     const size_t row = blockIdx.x;
     for (int i = threadIdx.x; i < heads * vd; i += blockDim.x) {
-        float v = x[row * heads * vd + i];
+        float v = x[((size_t)(i / vd) * gridDim.x + row) * vd + i % vd];
         if (gate != nullptr) v *= 1.0f / (1.0f + expf(-fr_load(gate + row * ld_gate + gate_off + i / vd)));
         fr_store(out + row * heads * vd + i, v);
     }
@@ -631,10 +631,10 @@ FR_EXPORT int attention_latent_gather(const void* c_pool, const void* r_pool, co
 }
 
 // hi and lo: rows of ld_p numbers each (the two may be halves of one buffer's rows)
-FR_EXPORT int attention_latent_softmax_split(const float* scores, int ld, int rows, int n_pad, int pos0, float scale, const void* sink,
+FR_EXPORT int attention_latent_softmax_split(const float* scores, int ld, int rows, int heads, int n_pad, int pos0, float scale, const void* sink,
                                              int sink_dtype, int head, void* hi, void* lo, int ld_p, cudaStream_t stream) {
-    if (rows <= 0) return FR_OK;
-    FR_CUDA(fr_launch(softmax_split_kernel, dim3(rows), dim3(256), 0, stream, scores, ld, n_pad, pos0, scale, sink, sink_dtype, head,
+    if (rows <= 0 || heads <= 0) return FR_OK;
+    FR_CUDA(fr_launch(softmax_split_kernel, dim3((unsigned)((long long)rows * heads)), dim3(256), 0, stream, scores, ld, rows, n_pad, pos0, scale, sink, sink_dtype, head,
                       (bf16*)hi, (bf16*)lo, ld_p));
     FR_CHECK_LAUNCH("softmax_split");
     return FR_OK;

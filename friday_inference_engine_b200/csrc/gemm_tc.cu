@@ -89,8 +89,9 @@ struct GemmParams {
                         // ACT_RELU_SQUARED: max(x, 0)^2 of every column
     int tiles_p, tiles_q, splits, kb_total, kb_per;
     int group_p;        // pairs of SMs: row tiles that go together (gemm_tc_pair.cuh)
-    const int* group_rows;      // rows in groups with weights of their own: [groups + 1], where they begin (null: one group)
-    int groups;
+    const int* group_rows;      // rows in groups with weights of their own: [groups + 1], where they begin (null: group_size rows each)
+    int groups, group_size;
+    int x_planes;               // the groups' rows of x lie in planes of their own
     // Work decomposition.  The first dp_tiles tiles are cut into `splits` equal k ranges each and dealt out round
     // robin (splits = 1: whole tiles).  The remaining sk_tiles tiles ("stream-k"): their k blocks, laid end to end,
     // are cut into one contiguous run of sk_units per CTA, so that a last, partial wave of tiles keeps every SM busy.
@@ -1273,18 +1274,21 @@ FR_EXPORT int gemm_tc_fused(const void* x, const void* w, void* out, int out_dty
 // group left most pairs idle (eight experts of some 512 rows, 2048 x 4096 and 2048 x 2048, bf16: 16 launches, 315 us in all
 // on a B200; two of this kernel 154).
 // row_tiles: how many tiles of 256 rows the groups have in all, as far as the caller knows (for the width of the tiles).
-// act as in gemm_tc_act; rows beyond the last group are left as they are.
-FR_EXPORT int gemm_tc_grouped(const void* x, const void* w, long long w_group, void* out, int out_dtype, const int* offsets, int groups, int rows,
+// act as in gemm_tc_act; rows beyond the last group are left as they are.  offsets null: the groups have rows / groups rows each;
+// x_group not zero (only then): group g's rows begin x_group * g elements after the first's (heads side by side in one row).
+FR_EXPORT int gemm_tc_grouped(const void* x, long long x_group, const void* w, long long w_group, void* out, int out_dtype, const int* offsets, int groups, int rows,
                               int n, int k, int lda, int ldw, int ldo, int row_tiles, int act, float act_limit, float act_slope, int* status, int sm_count,
                               cudaStream_t stream) {
     if (rows <= 0 || n <= 0 || groups <= 0) return FR_OK;
     if (act < 0 || act > ACT_RELU_SQUARED || (act && ((n % 2 && act != ACT_RELU_SQUARED) || out_dtype != FR_BF16)))
         FR_REFUSE("gemm_tc_grouped: an activation (%d) needs bf16 output, a gated one an even n", act);
     if (act == 3 && !(act_limit > 0.f)) FR_REFUSE("gemm_tc_grouped: the clipped gated unit needs its limit");
+    if (x_group < 0 || x_group % 8 || (offsets == nullptr ? rows % groups : x_group))
+        FR_REFUSE("gemm_tc_grouped: %d rows in %d groups, %lld elements apart: without offsets the groups are alike, with them the rows follow one another", rows, groups, x_group);
     if (k <= 0 || k % 8 || lda % 8 || ldw % 8 || w_group % 8 || w_group <= 0 || (((uintptr_t)x | (uintptr_t)w) & 15))
         FR_REFUSE("gemm_tc_grouped: k = %d, the strides (%d, %d, %lld) and the operands' starts must keep to 16 bytes", k, lda, ldw, w_group);
-    if (groups > MAX_GROUPS || sm_count < 2 || status == nullptr || offsets == nullptr)
-        FR_REFUSE("gemm_tc_grouped: %d groups (at most %d) need their offsets, a status word and two SMs", groups, MAX_GROUPS);
+    if (groups > MAX_GROUPS || sm_count < 2 || status == nullptr)
+        FR_REFUSE("gemm_tc_grouped: %d groups (at most %d) need a status word and two SMs", groups, MAX_GROUPS);
     GemmParams p;
     memset(&p, 0, sizeof p);
     p.f.act_limit = act_limit; p.f.act_slope = act_slope;
@@ -1296,8 +1300,10 @@ FR_EXPORT int gemm_tc_grouped(const void* x, const void* w, long long w_group, v
     p.splits = 1; p.kb_total = p.kb_per = (k + TILE_K - 1) / TILE_K;
     p.group_rows = offsets;
     p.groups = groups;
+    p.group_size = rows / groups;
+    p.x_planes = x_group > 0 ? 1 : 0;
     CUtensorMap mp, mq;
-    int rc = make_map(&mp, x, rows, k, lda, TILE_P);
+    int rc = x_group > 0 ? encode_group_map(&mp, x, groups, x_group, p.group_size, k, lda, TILE_P) : make_map(&mp, x, rows, k, lda, TILE_P);
     if (rc) return rc;
     rc = encode_group_map(&mq, w, groups, w_group, n, k, ldw, p.bn / 2);
     if (rc) return rc;

@@ -166,7 +166,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
     }
     if constexpr (GROUPED) {                               // where the groups lie is the predecessor's result
         fr_pdl_wait();
-        for (int g = threadIdx.x; g <= p.groups; g += PAIR_THREADS) s_off[g] = p.group_rows[g];
+        for (int g = threadIdx.x; g <= p.groups; g += PAIR_THREADS) s_off[g] = p.group_rows != nullptr ? p.group_rows[g] : g * p.group_size;
     }
     tc_fence_before();
     __syncthreads();
@@ -219,7 +219,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
                     if (rank == 0) mbar_expect_tx(full0 + 8 * stage, stage_tx);
                     load_weights(head, dst + P_BYTES, first_full0 + 8 * stage);
                 }
-                tma_load_2d_pair(dst, &map_p, head.kb * TILE_K, head.tiles.row0 + (int)rank * TILE_P, first_full0 + 8 * stage);
+                const int row = head.tiles.row0 + (int)rank * TILE_P;
+                if (GROUPED && p.x_planes)
+                    tma_load_3d_pair(dst, &map_p, head.kb * TILE_K, row - s_off[head.tiles.group], head.tiles.group, first_full0 + 8 * stage);
+                else tma_load_2d_pair(dst, &map_p, head.kb * TILE_K, row, first_full0 + 8 * stage);
                 if (++stage == STAGES) { stage = 0; phase ^= 1; }
             }
         }

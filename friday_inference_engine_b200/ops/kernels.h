@@ -41,7 +41,7 @@ struct GemmTc {
     int (*fused)(const void*, const void*, void*, int, const void*, int, const void*, int, int, int, int, int, int, float*,
                  long long, int*, int, int*, int, int, int, int, int, const GemmFusion*, cudaStream_t);
     int (*plan)(int, int, int, int, int, int, int, long long*);
-    int (*grouped)(const void*, const void*, long long, void*, int, const int*, int, int, int, int, int, int, int, int, int, float, float, int*, int,
+    int (*grouped)(const void*, long long, const void*, long long, void*, int, const int*, int, int, int, int, int, int, int, int, int, float, float, int*, int,
                    cudaStream_t);
 };
 struct AttentionSimt {
@@ -160,7 +160,7 @@ struct AttentionLatent {
     int (*run)(const float*, float*, const void*, const void*, const int*, int, int, const int*, const int*, const void*, int, int,
                int, int, int, float, int, float*, int, cudaStream_t);
     int (*gather)(const void*, const void*, const int*, int, int, int, int, int, void*, void*, int, cudaStream_t);
-    int (*softmax_split)(const float*, int, int, int, int, float, const void*, int, int, void*, void*, int, cudaStream_t);
+    int (*softmax_split)(const float*, int, int, int, int, int, float, const void*, int, int, void*, void*, int, cudaStream_t);
     int (*key_concat)(const void*, const void*, int, int, int, int, void*, int, cudaStream_t);
     int (*gate_cast)(const float*, const void*, int, int, int, int, int, void*, int, cudaStream_t);
 };

@@ -917,7 +917,7 @@ Tensor Ops::latent_attention_prompt(const Tensor& proj, const Tensor& w_uk, cons
         throw KernelError("latent_attention_prompt: bfloat16 rows and a step whose lengths the host knows");
     const auto& k = kernels::attention_latent();
     const int64_t hv = (int64_t)s.heads * s.vdim;
-    Tensor of = alloc(DType::F32, proj.rows(), hv);
+    Tensor of = alloc(DType::F32, proj.rows(), hv), out = alloc(proj.dtype, proj.rows(), hv);
     int64_t r0 = 0;
     for (int q = 0; q < ctx.n_seqs; ++q) {
         const int64_t T = ctx.q_lens[(size_t)q], n = ctx.kv_lens[(size_t)q], n_pad = (n + 7) / 8 * 8;
@@ -937,33 +937,61 @@ Tensor Ops::latent_attention_prompt(const Tensor& proj, const Tensor& w_uk, cons
                  "key_concat");
         }
         Tensor vt = linear(Rows(w_uv), c_all);                          // [heads * vdim, 2 n_pad]: values, transposed, twice side by side
-        Tensor scores = alloc(DType::F32, T, n_pad);
-        Tensor weights = alloc(DType::BF16, T, 2 * n_pad);              // every weight as two bf16 numbers: [hi | lo]
         const Tensor rows = proj.row_slice(r0, T);
-        for (int h = 0; h < s.heads; ++h) {
+        // Several heads at a time, as many as 64 MB of scores hold: a launch per product and one for their softmax (a head by
+        // itself was three launches of some 7 us each, whatever its size: 16 heads x 512 rows 16 x 19 us;
+        // together 46).  Rows of the
+        // projection off 16 bytes: head by head, on whatever kernel takes them.
+        const void* q0 = (const char*)rows.data + (size_t)s.q_off * 2;
+        const bool together = rows.ld % 8 == 0 && aligned16(q0) && hd % 8 == 0 && sms_ >= 2;
+        const int64_t fit = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(s.heads, 256), (int64_t)(64 << 20) / (T * n_pad * 4)));
+        const int64_t at_once = together ? fit : 1;
+        Tensor scores = alloc(DType::F32, at_once * T, n_pad);
+        Tensor weights = alloc(DType::BF16, at_once * T, 2 * n_pad);    // every weight as two bf16 numbers: [hi | lo]
+        auto softmax = [&](int h, int64_t n_heads) {
+            Timed t(*this, Attention);
+            call(launches_, k, k.softmax_split((const float*)scores.data, (int)scores.ld, (int)T, (int)n_heads, (int)n_pad, (int)(n - T), s.scale,
+                                               sink ? sink->data : nullptr, sink ? code(sink->dtype) : 0, h, weights.data,
+                                               (char*)weights.data + (size_t)n_pad * 2, (int)(2 * n_pad), stream_), "softmax_split");
+        };
+        // the heads' results: [heads][T][vdim] for this sequence, one plane per head
+        const auto& g = kernels::gemm_tc();
+        const int64_t tiles = (T + 255) / 256;
+        for (int64_t h = 0; together && h < s.heads; h += at_once) {
+            const int64_t c = std::min<int64_t>(at_once, s.heads - h);
+            {
+                Timed t(*this, Product);
+                call(launches_, g, g.grouped((const char*)q0 + (size_t)h * hd * 2, hd, (const char*)kcat.data + (size_t)h * hd * 2, hd, scores.data,
+                                             code(DType::F32), nullptr, (int)c, (int)(c * T), (int)n_pad, (int)hd, (int)rows.ld, (int)kcat.ld, (int)n_pad,
+                                             (int)(c * tiles), 0, 0.f, 0.f, (int*)status_.get(), sms_, stream_), "gemm_tc_grouped");
+            }
+            softmax((int)h, c);
+            {
+                Timed t(*this, Product);
+                call(launches_, g, g.grouped(weights.data, 0, (const char*)vt.data + (size_t)h * s.vdim * vt.ld * 2, (long long)s.vdim * vt.ld,
+                                             (float*)of.data + (size_t)r0 * hv + (size_t)h * T * s.vdim, code(DType::F32), nullptr, (int)c, (int)(c * T),
+                                             s.vdim, (int)(2 * n_pad), (int)(2 * n_pad), (int)vt.ld, s.vdim, (int)(c * tiles), 0, 0.f, 0.f,
+                                             (int*)status_.get(), sms_, stream_), "gemm_tc_grouped");
+            }
+        }
+        for (int h = 0; !together && h < s.heads; ++h) {
             Tensor qh = rows, kh = kcat, vh = vt.row_slice((int64_t)h * s.vdim, s.vdim);
             qh.data = (char*)rows.data + (size_t)(s.q_off + (int64_t)h * hd) * 2;
             qh.shape[1] = hd;
             kh.data = (char*)kcat.data + (size_t)h * hd * 2;
             kh.shape[1] = hd;
             linear(Rows(qh), kh, nullptr, nullptr, (int)DType::F32, &scores);
-            {
-                Timed t(*this, Attention);
-                call(launches_, k, k.softmax_split((const float*)scores.data, (int)scores.ld, (int)T, (int)n_pad, (int)(n - T), s.scale,
-                                                   sink ? sink->data : nullptr, sink ? code(sink->dtype) : 0, h, weights.data,
-                                                   (char*)weights.data + (size_t)n_pad * 2, (int)(2 * n_pad), stream_), "softmax_split");
-            }
-            Tensor oh = of.row_slice(r0, T);
-            oh.data = (char*)oh.data + (size_t)h * s.vdim * 4;
-            oh.shape[1] = s.vdim;
+            softmax(h, 1);
+            Tensor oh = Tensor::make((float*)of.data + (size_t)r0 * hv + (size_t)h * T * s.vdim, DType::F32, {T, (int64_t)s.vdim});
             linear(Rows(weights), vh, nullptr, nullptr, (int)DType::F32, &oh);
+        }
+        {
+            Timed t(*this, Other);
+            call(launches_, k, k.gate_cast((const float*)of.data + (size_t)r0 * hv, s.gate_off >= 0 ? rows.data : nullptr, (int)proj.ld, (int)s.gate_off,
+                                           (int)T, s.heads, s.vdim, out.row_slice(r0, T).data, code(proj.dtype), stream_), "gate_cast");
         }
         r0 += T;
     }
-    Tensor out = alloc(proj.dtype, proj.rows(), hv);
-    Timed t(*this, Other);
-    call(launches_, k, k.gate_cast((const float*)of.data, s.gate_off >= 0 ? proj.data : nullptr, (int)proj.ld, (int)s.gate_off,
-                                   (int)proj.rows(), s.heads, s.vdim, out.data, code(proj.dtype), stream_), "gate_cast");
     return out;
 }
 
@@ -1097,13 +1125,13 @@ Tensor Ops::experts_grouped(const Tensor& h, const Routing& r, const Tensor& w_g
     Tensor act = alloc(DType::BF16, n_pairs, inner), part = alloc(DType::F32, n_pairs, width);
     {
         Timed t(*this, Product);
-        call(launches_, g, g.grouped(gathered.data, w_gate_up.data, 2 * (long long)inner * width, act.data, code(act.dtype), offsets, experts, (int)n_pairs,
+        call(launches_, g, g.grouped(gathered.data, 0, w_gate_up.data, 2 * (long long)inner * width, act.data, code(act.dtype), offsets, experts, (int)n_pairs,
                                      2 * inner, (int)width, (int)gathered.ld, (int)w_gate_up.ld, (int)act.ld, row_tiles, unit, limit, slope,
                                      (int*)status_.get(), sms_, stream_), "gemm_tc_grouped");
     }
     {
         Timed t(*this, Product);
-        call(launches_, g, g.grouped(act.data, w_down.data, inner, part.data, code(part.dtype), offsets, experts, (int)n_pairs, (int)width, inner,
+        call(launches_, g, g.grouped(act.data, 0, w_down.data, inner, part.data, code(part.dtype), offsets, experts, (int)n_pairs, (int)width, inner,
                                      (int)act.ld, (int)w_down.ld, (int)part.ld, row_tiles, 0, 0.f, 0.f, (int*)status_.get(), sms_, stream_),
              "gemm_tc_grouped");
     }

@@ -74,7 +74,7 @@ def test_streamed_experts(rows, top, experts, spread, width, inner):
 @pytest.mark.parametrize("side_by_side", [False, True])
 def test_grouped_product(sizes, n, k, act, side_by_side):
     g = lib.family("gemm_tc")
-    g.declare("gemm_tc_grouped", [P, P, L, P, I, P, I, I, I, I, I, I, I, I, I, F, F, P, I, P])
+    g.declare("gemm_tc_grouped", [P, L, P, L, P, I, P, I, I, I, I, I, I, I, I, I, F, F, P, I, P])
     groups, used = len(sizes), sum(sizes)
     rows = used + 5
     x = rnd((rows, k), 7)
@@ -90,7 +90,7 @@ def test_grouped_product(sizes, n, k, act, side_by_side):
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     if side_by_side and not act:
         parts[0].fill_(float("nan"))           # reaches no other group's sums
-    g.call("gemm_tc_grouped", ptr(x), ptr(w), step, ptr(out), 1 if act else 0, ptr(offsets), groups, rows, n, k, k, ldw, out.shape[1],
+    g.call("gemm_tc_grouped", ptr(x), 0, ptr(w), step, ptr(out), 1 if act else 0, ptr(offsets), groups, rows, n, k, k, ldw, out.shape[1],
            sum((s + 255) // 256 for s in sizes), act, 2.0, 1.702, ptr(status), sms, stream())
     assert int(status) == 0
     assert bool((out[used:] == 7.0).all())
@@ -109,3 +109,20 @@ def test_grouped_product(sizes, n, k, act, side_by_side):
             assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + slack + 1e-6).all())
         else:
             assert bool(((got - z).abs() <= k * 2.0 ** -23 * mag).all())
+
+
+# groups of equal size whose rows lie side by side (heads), no offsets: rows and columns around the tiles, k around the blocks
+@pytest.mark.parametrize("groups,size,n,k", [(1, 1, 8, 8), (3, 40, 520, 192), (16, 257, 264, 24), (5, 600, 128, 72)])
+def test_grouped_product_of_planes(groups, size, n, k):
+    g = lib.family("gemm_tc")
+    g.declare("gemm_tc_grouped", [P, L, P, L, P, I, P, I, I, I, I, I, I, I, I, I, F, F, P, I, P])
+    x, w = rnd((size, groups * k + 8), 9), rnd((n, groups * k), 10, 0.3)
+    out = torch.empty((groups * size, n), device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    g.call("gemm_tc_grouped", ptr(x), k, ptr(w), k, ptr(out), 0, None, groups, groups * size, n, k, groups * k + 8, groups * k, n,
+           groups * ((size + 255) // 256), 0, 0.0, 0.0, ptr(status), sms, stream())
+    assert int(status) == 0
+    for e in range(groups):
+        a, b = x[:, e * k:(e + 1) * k].double(), w[:, e * k:(e + 1) * k].double()
+        assert bool(((out[e * size:(e + 1) * size].double() - a @ b.T).abs() <= k * 2.0 ** -23 * (a.abs() @ b.abs().T)).all())
