@@ -29,7 +29,7 @@ FR_EXPORT const char* attention_simt_last_error() { return fr_error_text; }
 
 namespace {
 
-constexpr int MAX_PER_LANE = 8;   // head sizes up to 256
+constexpr int MOST_PER_LANE = 8;   // head sizes up to 256
 
 struct AttnArgs {
     const void* q;        // [rows][q_stride] ; head h at h*hd
@@ -46,13 +46,19 @@ struct AttnArgs {
     float out_scale;      // the result is multiplied by this
 };
 
-template <typename T>
+// MAX_PER_LANE: dimensions per lane; KEYS keys at a time: their loads are issued together, so that a warp waits for memory once
+// per KEYS keys.  Small heads take more of them: a step of a window of 24 keys over heads of 32 took 7.8 us at four at a time,
+// 6.6 at sixteen; a prompt of 333 rows over 28 heads of 128 229
+// and 184 (eight).
+template <typename T, int MAX_PER_LANE, int KEYS>
 __global__ void __launch_bounds__(128) attention_kernel(AttnArgs p) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int item = blockIdx.x * 4 + warp;          // (row, head)
     if (item >= p.rows * p.nq) return;
     const int row = item / p.nq, h = item - row * p.nq;
     const int split = blockIdx.y;
+    fr_pdl_wait();
+    fr_pdl_launch();
     const int seq = p.row_seq[row];
     T* o_row = (T*)p.out + (size_t)row * p.nq * p.vd + (size_t)h * p.vd;
     float* part = p.splits > 1 ? p.part + ((size_t)item * p.splits + split) * (p.vd + 2) : nullptr;
@@ -78,56 +84,46 @@ __global__ void __launch_bounds__(128) attention_kernel(AttnArgs p) {
             qv[i] = d < p.hd ? fr_load(q + d) * p.scale : 0.f;
         }
         const int* table = p.block_table + (size_t)seq * p.table_width;
-        // four keys at a time: their loads are issued together, so that a warp waits for memory once per four keys
-        for (int i = i0; i < i1; i += 4) {
-            const T* kr[4];
-            const T* vr[4];
-            float s4[4];
+        for (int i = i0; i < i1; i += KEYS) {
+            float sk[KEYS], vv[KEYS][MAX_PER_LANE];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
+            for (int u = 0; u < KEYS; ++u) {
                 const int iu = min(i + u, i1 - 1);           // past the end: the last key again (its weight is set to zero)
                 const int j = iu < kept ? iu : lo + (iu - kept);
                 const size_t at = ((size_t)table[j / p.page] * p.page + j % p.page) * p.nkv + kvh;
-                kr[u] = (const T*)p.k_pool + at * p.hd;
-                vr[u] = (const T*)p.v_pool + at * p.vd;
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
+                const T* kr = (const T*)p.k_pool + at * p.hd;
+                const T* vr = (const T*)p.v_pool + at * p.vd;
                 float s = 0.f;
 #pragma unroll
                 for (int c = 0; c < MAX_PER_LANE; ++c) {
                     const int d = lane + 32 * c;
-                    if (d < p.hd) s = fmaf(qv[c], fr_load(kr[u] + d), s);
+                    if (d < p.hd) s = fmaf(qv[c], fr_load(kr + d), s);
+                    vv[u][c] = d < p.vd ? fr_load(vr + d) : 0.f;
                 }
-                s4[u] = s;
+                sk[u] = s;
             }
-            float vv[4][MAX_PER_LANE];
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int c = 0; c < MAX_PER_LANE; ++c) {
-                    const int d = lane + 32 * c;
-                    vv[u][c] = d < p.vd ? fr_load(vr[u] + d) : 0.f;
-                }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-                for (int u = 0; u < 4; ++u) s4[u] += __shfl_xor_sync(0xffffffffu, s4[u], o);
+                for (int u = 0; u < KEYS; ++u) sk[u] += __shfl_xor_sync(0xffffffffu, sk[u], o);
             float m_new = m;
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (i + u < i1) m_new = fmaxf(m_new, s4[u]);
+            for (int u = 0; u < KEYS; ++u)
+                if (i + u < i1) m_new = fmaxf(m_new, sk[u]);
             const float alpha = expf(m - m_new);      // exp(-inf) = 0 on the first keys
-            float e4[4];
+            float sum = 0.f, add[MAX_PER_LANE];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) e4[u] = i + u < i1 ? expf(s4[u] - m_new) : 0.f;
-            l = l * alpha + ((e4[0] + e4[1]) + (e4[2] + e4[3]));
+            for (int c = 0; c < MAX_PER_LANE; ++c) add[c] = 0.f;
 #pragma unroll
-            for (int c = 0; c < MAX_PER_LANE; ++c) {
-                const int d = lane + 32 * c;
-                if (d < p.vd)
-                    acc[c] = acc[c] * alpha + ((e4[0] * vv[0][c] + e4[1] * vv[1][c]) + (e4[2] * vv[2][c] + e4[3] * vv[3][c]));
+            for (int u = 0; u < KEYS; ++u) {
+                const float e = i + u < i1 ? expf(sk[u] - m_new) : 0.f;
+                sum += e;
+#pragma unroll
+                for (int c = 0; c < MAX_PER_LANE; ++c) add[c] = fmaf(e, vv[u][c], add[c]);
             }
+            l = l * alpha + sum;
+#pragma unroll
+            for (int c = 0; c < MAX_PER_LANE; ++c) acc[c] = acc[c] * alpha + add[c];
             m = m_new;
         }
     }
@@ -151,6 +147,15 @@ __global__ void __launch_bounds__(128) attention_kernel(AttnArgs p) {
     }
 }
 
+template <typename T>
+cudaError_t launch_attention(const AttnArgs& p, dim3 grid, cudaStream_t stream) {
+    const int size = p.hd > p.vd ? p.hd : p.vd;
+    if (size <= 32) return fr_launch(attention_kernel<T, 1, 16>, grid, dim3(128), 0, stream, p);
+    if (size <= 64) return fr_launch(attention_kernel<T, 2, 8>, grid, dim3(128), 0, stream, p);
+    if (size <= 128) return fr_launch(attention_kernel<T, 4, 8>, grid, dim3(128), 0, stream, p);
+    return fr_launch(attention_kernel<T, 8, 4>, grid, dim3(128), 0, stream, p);
+}
+
 }  // namespace
 
 // Scratch floats needed for `splits` > 1 (vd: the size of a value head).
@@ -165,8 +170,8 @@ FR_EXPORT int attention_simt_masked(const void* q, int q_stride, void* out, cons
                                     const int* row_pos, int rows, int nq, int nkv, int hd, int vd, int window, int keep_first,
                                     float scale, float out_scale, int splits, float* scratch, int dtype, cudaStream_t stream) {
     if (rows <= 0) return FR_OK;
-    if (hd <= 0 || hd > 32 * MAX_PER_LANE) FR_REFUSE("attention: head size %d is outside 1..%d", hd, 32 * MAX_PER_LANE);
-    if (vd <= 0 || vd > 32 * MAX_PER_LANE) FR_REFUSE("attention: value size %d is outside 1..%d", vd, 32 * MAX_PER_LANE);
+    if (hd <= 0 || hd > 32 * MOST_PER_LANE) FR_REFUSE("attention: head size %d is outside 1..%d", hd, 32 * MOST_PER_LANE);
+    if (vd <= 0 || vd > 32 * MOST_PER_LANE) FR_REFUSE("attention: value size %d is outside 1..%d", vd, 32 * MOST_PER_LANE);
     if (nkv <= 0 || nq % nkv != 0) FR_REFUSE("attention: %d heads cannot share %d key/value heads", nq, nkv);
     if (splits < 1 || splits > 65535) FR_REFUSE("attention: %d splits", splits);
     if (splits > 1 && scratch == nullptr) FR_REFUSE("attention: splits need a scratch buffer");
@@ -177,13 +182,13 @@ FR_EXPORT int attention_simt_masked(const void* q, int q_stride, void* out, cons
     MergeArgs mp{scratch, out, rows, nq, vd, splits, out_scale};
     dim3 grid((items + 3) / 4, splits);
     if (dtype == FR_F32) {
-        attention_kernel<float><<<grid, 128, 0, stream>>>(p);
+        FR_CUDA(launch_attention<float>(p, grid, stream));
         FR_CHECK_LAUNCH("attention");
-        if (splits > 1) attention_merge_kernel<float><<<(items + 3) / 4, 128, 0, stream>>>(mp);
+        if (splits > 1) FR_CUDA(fr_launch(attention_merge_kernel<float>, dim3((items + 3) / 4), dim3(128), 0, stream, mp));
     } else if (dtype == FR_BF16) {
-        attention_kernel<__nv_bfloat16><<<grid, 128, 0, stream>>>(p);
+        FR_CUDA(launch_attention<__nv_bfloat16>(p, grid, stream));
         FR_CHECK_LAUNCH("attention");
-        if (splits > 1) attention_merge_kernel<__nv_bfloat16><<<(items + 3) / 4, 128, 0, stream>>>(mp);
+        if (splits > 1) FR_CUDA(fr_launch(attention_merge_kernel<__nv_bfloat16>, dim3((items + 3) / 4), dim3(128), 0, stream, mp));
     } else {
         FR_REFUSE("attention: unknown dtype %d", dtype);
     }

@@ -236,9 +236,10 @@ few_rows_kernel(const F32Args p) {
     constexpr int V = MR * NC;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n0 = (blockIdx.x * 4 + warp) * NC, m0 = blockIdx.y * MR;
-    fr_pdl_wait();
-    fr_pdl_launch();
-    if (n0 >= p.n) return;
+    if (n0 >= p.n) {
+        fr_pdl_wait();                                       // (no kernel ends before its predecessor)
+        return;
+    }
     Pair acc[V];
 #pragma unroll
     for (int v = 0; v < V; ++v) acc[v] = 0ull;
@@ -248,11 +249,17 @@ few_rows_kernel(const F32Args p) {
     for (int c = 0; c < NC; ++c) w[c] = (const ulonglong2*)(p.w + (size_t)min(n0 + c, p.n - 1) * p.ldw);
 #pragma unroll
     for (int r = 0; r < MR; ++r) x[r] = (const ulonglong2*)(p.a + (size_t)min(m0 + r, p.m - 1) * p.lda);
+    // the first piece of the weights, which do not depend on the kernel before this one, ahead of the wait for it
+    ulonglong2 first[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) first[c] = lane < p.k / 4 ? __ldg(w[c] + lane) : make_ulonglong2(0, 0);
+    fr_pdl_wait();
+    fr_pdl_launch();
 #pragma unroll 2
     for (int q = lane; q < p.k / 4; q += 32) {
         ulonglong2 y[NC];
 #pragma unroll
-        for (int c = 0; c < NC; ++c) y[c] = __ldg(w[c] + q);
+        for (int c = 0; c < NC; ++c) y[c] = q == lane ? first[c] : __ldg(w[c] + q);
 #pragma unroll
         for (int r = 0; r < MR; ++r) {
             const ulonglong2 z = x[r][q];

@@ -50,7 +50,7 @@ FR_EXPORT int rowwise_embedding(const int* tokens, const void* table, void* out,
                                 int dtype, cudaStream_t stream) {
     if (n_rows <= 0) return FR_OK;
     if (dtype == FR_F32)
-        embedding_kernel<float><<<n_rows, 256, 0, stream>>>(tokens, (const float*)table, (float*)out, width, vocab);
+        FR_CUDA(fr_launch(embedding_kernel<float>, dim3(n_rows), dim3(256), 0, stream, tokens, (const float*)table, (float*)out, width, vocab));
     else if (dtype == FR_BF16)
         FR_CUDA(fr_launch(embedding_kernel<__nv_bfloat16>, dim3(n_rows), dim3(256), 0, stream, tokens,
                           (const __nv_bfloat16*)table, (__nv_bfloat16*)out, width, vocab));
@@ -73,7 +73,7 @@ FR_EXPORT int rowwise_gather_rows(const int* rows, const void* src, void* out, i
                                   cudaStream_t stream) {
     if (n_rows <= 0) return FR_OK;
     if (dtype == FR_F32)
-        gather_rows_kernel<float><<<n_rows, 256, 0, stream>>>(rows, (const float*)src, (float*)out, width);
+        FR_CUDA(fr_launch(gather_rows_kernel<float>, dim3(n_rows), dim3(256), 0, stream, rows, (const float*)src, (float*)out, width));
     else if (dtype == FR_BF16)
         FR_CUDA(fr_launch(gather_rows_kernel<__nv_bfloat16>, dim3(n_rows), dim3(256), 0, stream, rows,
                           (const __nv_bfloat16*)src, (__nv_bfloat16*)out, width));
@@ -162,7 +162,7 @@ FR_EXPORT int rowwise_rmsnorm(const void* x, const void* w, int w_dtype, void* y
     if (n_rows <= 0) return FR_OK;
     FrVec wv{w, w_dtype};
     if (dtype == FR_F32)
-        rmsnorm_kernel<float><<<n_rows, 256, 0, stream>>>((const float*)x, wv, (float*)y, width, eps);
+        FR_CUDA(fr_launch(rmsnorm_kernel<float>, dim3(n_rows), dim3(256), 0, stream, (const float*)x, wv, (float*)y, width, eps));
     else if (dtype == FR_BF16 && width % 8 == 0 && width <= 8 * 256 * RMS_CHUNKS && (((uintptr_t)x | (uintptr_t)y) & 15) == 0)
         FR_CUDA(fr_launch(rmsnorm_bf16_kernel, dim3(n_rows), dim3(256), 0, stream, (const __nv_bfloat16*)x, wv,
                           (__nv_bfloat16*)y, width, eps));
@@ -199,7 +199,7 @@ FR_EXPORT int rowwise_gated_act(const void* gu, void* out, int n_rows, int inner
     const long long cap = (long long)(fr_sm_count() > 0 ? fr_sm_count() : 128) * 16;       // a few waves of the device
     const int blocks = (int)((long long)((total + 255) / 256) < cap ? (total + 255) / 256 : cap);
     if (dtype == FR_F32)
-        swiglu_kernel<float><<<blocks, 256, 0, stream>>>((const float*)gu, (float*)out, inner, total, act, limit, slope);
+        FR_CUDA(fr_launch(swiglu_kernel<float>, dim3(blocks), dim3(256), 0, stream, (const float*)gu, (float*)out, inner, total, act, limit, slope));
     else if (dtype == FR_BF16)
         FR_CUDA(fr_launch(swiglu_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, (const __nv_bfloat16*)gu,
                           (__nv_bfloat16*)out, inner, total, act, limit, slope));
@@ -353,9 +353,8 @@ FR_EXPORT int rowwise_rope_kv_write(void* qkv, const int* row_seq, const int* ro
     const dim3 grid(n_rows, n_rows < 64 ? (heads < 4 ? heads : 4) : 1);     // few rows: spread the heads over more SMs
     const size_t smem = (size_t)(rot > 0 ? rot : 2) * sizeof(float);
     if (dtype == FR_F32)
-        rope_kv_write_kernel<float><<<grid, threads, smem, stream>>>((float*)qkv, row_seq, row_pos, denom, rot, nq, nkv,
-                                                                     hd, (float*)k_pool, (float*)v_pool, block_table,
-                                                                     table_width, page, write);
+        FR_CUDA(fr_launch(rope_kv_write_kernel<float>, grid, dim3(threads), smem, stream, (float*)qkv, row_seq, row_pos, denom, rot,
+                          nq, nkv, hd, (float*)k_pool, (float*)v_pool, block_table, table_width, page, write));
     else if (dtype == FR_BF16)
         FR_CUDA(fr_launch(rope_kv_write_kernel<__nv_bfloat16>, grid, dim3(threads), smem, stream,
                           (__nv_bfloat16*)qkv, row_seq, row_pos, denom, rot, nq, nkv, hd, (__nv_bfloat16*)k_pool,
