@@ -228,6 +228,171 @@ __global__ void __launch_bounds__(128) head_linear_nk_kernel(HeadLinearArgs p) {
     }
 }
 
+// The same two products for bf16 weights in 16-byte pieces, with the weights of a thread on their way before the predecessor has
+// finished: a decoding step runs one round of blocks, so the chain of waits is the cost (8 rows, 16 heads, 128 x 512: 22 us each
+// with the kernels above, 5.8 and 8.8 with these).
+__device__ __forceinline__ void eight_of(const uint4& v, float (&f)[8]) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        f[2 * i] = __uint_as_float(w[i] << 16);
+        f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+    }
+}
+template <typename TX>
+__device__ __forceinline__ void stage_rows(const HeadLinearArgs& p, int h, int row0, int nr, float* sx) {
+    for (int idx = threadIdx.x; idx < HL_ROWS * p.k; idx += blockDim.x) {
+        const int r = idx / p.k, i = idx - r * p.k;
+        sx[idx] = r < nr ? fr_load((const TX*)p.x + (size_t)(row0 + r) * p.ld_x + p.x_off + (size_t)h * p.x_stride + i) : 0.f;
+    }
+}
+template <typename TO>
+__device__ __forceinline__ void head_out(const HeadLinearArgs& p, int row, int h, int n, float v) {
+    if (p.row_seq != nullptr && p.row_seq[row] < 0) return;
+    if (p.gate != nullptr) {
+        const float g = fr_load((const TO*)p.gate + (size_t)row * p.ld_gate + p.gate_off + h);
+        v *= 1.0f / (1.0f + expf(-g));
+    }
+    fr_store((TO*)p.out + (size_t)row * p.ld_out + (size_t)h * p.out_stride + n, v);
+}
+
+// layout 0: 128 columns per block, eight per thread; sixteen groups of threads share k
+template <typename TX, typename TO>
+__global__ void __launch_bounds__(256) head_kn_kernel(HeadLinearArgs p) {
+    extern __shared__ __align__(16) float sx[];          // [HL_ROWS][k], then [8 warps][HL_ROWS][128]
+    float* red = sx + HL_ROWS * p.k;
+    const int h = blockIdx.y, row0 = blockIdx.z * HL_ROWS, nr = min(HL_ROWS, p.rows - row0);
+    const int group = threadIdx.x >> 4, c0 = (threadIdx.x & 15) * 8, n0 = blockIdx.x * 128;
+    const bool inside = n0 + c0 < p.n;
+    const bf16* w = (const bf16*)p.w + (size_t)h * p.k * p.n + (inside ? n0 + c0 : 0);
+    uint4 wv[8];
+    auto fetch = [&](int i0) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int i = i0 + group + 16 * u;
+            wv[u] = i < p.k ? __ldg((const uint4*)(w + (size_t)i * p.n)) : make_uint4(0, 0, 0, 0);
+        }
+    };
+    fetch(0);
+    fr_pdl_wait();
+    fr_pdl_launch();
+    stage_rows<TX>(p, h, row0, nr, sx);
+    __syncthreads();
+    float acc[HL_ROWS][8];
+#pragma unroll
+    for (int r = 0; r < HL_ROWS; ++r)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[r][e] = 0.f;
+    for (int i0 = 0; i0 < p.k; i0 += 128) {
+        if (i0 > 0) fetch(i0);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int i = i0 + group + 16 * u;
+            if (i >= p.k) break;
+            float f[8];
+            eight_of(wv[u], f);
+#pragma unroll
+            for (int r = 0; r < HL_ROWS; ++r) {
+                const float x = sx[r * p.k + i];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) acc[r][e] = fmaf(x, f[e], acc[r][e]);
+            }
+        }
+    }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+    for (int r = 0; r < HL_ROWS; ++r)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const float v = acc[r][e] + __shfl_xor_sync(0xffffffffu, acc[r][e], 16);
+            if (lane < 16) red[(warp * HL_ROWS + r) * 128 + c0 + e] = v;
+        }
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < nr * 128; idx += 256) {
+        const int r = idx >> 7, c = idx & 127;
+        if (n0 + c >= p.n) continue;
+        float v = 0.f;
+#pragma unroll
+        for (int g = 0; g < 8; ++g) v += red[(g * HL_ROWS + r) * 128 + c];
+        head_out<TO>(p, row0 + r, h, n0 + c, v);
+    }
+}
+
+// layout 1: sixteen columns per block, two per warp; the lanes share k
+template <typename TX, typename TO>
+__global__ void __launch_bounds__(256) head_nk_kernel(HeadLinearArgs p) {
+    extern __shared__ __align__(16) float sx[];          // [HL_ROWS][k]
+    const int h = blockIdx.y, row0 = blockIdx.z * HL_ROWS, nr = min(HL_ROWS, p.rows - row0);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n0 = blockIdx.x * 16 + 2 * warp;
+    const uint4* w[2];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) w[c] = (const uint4*)((const bf16*)p.w + ((size_t)h * p.n + min(n0 + c, p.n - 1)) * p.k);
+    const int pieces = p.k >> 3;
+    uint4 wv[2][2];
+    auto fetch = [&](int q0) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int u = 0; u < 2; ++u) wv[c][u] = q0 + lane + 32 * u < pieces ? __ldg(w[c] + q0 + lane + 32 * u) : make_uint4(0, 0, 0, 0);
+    };
+    fetch(0);
+    fr_pdl_wait();
+    fr_pdl_launch();
+    stage_rows<TX>(p, h, row0, nr, sx);
+    __syncthreads();
+    float acc[2 * HL_ROWS];                              // [row][column]
+#pragma unroll
+    for (int v = 0; v < 2 * HL_ROWS; ++v) acc[v] = 0.f;
+    for (int q0 = 0; q0 < pieces; q0 += 64) {
+        if (q0 > 0) fetch(q0);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int q = q0 + lane + 32 * u;
+            if (q >= pieces) break;
+            float f[2][8];
+            eight_of(wv[0][u], f[0]);
+            eight_of(wv[1][u], f[1]);
+#pragma unroll
+            for (int r = 0; r < HL_ROWS; ++r) {
+                const float4 a = *(const float4*)(sx + r * p.k + 8 * q), b = *(const float4*)(sx + r * p.k + 8 * q + 4);
+                const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+                for (int c = 0; c < 2; ++c)
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) acc[2 * r + c] = fmaf(x[e], f[c][e], acc[2 * r + c]);
+            }
+        }
+    }
+    // sums over the lanes: halve the values and double the lanes behind each; lanes 2 v and 2 v + 1 end with value v
+#pragma unroll
+    for (int half = HL_ROWS, bit = 16; half > 0; half >>= 1, bit >>= 1)
+#pragma unroll
+        for (int v = 0; v < HL_ROWS; ++v)
+            if (v < half) {
+                const bool upper = (lane & bit) != 0;
+                const float give = upper ? acc[v] : acc[v + half], keep = upper ? acc[v + half] : acc[v];
+                acc[v] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+            }
+    acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
+    const int value = lane >> 1, r = value >> 1, n = n0 + (value & 1);
+    if ((lane & 1) == 0 && r < nr && n < p.n) head_out<TO>(p, row0 + r, h, n, acc[0]);
+}
+
+template <typename TX, typename TO>
+int launch_head_pieces(const HeadLinearArgs& p, int layout, cudaStream_t stream) {
+    const int row_blocks = (p.rows + HL_ROWS - 1) / HL_ROWS;
+    const size_t rows = (size_t)HL_ROWS * p.k * sizeof(float);
+    if (layout == 0) {
+        const size_t smem = rows + 8 * HL_ROWS * 128 * sizeof(float);
+        if (smem > 48 * 1024) FR_CUDA(cudaFuncSetAttribute(head_kn_kernel<TX, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        FR_CUDA(fr_launch(head_kn_kernel<TX, TO>, dim3((p.n + 127) / 128, p.heads, row_blocks), dim3(256), smem, stream, p));
+    } else {
+        FR_CUDA(fr_launch(head_nk_kernel<TX, TO>, dim3((p.n + 15) / 16, p.heads, row_blocks), dim3(256), rows, stream, p));
+    }
+    FR_CHECK_LAUNCH("head_linear (pieces)");
+    return FR_OK;
+}
+
 template <typename TX, typename TW, typename TO>
 int launch_head_linear(const HeadLinearArgs& p, int layout, cudaStream_t stream) {
     const size_t smem = (size_t)HL_ROWS * p.k * sizeof(float);
@@ -393,51 +558,230 @@ __global__ void __launch_bounds__(128) latent_attention_kernel(AttnArgs p) {
         }
 }
 
-__global__ void __launch_bounds__(128) latent_merge_kernel(AttnArgs p) {
+// The same for a bf16 cache, all heads of a row in one block: the block brings KEYS cached rows at a time into shared memory (the
+// next ones on their way meanwhile), and its warps take the heads in turn, NH each.  A warp per (row, head) read every cached
+// row once per head, two at a time: 8 rows, 16 heads, up to
+// 540 keys took 47 us, 20 here.
+constexpr int KEYS = 16;
+template <int NH>
+__global__ void __launch_bounds__(256, NH <= 2 ? 2 : 1) latent_rows_kernel(AttnArgs p) {
+    extern __shared__ __align__(16) unsigned char keys_raw[];            // [2][KEYS][rank + rot] bf16
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, row = blockIdx.x, split = blockIdx.y;
+    const int width = p.rank + p.rot;
+    bf16* keys = (bf16*)keys_raw;
     fr_pdl_wait();
     fr_pdl_launch();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int item = blockIdx.x * 4 + warp;
-    if (item >= p.rows * p.heads) return;
-    const int h = item % p.heads;
-    const float* part = p.part + (size_t)item * p.splits * (p.rank + 2);
-    // every lane takes the maximum and the sum of some splits: their loads are in flight together
-    float top = -INFINITY;
-    for (int s = lane; s < p.splits; s += 32) top = fmaxf(top, part[(size_t)s * (p.rank + 2) + p.rank]);
-    top = fr_warp_max(top);
-    const bool live = p.row_seq[item / p.heads] >= 0;
-    float sk = -INFINITY;
-    if (p.sink != nullptr && live) {
-        sk = FrVec{p.sink, p.sink_dtype}.at(h);
-        top = fmaxf(top, sk);
-    }
-    float l = 0.f;
-    for (int s = lane; s < p.splits; s += 32) {
-        const float ls = part[(size_t)s * (p.rank + 2) + p.rank + 1];
-        if (ls > 0.f) l += ls * expf(part[(size_t)s * (p.rank + 2) + p.rank] - top);
-    }
-    l = fr_warp_sum(l);
-    float acc[C_PER_LANE];
+    const int seq = p.row_seq[row];
+    const int n = seq >= 0 ? p.row_pos[row] + 1 : 0, chunk = (n + p.splits - 1) / p.splits;
+    const int i0 = min(split * chunk, n), i1 = min(i0 + chunk, n);
+    const int* table = p.block_table + (size_t)max(seq, 0) * p.table_width;
+    auto fetch = [&](int j0, int buf) {                                  // cached rows j0 .. j0 + KEYS - 1 of this split
+        const int per = width >> 3;
+        for (int idx = threadIdx.x; idx < KEYS * per; idx += 256) {
+            const int u = idx / per, c = (idx - u * per) * 8;
+            if (j0 + u >= i1) break;
+            const size_t at = (size_t)table[(j0 + u) / p.page] * p.page + (j0 + u) % p.page;
+            const bf16* src = c < p.rank ? (const bf16*)p.c_pool + at * p.rank + c : (const bf16*)p.r_pool + at * p.rot + (c - p.rank);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(keys + ((size_t)buf * KEYS + u) * width + c)), "l"(src) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(i0, 0);
+    // lane l has dimensions 2 l, 2 l + 1 of every 64
+    float q[NH][C_PER_LANE + R_PER_LANE], acc[NH][C_PER_LANE], m[NH], l[NH];
 #pragma unroll
-    for (int i = 0; i < C_PER_LANE; ++i) acc[i] = 0.f;
-    for (int s = 0; s < p.splits; ++s) {
-        const float* ps = part + (size_t)s * (p.rank + 2);
-        const float ls = ps[p.rank + 1];
-        const float f = ls > 0.f ? expf(ps[p.rank] - top) : 0.f;
+    for (int a = 0; a < NH; ++a) {
+        const int h = warp + 8 * a;
+        const float* qh = p.q + ((size_t)row * p.heads + min(h, p.heads - 1)) * width;
 #pragma unroll
-        for (int i = 0; i < C_PER_LANE; ++i) {
-            const int d = lane + 32 * i;
-            if (d < p.rank) acc[i] += ps[d] * f;
+        for (int i = 0; i < C_PER_LANE / 2; ++i) {
+            const int d = 2 * lane + 64 * i;
+            q[a][2 * i] = d < p.rank ? qh[d] * p.scale : 0.f;
+            q[a][2 * i + 1] = d < p.rank ? qh[d + 1] * p.scale : 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < R_PER_LANE / 2; ++i) {
+            const int d = 2 * lane + 64 * i;
+            q[a][C_PER_LANE + 2 * i] = d < p.rot ? qh[p.rank + d] * p.scale : 0.f;
+            q[a][C_PER_LANE + 2 * i + 1] = d < p.rot ? qh[p.rank + d + 1] * p.scale : 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < C_PER_LANE; ++i) acc[a][i] = 0.f;
+        m[a] = -INFINITY;
+        l[a] = 0.f;
+    }
+    int buf = 0;
+    for (int j0 = i0; j0 < i1; j0 += KEYS, buf ^= 1) {
+        fetch(j0 + KEYS, buf ^ 1);                                       // (nothing beyond the split's end)
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();
+        const bf16* rows = keys + (size_t)buf * KEYS * width;
+        const int count = min(KEYS, i1 - j0);
+        // (four keys of the round at a time: unrolled over all of them the loop was longer than the instruction cache, 40 us)
+#pragma unroll 1
+        for (int g = 0; g < count; g += 4) {
+            const bf16* group = rows + (size_t)g * width + 2 * lane;
+            const int live = count - g;
+#pragma unroll
+            for (int a = 0; a < NH; ++a) {
+                if (warp + 8 * a >= p.heads) break;
+                float s[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    s[u] = 0.f;
+                    const bf16* kr = group + (size_t)(u < live ? u : 0) * width;
+#pragma unroll
+                    for (int i = 0; i < C_PER_LANE / 2; ++i) {
+                        if (2 * lane + 64 * i < p.rank) {
+                            const float2 c = __bfloat1622float2(*(const __nv_bfloat162*)(kr + 64 * i));
+                            s[u] = fmaf(q[a][2 * i], c.x, s[u]);
+                            s[u] = fmaf(q[a][2 * i + 1], c.y, s[u]);
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < R_PER_LANE / 2; ++i) {
+                        if (2 * lane + 64 * i < p.rot) {
+                            const float2 c = __bfloat1622float2(*(const __nv_bfloat162*)(kr + p.rank + 64 * i));
+                            s[u] = fmaf(q[a][C_PER_LANE + 2 * i], c.x, s[u]);
+                            s[u] = fmaf(q[a][C_PER_LANE + 2 * i + 1], c.y, s[u]);
+                        }
+                    }
+                }
+                // sums over the lanes: eight lanes in a row end with one key's score
+                const bool up16 = (lane & 16) != 0, up8 = (lane & 8) != 0;
+                const float a0 = (up16 ? s[2] : s[0]) + __shfl_xor_sync(0xffffffffu, up16 ? s[0] : s[2], 16);
+                const float a1 = (up16 ? s[3] : s[1]) + __shfl_xor_sync(0xffffffffu, up16 ? s[1] : s[3], 16);
+                float mine = (up8 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, up8 ? a0 : a1, 8);
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+                if ((lane >> 3) >= live) mine = -INFINITY;
+                float m_new = fmaxf(mine, __shfl_xor_sync(0xffffffffu, mine, 16));
+                m_new = fmaxf(m[a], fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, 8)));
+                const float e = (lane >> 3) < live ? expf(mine - m_new) : 0.f, alpha = expf(m[a] - m_new);
+                float w[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) w[u] = __shfl_sync(0xffffffffu, e, 8 * u);
+                l[a] = l[a] * alpha + ((w[0] + w[1]) + (w[2] + w[3]));
+                m[a] = m_new;
+#pragma unroll
+                for (int i = 0; i < C_PER_LANE / 2; ++i) {
+                    if (2 * lane + 64 * i < p.rank) {
+                        float x = acc[a][2 * i] * alpha, y = acc[a][2 * i + 1] * alpha;
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const float2 c = __bfloat1622float2(*(const __nv_bfloat162*)(group + (size_t)(u < live ? u : 0) * width + 64 * i));
+                            x = fmaf(w[u], c.x, x);
+                            y = fmaf(w[u], c.y, y);
+                        }
+                        acc[a][2 * i] = x;
+                        acc[a][2 * i + 1] = y;
+                    }
+                }
+            }
+        }
+        __syncthreads();                                                 // all have read what the next turn overwrites
+    }
+#pragma unroll
+    for (int a = 0; a < NH; ++a) {
+        const int h = warp + 8 * a;
+        if (h >= p.heads) break;
+        const size_t item = (size_t)row * p.heads + h;
+        float f = 1.f;
+        float* o = p.out + item * p.rank;
+        if (p.splits > 1) {
+            o = p.part + (item * p.splits + split) * (p.rank + 2);
+            if (lane == 0) {
+                o[p.rank] = m[a];
+                o[p.rank + 1] = l[a];
+            }
+        } else {
+            float denom = l[a], g = 1.f;
+            if (p.sink != nullptr && seq >= 0) {
+                const float sk = FrVec{p.sink, p.sink_dtype}.at(h), top = fmaxf(m[a], sk);
+                g = expf(m[a] - top);
+                denom = l[a] * g + expf(sk - top);
+            }
+            f = denom > 0.f ? g / denom : 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < C_PER_LANE / 2; ++i) {
+            const int d = 2 * lane + 64 * i;
+            if (d < p.rank) {
+                o[d] = acc[a][2 * i] * f;
+                o[d + 1] = acc[a][2 * i + 1] * f;
+            }
         }
     }
+}
+
+// A block per (row, head): the splits' factors through shared memory, then every thread's dimensions with their loads in flight
+// together (a warp per item walked the splits one by one: 21 us for 128 items, 7 here).
+__global__ void __launch_bounds__(256) latent_merge_kernel(AttnArgs p) {
+    __shared__ float factor[256];
+    fr_pdl_wait();
+    fr_pdl_launch();
+    const int lane = threadIdx.x & 31, item = blockIdx.x, h = item % p.heads;
+    const size_t step = p.rank + 2;
+    const float* part = p.part + (size_t)item * p.splits * step;
+    // thread s has split s (and s + 256, ...): the maximum over the block, then the factors and the sum of the weights
+    __shared__ float over[2][8];
+    float m_of = -INFINITY, l_of = 0.f;
+    if ((int)threadIdx.x < p.splits) {
+        m_of = part[threadIdx.x * step + p.rank];
+        l_of = part[threadIdx.x * step + p.rank + 1];
+    }
+    float top = m_of;
+    for (int s = threadIdx.x + 256; s < p.splits; s += 256) top = fmaxf(top, part[s * step + p.rank]);
+    const bool live = p.row_seq[item / p.heads] >= 0;
+    const float sk = p.sink != nullptr && live ? FrVec{p.sink, p.sink_dtype}.at(h) : -INFINITY;
+    top = fr_warp_max(top);
+    if (lane == 0) over[0][threadIdx.x >> 5] = top;
+    __syncthreads();
+    top = sk;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) top = fmaxf(top, over[0][i]);
+    float l = l_of > 0.f ? l_of * expf(m_of - top) : 0.f;
+    for (int s = threadIdx.x + 256; s < p.splits; s += 256) {
+        const float ls = part[s * step + p.rank + 1];
+        if (ls > 0.f) l += ls * expf(part[s * step + p.rank] - top);
+    }
+    l = fr_warp_sum(l);
+    if (lane == 0) over[1][threadIdx.x >> 5] = l;
+    static_assert(32 * C_PER_LANE <= 512, "two dimensions per thread");
+    const int d0 = threadIdx.x, d1 = threadIdx.x + 256;
+    float a0 = 0.f, a1 = 0.f;
+    for (int s0 = 0; s0 < p.splits; s0 += 256) {
+        const int s = s0 + threadIdx.x, count = min(256, p.splits - s0);
+        if (s0 > 0) {
+            __syncthreads();
+            m_of = s < p.splits ? part[s * step + p.rank] : -INFINITY;
+            l_of = s < p.splits ? part[s * step + p.rank + 1] : 0.f;
+        }
+        factor[threadIdx.x] = l_of > 0.f ? expf(m_of - top) : 0.f;
+        __syncthreads();
+        const float* ps = part + s0 * step;
+#pragma unroll 16
+        for (int u = 0; u < count; ++u) {
+            if (d0 < p.rank) a0 = fmaf(ps[u * step + d0], factor[u], a0);
+            if (d1 < p.rank) a1 = fmaf(ps[u * step + d1], factor[u], a1);
+        }
+    }
+    l = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) l += over[1][i];
     if (p.sink != nullptr && live) l += expf(sk - top);
     const float inv = l > 0.f ? 1.0f / l : 0.f;
     float* o = p.out + (size_t)item * p.rank;
-#pragma unroll
-    for (int i = 0; i < C_PER_LANE; ++i) {
-        const int d = lane + 32 * i;
-        if (d < p.rank) o[d] = acc[i] * inv;
-    }
+    if (d0 < p.rank) o[d0] = a0 * inv;
+    if (d1 < p.rank) o[d1] = a1 * inv;
+}
+
+// Whether latent_rows_kernel takes a cache: bf16 rows in 16-byte pieces, at most 32 heads.
+inline bool shared_rows(int heads, int rank, int rot, int dtype) { return dtype == FR_BF16 && heads <= 32 && rank % 8 == 0 && rot % 8 == 0; }
+
+template <int NH>
+cudaError_t launch_rows(const AttnArgs& p, cudaStream_t stream) {
+    return fr_launch(latent_rows_kernel<NH>, dim3(p.rows, p.splits), dim3(256), (size_t)2 * KEYS * (p.rank + p.rot) * 2, stream, p);
 }
 
 // ------------------------------------------------------------------ prompts: the pieces between tensor-core products
@@ -581,6 +925,13 @@ FR_EXPORT int attention_latent_head_linear(const void* x, int x_dtype, int ld_x,
     if (heads <= 0 || k <= 0 || n <= 0) FR_REFUSE("head_linear: %d heads, k %d, n %d", heads, k, n);
     HeadLinearArgs p{x, w, out, gate, row_seq, rows, heads, k, n, ld_x, x_off, x_stride, ld_out, out_stride, ld_gate, gate_off};
     const int key = x_dtype * 4 + w_dtype * 2 + out_dtype;
+    // bf16 weights whose rows (of n numbers in layout 0, of k in layout 1) are whole 16-byte pieces
+    if (w_dtype == FR_BF16 && (layout == 0 ? n : k) % 8 == 0 && ((uintptr_t)w & 15) == 0 && (size_t)HL_ROWS * k * sizeof(float) <= 48 * 1024) {
+        if (key == 6) return launch_head_pieces<bf16, float>(p, layout, stream);
+        if (key == 3) return launch_head_pieces<float, bf16>(p, layout, stream);
+        if (key == 2) return launch_head_pieces<float, float>(p, layout, stream);
+        if (key == 7) return launch_head_pieces<bf16, bf16>(p, layout, stream);
+    }
     switch (key) {
         case 0: return launch_head_linear<float, float, float>(p, layout, stream);
         case 4 + 2 + 0: return launch_head_linear<bf16, bf16, float>(p, layout, stream);
@@ -589,6 +940,16 @@ FR_EXPORT int attention_latent_head_linear(const void* x, int x_dtype, int ld_x,
         case 4 + 2 + 1: return launch_head_linear<bf16, bf16, bf16>(p, layout, stream);
         default: FR_REFUSE("head_linear: dtypes x %d, weights %d, out %d are not a combination that is built", x_dtype, w_dtype, out_dtype);
     }
+}
+
+// Splits of the keys for a call of `rows` rows that see at most `keys`: two blocks per SM, at least one round of keys each; 0: the
+// cache is not one for the kernel whose blocks have all heads of a row (then a split is a warp's work).
+FR_EXPORT int attention_latent_splits(int rows, int heads, int keys, int rank, int rot, int dtype) {
+    if (rows <= 0 || !shared_rows(heads, rank, rot, dtype)) return 0;
+    const int sms = fr_sm_count() > 0 ? fr_sm_count() : 148;
+    int splits = 2 * sms / rows;
+    if (splits > (keys + KEYS - 1) / KEYS) splits = (keys + KEYS - 1) / KEYS;
+    return splits < 1 ? 1 : splits;
 }
 
 FR_EXPORT int attention_latent(const float* q, float* out, const void* c_pool, const void* r_pool, const int* block_table,
@@ -604,6 +965,17 @@ FR_EXPORT int attention_latent(const float* q, float* out, const void* c_pool, c
                rot, splits, scale};
     const int items = rows * heads;
     const dim3 grid((items + 3) / 4, splits);
+    if (shared_rows(heads, rank, rot, dtype) && (((uintptr_t)c_pool | (uintptr_t)r_pool) & 15) == 0) {
+        if (heads <= 8) FR_CUDA(launch_rows<1>(p, stream));
+        else if (heads <= 16) FR_CUDA(launch_rows<2>(p, stream));
+        else FR_CUDA(launch_rows<4>(p, stream));
+        FR_CHECK_LAUNCH("latent attention (shared rows)");
+        if (splits > 1) {
+            FR_CUDA(fr_launch(latent_merge_kernel, dim3(items), dim3(256), 0, stream, p));
+            FR_CHECK_LAUNCH("latent attention merge");
+        }
+        return FR_OK;
+    }
     const bool pairs = rank % 2 == 0 && rot % 2 == 0 && (((uintptr_t)c_pool | (uintptr_t)r_pool) & 7) == 0;
     if (dtype == FR_F32 && pairs) FR_CUDA(fr_launch(latent_attention_kernel<float, 2>, grid, dim3(128), 0, stream, p));
     else if (dtype == FR_F32) FR_CUDA(fr_launch(latent_attention_kernel<float, 1>, grid, dim3(128), 0, stream, p));
@@ -612,7 +984,7 @@ FR_EXPORT int attention_latent(const float* q, float* out, const void* c_pool, c
     else FR_REFUSE("latent attention: unknown dtype %d", dtype);
     FR_CHECK_LAUNCH("latent attention");
     if (splits > 1) {
-        FR_CUDA(fr_launch(latent_merge_kernel, dim3((items + 3) / 4), dim3(128), 0, stream, p));
+        FR_CUDA(fr_launch(latent_merge_kernel, dim3(items), dim3(256), 0, stream, p));
         FR_CHECK_LAUNCH("latent attention merge");
     }
     return FR_OK;

@@ -479,7 +479,7 @@ FR_EXPORT int delta_scan(const float* qkv, const void* a_raw, int ld_a, const vo
 // query and key head form a cluster: its first block moves their history on once all have read it.
 //
 // Bound by the matrices' bytes (8 sequences, 16 heads of 128 x 128: 16.8 MB, 2.6 us) and a chain of five barriers
-// (10.1 us; conv_prepare, scan and head_norm_gate took 25 us in a decoding
+// (8.3 to 9.4 us; conv_prepare, scan and head_norm_gate took 25 us in a decoding
 // step, 36 with a decay per channel).
 namespace {
 
@@ -509,10 +509,12 @@ __global__ void __launch_bounds__(256) delta_step_kernel(const StepArgs p) {
     const int head = blockIdx.x, seq = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int share = p.heads / c.qk_heads, group = head / share, dk = c.dk, dv = p.dv;
     const int qk = c.qk_heads * dk, channels = 2 * qk + c.v_channels, keep = c.taps - 1;
-    fr_pdl_wait();
-    fr_pdl_launch();
+    // the step's geometry is final, and the matrix was written a step ago: both are read while the predecessor still runs
     const int row = c.seq_start[seq];
-    if (c.seq_qlen[seq] <= 0 || c.row_seq[row] < 0) return;                 // (the whole cluster: its blocks have one sequence)
+    if (c.seq_qlen[seq] <= 0 || c.row_seq[row] < 0) {                       // (the whole cluster: its blocks have one sequence)
+        fr_pdl_wait();                                                      // (this kernel must not end before its predecessor)
+        return;
+    }
     float* hist = c.state + (size_t)c.seq_slots[seq] * c.state_stride;
     float4* S = (float4*)(hist + p.s_off + (size_t)head * dk * dv);
     // this thread's part of the matrix: columns 4 c4 .. 4 c4 + 3 of rows rg, rg + groups, ...
@@ -523,6 +525,8 @@ __global__ void __launch_bounds__(256) delta_step_kernel(const StepArgs p) {
         const int i = rg + j * groups;
         s[j] = rg < groups && i < dk ? S[(size_t)i * across + c4] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
+    fr_pdl_wait();
+    fr_pdl_launch();
     const T* x = (const T*)c.x + (size_t)row * c.ld;
     auto place = [&](int n, int& src, int& channel) {                       // the n-th of this head's q, k, v channels
         const int which = n < dk ? 0 : n < 2 * dk ? 1 : 2, d = n - which * dk;

@@ -163,6 +163,7 @@ struct AttentionLatent {
     int (*softmax_split)(const float*, int, int, int, int, int, float, const void*, int, int, void*, void*, int, cudaStream_t);
     int (*key_concat)(const void*, const void*, int, int, int, int, void*, int, cudaStream_t);
     int (*gate_cast)(const float*, const void*, int, int, int, int, int, void*, int, cudaStream_t);
+    int (*splits)(int, int, int, int, int, int);
 };
 struct Routed {
     last_error_fn last_error;

@@ -899,9 +899,10 @@ Tensor Ops::latent_attention(const Tensor& qf, const Tensor* sink, const LatentS
         throw KernelError("latent_attention: the cache keeps one row [latent | key part] per position, the sink one number per head");
     const int rows = (int)qf.rows();
     Tensor out = alloc(DType::F32, rows, (int64_t)s.heads * s.rank);
-    const int splits = attention_splits(rows, s.heads, ctx.max_kv_len);
-    float* scratch = splits > 1 ? scratch_floats((int64_t)rows * s.heads * splits * (s.rank + 2)) : nullptr;
     const auto& k = kernels::attention_latent();
+    int splits = k.splits(rows, s.heads, ctx.max_kv_len, s.rank, s.rot, code(view.dtype));
+    if (splits < 1) splits = attention_splits(rows, s.heads, ctx.max_kv_len);
+    float* scratch = splits > 1 ? scratch_floats((int64_t)rows * s.heads * splits * (s.rank + 2)) : nullptr;
     Timed t(*this, Attention);
     call(launches_, k, k.run((const float*)qf.data, (float*)out.data, view.k_pool, view.v_pool, view.block_table, view.table_width,
                              view.page_size, ctx.row_seq, ctx.row_pos, sink ? sink->data : nullptr, sink ? code(sink->dtype) : 0, rows,
