@@ -16,7 +16,8 @@
 //                  (fp32) behind the place of qc
 //   head_linear    a product per head: out[row][h][n] = sum_k x[row][h][k] W_h[k][n] (weights [heads * k][n], layout 0) or
 //                  sum_k x[row][h][k] W_h[n][k] (weights [heads * n][k], layout 1), optionally times sigmoid(gate[row][h])
-//   attention      a warp per (row, head, split of the keys): online softmax in fp32 over the paged cache
+//   attention      a block per (row, split of the keys) that stages the cached rows for all heads (bf16, up to 32 heads), else a
+//                  warp per (row, head, split): online softmax in fp32 over the paged cache
 //                  (c in the key pool [pages][page][rank], r in the value pool [pages][page][rot]); a merge kernel when the
 //                  keys were split; the sink joins the denominator at the end
 //

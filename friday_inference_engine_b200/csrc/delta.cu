@@ -18,6 +18,7 @@
 //                  memory meanwhile.  beta = sigmoid(raw),
 //                  g = exp(-exp(A_log) * softplus(raw + dt_bias)) are formed here in fp32.  Columns of S never mix, so
 //                  any split of the value channels over blocks is exact.
+//   step           all of it and the heads' gated norm for one token per sequence (below)
 //
 // State of a sequence: [taps-1][channels] history (channel order of the stacked projection: q, k, v), then the heads'
 // matrices [heads][dk][dv], all fp32.  Everything here is fp32 arithmetic; only the projection's rows may be bf16.
