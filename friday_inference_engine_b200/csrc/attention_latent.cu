@@ -142,6 +142,7 @@ struct HeadLinearArgs {
     const void* gate;         // [rows][ld_gate] at gate_off + h: the result is multiplied by its sigmoid (or null)
     const int* row_seq;
     int rows, heads, k, n, ld_x, x_off, x_stride, ld_out, out_stride, ld_gate, gate_off;
+    int fixed_weights;        // no kernel writes w any more: it may be read ahead of the wait for the kernel before
 };
 
 constexpr int HL_ROWS = 8;        // rows per block
@@ -229,8 +230,8 @@ __global__ void __launch_bounds__(128) head_linear_nk_kernel(HeadLinearArgs p) {
     }
 }
 
-// The same two products for bf16 weights in 16-byte pieces, with the weights of a thread on their way before the predecessor has
-// finished: a decoding step runs one round of blocks, so the chain of waits is the cost (8 rows, 16 heads, 128 x 512: 22 us each
+// The same two products for bf16 weights in 16-byte pieces, with the weights of a thread (fixed ones) on their way before the
+// predecessor has finished: a decoding step runs one round of blocks, so the chain of waits is the cost (8 rows, 16 heads, 128 x 512: 22 us each
 // with the kernels above, 5.8 and 8.8 with these).
 __device__ __forceinline__ void eight_of(const uint4& v, float (&f)[8]) {
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
@@ -274,6 +275,7 @@ __global__ void __launch_bounds__(256) head_kn_kernel(HeadLinearArgs p) {
             wv[u] = i < p.k ? __ldg((const uint4*)(w + (size_t)i * p.n)) : make_uint4(0, 0, 0, 0);
         }
     };
+    if (!p.fixed_weights) fr_pdl_wait();
     fetch(0);
     fr_pdl_wait();
     fr_pdl_launch();
@@ -336,6 +338,7 @@ __global__ void __launch_bounds__(256) head_nk_kernel(HeadLinearArgs p) {
 #pragma unroll
             for (int u = 0; u < 2; ++u) wv[c][u] = q0 + lane + 32 * u < pieces ? __ldg(w[c] + q0 + lane + 32 * u) : make_uint4(0, 0, 0, 0);
     };
+    if (!p.fixed_weights) fr_pdl_wait();
     fetch(0);
     fr_pdl_wait();
     fr_pdl_launch();
@@ -918,13 +921,14 @@ FR_EXPORT int attention_latent_prepare(const void* x, int ld, int q_off, int kv_
 }
 
 // x_dtype / w_dtype / out_dtype: FR_F32 or FR_BF16 each; the gate (if any) is stored in the result's dtype.
-FR_EXPORT int attention_latent_head_linear(const void* x, int x_dtype, int ld_x, int x_off, int x_stride, const void* w, int w_dtype,
-                                           int layout, void* out, int out_dtype, int ld_out, int out_stride, const void* gate,
-                                           int ld_gate, int gate_off, const int* row_seq, int rows, int heads, int k, int n,
-                                           cudaStream_t stream) {
+// fixed_weights not zero: w is memory that no kernel writes any more, and may be read while the kernel before still runs.
+FR_EXPORT int attention_latent_head_linear_weights(const void* x, int x_dtype, int ld_x, int x_off, int x_stride, const void* w, int w_dtype,
+                                                   int layout, void* out, int out_dtype, int ld_out, int out_stride, const void* gate,
+                                                   int ld_gate, int gate_off, const int* row_seq, int rows, int heads, int k, int n,
+                                                   int fixed_weights, cudaStream_t stream) {
     if (rows <= 0) return FR_OK;
     if (heads <= 0 || k <= 0 || n <= 0) FR_REFUSE("head_linear: %d heads, k %d, n %d", heads, k, n);
-    HeadLinearArgs p{x, w, out, gate, row_seq, rows, heads, k, n, ld_x, x_off, x_stride, ld_out, out_stride, ld_gate, gate_off};
+    HeadLinearArgs p{x, w, out, gate, row_seq, rows, heads, k, n, ld_x, x_off, x_stride, ld_out, out_stride, ld_gate, gate_off, fixed_weights};
     const int key = x_dtype * 4 + w_dtype * 2 + out_dtype;
     // bf16 weights whose rows (of n numbers in layout 0, of k in layout 1) are whole 16-byte pieces
     if (w_dtype == FR_BF16 && (layout == 0 ? n : k) % 8 == 0 && ((uintptr_t)w & 15) == 0 && (size_t)HL_ROWS * k * sizeof(float) <= 48 * 1024) {
@@ -941,6 +945,15 @@ FR_EXPORT int attention_latent_head_linear(const void* x, int x_dtype, int ld_x,
         case 4 + 2 + 1: return launch_head_linear<bf16, bf16, bf16>(p, layout, stream);
         default: FR_REFUSE("head_linear: dtypes x %d, weights %d, out %d are not a combination that is built", x_dtype, w_dtype, out_dtype);
     }
+}
+
+// The same for weights that any earlier kernel of the stream may have made.
+FR_EXPORT int attention_latent_head_linear(const void* x, int x_dtype, int ld_x, int x_off, int x_stride, const void* w, int w_dtype,
+                                           int layout, void* out, int out_dtype, int ld_out, int out_stride, const void* gate,
+                                           int ld_gate, int gate_off, const int* row_seq, int rows, int heads, int k, int n,
+                                           cudaStream_t stream) {
+    return attention_latent_head_linear_weights(x, x_dtype, ld_x, x_off, x_stride, w, w_dtype, layout, out, out_dtype, ld_out, out_stride,
+                                                gate, ld_gate, gate_off, row_seq, rows, heads, k, n, 0, stream);
 }
 
 // Splits of the keys for a call of `rows` rows that see at most `keys`: two blocks per SM, at least one round of keys each; 0: the

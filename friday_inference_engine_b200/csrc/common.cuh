@@ -141,7 +141,9 @@ __device__ __forceinline__ float fr_warp_max(float v) {
 // follows one of these in a stream but was launched the ordinary way is fully serialised,
 // as always.  FRIDAY_PDL=0 in the environment switches the launch attribute off.
 //
-// What may be read ahead of the wait: memory that only copies from the host write (page tables), and the
+// What may be read ahead of the wait: memory that only copies from the host write (page tables), weights that the
+// caller calls fixed (the launchers' `fixed_weights`: no kernel writes them any more; other weights may be the
+// result of the kernel before, and are read after the wait), and the
 // geometry of the step (rows, positions, ended sequences), which is final before the step's first kernel
 // starts.  The latter holds because the row-wise kernels that open every step (embedding, the first norm)
 // wait before they let their dependents launch: whatever runs after them was launched after the step before

@@ -110,6 +110,7 @@ struct F32Args {
     const float* residual;
     int m, n, k, lda, ldw, ldo;
     int splits, kb_per;          // CTAs of the cluster that share a tile's k, k blocks of each
+    int fixed_weights;           // no kernel writes them any more: they may be read ahead of the wait for the kernel before
 };
 
 __device__ __forceinline__ void finish(const F32Args& p, int gm, int gn, float v) {
@@ -249,7 +250,8 @@ few_rows_kernel(const F32Args p) {
     for (int c = 0; c < NC; ++c) w[c] = (const ulonglong2*)(p.w + (size_t)min(n0 + c, p.n - 1) * p.ldw);
 #pragma unroll
     for (int r = 0; r < MR; ++r) x[r] = (const ulonglong2*)(p.a + (size_t)min(m0 + r, p.m - 1) * p.lda);
-    // the first piece of the weights, which do not depend on the kernel before this one, ahead of the wait for it
+    // the first piece of fixed weights, which do not depend on the kernel before this one, ahead of the wait for it
+    if (!p.fixed_weights) fr_pdl_wait();
     ulonglong2 first[NC];
 #pragma unroll
     for (int c = 0; c < NC; ++c) first[c] = lane < p.k / 4 ? __ldg(w[c] + lane) : make_ulonglong2(0, 0);
@@ -370,9 +372,10 @@ int run_f32(F32Args p, cudaStream_t stream) {
 // a: [m][k] (row stride lda), w: [n][k] (row stride ldw), out and residual: [m][n]
 // (row stride ldo; residual may be `out` itself).  bias may be null; its dtype is
 // given apart from the others because a bias stored in 32-bit stays so.
-FR_EXPORT int gemm_simt(const void* a, int a_dtype, const void* w, int w_dtype, void* out, int out_dtype,
-                        const void* bias, int bias_dtype, const void* residual, int m, int n, int k, int lda,
-                        int ldw, int ldo, cudaStream_t stream) {
+// fixed_weights not zero: w is memory that no kernel writes any more, and may be read while the kernel before still runs.
+FR_EXPORT int gemm_simt_weights(const void* a, int a_dtype, const void* w, int w_dtype, void* out, int out_dtype,
+                                const void* bias, int bias_dtype, const void* residual, int m, int n, int k, int lda,
+                                int ldw, int ldo, int fixed_weights, cudaStream_t stream) {
     if (m <= 0 || n <= 0) return FR_OK;
     if (k <= 0) FR_REFUSE("gemm_simt: k = %d", k);
     FrVec bv{bias, bias_dtype};
@@ -380,7 +383,7 @@ FR_EXPORT int gemm_simt(const void* a, int a_dtype, const void* w, int w_dtype, 
     // rows in 16-byte pieces (and no grid beyond the launch limits): the fp32 kernels
     if (a_dtype == FR_F32 && w_dtype == FR_F32 && out_dtype == FR_F32 && !((k | lda | ldw) & 3) && !(((uintptr_t)a | (uintptr_t)w) & 15) &&
         m <= 65535 * 32)
-        return run_f32(F32Args{(const float*)a, (const float*)w, (float*)out, bv, (const float*)residual, m, n, k, lda, ldw, ldo, 1, 0}, stream);
+        return run_f32(F32Args{(const float*)a, (const float*)w, (float*)out, bv, (const float*)residual, m, n, k, lda, ldw, ldo, 1, 0, fixed_weights}, stream);
     const int key = a_dtype * 4 + w_dtype * 2 + out_dtype;
     switch (key) {
         case 0: return launch<float, float, float>(a, w, out, bv, residual, m, n, k, lda, ldw, ldo, stream);
@@ -390,4 +393,11 @@ FR_EXPORT int gemm_simt(const void* a, int a_dtype, const void* w, int w_dtype, 
         case 7: return launch<bf16, bf16, bf16>(a, w, out, bv, residual, m, n, k, lda, ldw, ldo, stream);
         default: FR_REFUSE("gemm_simt: no kernel for dtypes a=%d w=%d out=%d", a_dtype, w_dtype, out_dtype);
     }
+}
+
+// The same for weights that any earlier kernel of the stream may have made.
+FR_EXPORT int gemm_simt(const void* a, int a_dtype, const void* w, int w_dtype, void* out, int out_dtype,
+                        const void* bias, int bias_dtype, const void* residual, int m, int n, int k, int lda,
+                        int ldw, int ldo, cudaStream_t stream) {
+    return gemm_simt_weights(a, a_dtype, w, w_dtype, out, out_dtype, bias, bias_dtype, residual, m, n, k, lda, ldw, ldo, 0, stream);
 }

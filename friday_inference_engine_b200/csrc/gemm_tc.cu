@@ -286,8 +286,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
                     if (++kb >= item.kb1) open(pp);
                 }
             };
-            // The weights do not depend on the kernel before this one; the activations do.  Fill the ring with
+            // Fixed weights do not depend on the kernel before this one; the activations do.  Fill the ring with
             // weight slices first, then wait for the predecessor, then add the activation slices.
+            if (!p.f.fixed_weights) fr_pdl_wait();
             const uint32_t stage_tx = P_BYTES + bn * TILE_K * 2;       // bytes that land in a stage
             const CUtensorMap* map_w = p.swapped ? &map_p : &map_q;
             const CUtensorMap* map_x = p.swapped ? &map_q : &map_p;

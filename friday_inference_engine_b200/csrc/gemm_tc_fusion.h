@@ -37,6 +37,9 @@ struct GemmFusion {
     unsigned long long* trace;
     // (5) Constants of the activation: limit and slope of the clipped gated unit.
     float act_limit, act_slope;
+    // (6) Not zero: the weights are memory that no kernel writes any more, and may be read while the kernel before this one still
+    // runs.  Zero: any earlier kernel of the stream may have made them, and they are read after it has finished.
+    int fixed_weights;
 };
 
 // For `swap`: the launcher chooses, also a kernel whose sums differ in order from the fused forms' (a product that has none).

@@ -196,8 +196,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
                 if constexpr (GROUPED) tma_load_3d_pair(dst, &map_q, at.kb * TILE_K, row, at.tiles.group, bar);
                 else tma_load_2d_pair(dst, &map_q, at.kb * TILE_K, row, bar);
             };
-            // The weights do not depend on the kernel before this one; the activations do.  Fill the ring with
+            // Fixed weights do not depend on the kernel before this one; the activations do.  Fill the ring with
             // weight slices first, then wait for the predecessor, then add the activation slices.
+            if (!p.f.fixed_weights) fr_pdl_wait();
             const uint32_t stage_tx = 2u * (P_BYTES + (uint32_t)half * TILE_K * 2);      // both CTAs' bytes of a stage
             Walk head(p, s_off, pair, pairs);
             Walk ahead(p, s_off, pair, pairs);

@@ -2,7 +2,7 @@
 //
 // What such a product costs on the tcgen05 kernel is a chain of waits: a ring that fills, instructions, partial tiles, their
 // counter, their sum.  Here a block owns 16 columns of the output and its warps share k: every lane fetches its pieces of the
-// weights with 16-byte loads that are all on their way before the predecessor has finished, then the rows' pieces, multiplies
+// weights with 16-byte loads that are all on their way before the predecessor has finished (fixed weights), then the rows' pieces, multiplies
 // with mma.sync.m16n8k16 (the columns on its M side, up to 8 rows on its N side, fp32 sums), and the warps' sums meet in
 // shared memory.  A lane's 16 bytes are eight consecutive k; which k an instruction takes from which place is free as long as
 // both operands agree, so two instructions take them as they lie.
@@ -17,7 +17,7 @@ constexpr int SKINNY_STEPS = 8;              // pieces of 32 k per warp that are
 constexpr int SKINNY_K = SKINNY_STEPS * 32;  // k per warp and turn
 
 struct SkinnyParams {
-    GemmFusion f;                            // the activation's constants
+    GemmFusion f;                            // the activation's constants, whether the weights are fixed
     const __nv_bfloat16* x;
     const __nv_bfloat16* w;
     void* out;
@@ -50,6 +50,7 @@ gemm_skinny_kernel(const SkinnyParams p) {
 #pragma unroll
     for (int i = 0; i < MT; ++i) xr[i] = p.x + (size_t)min(i * 8 + g, p.m - 1) * p.lda;
     fr_pdl_launch();
+    if (!p.f.fixed_weights) fr_pdl_wait();
     float acc[MT][4];
 #pragma unroll
     for (int i = 0; i < MT; ++i)
@@ -67,7 +68,7 @@ gemm_skinny_kernel(const SkinnyParams p) {
                 hi[s] = load_weights(wh + k);
             }
         }
-        if (k0 < WARPS * SKINNY_K) fr_pdl_wait();        // the weights do not depend on the kernel before this one; the rows do
+        if (k0 < WARPS * SKINNY_K) fr_pdl_wait();        // fixed weights do not depend on the kernel before this one; the rows do
 #pragma unroll
         for (int s = 0; s < SKINNY_STEPS; ++s) {
             const int k = k0 + s * 32 + t * 8;

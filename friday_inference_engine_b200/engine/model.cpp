@@ -129,6 +129,7 @@ std::vector<StoredParam> plan_storage(const std::vector<Part::Named>& all, const
 
 size_t load_params(const std::vector<StoredParam>& plan, WeightSource& source, Ops& ops) {
     size_t bytes = 0;
+    std::vector<std::shared_ptr<DeviceBuffer>> made;
     for (const auto& s : plan) {          // stacked tensors first
         const Part::Named& e = s.param;
         if (e.decl.into.empty() || e.owner->tensors.count(e.decl.into)) continue;
@@ -140,6 +141,7 @@ size_t load_params(const std::vector<StoredParam>& plan, WeightSource& source, O
         auto mem = std::make_shared<DeviceBuffer>((size_t)(*shape)[0] * (*shape)[1] * dtype_size(s.dtype), true);
         e.owner->set_tensor(e.decl.into, Tensor::make(mem->get(), s.dtype, *shape));
         e.owner->hold(mem);
+        made.push_back(mem);
         bytes += mem->bytes();
     }
     for (const auto& s : plan) {
@@ -153,6 +155,7 @@ size_t load_params(const std::vector<StoredParam>& plan, WeightSource& source, O
             Tensor t = Tensor::make(mem->get(), s.dtype, e.decl.shape);
             e.owner->set_tensor(e.local, t);
             e.owner->hold(mem);
+            made.push_back(mem);
             bytes += mem->bytes();
             dst = t;
             dst.ld = cols;
@@ -174,6 +177,7 @@ size_t load_params(const std::vector<StoredParam>& plan, WeightSource& source, O
         source.load(e.name, dst, ops.stream());
     }
     cuda_check(cudaStreamSynchronize(ops.stream()), "cudaStreamSynchronize");
+    for (const auto& mem : made) ops.declare_fixed(mem);
     return bytes;
 }
 

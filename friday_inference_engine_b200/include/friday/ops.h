@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include <map>
+#include <memory>
 #include <string>
 #include <tuple>
 #include <vector>
@@ -100,6 +101,12 @@ public:
     Arena* arena = nullptr;                                   // where results come from
     Tensor alloc(DType dtype, int64_t rows, int64_t cols);
     float* scratch_floats(int64_t n);                         // from the arena
+
+    // Memory that no kernel writes any more (a loaded model's parameters).  A product whose weights (its second operand, and
+    // head_linear's) lie in such memory reads them while the kernel before it still runs; weights anywhere else may be the
+    // result of the kernel before, and are read after it has finished.  Only what is still allocated counts.
+    void declare_fixed(const std::shared_ptr<DeviceBuffer>& memory);
+    bool fixed(const Tensor& weight) const;
 
     // ---- row-wise
     Tensor embedding(const int* tokens, int64_t n, const Tensor& table, Tensor* out = nullptr);
@@ -344,7 +351,8 @@ public:
     Tensor experts_grouped(const Tensor& h, const Routing& r, const Tensor& w_gate_up, const Tensor& w_down, const Tensor& residual,
                            int top, int inner, int act = 1, float limit = 0.f, float slope = 1.f, int row_tiles = 0);
 
-    // ---- matrix products: x [rows, k] @ weight [n, k]^T (+ bias [n]) (+ residual [rows, n])
+    // ---- matrix products: x [rows, k] @ weight [n, k]^T (+ bias [n]) (+ residual [rows, n]); weight may be any kernel's result,
+    // also the last one's (declare_fixed says when it is read early)
     Tensor linear(const Rows& x, const Tensor& weight, const Tensor* bias = nullptr, const Tensor* residual = nullptr,
                   int out_dtype = -1, Tensor* out = nullptr);
     // The same for a product that has no fused form to agree with bit by bit (linear_norm, qkv_rope_write): few rows may run on
@@ -426,6 +434,12 @@ public:
 private:
     struct Timed;
     friend struct Timed;
+    struct Fixed {
+        const char* begin;
+        const char* end;
+        std::weak_ptr<DeviceBuffer> memory;
+    };
+    std::vector<Fixed> fixed_;                                // by address
     bool few_rows_tile_ok(const Tensor& x, const Tensor& weight, const Tensor& out, const Tensor* residual,
                           int64_t max_rows, int columns = 128) const;
     void fusion_in(const Rows& x, GemmFusion& f) const;

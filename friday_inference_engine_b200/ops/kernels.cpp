@@ -95,7 +95,7 @@ FAMILY(Rowwise, rowwise, "rowwise",
        resolve(h, fam, "rowwise_rope_kv_write", t.rope_kv_write); resolve(h, fam, "rowwise_advance", t.advance);
        resolve(h, fam, "rowwise_scale_rows", t.scale_rows); resolve(h, fam, "rowwise_finish_logits", t.finish_logits);
        resolve(h, fam, "rowwise_random_normal", t.random_normal);)
-FAMILY(GemmSimt, gemm_simt, "gemm_simt", resolve(h, fam, "gemm_simt", t.gemm);)
+FAMILY(GemmSimt, gemm_simt, "gemm_simt", resolve(h, fam, "gemm_simt_weights", t.gemm);)
 FAMILY(GemmTc, gemm_tc, "gemm_tc", resolve(h, fam, "gemm_tc_fused", t.fused); resolve(h, fam, "gemm_tc_plan", t.plan);
        resolve(h, fam, "gemm_tc_grouped", t.grouped);)
 FAMILY(AttentionSimt, attention_simt, "attention_simt", resolve(h, fam, "attention_simt", t.run);
@@ -137,7 +137,7 @@ FAMILY(Delta, delta, "delta", resolve(h, fam, "delta_conv_prepare", t.conv_prepa
        resolve(h, fam, "delta_general_prepare", t.general_prepare); resolve(h, fam, "delta_general_scan", t.general_scan);
        resolve(h, fam, "delta_step_supports", t.step_supports); resolve(h, fam, "delta_step", t.step);)
 FAMILY(AttentionLatent, attention_latent, "attention_latent", resolve(h, fam, "attention_latent_rotate_pairs", t.rotate_pairs);
-       resolve(h, fam, "attention_latent_prepare", t.prepare); resolve(h, fam, "attention_latent_head_linear", t.head_linear);
+       resolve(h, fam, "attention_latent_prepare", t.prepare); resolve(h, fam, "attention_latent_head_linear_weights", t.head_linear);
        resolve(h, fam, "attention_latent", t.run); resolve(h, fam, "attention_latent_gather", t.gather);
        resolve(h, fam, "attention_latent_softmax_split", t.softmax_split);
        resolve(h, fam, "attention_latent_splits", t.splits); resolve(h, fam, "attention_latent_gate_cast", t.gate_cast);

@@ -34,7 +34,7 @@ struct Rowwise {
 struct GemmSimt {
     last_error_fn last_error;
     int (*gemm)(const void*, int, const void*, int, void*, int, const void*, int, const void*, int, int, int, int, int, int,
-                cudaStream_t);
+                int, cudaStream_t);
 };
 struct GemmTc {
     last_error_fn last_error;
@@ -156,7 +156,7 @@ struct AttentionLatent {
     int (*prepare)(const void*, int, int, int, void*, float*, const void*, int, float, const int*, const int*, const float*, float, int,
                    int, int, int, int, int, int, cudaStream_t);
     int (*head_linear)(const void*, int, int, int, int, const void*, int, int, void*, int, int, int, const void*, int, int, const int*,
-                       int, int, int, int, cudaStream_t);
+                       int, int, int, int, int, cudaStream_t);
     int (*run)(const float*, float*, const void*, const void*, const int*, int, int, const int*, const int*, const void*, int, int,
                int, int, int, float, int, float*, int, cudaStream_t);
     int (*gather)(const void*, const void*, const int*, int, int, int, int, int, void*, void*, int, cudaStream_t);

@@ -103,6 +103,23 @@ Tensor Ops::alloc(DType dtype, int64_t rows, int64_t cols) {
     return Tensor::make(p, dtype, {rows, cols});
 }
 
+void Ops::declare_fixed(const std::shared_ptr<DeviceBuffer>& memory) {
+    const char* begin = (const char*)memory->get();
+    const Fixed entry{begin, begin + memory->bytes(), memory};
+    if (entry.begin == entry.end) return;
+    // (what overlaps has been freed: its address came back)
+    fixed_.erase(std::remove_if(fixed_.begin(), fixed_.end(), [&](const Fixed& f) { return f.begin < entry.end && entry.begin < f.end; }), fixed_.end());
+    fixed_.insert(std::upper_bound(fixed_.begin(), fixed_.end(), entry, [](const Fixed& a, const Fixed& b) { return a.begin < b.begin; }), entry);
+}
+
+bool Ops::fixed(const Tensor& weight) const {
+    const char* at = (const char*)weight.data;
+    auto it = std::upper_bound(fixed_.begin(), fixed_.end(), at, [](const char* p, const Fixed& f) { return p < f.begin; });
+    if (it == fixed_.begin()) return false;
+    --it;
+    return at < it->end && !it->memory.expired();
+}
+
 float* Ops::scratch_floats(int64_t n) {
     if (!arena) throw KernelError("internal: an operation needs scratch memory and no arena is set");
     return (float*)arena->alloc((size_t)(n > 0 ? n : 1) * sizeof(float));
@@ -889,7 +906,7 @@ void Ops::head_linear(const Tensor& x, int64_t x_off, int64_t x_stride, const Te
     call(launches_, k, k.head_linear(x.data, code(x.dtype), (int)x.ld, (int)x_off, (int)x_stride, w.data, code(w.dtype),
                                      per_head_rows_k ? 0 : 1, out.data, code(out.dtype), (int)out.ld, (int)out_stride,
                                      gate ? gate->data : nullptr, gate ? (int)gate->ld : 0, (int)gate_off, ctx.row_seq, (int)x.rows(),
-                                     heads, k_, n, stream_), "head_linear");
+                                     heads, k_, n, fixed(w) ? 1 : 0, stream_), "head_linear");
 }
 
 Tensor Ops::latent_attention(const Tensor& qf, const Tensor* sink, const LatentSpec& s, const CacheView& view, const StepContext& ctx) {
@@ -1191,19 +1208,17 @@ Tensor Ops::linear_tc(const Tensor& x, const Tensor& weight, const Tensor* bias,
                       int swap, int bn, int splits, int act, GemmFusion* fusion) {
     const auto& g = kernels::gemm_tc();
     Timed t(*this, Product);
-    GemmFusion traced;
-    if (trace_ && trace_next_ < trace_left_) {
-        if (fusion) traced = *fusion;
-        else memset(&traced, 0, sizeof traced);
-        traced.trace = trace_ + (size_t)trace_next_++ * sms_ * 16;
-        fusion = &traced;
-    }
+    GemmFusion f;
+    if (fusion) f = *fusion;
+    else memset(&f, 0, sizeof f);
+    f.fixed_weights = fixed(weight) ? 1 : 0;
+    if (trace_ && trace_next_ < trace_left_) f.trace = trace_ + (size_t)trace_next_++ * sms_ * 16;
     call(launches_, g,
          g.fused(x.data, weight.data, out.data, code(out.dtype), bias ? bias->data : nullptr, bias ? code(bias->dtype) : 0,
                  residual ? residual->data : nullptr, (int)x.rows(), (int)weight.rows(), (int)x.cols(), (int)x.ld,
                  (int)weight.ld, (int)out.ld, (float*)tc_scratch_.get(), (long long)(tc_scratch_.bytes() / sizeof(float)),
                  (int*)tc_counters_.get(), (int)(tc_counters_.bytes() / sizeof(int)), (int*)status_.get(), sms_, swap, bn,
-                 splits, act, fusion, stream_),
+                 splits, act, &f, stream_),
          "gemm_tc_fused");
     return out;
 }
@@ -1214,7 +1229,7 @@ Tensor Ops::linear_simt(const Tensor& x, const Tensor& weight, const Tensor* bia
     call(launches_, g,
          g.gemm(x.data, code(x.dtype), weight.data, code(weight.dtype), out.data, code(out.dtype),
                 bias ? bias->data : nullptr, bias ? code(bias->dtype) : 0, residual ? residual->data : nullptr,
-                (int)x.rows(), (int)weight.rows(), (int)x.cols(), (int)x.ld, (int)weight.ld, (int)out.ld, stream_),
+                (int)x.rows(), (int)weight.rows(), (int)x.cols(), (int)x.ld, (int)weight.ld, (int)out.ld, fixed(weight) ? 1 : 0, stream_),
          "gemm_simt");
     return out;
 }
