@@ -161,10 +161,13 @@ __device__ __forceinline__ void mark(const GemmParams& p, int point) {
 }
 
 // Rows on the M side, the RMSNorm of the output begun: 16 whole columns gj0.. of row gi (the launcher has seen to
-// n % 16 == 0 and 16-byte aligned rows): bias, residual, rounding, store; then the rounded values' squares into ss and,
-// times the norm's weights g16[0..15], into norm_out.  pre_added: bias and residual are in v already.
-__device__ __forceinline__ void finish16_begin_norm(const GemmParams& p, const float* g16, int gi, int gj0, float (&v)[16],
-                                                    float& ss, bool pre_added = false) {
+// n % 16 == 0 and 16-byte aligned rows): bias, residual, rounding, store; then the rounded values, times the norm's weights
+// g16[0..15], into norm_out.  w gets the rounded values in pairs, zeros for columns or rows beyond the result.
+// pre_added: bias and residual are in v already.
+__device__ __forceinline__ void finish16_scaled(const GemmParams& p, const float* g16, int gi, int gj0, float (&v)[16],
+                                                uint32_t (&w)[8], bool pre_added) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) w[j] = 0u;
     if (gi >= p.p_rows || gj0 >= p.q_rows) return;
     const size_t base = (size_t)gi * p.ldo + gj0;
     if (p.bias != nullptr && !pre_added)
@@ -180,14 +183,11 @@ __device__ __forceinline__ void finish16_begin_norm(const GemmParams& p, const f
             v[2 * j + 1] += __uint_as_float(rw[j] & 0xffff0000u);
         }
     }
-    uint32_t w[8], h[8];
+    uint32_t h[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         w[j] = pack2(v[2 * j], v[2 * j + 1]);
-        const float x0 = __uint_as_float(w[j] << 16), x1 = __uint_as_float(w[j] & 0xffff0000u);
-        ss += x0 * x0;
-        ss += x1 * x1;
-        h[j] = pack2(x0 * g16[2 * j], x1 * g16[2 * j + 1]);
+        h[j] = pack2(__uint_as_float(w[j] << 16) * g16[2 * j], __uint_as_float(w[j] & 0xffff0000u) * g16[2 * j + 1]);
     }
     uint4* o = (uint4*)((__nv_bfloat16*)p.out + base);
     o[0] = make_uint4(w[0], w[1], w[2], w[3]);
@@ -195,6 +195,21 @@ __device__ __forceinline__ void finish16_begin_norm(const GemmParams& p, const f
     uint4* ho = (uint4*)((__nv_bfloat16*)p.f.norm_out + base);
     ho[0] = make_uint4(h[0], h[1], h[2], h[3]);
     ho[1] = make_uint4(h[4], h[5], h[6], h[7]);
+}
+// The squares of 16 rounded values into a row's sum, column by column: every kernel adds a tile's columns in this order.
+__device__ __forceinline__ void add_squares(const uint32_t (&w)[8], float& ss) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const float x0 = __uint_as_float(w[j] << 16), x1 = __uint_as_float(w[j] & 0xffff0000u);
+        ss += x0 * x0;
+        ss += x1 * x1;
+    }
+}
+__device__ __forceinline__ void finish16_begin_norm(const GemmParams& p, const float* g16, int gi, int gj0, float (&v)[16],
+                                                    float& ss, bool pre_added = false) {
+    uint32_t w[8];
+    finish16_scaled(p, g16, gi, gj0, v, w, pre_added);
+    add_squares(w, ss);
 }
 
 template <int BN, int STAGES>

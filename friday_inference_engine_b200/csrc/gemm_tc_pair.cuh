@@ -137,7 +137,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
     uint32_t* tmem_slot = (uint32_t*)(bars + 2 * STAGES + 4);
     volatile int* s_gave_up = (volatile int*)(tmem_slot + 1);               // a finisher of this CTA has stopped waiting
     float* s_gw = (float*)((uint8_t*)(bars + 2 * STAGES + 4) + 64);         // [BN] norm weights of the tile's columns
-    float* s_ss = s_gw + BN;                                                // [128] sums of squares that a row's other warp found
+    float* s_ss = s_gw + BN;                                                // [128] the rows' sums of squares over a tile's first half
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = fr_cluster_rank();                                 // 0: the CTA that issues the instructions
     const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
@@ -281,7 +281,6 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
                 row_scale = 1.0f / sqrtf(ss / f.in_width + f.in_eps);
                 scale_row = gi;
             }
-            float ss_row = 0.f;                            // with a norm begun: this row's sum of squares over the tile
             if (norm_rows) {
                 asm volatile("bar.sync 1, 256;" ::: "memory");
                 for (int i = et; i < bn; i += PAIR_FINISHERS) {
@@ -300,28 +299,57 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
             if (!ok) break;
             tc_fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + a * BN;
-#pragma unroll 1
-            for (int c = share; c < bn / 16; c += 2) {
+            auto sums16 = [&](int c, float (&v)[16]) {
                 uint32_t r[16];
                 tc_ld16(taddr + c * 16, r);
                 tc_ld_wait();
-                float v[16];
 #pragma unroll
                 for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
                 if (f.in_ssq != nullptr)
 #pragma unroll
                     for (int j = 0; j < 16; ++j) v[j] *= row_scale;
-                const int gj0 = q_blk * bn + c * 16;
-                if (norm_rows) finish16_begin_norm(p, s_gw + c * 16, gi, gj0, v, ss_row);
-                else if (!GROUPED || gi < tiles.row_end) finish16(p, gi, gj0, v);
+            };
+            // With a norm begun, a row's two warps have its columns' first and second half: the second adds its squares to
+            // the sum of the first, so that a row's sum has the order that it has everywhere (its values wait in registers).
+            uint32_t kept[GROUPED ? 1 : PAIR_BN / 32][8];
+            if (!GROUPED && norm_rows) {
+                const int first = (bn / 16 + 1) / 2, c0 = share == 0 ? 0 : first, c1 = share == 0 ? first : bn / 16;
+#pragma unroll
+                for (int i = 0; i < (GROUPED ? 1 : PAIR_BN / 32); ++i) {
+                    const int c = c0 + i;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) kept[i][j] = 0u;
+                    if (c < c1) {
+                        float v[16];
+                        sums16(c, v);
+                        finish16_scaled(p, s_gw + c * 16, gi, q_blk * bn + c * 16, v, kept[i], false);
+                    }
+                }
+            } else {
+#pragma unroll 1
+                for (int c = share; c < bn / 16; c += 2) {
+                    float v[16];
+                    sums16(c, v);
+                    if (!GROUPED || gi < tiles.row_end) finish16(p, gi, q_blk * bn + c * 16, v);
+                }
             }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(first_acce0 + 8 * a);     // the accumulator may be overwritten
-            if (norm_rows) {                               // a row's two shares, the columns' even groups first
-                if (share == 1) s_ss[i_local] = ss_row;
+            if (!GROUPED && norm_rows) {
+                float ss = 0.f;
+                if (share == 0) {
+#pragma unroll
+                    for (int i = 0; i < (GROUPED ? 1 : PAIR_BN / 32); ++i) add_squares(kept[i], ss);
+                    s_ss[i_local] = ss;
+                }
                 asm volatile("bar.sync 1, 256;" ::: "memory");
-                if (share == 0 && gi < p.p_rows) f.out_ssq[(size_t)q_blk * p.p_rows + gi] = ss_row + s_ss[i_local];
+                if (share == 1) {
+                    ss = s_ss[i_local];
+#pragma unroll
+                    for (int i = 0; i < (GROUPED ? 1 : PAIR_BN / 32); ++i) add_squares(kept[i], ss);
+                    if (gi < p.p_rows) f.out_ssq[(size_t)q_blk * p.p_rows + gi] = ss;
+                }
             }
         }
     }
