@@ -936,9 +936,27 @@ Tensor Ops::latent_attention_prompt(const Tensor& proj, const Tensor& w_uk, cons
     const auto& k = kernels::attention_latent();
     const int64_t hv = (int64_t)s.heads * s.vdim;
     Tensor of = alloc(DType::F32, proj.rows(), hv), out = alloc(proj.dtype, proj.rows(), hv);
+    const int64_t hd = (int64_t)s.dim + s.rot;
+    // Several heads at a time, as many as 64 MB of scores hold: a launch per product and one for their softmax (a head by
+    // itself was three launches of some 7 us each, whatever its size: 16 heads x 512 rows 16 x 19 us; together 46).  Rows of
+    // the projection off 16 bytes: head by head, on whatever kernel takes them.
+    const bool together = proj.ld % 8 == 0 && aligned16((const char*)proj.data + (size_t)s.q_off * 2) && hd % 8 == 0 && sms_ >= 2;
+    auto padded = [](int64_t n) { return (n + 7) / 8 * 8; };
+    auto heads_at_once = [&](int64_t T, int64_t n_pad) {
+        return together ? std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(s.heads, 256), (int64_t)(64 << 20) / (T * n_pad * 4))) : 1;
+    };
+    // The scores, and every weight as two bf16 numbers [hi | lo]: one pair of buffers for all sequences, whose kernels follow one
+    // another on the stream, so that the batch costs no more memory than its longest sequence.
+    int64_t most = 0;
+    for (int q = 0; q < ctx.n_seqs; ++q) {
+        const int64_t T = ctx.q_lens[(size_t)q], n_pad = padded(ctx.kv_lens[(size_t)q]);
+        if (T > 0) most = std::max(most, heads_at_once(T, n_pad) * T * n_pad);
+    }
+    float* score_memory = scratch_floats(most);
+    float* weight_memory = scratch_floats(most);
     int64_t r0 = 0;
     for (int q = 0; q < ctx.n_seqs; ++q) {
-        const int64_t T = ctx.q_lens[(size_t)q], n = ctx.kv_lens[(size_t)q], n_pad = (n + 7) / 8 * 8;
+        const int64_t T = ctx.q_lens[(size_t)q], n = ctx.kv_lens[(size_t)q], n_pad = padded(n);
         if (T <= 0) continue;
         Tensor c_all = alloc(DType::BF16, 2 * n_pad, s.rank), r_all = alloc(DType::BF16, n_pad, s.rot);
         {
@@ -946,7 +964,6 @@ Tensor Ops::latent_attention_prompt(const Tensor& proj, const Tensor& w_uk, cons
             call(launches_, k, k.gather(view.k_pool, view.v_pool, view.block_table + (size_t)q * view.table_width, view.page_size, (int)n,
                                         (int)n_pad, s.rank, s.rot, c_all.data, r_all.data, code(DType::BF16), stream_), "latent gather");
         }
-        const int64_t hd = (int64_t)s.dim + s.rot;
         Tensor kn = linear(Rows(c_all.row_slice(0, n_pad)), w_uk);      // [n_pad, heads * dim]: every head's unrotated keys
         Tensor kcat = alloc(DType::BF16, n_pad, s.heads * hd);          // [n_pad, heads, dim + rot]: whole keys, head by head
         {
@@ -956,16 +973,10 @@ Tensor Ops::latent_attention_prompt(const Tensor& proj, const Tensor& w_uk, cons
         }
         Tensor vt = linear(Rows(w_uv), c_all);                          // [heads * vdim, 2 n_pad]: values, transposed, twice side by side
         const Tensor rows = proj.row_slice(r0, T);
-        // Several heads at a time, as many as 64 MB of scores hold: a launch per product and one for their softmax (a head by
-        // itself was three launches of some 7 us each, whatever its size: 16 heads x 512 rows 16 x 19 us;
-        // together 46).  Rows of the
-        // projection off 16 bytes: head by head, on whatever kernel takes them.
         const void* q0 = (const char*)rows.data + (size_t)s.q_off * 2;
-        const bool together = rows.ld % 8 == 0 && aligned16(q0) && hd % 8 == 0 && sms_ >= 2;
-        const int64_t fit = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(s.heads, 256), (int64_t)(64 << 20) / (T * n_pad * 4)));
-        const int64_t at_once = together ? fit : 1;
-        Tensor scores = alloc(DType::F32, at_once * T, n_pad);
-        Tensor weights = alloc(DType::BF16, at_once * T, 2 * n_pad);    // every weight as two bf16 numbers: [hi | lo]
+        const int64_t at_once = heads_at_once(T, n_pad);
+        Tensor scores = Tensor::make(score_memory, DType::F32, {at_once * T, n_pad});
+        Tensor weights = Tensor::make(weight_memory, DType::BF16, {at_once * T, 2 * n_pad});
         auto softmax = [&](int h, int64_t n_heads) {
             Timed t(*this, Attention);
             call(launches_, k, k.softmax_split((const float*)scores.data, (int)scores.ld, (int)T, (int)n_heads, (int)n_pad, (int)(n - T), s.scale,
