@@ -345,11 +345,17 @@ public:
     Tensor expert_gate_up(const Tensor& h, const Routing& r, const Tensor& w_gate_up, int top, int inner, int act = 1, float limit = 0.f,
                           float slope = 1.f);
     Tensor expert_down_combine(const Tensor& act, const Routing& r, const Tensor& w_down, const Tensor& residual, int top, int inner);
-    // Many rows: the rows are gathered expert by expert and every expert runs its two products on the tensor cores over its
-    // own rows only, all experts in one launch per product.  row_tiles: how many tiles of 256 rows that makes, as far as the
-    // caller knows.  bf16.  w_gate_up [experts * 2 * inner, width] (gate and up row by row in turn), w_down [width, experts * inner].
+    // Many rows: the rows are gathered expert by expert and every expert runs its two products over its own rows only.  bf16 rows
+    // and weights in 16-byte pieces: on the tensor cores, all experts in one launch per product.  Anything else: expert by expert,
+    // on whatever kernel takes the sizes; the host then reads the experts' row counts (one small copy and a wait per call) unless
+    // it knows them already, so that form is for prompts, never inside a captured step.  counts: a number of choices per expert,
+    // where the host knows them.  w_gate_up [experts * 2 * inner, width] (gate and up row by row in turn), w_down
+    // [width, experts * inner].
     Tensor experts_grouped(const Tensor& h, const Routing& r, const Tensor& w_gate_up, const Tensor& w_down, const Tensor& residual,
-                           int top, int inner, int act = 1, float limit = 0.f, float slope = 1.f, int row_tiles = 0);
+                           int top, int inner, int act = 1, float limit = 0.f, float slope = 1.f, const std::vector<int>* counts = nullptr);
+    // Tiles of 256 rows that the experts' own rows make: exact with counts, else what `pairs` choices make on average (half a tile
+    // is left over per expert that has any).
+    static int64_t expert_tiles(int64_t pairs, int experts, const std::vector<int>* counts);
 
     // ---- matrix products: x [rows, k] @ weight [n, k]^T (+ bias [n]) (+ residual [rows, n]); weight may be any kernel's result,
     // also the last one's (declare_fixed says when it is read early)

@@ -1135,8 +1135,18 @@ Tensor Ops::expert_down_combine(const Tensor& act, const Routing& r, const Tenso
     return out;
 }
 
+int64_t Ops::expert_tiles(int64_t pairs, int experts, const std::vector<int>* counts) {
+    int64_t tiles = 0;
+    if (counts) {
+        for (int n : *counts) tiles += (n + 255) / 256;
+        return tiles;
+    }
+    const int64_t some = std::min<int64_t>(experts, pairs);
+    return std::max(some, pairs / 256 + some / 2);
+}
+
 Tensor Ops::experts_grouped(const Tensor& h, const Routing& r, const Tensor& w_gate_up, const Tensor& w_down, const Tensor& residual,
-                            int top, int inner, int unit, float limit, float slope, int row_tiles) {
+                            int top, int inner, int unit, float limit, float slope, const std::vector<int>* counts) {
     const int64_t rows = h.rows(), width = h.cols(), n_pairs = rows * top;
     const int experts = (int)(w_gate_up.rows() / (2 * (int64_t)inner));
     const auto& k = kernels::routed();
@@ -1147,22 +1157,43 @@ Tensor Ops::experts_grouped(const Tensor& h, const Routing& r, const Tensor& w_g
         Timed t(*this, Other);
         call(launches_, k, k.sort_pairs((const int*)r.ids.data, (int)rows, top, experts, offsets, pos, row_at, stream_), "sort_pairs");
     }
-    if (h.dtype != DType::BF16 || w_gate_up.dtype != DType::BF16 || w_down.dtype != DType::BF16 || !w_gate_up.contiguous())
-        throw KernelError("experts_grouped: bf16 rows and weights");
-    const auto& g = kernels::gemm_tc();
-    Tensor gathered = gather_rows(row_at, n_pairs, h);
-    Tensor act = alloc(DType::BF16, n_pairs, inner), part = alloc(DType::F32, n_pairs, width);
-    {
+    if (counts && (int)counts->size() != experts) throw KernelError("experts_grouped: a number of choices per expert");
+    Tensor part = alloc(DType::F32, n_pairs, width);
+    const bool one_launch = h.dtype == DType::BF16 && w_gate_up.dtype == DType::BF16 && w_down.dtype == DType::BF16 && width % 8 == 0 &&
+                            inner % 8 == 0 && w_gate_up.ld % 8 == 0 && w_down.ld % 8 == 0 && aligned16(w_gate_up.data) &&
+                            aligned16(w_down.data) && sms_ >= 2;
+    if (one_launch) {
+        const auto& g = kernels::gemm_tc();
+        const int row_tiles = (int)expert_tiles(n_pairs, experts, counts);
+        Tensor gathered = gather_rows(row_at, n_pairs, h);
+        Tensor act = alloc(DType::BF16, n_pairs, inner);
         Timed t(*this, Product);
-        call(launches_, g, g.grouped(gathered.data, 0, w_gate_up.data, 2 * (long long)inner * width, act.data, code(act.dtype), offsets, experts, (int)n_pairs,
-                                     2 * inner, (int)width, (int)gathered.ld, (int)w_gate_up.ld, (int)act.ld, row_tiles, unit, limit, slope,
+        call(launches_, g, g.grouped(gathered.data, 0, w_gate_up.data, 2 * (long long)inner * w_gate_up.ld, act.data, code(act.dtype), offsets, experts,
+                                     (int)n_pairs, 2 * inner, (int)width, (int)gathered.ld, (int)w_gate_up.ld, (int)act.ld, row_tiles, unit, limit, slope,
                                      (int*)status_.get(), sms_, stream_), "gemm_tc_grouped");
-    }
-    {
-        Timed t(*this, Product);
         call(launches_, g, g.grouped(act.data, 0, w_down.data, inner, part.data, code(part.dtype), offsets, experts, (int)n_pairs, (int)width, inner,
                                      (int)act.ld, (int)w_down.ld, (int)part.ld, row_tiles, 0, 0.f, 0.f, (int*)status_.get(), sms_, stream_),
              "gemm_tc_grouped");
+    } else {
+        std::vector<int> off((size_t)experts + 1);
+        if (counts) {
+            for (int e = 0; e < experts; ++e) off[(size_t)e + 1] = off[(size_t)e] + (*counts)[(size_t)e];
+        } else {
+            cuda_check(cudaMemcpyAsync(off.data(), offsets, off.size() * sizeof(int), cudaMemcpyDeviceToHost, stream_), "cudaMemcpyAsync");
+            cuda_check(cudaStreamSynchronize(stream_), "cudaStreamSynchronize");
+        }
+        // (fewer places than pairs where some choices are no expert of this table: only the places that exist are gathered)
+        Tensor gathered = off.back() > 0 ? gather_rows(row_at, off.back(), h) : Tensor();
+        for (int e = 0; e < experts; ++e) {
+            const int64_t lo = off[(size_t)e], n = off[(size_t)e + 1] - lo;
+            if (n <= 0) continue;
+            Tensor act = linear_swiglu(Rows(gathered.row_slice(lo, n)), w_gate_up.row_slice((int64_t)e * 2 * inner, 2 * (int64_t)inner), unit, limit, slope);
+            Tensor wd = w_down;                          // this expert's columns, the matrix's row stride
+            wd.data = (char*)w_down.data + (size_t)e * inner * dtype_size(w_down.dtype);
+            wd.shape[1] = inner;
+            Tensor out = part.row_slice(lo, n);
+            linear(Rows(act), wd, nullptr, nullptr, (int)DType::F32, &out);
+        }
     }
     Tensor result = alloc(residual.dtype, residual.rows(), residual.cols());
     Timed t(*this, Other);

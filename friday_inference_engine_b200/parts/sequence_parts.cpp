@@ -503,12 +503,7 @@ public:
         // inner size 2048, 8 experts, 2 chosen: 3,006 us a pass of seven layers, 3,560 in the dense form).  Without a table only the device knows how the
         // rows fall, half a tile per expert is left over on average.  Grouping is for prompts: a one-token step never groups.
         const std::vector<int> counts = choices_per_expert(ctx);          // empty: only the device knows
-        const int64_t pairs = x.rows() * top_, some = std::min<int64_t>(experts_, pairs);
-        int64_t grouped_tiles = std::max(some, pairs / 256 + some / 2);
-        if (!counts.empty()) {
-            grouped_tiles = 0;
-            for (int n : counts) grouped_tiles += (n + 255) / 256;
-        }
+        const int64_t grouped_tiles = Ops::expert_tiles(x.rows() * top_, experts_, counts.empty() ? nullptr : &counts);
         const int64_t dense_tiles = (x.rows() + 255) / 256 * experts_;
         // FRIDAY_EXPERTS=grouped|dense|pairs forces a form where it can run (for comparisons and tests)
         const char* force = getenv("FRIDAY_EXPERTS");
@@ -541,7 +536,7 @@ public:
             residual = with_shared(residual_in);
         }
         if (grouped)
-            return PartOut(ops.experts_grouped(x, r, tensor("w_gate_up"), tensor("w_down"), residual, top_, inner_, act_, limit_, slope_, (int)grouped_tiles));
+            return PartOut(ops.experts_grouped(x, r, tensor("w_gate_up"), tensor("w_down"), residual, top_, inner_, act_, limit_, slope_, counts.empty() ? nullptr : &counts));
         if (dense) {
             Tensor act = ops.linear_swiglu(Rows(x), tensor("w_gate_up"), act_, limit_, slope_);
             ops.scale_by_route(act, r.dense, experts_, inner_);
