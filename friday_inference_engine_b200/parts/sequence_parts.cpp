@@ -497,11 +497,13 @@ public:
         }
         const bool tensor_cores = x.dtype == DType::BF16 && x.rows() > 32 && tensor("w_gate_up").dtype == DType::BF16 &&
                                   x.cols() % 8 == 0 && inner_ % 8 == 0;
-        // The dense form (all experts for every row) against the grouped one, in tiles of 256 rows of a product.  As far as 256 rows
-        // both read every expert's weights once, and the dense form needs no sorting; from there the grouped form has fewer tiles
-        // (a prompt of 2,048 rows, width and
-        // inner size 2048, 8 experts, 2 chosen: 3,006 us a pass of seven layers, 3,560 in the dense form).  Without a table only the device knows how the
-        // rows fall, half a tile per expert is left over on average.  Grouping is for prompts: a one-token step never groups.
+        // Rows for the tensor cores: the dense form (all experts for every row) or the grouped one, by their tiles of 256 rows of a
+        // product.  As far as 256 rows both read every expert's weights once, and the dense form needs no sorting; from there the
+        // grouped form has fewer tiles (a prompt of 2,048 rows, width and inner size 2048, 8 experts, 2 chosen: 3,006 us a pass of
+        // seven layers, 3,560 in the dense form).  More than 16 experts per choice are never run for every row: such rows are
+        // grouped, whatever their number (64 experts of those sizes, 2 chosen, on a B200: 33 rows 1,350 us a pass, 2,381 when every
+        // choice reads its expert for itself; 256 rows 1,874 and 10,917).  Without a table only the device knows how the rows fall.
+        // Grouping is for prompts: a one-token step never groups.
         const std::vector<int> counts = choices_per_expert(ctx);          // empty: only the device knows
         const int64_t grouped_tiles = Ops::expert_tiles(x.rows() * top_, experts_, counts.empty() ? nullptr : &counts);
         const int64_t dense_tiles = (x.rows() + 255) / 256 * experts_;
@@ -509,8 +511,9 @@ public:
         const char* force = getenv("FRIDAY_EXPERTS");
         const std::string forced = force ? force : "";
         const bool may_group = tensor_cores && tensor("w_down").dtype == DType::BF16 && !ctx.decode && ctx.rows == (int)x.rows() && ctx.n_seqs > 0;
-        const bool grouped = may_group && (forced == "grouped" || (forced.empty() && grouped_tiles < dense_tiles && x.rows() > 256));
-        const bool dense = tensor_cores && !grouped && (forced == "dense" || (forced.empty() && experts_ <= 16 * top_));
+        const bool may_dense = tensor_cores && experts_ <= 16 * top_;
+        const bool grouped = may_group && (forced == "grouped" || (forced.empty() && (!may_dense || (grouped_tiles < dense_tiles && x.rows() > 256))));
+        const bool dense = tensor_cores && !grouped && (forced == "dense" || (forced.empty() && may_dense));
         Ops::Routing r = tabled_ ? ops.route_table(ctx.tokens, x.rows(), tensor("table"), experts_, dense)
                         : sigmoid_ ? ops.route_scored(logits, top_, choice_bias_.empty() ? nullptr : &tensor(choice_bias_), groups_, keep_,
                                                      weight_scale_, dense)
