@@ -1023,8 +1023,14 @@ static int tile_width(long long tiles_p, int q_rows, long long units, int narrow
 // (us a product, tcgen05 against this one): 8 rows: 64 x 2048 8.0 / 2.1, 2048 x 2048 6.5 / 3.4, 4608 x 3584 9.9 / 7.0,
 // 12288 x 2048 12.2 / 11.1, 3584 x 18944 27.5 / 27.4, 32768 x 2048 24.8 / 25.6.  16 rows: 64 x 2048 8.2 / 2.4, 4096 x 2048
 // 8.2 / 6.7, 2048 x 6144 9.3 / 7.7, 7168 x 2048 11.0 / 11.8, 3584 x 3584 9.3 / 11.0.
+// A block walks all of k, so with few blocks a long k is the other kernel's, which splits it: 256 x 12288 12.0 / 7.9 at 8 rows and
+// 12.2 / 9.6 at 16, 512 x 18944 12.8 / 11.2 and 12.9 / 14.6, 512 x 32768 14.6 / 16.7 and 14.7 / 22.7; one or two tiles of columns
+// are split less well: 128 x 18944 14.1 / 10.9 and 14.0 / 14.2, 256 x 32768 16.4 / 16.4 and 15.8 / 22.3, x 65536 18.8 / 29.8.
+// Not so where the columns are no multiple of its tile of 128, whose partial tiles one CTA then sums alone: 64 x 18944 30.3 / 10.7
+// and 30.3 / 13.8, 192 x 32768 33.1 / 16.4 and 33.3 / 22.2.
 static bool skinny_shape(int m, int n, int k, int sm_count) {
     const long long size = (long long)n * k;
+    if (n % TILE_P == 0 && k > (m <= 8 ? 24576 : 16384) * (n <= 2 * TILE_P ? 1.5 : 1.0)) return false;
     if (m <= 8) return size <= (32ll << 20);
     return m <= 16 && (size <= (8ll << 20) || (size <= (16ll << 20) && n <= SKINNY_N * sm_count));
 }
