@@ -147,7 +147,9 @@ __device__ __forceinline__ float fr_warp_max(float v) {
 // geometry of the step (rows, positions, ended sequences), which is final before the step's first kernel
 // starts.  The latter holds because the row-wise kernels that open every step (embedding, the first norm)
 // wait before they let their dependents launch: whatever runs after them was launched after the step before
-// had finished.  Kernels that let dependents launch before their own wait (the products) never open a step.
+// had finished.  For the same reason a one-token step may read a recurrent state ahead of the wait (delta_step)
+// if it is the only program entry that writes the state's cache entry: the state is then from the step before.
+// Kernels that let dependents launch before their own wait (the products) never open a step.
 __device__ __forceinline__ void fr_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void fr_pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -220,7 +220,8 @@ public:
     Tensor delta_scan(const Tensor& qkv, const Tensor& a_raw, const Tensor& b_raw, const Tensor& a_log, const Tensor& dt_bias,
                       const DeltaSpec& spec, const CacheView& view, const StepContext& ctx);
     // conv_silu_unit, delta_scan and head_norm_gate (a weight shared by the heads) in one kernel, for steps of one token per
-    // sequence whose sizes it takes and whose gate is in the projection's dtype; a_raw and b_raw fp32
+    // sequence whose sizes it takes and whose gate is in the projection's dtype; a_raw and b_raw fp32.  It reads the state while the
+    // kernel before still runs, so only for the one program entry that writes the state's cache entry (common.cuh)
     bool delta_step_ok(const Tensor& proj, const Tensor& a_raw, const Tensor& gate, const DeltaSpec& spec, const CacheView& view, const StepContext& ctx) const;
     Tensor delta_step(const Tensor& proj, const Tensor& taps, const Tensor& a_raw, const Tensor& b_raw, const Tensor& a_log, const Tensor& dt_bias,
                       const Tensor& gate, const Tensor& norm, float eps, float out_scale, bool gate_sigmoid, const DeltaSpec& spec,

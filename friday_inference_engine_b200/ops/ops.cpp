@@ -851,7 +851,7 @@ Tensor Ops::delta_scan(const Tensor& qkv, const Tensor& a_raw, const Tensor& b_r
 }
 
 bool Ops::delta_step_ok(const Tensor& proj, const Tensor& a_raw, const Tensor& gate, const DeltaSpec& s, const CacheView& view, const StepContext& ctx) const {
-    return ctx.decode && a_raw.dtype == DType::F32 && gate.dtype == proj.dtype && view.kind == CacheRequest::State && view.state.defined() &&
+    return ctx.decode && view.write && a_raw.dtype == DType::F32 && gate.dtype == proj.dtype && view.kind == CacheRequest::State && view.state.defined() &&
            view.state.dtype == DType::F32 && aligned16(view.state.data) && ctx.n_seqs <= 65535 &&
            kernels::delta().step_supports(s.heads, s.qk_heads, s.dk, s.dv, s.taps, view.state.numel() / view.state.shape[0]) != 0;
 }
