@@ -46,12 +46,17 @@ struct AttnArgs {
     float out_scale;      // the result is multiplied by this
 };
 
-// MAX_PER_LANE: dimensions per lane; KEYS keys at a time: their loads are issued together, so that a warp waits for memory once
-// per KEYS keys.  Small heads take more of them: a step of a window of 24 keys over heads of 32 took 7.8 us at four at a time,
-// 6.6 at sixteen; a prompt of 333 rows over 28 heads of 128 229
-// and 184 (eight).
+template <int N>
+struct Number {
+    static constexpr int value = N;
+};
+
+// MAX_PER_LANE: dimensions per lane; KEYS keys at a time, four where no more than four are left: their loads are issued together,
+// keys before values (bf16 heads of 65 to 128: key by key, a tenth faster), so that a warp waits for memory once per round.  fp32, us, four at a time / as launched below: 28 heads of 32,
+// 4 rows, a window of 24 keys 8.3 / 5.3; of 64, 333 rows 267 / 181, 8 rows x 4,000 keys 166 / 114; of 128, 333 rows 275 / 209.
 template <typename T, int MAX_PER_LANE, int KEYS>
 __global__ void __launch_bounds__(128) attention_kernel(AttnArgs p) {
+    constexpr bool VALUES_LAST = sizeof(T) == 4 || MAX_PER_LANE != 4;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int item = blockIdx.x * 4 + warp;          // (row, head)
     if (item >= p.rows * p.nq) return;
@@ -84,48 +89,75 @@ __global__ void __launch_bounds__(128) attention_kernel(AttnArgs p) {
             qv[i] = d < p.hd ? fr_load(q + d) * p.scale : 0.f;
         }
         const int* table = p.block_table + (size_t)seq * p.table_width;
-        for (int i = i0; i < i1; i += KEYS) {
-            float sk[KEYS], vv[KEYS][MAX_PER_LANE];
+        // this lane's share of a key's score; its value too where v is given
+        auto dot = [&](const T* k, const T* v, float& score, float (&value)[MAX_PER_LANE]) {
+            float s = 0.f;
 #pragma unroll
-            for (int u = 0; u < KEYS; ++u) {
+            for (int c = 0; c < MAX_PER_LANE; ++c) {
+                const int d = lane + 32 * c;
+                if (d < p.hd) s = fmaf(qv[c], fr_load(k + d), s);
+                if (!VALUES_LAST) value[c] = d < p.vd ? fr_load(v + d) : 0.f;
+            }
+            score = s;
+        };
+        auto round = [&](auto number, int i) {
+            constexpr int N = decltype(number)::value;
+            const T* kr[N];
+            const T* vr[N];
+            float sk[N], vv[N][MAX_PER_LANE];
+#pragma unroll
+            for (int u = 0; u < N; ++u) {
                 const int iu = min(i + u, i1 - 1);           // past the end: the last key again (its weight is set to zero)
                 const int j = iu < kept ? iu : lo + (iu - kept);
                 const size_t at = ((size_t)table[j / p.page] * p.page + j % p.page) * p.nkv + kvh;
-                const T* kr = (const T*)p.k_pool + at * p.hd;
-                const T* vr = (const T*)p.v_pool + at * p.vd;
-                float s = 0.f;
+                kr[u] = (const T*)p.k_pool + at * p.hd;
+                vr[u] = (const T*)p.v_pool + at * p.vd;
+                if (!VALUES_LAST) dot(kr[u], vr[u], sk[u], vv[u]);
+            }
+            if (VALUES_LAST) {
 #pragma unroll
-                for (int c = 0; c < MAX_PER_LANE; ++c) {
-                    const int d = lane + 32 * c;
-                    if (d < p.hd) s = fmaf(qv[c], fr_load(kr + d), s);
-                    vv[u][c] = d < p.vd ? fr_load(vr + d) : 0.f;
-                }
-                sk[u] = s;
+                for (int u = 0; u < N; ++u) dot(kr[u], nullptr, sk[u], vv[u]);
+#pragma unroll
+                for (int u = 0; u < N; ++u)
+#pragma unroll
+                    for (int c = 0; c < MAX_PER_LANE; ++c) {
+                        const int d = lane + 32 * c;
+                        vv[u][c] = d < p.vd ? fr_load(vr[u] + d) : 0.f;
+                    }
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-                for (int u = 0; u < KEYS; ++u) sk[u] += __shfl_xor_sync(0xffffffffu, sk[u], o);
+                for (int u = 0; u < N; ++u) sk[u] += __shfl_xor_sync(0xffffffffu, sk[u], o);
             float m_new = m;
 #pragma unroll
-            for (int u = 0; u < KEYS; ++u)
+            for (int u = 0; u < N; ++u)
                 if (i + u < i1) m_new = fmaxf(m_new, sk[u]);
             const float alpha = expf(m - m_new);      // exp(-inf) = 0 on the first keys
-            float sum = 0.f, add[MAX_PER_LANE];
+            float e[N], sum = 0.f;
 #pragma unroll
-            for (int c = 0; c < MAX_PER_LANE; ++c) add[c] = 0.f;
-#pragma unroll
-            for (int u = 0; u < KEYS; ++u) {
-                const float e = i + u < i1 ? expf(sk[u] - m_new) : 0.f;
-                sum += e;
-#pragma unroll
-                for (int c = 0; c < MAX_PER_LANE; ++c) add[c] = fmaf(e, vv[u][c], add[c]);
+            for (int u = 0; u < N; ++u) {
+                e[u] = i + u < i1 ? expf(sk[u] - m_new) : 0.f;
+                sum += e[u];
             }
             l = l * alpha + sum;
 #pragma unroll
-            for (int c = 0; c < MAX_PER_LANE; ++c) acc[c] = acc[c] * alpha + add[c];
+            for (int c = 0; c < MAX_PER_LANE; ++c) {
+                // (large heads: the sums under the condition of their loads, which the compiler then keeps together; without it
+                // heads of 192 and 256 took half as long again, with it smaller ones a tenth longer)
+                if (MAX_PER_LANE < 8 || lane + 32 * c < p.vd) {
+                    float add = 0.f;
+#pragma unroll
+                    for (int u = 0; u < N; ++u) add = fmaf(e[u], vv[u][c], add);
+                    acc[c] = acc[c] * alpha + add;
+                }
+            }
             m = m_new;
-        }
+        };
+        int i = i0;
+        if (KEYS > 4)
+            for (; i1 - i > 4; i += KEYS) round(Number<KEYS>{}, i);
+        for (; i < i1; i += 4) round(Number<4>{}, i);
     }
     if (part == nullptr) {
         const float inv = l > 0.f ? p.out_scale / l : 0.f;
@@ -150,10 +182,15 @@ __global__ void __launch_bounds__(128) attention_kernel(AttnArgs p) {
 template <typename T>
 cudaError_t launch_attention(const AttnArgs& p, dim3 grid, cudaStream_t stream) {
     const int size = p.hd > p.vd ? p.hd : p.vd;
-    if (size <= 32) return fr_launch(attention_kernel<T, 1, 16>, grid, dim3(128), 0, stream, p);
-    if (size <= 64) return fr_launch(attention_kernel<T, 2, 8>, grid, dim3(128), 0, stream, p);
-    if (size <= 128) return fr_launch(attention_kernel<T, 4, 8>, grid, dim3(128), 0, stream, p);
-    return fr_launch(attention_kernel<T, 8, 4>, grid, dim3(128), 0, stream, p);
+    void (*kernel)(AttnArgs) = size <= 32 ? attention_kernel<T, 1, 8> : size <= 64 ? attention_kernel<T, 2, 16>
+                             : size <= 128 ? attention_kernel<T, 4, 8> : attention_kernel<T, 8, 4>;
+    // Blocks that start while the predecessor still runs go to whichever SMs are free first.  A few blocks per SM then lie
+    // unevenly for the whole call (64 rows x 28 heads of 192, 700 keys: 355 us, 274 after the predecessor's end), so only a call
+    // of at most two per SM starts early.
+    const int sms = fr_sm_count() > 0 ? fr_sm_count() : 148;
+    if ((long long)grid.x * grid.y <= 2ll * sms) return fr_launch(kernel, grid, dim3(128), 0, stream, p);
+    kernel<<<grid, 128, 0, stream>>>(p);
+    return cudaGetLastError();
 }
 
 }  // namespace
