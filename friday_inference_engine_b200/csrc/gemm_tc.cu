@@ -1028,8 +1028,11 @@ static int tile_width(long long tiles_p, int q_rows, long long units, int narrow
 // are split less well: 128 x 18944 14.1 / 10.9 and 14.0 / 14.2, 256 x 32768 16.4 / 16.4 and 15.8 / 22.3, x 65536 18.8 / 29.8.
 // Not so where the columns are no multiple of its tile of 128, whose partial tiles one CTA then sums alone: 64 x 18944 30.3 / 10.7
 // and 30.3 / 13.8, 192 x 32768 33.1 / 16.4 and 33.3 / 22.2.
+// Many columns beside a short k are many blocks that do little each: 8 rows, 32-bit results: 4096 x 128 2.7 / 1.6, 8192 x 128 2.7 /
+// 2.9, 8192 x 512 6.5 / 3.9, 12288 x 512 4.5 / 5.8, 12288 x 1024 7.5 / 7.2, 16384 x 1024 7.6 / 8.7, 131072 x 256 12.6 / 43.
 static bool skinny_shape(int m, int n, int k, int sm_count) {
     const long long size = (long long)n * k;
+    if (n > 4096 + 8ll * k) return false;
     if (n % TILE_P == 0 && k > (m <= 8 ? 24576 : 16384) * (n <= 2 * TILE_P ? 1.5 : 1.0)) return false;
     if (m <= 8) return size <= (32ll << 20);
     return m <= 16 && (size <= (8ll << 20) || (size <= (16ll << 20) && n <= SKINNY_N * sm_count));

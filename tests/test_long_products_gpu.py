@@ -1,4 +1,5 @@
-"""Products of few rows with a few columns and a long k, on both sides of the lines where the kernel for small matrices ends."""
+"""Products of few rows with few columns and a long k, or many columns and a short k, on both sides of the lines where the kernel for
+small matrices ends."""
 import pytest
 import torch
 
@@ -9,8 +10,9 @@ DEV = "cuda:0"
 
 
 @pytest.mark.parametrize("m", [1, 8, 9, 16])
-@pytest.mark.parametrize("n,k", [(64, 65536), (127, 24584), (128, 24576), (128, 24584), (200, 32768), (256, 36864), (256, 36872), (384, 16384), (384, 16392), (384, 24576), (384, 24584)])
-def test_few_columns_long_k(m, n, k):
+@pytest.mark.parametrize("n,k", [(64, 65536), (127, 24584), (128, 24576), (128, 24584), (200, 32768), (256, 36864), (256, 36872), (384, 16384), (384, 16392), (384, 24576), (384, 24584),
+                                 (4608, 64), (4616, 64), (6145, 256), (12288, 1024), (12304, 1024)])
+def test_few_rows_at_the_lines(m, n, k):
     g = torch.Generator().manual_seed(m * n)
     x, w = (torch.randn(s, generator=g).bfloat16().to(DEV) for s in ((m, k), (n, k)))
     got = ops.linear(x, w, out_dtype=torch.float32)
