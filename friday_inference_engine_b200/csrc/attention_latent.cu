@@ -564,8 +564,7 @@ __global__ void __launch_bounds__(128) latent_attention_kernel(AttnArgs p) {
 
 // The same for a bf16 cache, all heads of a row in one block: the block brings KEYS cached rows at a time into shared memory (the
 // next ones on their way meanwhile), and its warps take the heads in turn, NH each.  A warp per (row, head) read every cached
-// row once per head, two at a time: 8 rows, 16 heads, up to
-// 540 keys took 47 us, 20 here.
+// row once per head, two at a time: 8 rows, 16 heads, up to 540 keys took 47 us, 20 here.
 constexpr int KEYS = 16;
 template <int NH>
 __global__ void __launch_bounds__(256, NH <= 2 ? 2 : 1) latent_rows_kernel(AttnArgs p) {
@@ -920,6 +919,17 @@ FR_EXPORT int attention_latent_prepare(const void* x, int ld, int q_off, int kv_
     return FR_OK;
 }
 
+// Whether the products in 16-byte pieces are the faster form: up to a few rounds of blocks, where the chain of waits is the cost.
+// Beyond, a block's set-up and its sums over the groups or lanes count (layout 0: until k is long, layout 1: where it is).  us, a column
+// at a time / in pieces: layout 0, 16 x 24 2.5 / 2.8; 64 x 64, 64 rows x 32 heads 3.5 / 3.0, 300 x 32 9.8 / 22.9; 128 x 512, 31 x 32 1.2
+// times as fast, 300 x 32 91 / 108; 256 x 512 1.03 to 3.2 times; layout 1, 64 x 64 1.2 to 2.8 times; 512 x 128, 64 x 32 1.0 times,
+// 300 x 32 209 / 233.
+static bool pieces_pay(int layout, int rows, int heads, int k, int n) {
+    const long long blocks = (long long)((rows + HL_ROWS - 1) / HL_ROWS) * heads * (layout == 0 ? (n + 127) / 128 : (n + 15) / 16);
+    if (layout == 0) return k >= 192 || (k >= 32 && blocks <= (long long)k * k / 12);
+    return k <= 128 || blocks * k <= 1 << 20;
+}
+
 // x_dtype / w_dtype / out_dtype: FR_F32 or FR_BF16 each; the gate (if any) is stored in the result's dtype.
 // fixed_weights not zero: w is memory that no kernel writes any more, and may be read while the kernel before still runs.
 FR_EXPORT int attention_latent_head_linear_weights(const void* x, int x_dtype, int ld_x, int x_off, int x_stride, const void* w, int w_dtype,
@@ -930,8 +940,9 @@ FR_EXPORT int attention_latent_head_linear_weights(const void* x, int x_dtype, i
     if (heads <= 0 || k <= 0 || n <= 0) FR_REFUSE("head_linear: %d heads, k %d, n %d", heads, k, n);
     HeadLinearArgs p{x, w, out, gate, row_seq, rows, heads, k, n, ld_x, x_off, x_stride, ld_out, out_stride, ld_gate, gate_off, fixed_weights};
     const int key = x_dtype * 4 + w_dtype * 2 + out_dtype;
-    // bf16 weights whose rows (of n numbers in layout 0, of k in layout 1) are whole 16-byte pieces
-    if (w_dtype == FR_BF16 && (layout == 0 ? n : k) % 8 == 0 && ((uintptr_t)w & 15) == 0 && (size_t)HL_ROWS * k * sizeof(float) <= 48 * 1024) {
+    // bf16 weights whose rows (of n numbers in layout 0, of k in layout 1) are whole 16-byte pieces, where pieces_pay
+    if (w_dtype == FR_BF16 && (layout == 0 ? n : k) % 8 == 0 && ((uintptr_t)w & 15) == 0 && (size_t)HL_ROWS * k * sizeof(float) <= 48 * 1024 &&
+        pieces_pay(layout, rows, heads, k, n)) {
         if (key == 6) return launch_head_pieces<bf16, float>(p, layout, stream);
         if (key == 3) return launch_head_pieces<float, bf16>(p, layout, stream);
         if (key == 2) return launch_head_pieces<float, float>(p, layout, stream);
@@ -956,20 +967,34 @@ FR_EXPORT int attention_latent_head_linear(const void* x, int x_dtype, int ld_x,
                                                 gate, ld_gate, gate_off, row_seq, rows, heads, k, n, 0, stream);
 }
 
-// Splits of the keys for a call of `rows` rows that see at most `keys`: two blocks per SM, at least one round of keys each; 0: the
-// cache is not one for the kernel whose blocks have all heads of a row (then a split is a warp's work).
+// Whether blocks with all heads of a row are the faster form.  Their time hardly depends on the heads (a warp has one of 1 to 8,
+// two of 9 to 16, up to four of 17 to 32), that of a warp per head grows with them, and a block's rounds are a chain, so that few
+// heads want few keys per block and several per warp many keys.  Latent 512 + 64, us, a warp per head / a block per row: 1 head, 8 rows x 2,000 keys 49 / 15,
+// 64 x 2,000 116 / 159, 1,000 x 600 174 / 703; 4 heads, 64 x 2,000 1.1 times as fast, 256 x 600 173 / 204; 8 heads and 16: 1.0 to
+// 3.8 times from 150 keys on, 8 rows x 20 keys 1.1 times and 10.1 / 12.8; 17 heads, 8 rows x 600 1.2 times, 64 x 600 176 / 237;
+// 24 heads, 64 x 600 1.5 times, 256 x 600 0.95 times, 8 x 20 10.2 / 15.9.
+static bool rows_pay(int rows, int heads, int keys) {
+    if (heads <= 4) return rows <= 16 || (rows <= 256 && (long long)rows * keys <= (rows <= 64 ? 32768ll : 8192ll) * heads);
+    if (heads <= 8) return rows <= 32 || keys >= 48;
+    if (heads <= 16) return keys >= 4 * heads;
+    return (rows <= 8 && keys >= 4 * heads) || (heads >= 22 && rows <= 64 && keys >= 256);
+}
+
+// Splits of the keys for a call of `rows` rows that see at most `keys`: two blocks per SM, at least one round of keys each; 0: not
+// a call for the kernel whose blocks have all heads of a row (then a split is a warp's work).
 FR_EXPORT int attention_latent_splits(int rows, int heads, int keys, int rank, int rot, int dtype) {
-    if (rows <= 0 || !shared_rows(heads, rank, rot, dtype)) return 0;
+    if (rows <= 0 || !shared_rows(heads, rank, rot, dtype) || !rows_pay(rows, heads, keys)) return 0;
     const int sms = fr_sm_count() > 0 ? fr_sm_count() : 148;
     int splits = 2 * sms / rows;
     if (splits > (keys + KEYS - 1) / KEYS) splits = (keys + KEYS - 1) / KEYS;
     return splits < 1 ? 1 : splits;
 }
 
-FR_EXPORT int attention_latent(const float* q, float* out, const void* c_pool, const void* r_pool, const int* block_table,
-                               int table_width, int page, const int* row_seq, const int* row_pos, const void* sink, int sink_dtype,
-                               int rows, int heads, int rank, int rot, float scale, int splits, float* scratch, int dtype,
-                               cudaStream_t stream) {
+// all_heads: blocks with all heads of a row, where the cache allows it (attention_latent_splits above 0 asks for it).
+FR_EXPORT int attention_latent_form(const float* q, float* out, const void* c_pool, const void* r_pool, const int* block_table,
+                                    int table_width, int page, const int* row_seq, const int* row_pos, const void* sink, int sink_dtype,
+                                    int rows, int heads, int rank, int rot, float scale, int splits, float* scratch, int dtype,
+                                    int all_heads, cudaStream_t stream) {
     if (rows <= 0) return FR_OK;
     if (rank <= 0 || rank > 32 * C_PER_LANE) FR_REFUSE("latent attention: latent size %d is outside 1..%d", rank, 32 * C_PER_LANE);
     if (rot < 0 || rot > 32 * R_PER_LANE) FR_REFUSE("latent attention: rotated part %d is outside 0..%d", rot, 32 * R_PER_LANE);
@@ -979,7 +1004,7 @@ FR_EXPORT int attention_latent(const float* q, float* out, const void* c_pool, c
                rot, splits, scale};
     const int items = rows * heads;
     const dim3 grid((items + 3) / 4, splits);
-    if (shared_rows(heads, rank, rot, dtype) && (((uintptr_t)c_pool | (uintptr_t)r_pool) & 15) == 0) {
+    if (all_heads && shared_rows(heads, rank, rot, dtype) && (((uintptr_t)c_pool | (uintptr_t)r_pool) & 15) == 0) {
         if (heads <= 8) FR_CUDA(launch_rows<1>(p, stream));
         else if (heads <= 16) FR_CUDA(launch_rows<2>(p, stream));
         else FR_CUDA(launch_rows<4>(p, stream));
@@ -1002,6 +1027,14 @@ FR_EXPORT int attention_latent(const float* q, float* out, const void* c_pool, c
         FR_CHECK_LAUNCH("latent attention merge");
     }
     return FR_OK;
+}
+
+FR_EXPORT int attention_latent(const float* q, float* out, const void* c_pool, const void* r_pool, const int* block_table,
+                               int table_width, int page, const int* row_seq, const int* row_pos, const void* sink, int sink_dtype,
+                               int rows, int heads, int rank, int rot, float scale, int splits, float* scratch, int dtype,
+                               cudaStream_t stream) {
+    return attention_latent_form(q, out, c_pool, r_pool, block_table, table_width, page, row_seq, row_pos, sink, sink_dtype, rows, heads, rank,
+                                 rot, scale, splits, scratch, dtype, 1, stream);
 }
 
 // One sequence's cached rows 0 .. n-1 (table: the sequence's row of the block table) as contiguous [2 n_pad][rank] (the

@@ -138,7 +138,7 @@ FAMILY(Delta, delta, "delta", resolve(h, fam, "delta_conv_prepare", t.conv_prepa
        resolve(h, fam, "delta_step_supports", t.step_supports); resolve(h, fam, "delta_step", t.step);)
 FAMILY(AttentionLatent, attention_latent, "attention_latent", resolve(h, fam, "attention_latent_rotate_pairs", t.rotate_pairs);
        resolve(h, fam, "attention_latent_prepare", t.prepare); resolve(h, fam, "attention_latent_head_linear_weights", t.head_linear);
-       resolve(h, fam, "attention_latent", t.run); resolve(h, fam, "attention_latent_gather", t.gather);
+       resolve(h, fam, "attention_latent_form", t.run); resolve(h, fam, "attention_latent_gather", t.gather);
        resolve(h, fam, "attention_latent_softmax_split", t.softmax_split);
        resolve(h, fam, "attention_latent_splits", t.splits); resolve(h, fam, "attention_latent_gate_cast", t.gate_cast);
        resolve(h, fam, "attention_latent_key_concat", t.key_concat);)

@@ -918,12 +918,13 @@ Tensor Ops::latent_attention(const Tensor& qf, const Tensor* sink, const LatentS
     Tensor out = alloc(DType::F32, rows, (int64_t)s.heads * s.rank);
     const auto& k = kernels::attention_latent();
     int splits = k.splits(rows, s.heads, ctx.max_kv_len, s.rank, s.rot, code(view.dtype));
-    if (splits < 1) splits = attention_splits(rows, s.heads, ctx.max_kv_len);
+    const bool all_heads = splits > 0;               // blocks with all heads of a row, else a warp per head
+    if (!all_heads) splits = attention_splits(rows, s.heads, ctx.max_kv_len);
     float* scratch = splits > 1 ? scratch_floats((int64_t)rows * s.heads * splits * (s.rank + 2)) : nullptr;
     Timed t(*this, Attention);
     call(launches_, k, k.run((const float*)qf.data, (float*)out.data, view.k_pool, view.v_pool, view.block_table, view.table_width,
                              view.page_size, ctx.row_seq, ctx.row_pos, sink ? sink->data : nullptr, sink ? code(sink->dtype) : 0, rows,
-                             s.heads, s.rank, s.rot, s.scale, splits, scratch, code(view.dtype), stream_), "attention_latent");
+                             s.heads, s.rank, s.rot, s.scale, splits, scratch, code(view.dtype), all_heads ? 1 : 0, stream_), "attention_latent");
     if (splits > 1) ++launches_;
     return out;
 }
