@@ -53,7 +53,7 @@ struct Number {
 
 // MAX_PER_LANE: dimensions per lane; KEYS keys at a time, four where no more than four are left: their loads are issued together,
 // keys before values (bf16 heads of 65 to 128: key by key, a tenth faster), so that a warp waits for memory once per round.  fp32, us, four at a time / as launched below: 28 heads of 32,
-// 4 rows, a window of 24 keys 8.3 / 5.3; of 64, 333 rows 267 / 181, 8 rows x 4,000 keys 166 / 114; of 128, 333 rows 275 / 209.
+// 4 rows, a window of 24 keys 8.0 / 4.6; of 64, 333 rows 267 / 183, 8 rows x 4,000 keys 166 / 113; of 128, 333 rows 275 / 207.
 template <typename T, int MAX_PER_LANE, int KEYS>
 __global__ void __launch_bounds__(128) attention_kernel(AttnArgs p) {
     constexpr bool VALUES_LAST = sizeof(T) == 4 || MAX_PER_LANE != 4;

@@ -480,8 +480,7 @@ FR_EXPORT int delta_scan(const float* qkv, const void* a_raw, int ld_a, const vo
 // query and key head form a cluster: its first block moves their history on once all have read it.
 //
 // Bound by the matrices' bytes (8 sequences, 16 heads of 128 x 128: 16.8 MB, 2.6 us) and a chain of five barriers
-// (8.3 to 9.4 us; conv_prepare, scan and head_norm_gate took 25 us in a decoding
-// step, 36 with a decay per channel).
+// (8.3 to 9.4 us; conv_prepare, scan and head_norm_gate took 25 us in a decoding step, 36 with a decay per channel).
 namespace {
 
 struct StepArgs {

@@ -6,11 +6,11 @@
 // innermost, which is how activations [rows][k] and projection weights [out][in] are
 // stored, so nothing is transposed.  Any m, n, k.  Three kernels:
 //
-//   gemm_f32_kernel    fp32 operands in 16-byte pieces, more than FEW_ROWS rows: tiles
-//                      in registers, k in two interleaved sums (fma.rn.f32x2), k split
+//   gemm_f32_kernel    fp32 operands in 16-byte pieces, more rows than the next one takes:
+//                      tiles in registers, k in two interleaved sums (fma.rn.f32x2), k split
 //                      over the CTAs of a cluster where there are few tiles;
-//   few_rows_kernel    the same operands, up to FEW_ROWS rows: a warp per few columns,
-//                      its lanes along k;
+//   few_rows_kernel    the same operands, up to FEW_ROWS rows (FEW_ROWS_WIDE from 8,192
+//                      columns on): a warp per few columns, its lanes along k;
 //   gemm_simt_kernel   everything else (mixed storage, unaligned rows).
 //
 // The reference's counterpart is its int8 tensor-core GEMM with the same epilogue
@@ -223,8 +223,9 @@ gemm_f32_kernel(const F32Args p) {
     fr_cluster_sync();                                       // nobody leaves while its shared memory is being read
 }
 
-// Bound by reading the weights once (or by the launch, for small ones).  Up to MR rows per block: a warp has NC columns, its lanes take 16-byte pieces of k in turn, every weight is read once per
-// block of rows; the MR * NC sums are then added over the lanes so that lane l ends with the l-th.
+// Bound by reading the weights once (or by the launch, for small ones).  Up to MR rows per block: a warp has NC columns, its lanes
+// take 16-byte pieces of k in turn, every weight is read once per block of rows; the MR * NC sums are then added over the lanes so
+// that lane l ends with the l-th.
 // Four columns per warp where there are enough of them to keep the SMs' loads in flight: a piece of x is then read once for
 // four weights (4 x 37888 x 3584: 108 us, 5.0 TB/s, against 129 with one column; 2 x 5000 x 3584 22 us either way).  Against
 // the general kernel: 694 and 338 us.  At 9 to 16 rows the weights are read twice, the second time from L2: up to 8,191
@@ -320,7 +321,10 @@ int launch_f32(const F32Args& p, cudaStream_t stream) {
     return FR_OK;
 }
 
-// Tile and split of k: the choice whose busiest SM has the least to do (a lone CTA leaves a third of the multiply-add rate).
+// Tile and split of k: the choice whose busiest SM has the least to do (a lone CTA leaves a third of the multiply-add rate).  The
+// cost of a k block is its multiply-adds, tm * tn, and 8 for what goes with them whatever the tile (barrier, copies, addresses); a
+// CTA's start and end count as four blocks of the largest tile, a cluster's exchange as four more.  These weights only rank the
+// choices; over 267 shapes (1 to 1,500 rows) the choice was never slower than the general kernel.
 // Measured on B200, this kernel against the general one below: 333 x 37888 x 3584 1,902 us (47.6 TFLOP/s; two thirds of the
 // rate at 1.88 GHz, whatever the tile and with plain multiply-adds too) against 3,998, 333 x 3584 x 18944 1,070 (7 x 8, four
 // splits) against 2,923, 64 x 3584 x 3584 57 against 338, 40 x 3584 x 18944 164 against 3,133.

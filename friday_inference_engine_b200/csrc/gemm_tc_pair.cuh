@@ -23,9 +23,10 @@ constexpr int PAIR_STAGES = 6;
 constexpr int PAIR_Q_BYTES = (PAIR_BN / 2) * TILE_K * 2;
 constexpr int PAIR_STAGE_BYTES = P_BYTES + PAIR_Q_BYTES;
 constexpr int PAIR_SMEM_BYTES = PAIR_STAGES * PAIR_STAGE_BYTES + 1024 + (2 * PAIR_STAGES + 4) * 8 + 64 + PAIR_BN * 4 + TILE_P * 4;
-// Eight warps finish a tile, two to each quarter of the accumulator's lanes, which take its groups of 16 columns in turn: with
-// one per quarter a gated tile's epilogue was longer than its products where k is short (2048 x 12288 x 2048: 107 us with one, 70 with two; eight experts
-// of some 512 rows, x 4096 x 2048: 113 and 70 to 76; prompts of the 7B shape 4 to 9 % less).
+// Eight warps finish a tile, two to each quarter of the accumulator's lanes, which take its groups of 16 columns in turn (with a norm
+// begun: a half each): with one per quarter a gated tile's epilogue was longer than its products where k is short (2048 x 12288 x
+// 2048: 107 us with one, 70 with two; eight experts of some 512 rows, x 4096 x 2048: 113 and 70 to 76; a prompt of 2,048 rows of the
+// 7B shape 5 % less).
 constexpr int PAIR_FINISHERS = 256, PAIR_THREADS = 64 + PAIR_FINISHERS;
 
 __device__ __forceinline__ uint32_t cluster_addr(uint32_t local, uint32_t rank) {

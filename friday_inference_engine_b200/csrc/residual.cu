@@ -152,8 +152,7 @@ layernorm_cast_kernel(const TI* __restrict__ x, FrVec w, FrVec b, TO* __restrict
 
 // Both norms for rows of whole groups of four numbers: what a thread has of the row, the weights and the bias is fetched at
 // once, before the first sum.  A decoding step has one block per row and nothing beside it, so the chain of waits is the cost
-// (8 rows of 2,048 in
-// a decoding step: 11 us with the kernels above, 2.3 to 3.4 with this one).
+// (8 rows of 2,048 in a decoding step: 11 us with the kernels above, 2.3 to 3.4 with this one).
 __device__ __forceinline__ void four_of(const float* p, int i, float (&v)[4]) {
     const float4 a = *(const float4*)(p + i);
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
