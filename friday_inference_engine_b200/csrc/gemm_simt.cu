@@ -15,9 +15,7 @@
 //
 // The reference's counterpart is its int8 tensor-core GEMM with the same epilogue
 // (bias, then residual, in place allowed): prefill_kernels.cu:156-171, 173-327.
-#include "common.cuh"
-
-#include <atomic>
+#include "gemm_f32_tc.cuh"
 
 FR_EXPORT const char* gemm_simt_last_error() { return fr_error_text; }
 
@@ -404,4 +402,34 @@ FR_EXPORT int gemm_simt(const void* a, int a_dtype, const void* w, int w_dtype, 
                         const void* bias, int bias_dtype, const void* residual, int m, int n, int k, int lda,
                         int ldw, int ldo, cudaStream_t stream) {
     return gemm_simt_weights(a, a_dtype, w, w_dtype, out, out_dtype, bias, bias_dtype, residual, m, n, k, lda, ldw, ldo, 0, stream);
+}
+
+// Products of fp32 operands on the tensor cores (gemm_f32_tc.cuh): whether gemm_simt_split takes this one with `scratch_bytes` of
+// scratch, and is the faster way.  It has two launches and a longer chain from its first load to its last store: below some 2^20
+// weights, or short k, the kernels of one launch are ahead (1024 x 512: 48 rows 10 us against 16; 1024 x 1024: 64 rows level, 128 rows
+// 21 against 16; 2048 x 1024: 48 rows 17 against 14; 200000 x 64: 96 rows 74 against 88).
+FR_EXPORT int gemm_simt_split_pays(const void* a, const void* w, int m, int n, int k, int lda, int ldw, long long scratch_bytes) {
+    if (((k | lda | ldw) & 3) || (((uintptr_t)a | (uintptr_t)w) & 15) || k < 1024 || n <= 0) return 0;
+    const bool few = m <= (n < 8192 ? FEW_ROWS : FEW_ROWS_WIDE);
+    if (few || split_rows_at_once(m, k, scratch_bytes) == 0) return 0;
+    const long long weights = (long long)n * k;
+    return weights >= 2ll << 20 ? m >= 48 || weights >= 6ll << 20 : weights >= 1ll << 20 && m > 64;
+}
+
+// scratch: 16-byte aligned, used by the kernels of this call only; status: a word that a wait that gave up is noted in.
+FR_EXPORT int gemm_simt_split(const float* a, const float* w, float* out, const void* bias, int bias_dtype, const float* residual, int m, int n,
+                              int k, int lda, int ldw, int ldo, int fixed_weights, void* scratch, long long scratch_bytes, int* status,
+                              cudaStream_t stream) {
+    if (m <= 0 || n <= 0) return FR_OK;
+    if (k <= 0) FR_REFUSE("gemm_simt: k = %d", k);
+    if (((k | lda | ldw) & 3) || (((uintptr_t)a | (uintptr_t)w | (uintptr_t)scratch) & 15)) FR_REFUSE("gemm_simt: rows are not in 16-byte pieces");
+    const int rows = split_rows_at_once(m, k, scratch_bytes);
+    if (rows == 0) FR_REFUSE("gemm_simt: %lld bytes of scratch are too few for rows of %d", scratch_bytes, k);
+    for (int r0 = 0; r0 < m; r0 += rows) {
+        const SplitArgs p{a + (size_t)r0 * lda, w, out + (size_t)r0 * ldo, FrVec{bias, bias_dtype}, residual ? residual + (size_t)r0 * ldo : nullptr,
+                          nullptr, m - r0 < rows ? m - r0 : rows, n, k, lda, ldw, ldo, 0, 0, 0, 1, 0, fixed_weights, status};
+        const int rc = run_split(p, scratch, stream);
+        if (rc) return rc;
+    }
+    return FR_OK;
 }

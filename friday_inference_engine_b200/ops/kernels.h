@@ -35,6 +35,9 @@ struct GemmSimt {
     last_error_fn last_error;
     int (*gemm)(const void*, int, const void*, int, void*, int, const void*, int, const void*, int, int, int, int, int, int,
                 int, cudaStream_t);
+    int (*split_pays)(const void*, const void*, int, int, int, int, int, long long);
+    int (*split)(const float*, const float*, float*, const void*, int, const float*, int, int, int, int, int, int, int, void*, long long, int*,
+                 cudaStream_t);
 };
 struct GemmTc {
     last_error_fn last_error;

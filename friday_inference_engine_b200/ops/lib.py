@@ -24,6 +24,8 @@ _SIGNATURES = {
     },
     "gemm_simt": {
         "gemm_simt": [P, I, P, I, P, I, P, I, P, I, I, I, I, I, I, P],
+        "gemm_simt_split": [P, P, P, P, I, P, I, I, I, I, I, I, I, P, c_longlong, P, P],
+        "gemm_simt_split_pays": [P, P, I, I, I, I, I, c_longlong],
     },
     "gemm_tc": {
         "gemm_tc": [P, P, P, I, P, I, P, I, I, I, I, I, I, P, c_longlong, P, I, P, I, I, I, I, P],

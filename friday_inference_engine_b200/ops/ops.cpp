@@ -1269,6 +1269,18 @@ Tensor Ops::linear_tc(const Tensor& x, const Tensor& weight, const Tensor* bias,
 Tensor Ops::linear_simt(const Tensor& x, const Tensor& weight, const Tensor* bias, const Tensor* residual, Tensor& out) {
     const auto& g = kernels::gemm_simt();
     Timed t(*this, Product);
+    const int m = (int)x.rows(), n = (int)weight.rows(), k = (int)x.cols();
+    const long long room = (long long)tc_scratch_.bytes();
+    if (x.dtype == DType::F32 && weight.dtype == DType::F32 && out.dtype == DType::F32 &&
+        g.split_pays(x.data, weight.data, m, n, k, (int)x.ld, (int)weight.ld, room)) {
+        call(launches_, g,
+             g.split((const float*)x.data, (const float*)weight.data, (float*)out.data, bias ? bias->data : nullptr, bias ? code(bias->dtype) : 0,
+                     residual ? (const float*)residual->data : nullptr, m, n, k, (int)x.ld, (int)weight.ld, (int)out.ld, fixed(weight) ? 1 : 0,
+                     tc_scratch_.get(), room, (int*)status_.get(), stream_),
+             "gemm_simt_split");
+        ++launches_;                                          // the rows' split and the product
+        return out;
+    }
     call(launches_, g,
          g.gemm(x.data, code(x.dtype), weight.data, code(weight.dtype), out.data, code(out.dtype),
                 bias ? bias->data : nullptr, bias ? code(bias->dtype) : 0, residual ? residual->data : nullptr,
