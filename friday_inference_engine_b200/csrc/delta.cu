@@ -18,11 +18,14 @@
 //                  memory meanwhile.  beta = sigmoid(raw),
 //                  g = exp(-exp(A_log) * softplus(raw + dt_bias)) are formed here in fp32.  Columns of S never mix, so
 //                  any split of the value channels over blocks is exact.
+//   scan_chunks    the recurrence of prompts, sixteen tokens at a time (delta_chunks.cuh)
 //   step           all of it and the heads' gated norm for one token per sequence (below)
 //
 // State of a sequence: [taps-1][channels] history (channel order of the stacked projection: q, k, v), then the heads'
 // matrices [heads][dk][dv], all fp32.  Everything here is fp32 arithmetic; only the projection's rows may be bf16.
 #include <math.h>
+
+#include <atomic>
 
 #include "common.cuh"
 
@@ -177,6 +180,10 @@ __device__ __forceinline__ float softplus_f(float z) { return fmaxf(z, 0.f) + lo
 
 template <typename TR>
 __device__ __forceinline__ float raw_at(const void* p, size_t i) { return fr_load((const TR*)p + i); }
+
+}  // namespace
+#include "delta_chunks.cuh"
+namespace {
 
 constexpr int STAGE_THREADS = 128;   // warps that only stage tokens, beside the warps that own value channels
 // Threads that share a value channel, each with its share of the key channels in registers.  Four: with sixteen (eight
@@ -471,6 +478,26 @@ FR_EXPORT int delta_scan(const float* qkv, const void* a_raw, int ld_a, const vo
     if (raw_dtype == FR_F32) return scan_by_size<float>(p, n_seqs, splits, stream);
     if (raw_dtype == FR_BF16) return scan_by_size<bf16>(p, n_seqs, splits, stream);
     FR_REFUSE("delta scan: unknown dtype %d", raw_dtype);
+}
+
+// Whether delta_scan_chunks takes these sizes (rows in 16-byte pieces, a head's keys within a chunk's tile).
+FR_EXPORT int delta_scan_chunks_supports(const float* qkv, int dk, int dv) {
+    return dk > 0 && dk <= CD && dk % 4 == 0 && dv > 0 && dv % 4 == 0 && ((uintptr_t)qkv & 15) == 0;
+}
+
+// delta_scan for prompts: the same arguments and results, sixteen tokens at a time (delta_chunks.cuh).
+FR_EXPORT int delta_scan_chunks(const float* qkv, const void* a_raw, int ld_a, const void* b_raw, int ld_b, int raw_dtype, const void* a_log,
+                                const void* dt_bias, int vec_dtype, float* out, float* state, long long state_stride, long long s_off,
+                                const int* row_seq, const int* seq_start, const int* seq_qlen, const int* seq_slots, int n_seqs, int heads,
+                                int qk_heads, int dk, int dv, int per_channel, cudaStream_t stream) {
+    if (n_seqs <= 0) return FR_OK;
+    if (heads <= 0 || qk_heads <= 0 || heads % qk_heads || !delta_scan_chunks_supports(qkv, dk, dv))
+        FR_REFUSE("delta chunks: %d heads on %d query/key heads, dk %d, dv %d", heads, qk_heads, dk, dv);
+    const ScanArgs p{qkv, a_raw, b_raw, raw_dtype, a_log, dt_bias, vec_dtype, out, state, state_stride, s_off, row_seq, seq_start, seq_qlen,
+                     seq_slots, ld_a, ld_b, heads, qk_heads, dk, dv, 0, per_channel ? 1 : 0};
+    if (raw_dtype == FR_F32) return per_channel ? launch_chunks<float, true>(p, n_seqs, stream) : launch_chunks<float, false>(p, n_seqs, stream);
+    if (raw_dtype == FR_BF16) return per_channel ? launch_chunks<bf16, true>(p, n_seqs, stream) : launch_chunks<bf16, false>(p, n_seqs, stream);
+    FR_REFUSE("delta chunks: unknown dtype %d", raw_dtype);
 }
 
 // ------------------------------------------------------------------ a step of one token per sequence

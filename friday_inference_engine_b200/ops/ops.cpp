@@ -830,6 +830,9 @@ Tensor Ops::conv_silu_unit(const Tensor& proj, const Tensor& taps, const DeltaSp
     return out;
 }
 
+// Tokens of the longest sequence from which on the delta rule goes in chunks of sixteen tokens.
+static constexpr int DELTA_CHUNKS_FROM = 32;
+
 Tensor Ops::delta_scan(const Tensor& qkv, const Tensor& a_raw, const Tensor& b_raw, const Tensor& a_log, const Tensor& dt_bias,
                        const DeltaSpec& s, const CacheView& view, const StepContext& ctx) {
     if (view.kind != CacheRequest::State || !view.state.defined() || view.state.dtype != DType::F32)
@@ -843,9 +846,10 @@ Tensor Ops::delta_scan(const Tensor& qkv, const Tensor& a_raw, const Tensor& b_r
     Tensor out = alloc(DType::F32, qkv.rows(), (int64_t)s.heads * s.dv);
     const auto& k = kernels::delta();
     Timed t(*this, Attention);
-    call(launches_, k, k.scan((const float*)qkv.data, a_raw.data, (int)a_raw.ld, b_raw.data, (int)b_raw.ld, code(a_raw.dtype), a_log.data,
-                              dt_bias.data, code(a_log.dtype), (float*)out.data, (float*)view.state.data, stride, s_off, ctx.row_seq,
-                              ctx.seq_start, ctx.seq_qlen, view.seq_slots, ctx.n_seqs, s.heads, s.qk_heads, s.dk, s.dv,
+    const bool chunks = !ctx.decode && ctx.max_q_len >= DELTA_CHUNKS_FROM && k.chunks_supports((const float*)qkv.data, s.dk, s.dv);
+    call(launches_, k, (chunks ? k.chunks : k.scan)((const float*)qkv.data, a_raw.data, (int)a_raw.ld, b_raw.data, (int)b_raw.ld, code(a_raw.dtype),
+                              a_log.data, dt_bias.data, code(a_log.dtype), (float*)out.data, (float*)view.state.data, stride, s_off,
+                              ctx.row_seq, ctx.seq_start, ctx.seq_qlen, view.seq_slots, ctx.n_seqs, s.heads, s.qk_heads, s.dk, s.dv,
                               s.per_channel ? 1 : 0, stream_), "delta_scan");
     return out;
 }
