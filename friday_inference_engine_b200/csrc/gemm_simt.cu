@@ -16,6 +16,7 @@
 // The reference's counterpart is its int8 tensor-core GEMM with the same epilogue
 // (bias, then residual, in place allowed): prefill_kernels.cu:156-171, 173-327.
 #include "gemm_f32_tc.cuh"
+#include "gemm_few_fusion.h"
 
 FR_EXPORT const char* gemm_simt_last_error() { return fr_error_text; }
 
@@ -303,6 +304,172 @@ int launch_few(const F32Args& p, cudaStream_t stream) {
     return FR_OK;
 }
 
+// The same with work of its neighbours at both ends (gemm_few_fusion.h).  A warp has NP pairs of columns: the two that a gated unit or a
+// rotation needs lie in one warp.  The norm of the input is finished after the sums: every warp reads all of its rows anyway and
+// adds up their squares on the way.
+enum FewEnd { FEW_PLAIN, FEW_GATED, FEW_ROTARY };
+
+// Columns of pair `pair` of a rotary product: (i, i + rot / 2) of a rotated head, neighbours elsewhere.
+__device__ __forceinline__ void rotary_columns(const GemmFewFusion& f, int pair, int& c0, int& c1, int& head, int& angle) {
+    const int per = f.hd >> 1;
+    head = pair / per;
+    const int i = pair - head * per, base = head * f.hd, half = f.rot >> 1;
+    angle = -1;
+    if (f.denom != nullptr && head < f.nq + f.nkv) {
+        if (i < half) {
+            angle = i;
+            c0 = base + i;
+            c1 = c0 + half;
+            return;
+        }
+        c0 = base + f.rot + 2 * (i - half);
+    } else {
+        c0 = base + 2 * i;
+    }
+    c1 = c0 + 1;
+}
+
+template <int MR, int NP, int END>
+__global__ void __launch_bounds__(128)
+few_fused_kernel(const F32Args p, const GemmFewFusion f) {
+    constexpr int NC = 2 * NP, V = MR * NC, SPARE = 32 / V;
+    static_assert(V <= 32, "a lane ends with one value");
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int pair0 = (blockIdx.x * 4 + warp) * NP, m0 = blockIdx.y * MR, pairs = (p.n + 1) >> 1;
+    if (pair0 >= pairs) {
+        fr_pdl_wait();                                       // (no kernel ends before its predecessor)
+        return;
+    }
+    int col[NC];
+#pragma unroll
+    for (int q = 0; q < NP; ++q) {
+        const int pair = min(pair0 + q, pairs - 1);
+        int head, angle;
+        if (END == FEW_ROTARY) {
+            rotary_columns(f, pair, col[2 * q], col[2 * q + 1], head, angle);
+        } else {
+            col[2 * q] = 2 * pair;
+            col[2 * q + 1] = min(2 * pair + 1, p.n - 1);
+        }
+    }
+    // what this lane finishes: value `at` of row m0 + at / NC and column at % NC of the warp's
+    const int at = lane / SPARE, my_row = m0 + at / NC, my_pair = pair0 + (at % NC) / 2, second = at & 1;
+    // its angle and cache row depend on the step's geometry alone
+    float cosine = 1.f, sine = 0.f;
+    float* cached = nullptr;
+    if (END == FEW_ROTARY && my_row < p.m && my_pair < pairs && f.row_seq[my_row] >= 0) {
+        int c0, c1, head, angle;
+        rotary_columns(f, my_pair, c0, c1, head, angle);
+        const int pos = f.row_pos[my_row];
+        if (angle >= 0) sincosf(__fdiv_rn((float)pos, f.denom[angle]), &sine, &cosine);
+        if (f.k_pool != nullptr && head >= f.nq) {
+            const int page = f.table[(size_t)f.row_seq[my_row] * f.table_width + pos / f.page];
+            const bool is_k = head < f.nq + f.nkv;
+            cached = (is_k ? f.k_pool : f.v_pool) + (((size_t)page * f.page + pos % f.page) * f.nkv + (head - f.nq - (is_k ? 0 : f.nkv))) * f.hd +
+                     (second ? c1 : c0) - head * f.hd;
+        }
+    }
+    const FrVec gain{f.norm_w, f.norm_w_dtype};
+    Pair acc[V];
+    float squares[MR];
+#pragma unroll
+    for (int v = 0; v < V; ++v) acc[v] = 0ull;
+#pragma unroll
+    for (int r = 0; r < MR; ++r) squares[r] = 0.f;
+    const ulonglong2* w[NC];
+    const float4* x[MR];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) w[c] = (const ulonglong2*)(p.w + (size_t)col[c] * p.ldw);
+#pragma unroll
+    for (int r = 0; r < MR; ++r) x[r] = (const float4*)(p.a + (size_t)min(m0 + r, p.m - 1) * p.lda);
+    if (!p.fixed_weights) fr_pdl_wait();
+    ulonglong2 first[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) first[c] = lane < p.k / 4 ? __ldg(w[c] + lane) : make_ulonglong2(0, 0);
+    fr_pdl_wait();
+    fr_pdl_launch();
+#pragma unroll 2
+    for (int q = lane; q < p.k / 4; q += 32) {
+        ulonglong2 y[NC];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) y[c] = q == lane ? first[c] : __ldg(w[c] + q);
+        float g[4] = {1.f, 1.f, 1.f, 1.f};
+        if (f.norm_w != nullptr) gain.four(4 * q, g);
+#pragma unroll
+        for (int r = 0; r < MR; ++r) {
+            float4 z = x[r][q];
+            if (f.norm_w != nullptr) {
+                squares[r] = fmaf(z.x, z.x, fmaf(z.y, z.y, fmaf(z.z, z.z, fmaf(z.w, z.w, squares[r]))));
+                z.x *= g[0]; z.y *= g[1]; z.z *= g[2]; z.w *= g[3];
+            }
+            const Pair lo = (Pair)__float_as_uint(z.x) | (Pair)__float_as_uint(z.y) << 32;
+            const Pair hi = (Pair)__float_as_uint(z.z) | (Pair)__float_as_uint(z.w) << 32;
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                fma_pair(acc[r * NC + c], lo, y[c].x);
+                fma_pair(acc[r * NC + c], hi, y[c].y);
+            }
+        }
+    }
+    float s[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) s[v] = pair_sum(acc[v]);
+    if (f.norm_w != nullptr) {
+#pragma unroll
+        for (int r = 0; r < MR; ++r) {
+            const float inv = 1.0f / sqrtf(fr_warp_sum(squares[r]) / (float)p.k + f.eps);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) s[r * NC + c] *= inv;
+        }
+    }
+#pragma unroll
+    for (int half = V / 2, bit = 16; bit > 0; bit >>= 1) {     // as in few_rows_kernel: lane l ends with value l / SPARE
+        if (half > 0) {
+            const bool upper = (lane & bit) != 0;
+#pragma unroll
+            for (int v = 0; v < V / 2; ++v)
+                if (v < half) {
+                    const float give = upper ? s[v] : s[v + half], keep = upper ? s[v + half] : s[v];
+                    s[v] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+                }
+            half >>= 1;
+        } else {
+            s[0] += __shfl_xor_sync(0xffffffffu, s[0], bit);
+        }
+    }
+    int c0 = 2 * my_pair, c1 = c0 + 1, head = 0, angle = -1;
+    if (END == FEW_ROTARY && my_pair < pairs) rotary_columns(f, my_pair, c0, c1, head, angle);
+    const int my_col = second ? c1 : c0;
+    const bool mine = lane % SPARE == 0 && my_row < p.m && my_pair < pairs && my_col < p.n;
+    float v = s[0];
+    if (mine && p.bias.p != nullptr) v += p.bias.at(my_col);
+    const float other = __shfl_xor_sync(0xffffffffu, v, SPARE);
+    if (!mine) return;
+    if (END == FEW_GATED) {
+        if (!second) p.out[(size_t)my_row * p.ldo + my_pair] = fr_gated(f.act, v, other, f.act_limit, f.act_slope);
+    } else {
+        if (END == FEW_ROTARY && angle >= 0 && f.row_seq[my_row] >= 0) {
+            float ra, rb;
+            fr_rotate(second ? other : v, second ? v : other, cosine, sine, ra, rb);
+            v = second ? rb : ra;
+        }
+        const size_t to = (size_t)my_row * p.ldo + my_col;
+        if (p.residual != nullptr) v += p.residual[to];
+        p.out[to] = v;
+        if (END == FEW_ROTARY && cached != nullptr) *cached = v;
+    }
+}
+
+template <int MR, int NP>
+int launch_few_fused(const F32Args& p, const GemmFewFusion& f, cudaStream_t stream) {
+    const dim3 grid(((p.n + 1) / 2 + 4 * NP - 1) / (4 * NP), (p.m + MR - 1) / MR);
+    if (f.nq > 0) FR_CUDA(fr_launch(few_fused_kernel<MR, NP, FEW_ROTARY>, grid, dim3(128), 0, stream, p, f));
+    else if (f.act) FR_CUDA(fr_launch(few_fused_kernel<MR, NP, FEW_GATED>, grid, dim3(128), 0, stream, p, f));
+    else FR_CUDA(fr_launch(few_fused_kernel<MR, NP, FEW_PLAIN>, grid, dim3(128), 0, stream, p, f));
+    FR_CHECK_LAUNCH("gemm_simt (few rows, fused)");
+    return FR_OK;
+}
+
 template <int TM, int TN>
 int launch_f32(const F32Args& p, cudaStream_t stream) {
     static std::atomic<unsigned long long> configured{0};    // devices (as bits) on which the limit has been raised
@@ -432,4 +599,27 @@ FR_EXPORT int gemm_simt_split(const float* a, const float* w, float* out, const 
         if (rc) return rc;
     }
     return FR_OK;
+}
+
+// Whether gemm_simt_few takes these rows and weights (as gemm_simt's kernel of few rows does).
+FR_EXPORT int gemm_simt_few_supports(const float* a, const float* w, int m, int n, int k, int lda, int ldw) {
+    return k > 0 && n > 0 && !((k | lda | ldw) & 3) && !(((uintptr_t)a | (uintptr_t)w) & 15) && m <= (n < 8192 ? FEW_ROWS : FEW_ROWS_WIDE);
+}
+
+// gemm_simt for few rows with the work that `fusion` asks for; out is [m][n], of a gated unit [m][n / 2].
+FR_EXPORT int gemm_simt_few(const float* a, const float* w, float* out, const void* bias, int bias_dtype, const float* residual, int m, int n,
+                            int k, int lda, int ldw, int ldo, const GemmFewFusion* fusion, cudaStream_t stream) {
+    if (m <= 0 || n <= 0) return FR_OK;
+    const GemmFewFusion& f = *fusion;
+    if (!gemm_simt_few_supports(a, w, m, n, k, lda, ldw)) FR_REFUSE("gemm_simt (few rows): %d x %d x %d, strides %d and %d", m, n, k, lda, ldw);
+    if (f.nq > 0 && (f.act || residual != nullptr || f.nkv <= 0 || f.hd <= 0 || (f.hd & 1) || (f.rot & 1) || f.rot < 0 || f.rot > f.hd ||
+                     n != (f.nq + 2 * f.nkv) * f.hd || f.row_seq == nullptr || f.row_pos == nullptr || (f.denom != nullptr && f.rot == 0)))
+        FR_REFUSE("gemm_simt (few rows): %d + 2 x %d heads of %d with %d rotated in %d columns", f.nq, f.nkv, f.hd, f.rot, n);
+    if (f.act && ((n & 1) || residual != nullptr)) FR_REFUSE("gemm_simt (few rows): a gated unit of %d columns", n);
+    const F32Args p{a, w, out, FrVec{bias, bias_dtype}, residual, m, n, k, lda, ldw, ldo, 1, 0, f.fixed_weights};
+    const bool wide = n >= 2368;                               // as many pairs per warp as keep the SMs' loads in flight
+    if (m == 1) return wide ? launch_few_fused<1, 2>(p, f, stream) : launch_few_fused<1, 1>(p, f, stream);
+    if (m == 2) return wide ? launch_few_fused<2, 2>(p, f, stream) : launch_few_fused<2, 1>(p, f, stream);
+    if (m <= 4) return wide ? launch_few_fused<4, 2>(p, f, stream) : launch_few_fused<4, 1>(p, f, stream);
+    return wide ? launch_few_fused<8, 2>(p, f, stream) : launch_few_fused<8, 1>(p, f, stream);
 }

@@ -18,6 +18,7 @@
 #include "friday/base.h"
 #include "friday/parts.h"
 
+struct GemmFewFusion;       // csrc/gemm_few_fusion.h: the same of the 32-bit product of few rows
 struct GemmFusion;          // csrc/gemm_tc_fusion.h: optional work at the two ends of the tensor-core product
 
 namespace friday {
@@ -68,8 +69,9 @@ private:
 // Rows on their way from one product to the next.  Plain rows are a tensor.  Deferred rows are rows whose
 // RMSNorm the product that made them has begun: `t` holds weight (*) x rounded to bf16, `ssq` [parts, rows]
 // each part's share of the rows' sums of squares; the product that takes them finishes the norm by scaling
-// its own rows with 1 / sqrt(sum / width + eps).  Anything else asks Ops::materialize, which runs the norm's
-// kernel on `source`.
+// its own rows with 1 / sqrt(sum / width + eps).  Deferred rows without `ssq` (few 32-bit rows) are `source` itself with
+// nothing of the norm begun: the product that takes them does all of it.  Anything else asks Ops::materialize, which runs
+// the norm's kernel on `source`.
 struct Rows {
     Tensor t;
     bool deferred = false;
@@ -419,6 +421,8 @@ public:
     Tensor linear_tc(const Tensor& x, const Tensor& weight, const Tensor* bias, const Tensor* residual, Tensor& out,
                      int swap = -1, int bn = -1, int splits = -1, int act = 0, GemmFusion* fusion = nullptr);
     Tensor linear_simt(const Tensor& x, const Tensor& weight, const Tensor* bias, const Tensor* residual, Tensor& out);
+    bool few_in(const Rows& x, const Tensor& weight, DType out, GemmFewFusion& f) const;
+    Tensor linear_few(const Rows& x, const Tensor& weight, const Tensor* bias, const Tensor* residual, Tensor& out, const GemmFewFusion& f);
     bool tensor_core_ok(const Tensor& x, const Tensor& weight, const Tensor& out, const Tensor* residual) const;
     void plan(int64_t rows, int64_t n, int64_t k, bool* swapped, int* bn, int* splits = nullptr);
     int decode_splits(int n_seqs, int n_heads, int n_kv_heads, int head_dim, int max_kv_len);

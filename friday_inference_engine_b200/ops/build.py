@@ -195,7 +195,7 @@ def _engine_inputs():
         units += sorted(os.path.join(folder, f) for f in os.listdir(folder) if f.endswith(".cpp"))
         headers += sorted(os.path.join(folder, f) for f in os.listdir(folder) if f.endswith(".h"))
     headers += sorted(os.path.join(INCLUDE, "friday", f) for f in os.listdir(os.path.join(INCLUDE, "friday")))
-    headers += [os.path.join(CSRC, "gemm_tc_fusion.h"), os.path.join(CSRC, "philox.h")]
+    headers += [os.path.join(CSRC, f) for f in ("gemm_tc_fusion.h", "gemm_few_fusion.h", "philox.h")]
     return units, headers
 
 

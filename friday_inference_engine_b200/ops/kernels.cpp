@@ -96,7 +96,8 @@ FAMILY(Rowwise, rowwise, "rowwise",
        resolve(h, fam, "rowwise_scale_rows", t.scale_rows); resolve(h, fam, "rowwise_finish_logits", t.finish_logits);
        resolve(h, fam, "rowwise_random_normal", t.random_normal);)
 FAMILY(GemmSimt, gemm_simt, "gemm_simt", resolve(h, fam, "gemm_simt_weights", t.gemm);
-       resolve(h, fam, "gemm_simt_split_pays", t.split_pays); resolve(h, fam, "gemm_simt_split", t.split);)
+       resolve(h, fam, "gemm_simt_split_pays", t.split_pays); resolve(h, fam, "gemm_simt_split", t.split);
+       resolve(h, fam, "gemm_simt_few_supports", t.few_supports); resolve(h, fam, "gemm_simt_few", t.few);)
 FAMILY(GemmTc, gemm_tc, "gemm_tc", resolve(h, fam, "gemm_tc_fused", t.fused); resolve(h, fam, "gemm_tc_plan", t.plan);
        resolve(h, fam, "gemm_tc_grouped", t.grouped);)
 FAMILY(AttentionSimt, attention_simt, "attention_simt", resolve(h, fam, "attention_simt", t.run);

@@ -10,6 +10,7 @@
 
 #include <string>
 
+#include "csrc/gemm_few_fusion.h"
 #include "csrc/gemm_tc_fusion.h"
 
 namespace friday {
@@ -38,6 +39,9 @@ struct GemmSimt {
     int (*split_pays)(const void*, const void*, int, int, int, int, int, long long);
     int (*split)(const float*, const float*, float*, const void*, int, const float*, int, int, int, int, int, int, int, void*, long long, int*,
                  cudaStream_t);
+    int (*few_supports)(const float*, const float*, int, int, int, int, int);
+    int (*few)(const float*, const float*, float*, const void*, int, const float*, int, int, int, int, int, int, const GemmFewFusion*,
+               cudaStream_t);
 };
 struct GemmTc {
     last_error_fn last_error;

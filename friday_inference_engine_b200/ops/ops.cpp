@@ -1314,8 +1314,39 @@ Tensor Ops::linear(const Rows& x, const Tensor& weight, const Tensor* bias, cons
         fusion_in(x, f);
         return linear_tc(xt, weight, bias, residual, o, -1, -1, -1, 0, x.deferred ? &f : nullptr);
     }
+    GemmFewFusion f;
+    if (x.deferred && few_in(x, weight, o.dtype, f)) return linear_few(x, weight, bias, residual, o, f);
     Tensor xin = x.deferred ? materialize(x) : xt;
     return linear_simt(xin, weight, bias, residual, o);
+}
+
+// Whether the 32-bit product of few rows takes x and weight; if so, f asks it for the norm that x has been promised.
+bool Ops::few_in(const Rows& x, const Tensor& weight, DType out, GemmFewFusion& f) const {
+    const Tensor& t = x.deferred ? x.source : x.t;
+    if (!t.defined() || t.dtype != DType::F32 || weight.dtype != DType::F32 || out != DType::F32 || t.rows() > 16 || !fusion_enabled()) return false;
+    if (!kernels::gemm_simt().few_supports((const float*)t.data, (const float*)weight.data, (int)t.rows(), (int)weight.rows(), (int)t.cols(),
+                                           (int)t.ld, (int)weight.ld))
+        return false;
+    memset(&f, 0, sizeof f);
+    if (x.deferred) {
+        f.norm_w = x.weight.data;
+        f.norm_w_dtype = code(x.weight.dtype);
+        f.eps = x.eps;
+    }
+    f.fixed_weights = fixed(weight) ? 1 : 0;
+    return true;
+}
+
+Tensor Ops::linear_few(const Rows& x, const Tensor& weight, const Tensor* bias, const Tensor* residual, Tensor& out, const GemmFewFusion& f) {
+    const Tensor& t = x.deferred ? x.source : x.t;
+    const auto& g = kernels::gemm_simt();
+    Timed timed(*this, Product);
+    call(launches_, g,
+         g.few((const float*)t.data, (const float*)weight.data, (float*)out.data, bias ? bias->data : nullptr, bias ? code(bias->dtype) : 0,
+               residual ? (const float*)residual->data : nullptr, (int)t.rows(), (int)weight.rows(), (int)t.cols(), (int)t.ld, (int)weight.ld,
+               (int)out.ld, &f, stream_),
+         "gemm_simt_few");
+    return out;
 }
 
 Tensor Ops::linear_alone(const Rows& x, const Tensor& weight, const Tensor* bias) {
@@ -1382,6 +1413,14 @@ std::pair<Tensor, Rows> Ops::linear_norm(const Rows& x, const Tensor& weight, co
         }
     }
     Tensor out = linear(x, weight, bias, residual);
+    if (out.dtype == DType::F32 && rows <= 16 && norm_weight.numel() == n && fusion_enabled()) {
+        Rows r(out);                                          // few 32-bit rows: the products that read them do their norm
+        r.deferred = true;
+        r.eps = eps;
+        r.source = out;
+        r.weight = norm_weight;
+        return {out, r};
+    }
     return {out, Rows(rmsnorm(out, norm_weight, eps))};
 }
 
@@ -1417,6 +1456,26 @@ Tensor Ops::qkv_rope_write(const Rows& x, const Tensor& weight, const Tensor* bi
             return linear_tc(xt, weight, bias, nullptr, out, -1, -1, -1, 0, &f);
         }
     }
+    GemmFewFusion few;
+    if (head_dim % 2 == 0 && rotary_dim % 2 == 0 && n == (int64_t)(n_heads + 2 * n_kv_heads) * head_dim && (denominators || write) &&
+        (!write || view->dtype == DType::F32) && few_in(x, weight, xt.dtype, few)) {
+        Tensor out = alloc(xt.dtype, xt.rows(), n);
+        few.row_seq = row_seq;
+        few.row_pos = row_pos;
+        few.denom = denominators;
+        few.rot = denominators ? rotary_dim : 0;
+        few.nq = n_heads;
+        few.nkv = n_kv_heads;
+        few.hd = head_dim;
+        if (write) {
+            few.k_pool = (float*)view->k_pool;
+            few.v_pool = (float*)view->v_pool;
+            few.table = view->block_table;
+            few.table_width = view->table_width;
+            few.page = view->page_size;
+        }
+        return linear_few(x, weight, bias, nullptr, out, few);
+    }
     Tensor qkv = linear(x, weight, bias);
     if (denominators || write) rope_kv_write(qkv, row_seq, row_pos, denominators, rotary_dim, n_heads, n_kv_heads, head_dim, view);
     return qkv;
@@ -1435,6 +1494,14 @@ Tensor Ops::linear_swiglu(const Rows& x, const Tensor& weight_pairs, int act, fl
         f.act_limit = limit;
         f.act_slope = slope;
         return linear_tc(xt, weight_pairs, nullptr, nullptr, out, -1, -1, -1, act, x.deferred || act == 3 ? &f : nullptr);
+    }
+    GemmFewFusion few;
+    if (act > 0 && act <= 3 && few_in(x, weight_pairs, xt.dtype, few)) {
+        Tensor out = alloc(xt.dtype, xt.rows(), inner);
+        few.act = act;
+        few.act_limit = limit;
+        few.act_slope = slope;
+        return linear_few(x, weight_pairs, nullptr, nullptr, out, few);
     }
     return swiglu(linear(x, weight_pairs), act, limit, slope);
 }
