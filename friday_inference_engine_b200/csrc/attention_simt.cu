@@ -22,6 +22,8 @@
 // a warp walks are the kept ones below the window's start followed by the window's.
 #include <math.h>
 
+#include <atomic>
+
 #include "attention_merge.cuh"
 #include "common.cuh"
 
@@ -179,6 +181,201 @@ __global__ void __launch_bounds__(128) attention_kernel(AttnArgs p) {
     }
 }
 
+// Prompts in fp32.  The kernel above reads every key and value for every query row; here a block takes 64 rows, the query heads
+// of one kv head for as many consecutive tokens as that makes, and walks 32 keys at a time, which pass through shared memory once for
+// all of them.  128 threads: a thread has four rows' scores with four keys, then the same rows' results in HD / 8
+// channels, so that a row's scores, maximum and weights stay within a warp.  Bound by the multiply-adds (each needs an eighth of a
+// 16-byte read from shared memory).
+constexpr int PT_ROWS = 64, PT_KEYS = 32, PT_THREADS = 128;
+
+struct PromptArgs {
+    const float* q;
+    float* out;
+    const float* k_pool;
+    const float* v_pool;
+    const int* block_table;
+    const int* row_seq;
+    const int* seq_start;
+    const int* seq_qlen;
+    const int* seq_pos0;
+    int table_width, page, nq, nkv, hd, q_stride, window;
+    float scale;
+};
+template <int HD>
+constexpr int prompt_smem() { return (PT_ROWS * (HD + 4) + 2 * PT_KEYS * (HD + 4) + 2 * PT_KEYS * HD + PT_ROWS * (PT_KEYS + 8)) * 4; }
+
+template <int HD>
+__global__ void __launch_bounds__(PT_THREADS) attention_prompt_kernel(const PromptArgs p) {
+    constexpr int LQ = HD + 4, LS = PT_KEYS + 8, CH = HD / 32;         // CH: groups of four channels per thread
+    extern __shared__ __align__(16) float pt[];
+    float* sq = pt;                                                    // [64][LQ]
+    float* sk = sq + PT_ROWS * LQ;                                     // [2][32][LQ]
+    float* sv = sk + 2 * PT_KEYS * LQ;                                 // [2][32][HD]
+    float* sp = sv + 2 * PT_KEYS * HD;                                 // [64][LS]
+    const int seq = blockIdx.z, kvh = blockIdx.y, group = p.nq / p.nkv, tokens = PT_ROWS / group;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, ty = lane >> 3, tx = lane & 7;
+    const int r0 = p.seq_start[seq], n = p.seq_qlen[seq], pos0 = p.seq_pos0[seq];
+    // the last tiles see the most keys: they start first
+    const int t0 = ((n + tokens - 1) / tokens - 1 - (int)blockIdx.x) * tokens;
+    fr_pdl_wait();
+    fr_pdl_launch();
+    if (t0 < 0 || n <= 0) return;
+    const int rows = min(tokens, n - t0) * group;
+    const bool ended = p.row_seq[r0] < 0;
+    const int last = pos0 + t0 + rows / group - 1, lo = p.window > 0 ? max(0, pos0 + t0 - p.window + 1) : 0;
+    const int steps = ended ? 0 : (last - lo) / PT_KEYS + 1;
+    const int* table = p.block_table + (size_t)seq * p.table_width;
+    auto copy = [&](float* dst, const float* src, bool there) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(there ? src : p.k_pool), "r"(there ? 16 : 0)
+                     : "memory");
+    };
+    auto fetch = [&](int step) {
+        float* dk = sk + (step & 1) * PT_KEYS * LQ;
+        float* dv = sv + (step & 1) * PT_KEYS * HD;
+        for (int idx = tid; idx < PT_KEYS * (HD / 4); idx += PT_THREADS) {
+            const int key = idx / (HD / 4), c = idx % (HD / 4) * 4, j = lo + step * PT_KEYS + key;
+            const bool there = j <= last && c < p.hd;
+            const int jj = min(j, last);
+            const size_t at = (((size_t)table[jj / p.page] * p.page + jj % p.page) * p.nkv + kvh) * p.hd + c;
+            copy(dk + key * LQ + c, p.k_pool + (there ? at : 0), there);
+            copy(dv + key * HD + c, p.v_pool + (there ? at : 0), there);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (steps > 0) fetch(0);
+    for (int idx = tid; idx < PT_ROWS * (HD / 4); idx += PT_THREADS) {
+        const int r = idx / (HD / 4), c = idx % (HD / 4) * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < rows && c < p.hd) v = *(const float4*)(p.q + (size_t)(r0 + t0 + r / group) * p.q_stride + (size_t)(kvh * group + r % group) * p.hd + c);
+        v.x *= p.scale; v.y *= p.scale; v.z *= p.scale; v.w *= p.scale;
+        *(float4*)(sq + r * LQ + c) = v;
+    }
+    // this thread's rows: row0 + 4 i (in shared memory four rows of a warp then lie in different banks)
+    const int row0 = warp * 16 + ty;
+    int pos[4];
+    float m[4], l[4], acc[4][4 * CH];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        pos[i] = pos0 + t0 + min(row0 + 4 * i, rows - 1) / group;
+        m[i] = -INFINITY;
+        l[i] = 0.f;
+#pragma unroll
+        for (int c = 0; c < 4 * CH; ++c) acc[i][c] = 0.f;
+    }
+    for (int step = 0; step < steps; ++step) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();                                               // this block of keys is here, and everyone is done with the one before
+        if (step + 1 < steps) fetch(step + 1);
+        const float* kb = sk + (step & 1) * PT_KEYS * LQ;
+        const float* vb = sv + (step & 1) * PT_KEYS * HD;
+        const int j0 = lo + step * PT_KEYS;
+        float s[4][4];                                                 // keys j0 + tx + 8 u
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) s[i][u] = 0.f;
+#pragma unroll 4
+        for (int d = 0; d < HD; d += 4) {
+            float4 a[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a[i] = *(const float4*)(sq + (row0 + 4 * i) * LQ + d);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const float4 b = *(const float4*)(kb + (tx + 8 * u) * LQ + d);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) s[i][u] = fmaf(a[i].x, b.x, fmaf(a[i].y, b.y, fmaf(a[i].z, b.z, fmaf(a[i].w, b.w, s[i][u]))));
+            }
+        }
+        // keys that some row of the tile does not see
+        const bool masked = j0 + PT_KEYS - 1 > pos0 + t0 || (p.window > 0 && j0 <= last - p.window);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (masked)
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int j = j0 + tx + 8 * u;
+                    if (j > pos[i] || (p.window > 0 && j <= pos[i] - p.window)) s[i][u] = -INFINITY;
+                }
+            float top = fmaxf(fmaxf(s[i][0], s[i][1]), fmaxf(s[i][2], s[i][3]));
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+            const float m_new = fmaxf(m[i], top), base = m_new == -INFINITY ? 0.f : m_new;      // (no key seen yet)
+            const float alpha = expf(m[i] - base);
+            float sum = 0.f;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const float e = expf(s[i][u] - base);
+                sum += e;
+                sp[(row0 + 4 * i) * LS + tx + 8 * u] = e;
+            }
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            l[i] = l[i] * alpha + sum;
+            m[i] = m_new;
+#pragma unroll
+            for (int c = 0; c < 4 * CH; ++c) acc[i][c] *= alpha;
+        }
+        __syncwarp();                                                  // a row's weights are its own warp's
+        auto add = [&](auto hidden) {
+#pragma unroll 2
+            for (int key = 0; key < PT_KEYS; key += 4) {
+                float4 w[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) w[i] = *(const float4*)(sp + (row0 + 4 * i) * LS + key);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+#pragma unroll
+                    for (int g = 0; g < CH; ++g) {
+                        const float4 v = *(const float4*)(vb + (key + u) * HD + 4 * tx + 32 * g);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const float e = u == 0 ? w[i].x : u == 1 ? w[i].y : u == 2 ? w[i].z : w[i].w;
+                            // (a key that the row does not see adds nothing, whatever its value is)
+                            if (decltype(hidden)::value == 0 || e != 0.f) {
+                                acc[i][4 * g] = fmaf(e, v.x, acc[i][4 * g]);
+                                acc[i][4 * g + 1] = fmaf(e, v.y, acc[i][4 * g + 1]);
+                                acc[i][4 * g + 2] = fmaf(e, v.z, acc[i][4 * g + 2]);
+                                acc[i][4 * g + 3] = fmaf(e, v.w, acc[i][4 * g + 3]);
+                            }
+                        }
+                    }
+                }
+            }
+        };
+        if (masked) add(Number<1>{});
+        else add(Number<0>{});
+        __syncwarp();
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = row0 + 4 * i;
+        if (r >= rows) continue;
+        const float inv = l[i] > 0.f ? 1.0f / l[i] : 0.f;
+        float* o = p.out + ((size_t)(r0 + t0 + r / group) * p.nq + kvh * group + r % group) * p.hd;
+#pragma unroll
+        for (int g = 0; g < CH; ++g) {
+            const int c = 4 * tx + 32 * g;
+            if (c < p.hd) *(float4*)(o + c) = make_float4(acc[i][4 * g] * inv, acc[i][4 * g + 1] * inv, acc[i][4 * g + 2] * inv, acc[i][4 * g + 3] * inv);
+        }
+    }
+}
+
+template <int HD>
+int launch_prompt(const PromptArgs& p, int n_seqs, int max_q_len, cudaStream_t stream) {
+    static std::atomic<unsigned long long> configured{0};     // devices (as bits) on which the limit has been raised
+    int device = 0;
+    FR_CUDA(cudaGetDevice(&device));
+    if (device < 0 || device >= 64) FR_REFUSE("attention: device %d is outside the table of 64", device);
+    if (!(configured.load(std::memory_order_acquire) & (1ull << device))) {
+        FR_CUDA(cudaFuncSetAttribute(attention_prompt_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, prompt_smem<HD>()));
+        configured.fetch_or(1ull << device, std::memory_order_release);
+    }
+    const int tokens = PT_ROWS / (p.nq / p.nkv);
+    FR_CUDA(fr_launch(attention_prompt_kernel<HD>, dim3((max_q_len + tokens - 1) / tokens, p.nkv, n_seqs), dim3(PT_THREADS), prompt_smem<HD>(), stream, p));
+    FR_CHECK_LAUNCH("attention (prompts)");
+    return FR_OK;
+}
+
 template <typename T>
 cudaError_t launch_attention(const AttnArgs& p, dim3 grid, cudaStream_t stream) {
     const int size = p.hd > p.vd ? p.hd : p.vd;
@@ -239,4 +436,25 @@ FR_EXPORT int attention_simt(const void* q, int q_stride, void* out, const void*
                              int splits, float* scratch, int dtype, cudaStream_t stream) {
     return attention_simt_masked(q, q_stride, out, k_pool, v_pool, block_table, table_width, page, row_seq, row_pos, rows, nq,
                                  nkv, hd, hd, window, 0, scale, 1.0f, splits, scratch, dtype, stream);
+}
+
+// Whether attention_simt_prompt takes these sizes (rows in 16-byte pieces, a kv head's query heads within a tile).
+FR_EXPORT int attention_simt_prompt_supports(const void* q, int q_stride, const void* out, const void* k_pool, const void* v_pool, int nq, int nkv,
+                                             int hd, int n_seqs) {
+    return hd > 0 && hd <= 128 && hd % 4 == 0 && nkv > 0 && nkv <= 65535 && nq % nkv == 0 && nq / nkv <= PT_ROWS && q_stride % 4 == 0 && n_seqs <= 65535 &&
+           (((uintptr_t)q | (uintptr_t)out | (uintptr_t)k_pool | (uintptr_t)v_pool) & 15) == 0;
+}
+
+// attention_simt for prompts in fp32: sequence s brings the rows seq_start[s] .. + seq_qlen[s] - 1 at positions from seq_pos0[s] on;
+// row_seq[seq_start[s]] < 0: it has ended (its rows become zeros).
+FR_EXPORT int attention_simt_prompt(const float* q, int q_stride, float* out, const float* k_pool, const float* v_pool, const int* block_table,
+                                    int table_width, int page, const int* row_seq, const int* seq_start, const int* seq_qlen, const int* seq_pos0,
+                                    int n_seqs, int max_q_len, int nq, int nkv, int hd, int window, float scale, cudaStream_t stream) {
+    if (n_seqs <= 0 || max_q_len <= 0) return FR_OK;
+    if (!attention_simt_prompt_supports(q, q_stride, out, k_pool, v_pool, nq, nkv, hd, n_seqs))
+        FR_REFUSE("attention (prompts): %d heads on %d of %d, stride %d", nq, nkv, hd, q_stride);
+    const PromptArgs p{q, out, k_pool, v_pool, block_table, row_seq, seq_start, seq_qlen, seq_pos0, table_width, page, nq, nkv, hd, q_stride, window, scale};
+    if (hd <= 32) return launch_prompt<32>(p, n_seqs, max_q_len, stream);
+    if (hd <= 64) return launch_prompt<64>(p, n_seqs, max_q_len, stream);
+    return launch_prompt<128>(p, n_seqs, max_q_len, stream);
 }

@@ -101,7 +101,8 @@ FAMILY(GemmSimt, gemm_simt, "gemm_simt", resolve(h, fam, "gemm_simt_weights", t.
 FAMILY(GemmTc, gemm_tc, "gemm_tc", resolve(h, fam, "gemm_tc_fused", t.fused); resolve(h, fam, "gemm_tc_plan", t.plan);
        resolve(h, fam, "gemm_tc_grouped", t.grouped);)
 FAMILY(AttentionSimt, attention_simt, "attention_simt", resolve(h, fam, "attention_simt", t.run);
-       resolve(h, fam, "attention_simt_masked", t.masked);)
+       resolve(h, fam, "attention_simt_masked", t.masked);
+       resolve(h, fam, "attention_simt_prompt_supports", t.prompt_supports); resolve(h, fam, "attention_simt_prompt", t.prompt);)
 FAMILY(AttentionWindow, attention_window, "attention_window", resolve(h, fam, "attention_window_fits", t.fits);
        resolve(h, fam, "attention_window", t.run);)
 FAMILY(Residual, residual, "residual", resolve(h, fam, "residual_norm_cast", t.norm_cast);

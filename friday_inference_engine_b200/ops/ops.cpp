@@ -1663,9 +1663,19 @@ void Ops::attention(const Tensor& q, int64_t q_stride, Tensor& out, const CacheV
              "attention_mma");
         return;
     }
+    const auto& k = kernels::attention_simt();
+    if (out.dtype == DType::F32 && geometry && !ctx.decode && ctx.max_q_len >= 16 && view.dtype == DType::F32 &&
+        k.prompt_supports(q.data, (int)q_stride, out.data, view.k_pool, view.v_pool, n_heads, n_kv_heads, head_dim, ctx.n_seqs)) {
+        Timed t(*this, Attention);
+        call(launches_, k,
+             k.prompt((const float*)q.data, (int)q_stride, (float*)out.data, (const float*)view.k_pool, (const float*)view.v_pool, view.block_table,
+                      view.table_width, view.page_size, ctx.row_seq, ctx.seq_start, ctx.seq_qlen, ctx.seq_pos0, ctx.n_seqs, ctx.max_q_len,
+                      n_heads, n_kv_heads, head_dim, window, scale, stream_),
+             "attention_simt_prompt");
+        return;
+    }
     const int splits = attention_splits(rows, n_heads, ctx.max_kv_len);
     float* scratch = splits > 1 ? scratch_floats((int64_t)rows * n_heads * splits * (head_dim + 2)) : nullptr;
-    const auto& k = kernels::attention_simt();
     Timed t(*this, Attention);
     call(launches_, k,
          k.run(q.data, (int)q_stride, out.data, view.k_pool, view.v_pool, view.block_table, view.table_width,
