@@ -128,6 +128,97 @@ __global__ void __launch_bounds__(256) conv_prepare_kernel(ConvArgs p) {
         out[2 * qk + d] = conv_at(p, x, p.v_off + d, 2 * qk + d, row, r0, hist, channels);
 }
 
+// The same for prompts: a warp takes a head, or 128 value channels, along CONV_RUN consecutive rows, four channels per lane, with the
+// taps and the rows before the present one in registers, so that an input is read once instead of once per tap.  Bound by
+// its bytes.
+constexpr int CONV_RUN = 16, CONV_RUN_TAPS = 4;
+template <typename T>
+__device__ __forceinline__ void load_four(const T* p, float (&v)[4]);
+template <>
+__device__ __forceinline__ void load_four<float>(const float* p, float (&v)[4]) {
+    const float4 a = *(const float4*)p;
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+}
+template <>
+__device__ __forceinline__ void load_four<bf16>(const bf16* p, float (&v)[4]) {
+    const uint2 a = *(const uint2*)p;
+    v[0] = __uint_as_float(a.x << 16); v[1] = __uint_as_float(a.x & 0xffff0000u);
+    v[2] = __uint_as_float(a.y << 16); v[3] = __uint_as_float(a.y & 0xffff0000u);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) conv_run_kernel(const ConvArgs p) {
+    fr_pdl_wait();
+    fr_pdl_launch();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int qk = p.qk_heads * p.dk, channels = 2 * qk + p.v_channels;
+    const int item = blockIdx.y * 8 + warp, items = 2 * p.qk_heads + (p.v_channels + 127) / 128;
+    if (item >= items) return;
+    const bool unit = item < 2 * p.qk_heads;
+    const int inside = 4 * lane, width = unit ? p.dk : min(128, p.v_channels - (item - 2 * p.qk_heads) * 128);
+    const bool live = inside < width;
+    const int c = (unit ? item * p.dk : 2 * qk + (item - 2 * p.qk_heads) * 128) + inside;       // channel in q|k|v order
+    const int src = c < qk ? p.q_off + c : c < 2 * qk ? p.k_off + (c - qk) : p.v_off + (c - 2 * qk);
+    const T* x = (const T*)p.x + src;
+    const int keep = p.taps - 1;                                                                // rows before the present one
+    const FrVec tw{p.taps_w, p.w_dtype};
+    float w[CONV_RUN_TAPS][4], past[CONV_RUN_TAPS - 1][4];                                      // past[b]: b + 1 rows before
+#pragma unroll
+    for (int b = 0; b < CONV_RUN_TAPS; ++b)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) w[b][e] = live && b <= keep ? tw.at((c + e) * p.taps + keep - b) : 0.f;
+    const int end = min(p.rows, (int)(blockIdx.x + 1) * CONV_RUN);
+    int seq = -1;
+    for (int row = blockIdx.x * CONV_RUN; row < end; ++row) {
+        const int of = p.row_seq[row];
+        if (of != seq && of >= 0) {                                                             // (the run's first row too)
+            const int r0 = p.seq_start[of];
+            const float* hist = p.state + (size_t)p.seq_slots[of] * p.state_stride + c;
+#pragma unroll
+            for (int b = 0; b < CONV_RUN_TAPS - 1; ++b) {
+                const int r = row - 1 - b;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) past[b][e] = 0.f;
+                if (live && b < keep) {
+                    if (r >= r0) load_four(x + (size_t)r * p.ld, past[b]);
+                    else {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) past[b][e] = hist[(size_t)(keep + (r - r0)) * channels + e];
+                    }
+                }
+            }
+        }
+        seq = of;
+        if (of < 0) continue;
+        float now[4] = {0.f, 0.f, 0.f, 0.f}, y[4];
+        if (live) load_four(x + (size_t)row * p.ld, now);
+        float ss = 0.f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            float acc = 0.f;
+#pragma unroll
+            for (int b = CONV_RUN_TAPS - 1; b > 0; --b) {
+                if (b <= keep) acc = fmaf(w[b][e], past[b - 1][e], acc);
+            }
+            acc = fmaf(w[0][e], now[e], acc);
+            y[e] = silu_f(acc);
+            ss = fmaf(y[e], y[e], ss);
+        }
+        if (unit) {
+            const float inv = (item < p.qk_heads ? p.q_scale : 1.0f) / sqrtf(fr_warp_sum(ss) + p.unit_eps);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) y[e] *= inv;
+        }
+        if (live) *(float4*)(p.out + (size_t)row * channels + c) = make_float4(y[0], y[1], y[2], y[3]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+#pragma unroll
+            for (int b = CONV_RUN_TAPS - 2; b > 0; --b) past[b][e] = past[b - 1][e];
+            past[0][e] = now[e];
+        }
+    }
+}
+
 // One block column per sequence: the history becomes the last taps-1 inputs of the sequence, this step's rows included.
 template <typename T>
 __global__ void __launch_bounds__(256) conv_state_kernel(ConvArgs p) {
@@ -424,6 +515,18 @@ FR_EXPORT int delta_conv_prepare(const void* x, int ld, int q_off, int k_off, in
                              nullptr, seq_slots, rows, qk_heads, dk, v_channels, taps, q_scale, unit_eps);
     if (rc != FR_OK) return rc;
     p.shift = shift_history && taps > 1 ? 1 : 0;
+    // prompts whose heads and rows lie in pieces of four channels: 16 rows per warp
+    const int piece = dtype == FR_F32 ? 16 : 8;
+    if (!p.shift && rows >= 4 * CONV_RUN && taps <= CONV_RUN_TAPS && dk <= 128 && dk % 4 == 0 && v_channels % 4 == 0 &&
+        ((q_off | k_off | v_off | ld) & 3) == 0 && (uintptr_t)x % piece == 0 && ((uintptr_t)out & 15) == 0 && (dtype == FR_F32 || dtype == FR_BF16)) {
+        const dim3 grid((rows + CONV_RUN - 1) / CONV_RUN, (2 * qk_heads + (v_channels + 127) / 128 + 7) / 8);
+        if (grid.y <= 65535) {
+            if (dtype == FR_F32) FR_CUDA(fr_launch(conv_run_kernel<float>, grid, dim3(256), 0, stream, p));
+            else FR_CUDA(fr_launch(conv_run_kernel<bf16>, grid, dim3(256), 0, stream, p));
+            FR_CHECK_LAUNCH("conv_prepare");
+            return FR_OK;
+        }
+    }
     int tiles = 1;
     if (rows < 128) {
         const int work = (2 * qk_heads + 7) / 8 + (v_channels + 255) / 256;      // rounds of a block's warps and threads

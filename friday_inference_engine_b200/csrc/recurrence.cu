@@ -321,6 +321,57 @@ __global__ void __launch_bounds__(128) head_norm_gate_kernel(NormGateArgs p) {
     }
 }
 
+// The same for heads of up to 128 channels in pieces of four: a head's channels are one load per lane and operand, all on their way
+// together.  Bound by its bytes.
+template <typename T>
+__device__ __forceinline__ void four_of(const T* p, float (&v)[4]);
+template <>
+__device__ __forceinline__ void four_of<float>(const float* p, float (&v)[4]) {
+    const float4 a = *(const float4*)p;
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+}
+template <>
+__device__ __forceinline__ void four_of<bf16>(const bf16* p, float (&v)[4]) {
+    const uint2 a = *(const uint2*)p;
+    v[0] = __uint_as_float(a.x << 16); v[1] = __uint_as_float(a.x & 0xffff0000u);
+    v[2] = __uint_as_float(a.y << 16); v[3] = __uint_as_float(a.y & 0xffff0000u);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) head_norm_gate_four_kernel(const NormGateArgs p) {
+    fr_pdl_wait();
+    fr_pdl_launch();
+    const int lane = threadIdx.x & 31;
+    const long long item = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (item >= (long long)p.rows * p.heads) return;
+    const int row = (int)(item / p.heads), head = (int)(item - (long long)row * p.heads), c = 4 * lane;
+    const bool live = c < p.dv;
+    const FrVec wv{p.weight, p.weight_dtype};
+    float o[4] = {0.f, 0.f, 0.f, 0.f}, g[4] = {0.f, 0.f, 0.f, 0.f}, w[4] = {0.f, 0.f, 0.f, 0.f};
+    if (live) {
+        four_of((const float*)p.o + (size_t)item * p.dv + c, o);
+        four_of((const T*)p.gate + (size_t)row * p.ld_gate + (size_t)head * p.dv + c, g);
+        wv.four(p.weight_per_head ? head * p.dv + c : c, w);
+    }
+    if (p.row_seq != nullptr && p.row_seq[row] < 0) return;
+    const float ss = fr_warp_sum(fmaf(o[0], o[0], fmaf(o[1], o[1], fmaf(o[2], o[2], o[3] * o[3]))));
+    const float inv = p.out_scale / sqrtf(ss / (float)p.dv + p.eps);
+    if (!live) return;
+    float y[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float sg = 1.0f / (1.0f + expf(-g[e]));
+        y[e] = o[e] * inv * w[e] * (p.gate_act == 1 ? sg : g[e] * sg);
+    }
+    T* out = (T*)p.out + (size_t)item * p.dv + c;
+    if (sizeof(T) == 4) {
+        *(float4*)out = make_float4(y[0], y[1], y[2], y[3]);
+    } else {
+        const __nv_bfloat162 a = __floats2bfloat162_rn(y[0], y[1]), b = __floats2bfloat162_rn(y[2], y[3]);
+        *(uint2*)out = make_uint2(*(const uint32_t*)&a, *(const uint32_t*)&b);
+    }
+}
+
 template <typename T, int DK>
 int launch_scan(const ScanArgs& p, int n_seqs, int splits, int threads, cudaStream_t stream) {
     const size_t smem = ((size_t)(3 * SCAN_TOKENS + 2) * DK + (size_t)SCAN_TOKENS * threads) * sizeof(float);
@@ -447,6 +498,15 @@ FR_EXPORT int recurrence_head_norm_gate(const float* o, const void* gate, int ld
     p.gate_act = gate_act;
     p.o = o; p.gate = gate; p.out = out; p.weight = weight; p.weight_dtype = weight_dtype; p.weight_per_head = weight_per_head;
     p.row_seq = row_seq; p.rows = rows; p.heads = heads; p.dv = dv; p.ld_gate = ld_gate; p.eps = eps; p.out_scale = out_scale;
+    const uintptr_t piece = dtype == FR_F32 ? 16 : 8;
+    if ((dtype == FR_F32 || dtype == FR_BF16) && dv <= 128 && dv % 4 == 0 && ld_gate % 4 == 0 && ((uintptr_t)o & 15) == 0 &&
+        (((uintptr_t)gate | (uintptr_t)out) & (piece - 1)) == 0) {
+        const dim3 grid((unsigned)(((long long)rows * heads + 7) / 8));
+        if (dtype == FR_F32) FR_CUDA(fr_launch(head_norm_gate_four_kernel<float>, grid, dim3(256), 0, stream, p));
+        else FR_CUDA(fr_launch(head_norm_gate_four_kernel<bf16>, grid, dim3(256), 0, stream, p));
+        FR_CHECK_LAUNCH("head_norm_gate");
+        return FR_OK;
+    }
     const int blocks = (rows * heads + 3) / 4;
     if (dtype == FR_F32) FR_CUDA(fr_launch(head_norm_gate_kernel<float>, dim3(blocks), dim3(128), 0, stream, p));
     else if (dtype == FR_BF16) FR_CUDA(fr_launch(head_norm_gate_kernel<bf16>, dim3(blocks), dim3(128), 0, stream, p));
