@@ -181,12 +181,13 @@ __global__ void __launch_bounds__(128) attention_kernel(AttnArgs p) {
     }
 }
 
-// Prompts in fp32.  The kernel above reads every key and value for every query row; here a block takes 64 rows, the query heads
-// of one kv head for as many consecutive tokens as that makes, and walks 32 keys at a time, which pass through shared memory once for
-// all of them.  128 threads: a thread has four rows' scores with four keys, then the same rows' results in HD / 8
-// channels, so that a row's scores, maximum and weights stay within a warp.  Bound by the multiply-adds (each needs an eighth of a
-// 16-byte read from shared memory).
-constexpr int PT_ROWS = 64, PT_KEYS = 32, PT_THREADS = 128;
+// Prompts in fp32.  The kernel above reads every key and value for every query row; here a block takes 16 RPT rows, the query
+// heads of one kv head for as many consecutive tokens as that makes, and walks 32 keys at a time, which pass through shared memory once
+// for all of them.  128 threads: a thread has RPT rows' scores with four keys, then the same rows' results in HD / 8
+// channels, so that a row's scores, maximum and weights stay within a warp.  Scores are summed 16 dimensions at a time, which keeps
+// their error that of the sums over lanes above.  Bound by the multiply-adds (each needs an eighth of a 16-byte read from shared
+// memory with four rows per thread) where blocks are many; two rows per thread where they are few.
+constexpr int PT_KEYS = 32, PT_THREADS = 128, PT_MOST_ROWS = 64;
 
 struct PromptArgs {
     const float* q;
@@ -201,17 +202,18 @@ struct PromptArgs {
     int table_width, page, nq, nkv, hd, q_stride, window;
     float scale;
 };
-template <int HD>
-constexpr int prompt_smem() { return (PT_ROWS * (HD + 4) + 2 * PT_KEYS * (HD + 4) + 2 * PT_KEYS * HD + PT_ROWS * (PT_KEYS + 8)) * 4; }
+template <int HD, int RPT>
+constexpr int prompt_smem() { return (16 * RPT * (HD + 4) + 2 * PT_KEYS * (HD + 4) + 2 * PT_KEYS * HD + 16 * RPT * (PT_KEYS + 8)) * 4; }
 
-template <int HD>
-__global__ void __launch_bounds__(PT_THREADS) attention_prompt_kernel(const PromptArgs p) {
+template <int HD, int RPT>
+__global__ void __launch_bounds__(PT_THREADS, 2) attention_prompt_kernel(const PromptArgs p) {
+    constexpr int PT_ROWS = 16 * RPT;
     constexpr int LQ = HD + 4, LS = PT_KEYS + 8, CH = HD / 32;         // CH: groups of four channels per thread
     extern __shared__ __align__(16) float pt[];
-    float* sq = pt;                                                    // [64][LQ]
+    float* sq = pt;                                                    // [PT_ROWS][LQ]
     float* sk = sq + PT_ROWS * LQ;                                     // [2][32][LQ]
     float* sv = sk + 2 * PT_KEYS * LQ;                                 // [2][32][HD]
-    float* sp = sv + 2 * PT_KEYS * HD;                                 // [64][LS]
+    float* sp = sv + 2 * PT_KEYS * HD;                                 // [PT_ROWS][LS]
     const int seq = blockIdx.z, kvh = blockIdx.y, group = p.nq / p.nkv, tokens = PT_ROWS / group;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, ty = lane >> 3, tx = lane & 7;
     const int r0 = p.seq_start[seq], n = p.seq_qlen[seq], pos0 = p.seq_pos0[seq];
@@ -251,11 +253,11 @@ __global__ void __launch_bounds__(PT_THREADS) attention_prompt_kernel(const Prom
         *(float4*)(sq + r * LQ + c) = v;
     }
     // this thread's rows: row0 + 4 i (in shared memory four rows of a warp then lie in different banks)
-    const int row0 = warp * 16 + ty;
-    int pos[4];
-    float m[4], l[4], acc[4][4 * CH];
+    const int row0 = warp * 4 * RPT + ty;
+    int pos[RPT];
+    float m[RPT], l[RPT], acc[RPT][4 * CH];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < RPT; ++i) {
         pos[i] = pos0 + t0 + min(row0 + 4 * i, rows - 1) / group;
         m[i] = -INFINITY;
         l[i] = 0.f;
@@ -269,27 +271,38 @@ __global__ void __launch_bounds__(PT_THREADS) attention_prompt_kernel(const Prom
         const float* kb = sk + (step & 1) * PT_KEYS * LQ;
         const float* vb = sv + (step & 1) * PT_KEYS * HD;
         const int j0 = lo + step * PT_KEYS;
-        float s[4][4];                                                 // keys j0 + tx + 8 u
+        float s[RPT][4];                                               // keys j0 + tx + 8 u
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < RPT; ++i)
 #pragma unroll
             for (int u = 0; u < 4; ++u) s[i][u] = 0.f;
-#pragma unroll 4
-        for (int d = 0; d < HD; d += 4) {
-            float4 a[4];
+#pragma unroll 1
+        for (int d0 = 0; d0 < HD; d0 += 16) {
+            float part[RPT][4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = *(const float4*)(sq + (row0 + 4 * i) * LQ + d);
+            for (int d = d0; d < d0 + 16; d += 4) {
+                float4 a[RPT];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const float4 b = *(const float4*)(kb + (tx + 8 * u) * LQ + d);
+                for (int i = 0; i < RPT; ++i) a[i] = *(const float4*)(sq + (row0 + 4 * i) * LQ + d);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) s[i][u] = fmaf(a[i].x, b.x, fmaf(a[i].y, b.y, fmaf(a[i].z, b.z, fmaf(a[i].w, b.w, s[i][u]))));
+                for (int u = 0; u < 4; ++u) {
+                    const float4 b = *(const float4*)(kb + (tx + 8 * u) * LQ + d);
+#pragma unroll
+                    for (int i = 0; i < RPT; ++i) {
+                        const float first = d == d0 ? a[i].w * b.w : fmaf(a[i].w, b.w, part[i][u]);
+                        part[i][u] = fmaf(a[i].x, b.x, fmaf(a[i].y, b.y, fmaf(a[i].z, b.z, first)));
+                    }
+                }
             }
+#pragma unroll
+            for (int i = 0; i < RPT; ++i)
+#pragma unroll
+                for (int u = 0; u < 4; ++u) s[i][u] += part[i][u];
         }
         // keys that some row of the tile does not see
         const bool masked = j0 + PT_KEYS - 1 > pos0 + t0 || (p.window > 0 && j0 <= last - p.window);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < RPT; ++i) {
             if (masked)
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
@@ -319,16 +332,16 @@ __global__ void __launch_bounds__(PT_THREADS) attention_prompt_kernel(const Prom
         auto add = [&](auto hidden) {
 #pragma unroll 2
             for (int key = 0; key < PT_KEYS; key += 4) {
-                float4 w[4];
+                float4 w[RPT];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) w[i] = *(const float4*)(sp + (row0 + 4 * i) * LS + key);
+                for (int i = 0; i < RPT; ++i) w[i] = *(const float4*)(sp + (row0 + 4 * i) * LS + key);
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
 #pragma unroll
                     for (int g = 0; g < CH; ++g) {
                         const float4 v = *(const float4*)(vb + (key + u) * HD + 4 * tx + 32 * g);
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) {
+                        for (int i = 0; i < RPT; ++i) {
                             const float e = u == 0 ? w[i].x : u == 1 ? w[i].y : u == 2 ? w[i].z : w[i].w;
                             // (a key that the row does not see adds nothing, whatever its value is)
                             if (decltype(hidden)::value == 0 || e != 0.f) {
@@ -347,7 +360,7 @@ __global__ void __launch_bounds__(PT_THREADS) attention_prompt_kernel(const Prom
         __syncwarp();
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < RPT; ++i) {
         const int r = row0 + 4 * i;
         if (r >= rows) continue;
         const float inv = l[i] > 0.f ? 1.0f / l[i] : 0.f;
@@ -360,20 +373,29 @@ __global__ void __launch_bounds__(PT_THREADS) attention_prompt_kernel(const Prom
     }
 }
 
-template <int HD>
-int launch_prompt(const PromptArgs& p, int n_seqs, int max_q_len, cudaStream_t stream) {
+template <int HD, int RPT>
+int launch_prompt_tiles(const PromptArgs& p, int n_seqs, int max_q_len, cudaStream_t stream) {
     static std::atomic<unsigned long long> configured{0};     // devices (as bits) on which the limit has been raised
     int device = 0;
     FR_CUDA(cudaGetDevice(&device));
     if (device < 0 || device >= 64) FR_REFUSE("attention: device %d is outside the table of 64", device);
     if (!(configured.load(std::memory_order_acquire) & (1ull << device))) {
-        FR_CUDA(cudaFuncSetAttribute(attention_prompt_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, prompt_smem<HD>()));
+        FR_CUDA(cudaFuncSetAttribute(attention_prompt_kernel<HD, RPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, prompt_smem<HD, RPT>()));
         configured.fetch_or(1ull << device, std::memory_order_release);
     }
-    const int tokens = PT_ROWS / (p.nq / p.nkv);
-    FR_CUDA(fr_launch(attention_prompt_kernel<HD>, dim3((max_q_len + tokens - 1) / tokens, p.nkv, n_seqs), dim3(PT_THREADS), prompt_smem<HD>(), stream, p));
+    const int tokens = 16 * RPT / (p.nq / p.nkv);
+    FR_CUDA(fr_launch(attention_prompt_kernel<HD, RPT>, dim3((max_q_len + tokens - 1) / tokens, p.nkv, n_seqs), dim3(PT_THREADS), prompt_smem<HD, RPT>(), stream, p));
     FR_CHECK_LAUNCH("attention (prompts)");
     return FR_OK;
+}
+
+// Tiles of 64 rows would leave SMs with fewer than two blocks: 32 rows, where the query heads of a kv head fit them.
+template <int HD>
+int launch_prompt(const PromptArgs& p, int n_seqs, int max_q_len, cudaStream_t stream) {
+    const int sms = fr_sm_count() > 0 ? fr_sm_count() : 148, group = p.nq / p.nkv, tokens = PT_MOST_ROWS / group;
+    const long long tiles = (long long)((max_q_len + tokens - 1) / tokens) * p.nkv * n_seqs;
+    if (group <= 32 && tiles < 4ll * sms) return launch_prompt_tiles<HD, 2>(p, n_seqs, max_q_len, stream);
+    return launch_prompt_tiles<HD, 4>(p, n_seqs, max_q_len, stream);
 }
 
 template <typename T>
@@ -441,7 +463,7 @@ FR_EXPORT int attention_simt(const void* q, int q_stride, void* out, const void*
 // Whether attention_simt_prompt takes these sizes (rows in 16-byte pieces, a kv head's query heads within a tile).
 FR_EXPORT int attention_simt_prompt_supports(const void* q, int q_stride, const void* out, const void* k_pool, const void* v_pool, int nq, int nkv,
                                              int hd, int n_seqs) {
-    return hd > 0 && hd <= 128 && hd % 4 == 0 && nkv > 0 && nkv <= 65535 && nq % nkv == 0 && nq / nkv <= PT_ROWS && q_stride % 4 == 0 && n_seqs <= 65535 &&
+    return hd > 0 && hd <= 128 && hd % 4 == 0 && nkv > 0 && nkv <= 65535 && nq % nkv == 0 && nq / nkv <= PT_MOST_ROWS && q_stride % 4 == 0 && n_seqs <= 65535 &&
            (((uintptr_t)q | (uintptr_t)out | (uintptr_t)k_pool | (uintptr_t)v_pool) & 15) == 0;
 }
 

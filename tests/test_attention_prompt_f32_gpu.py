@@ -56,7 +56,8 @@ class Case:
 
 
 @pytest.mark.parametrize("lens,pos0,nq,nkv,hd,window", [([9, 1, 70], [0, 5, 0], 28, 4, 128, 0), ([65, 33], [0, 0], 3, 1, 32, 24), ([100, 7], [5, 64], 6, 3, 20, 9),
-                                                        ([130], [70], 64, 1, 96, 0), ([40, 40], [0, 31], 2, 2, 64, 1), ([300], [0], 8, 4, 4, 100)])
+                                                        ([130], [70], 64, 1, 96, 0), ([40, 40], [0, 31], 2, 2, 64, 1), ([300], [0], 8, 4, 4, 100),
+                                                        ([70] * 10, [0] * 10, 64, 64, 36, 24)])
 @pytest.mark.parametrize("page", [64, 16])
 def test_prompt(lens, pos0, nq, nkv, hd, window, page):
     c = Case(lens, pos0, nq, nkv, hd, window, page)
