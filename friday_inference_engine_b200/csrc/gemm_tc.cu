@@ -404,21 +404,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
                                                    (size_t)p_blk * TILE_P + (idx & 15) * 8));
             }
         };
-        // the cosines and sines of rows t_lo .. t_lo + t_cnt - 1 of the tile (s_seq and s_pos were filled when it was taken); wider
-        // tiles hold those of one chunk of 16 rows at a time
-        int turned = -1;                                     // which chunk that is
-        auto make_turns = [&](int t_lo, int t_cnt) {
-            const int half = f.rot >> 1;
-            for (int idx = et; idx < t_cnt * half; idx += 128) {
-                const int t = idx / half, i = idx - t * half;
-                float sn = 0.f, cs = 1.f;
-                if (s_seq[t_lo + t] >= 0) sincosf(__fdiv_rn((float)s_pos[t_lo + t], s_den[i]), &sn, &cs);
-                s_cs[t * 64 + i] = make_float2(cs, sn);
-            }
-        };
-        // r_lo, r_cnt: the rows of the tile whose residual pieces this CTA will need first (16-wide tiles); chunk: the 16 rows that it will
-        // finish first (wider ones), whose angles are made while the products run
-        auto prefetch_tile = [&](int p_blk, int q_blk, int r_lo, int r_cnt, int chunk) {
+        // r_lo, r_cnt: the rows of the tile whose residual pieces this CTA will need first (16-wide tiles)
+        auto prefetch_tile = [&](int p_blk, int q_blk, int r_lo, int r_cnt) {
             const int nt = min(bn, p.q_rows - q_blk * bn);
             s_bias[et] = p.bias != nullptr ? bias_at(p, p_blk * TILE_P + et) : 0.f;
             if (f.norm_out != nullptr)
@@ -438,13 +425,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
                 s_crow[et] = crow;
             }
             asm volatile("bar.sync 1, 128;" ::: "memory");
-            turned = -1;
-            if (rope && f.denom != nullptr) {
-                if (BN == 16) {
-                    make_turns(0, nt);
-                } else if (chunk * 16 < nt) {
-                    make_turns(chunk * 16, min(16, nt - chunk * 16));
-                    turned = chunk;
+            if (BN == 16 && rope && f.denom != nullptr) {       // wider tiles make them 16 rows at a time, when they finish them
+                const int half = f.rot >> 1;
+                for (int idx = et; idx < nt * half; idx += 128) {
+                    const int token = idx / half, i = idx - token * half;
+                    float sn = 0.f, cs = 1.f;
+                    if (s_seq[token] >= 0) sincosf(__fdiv_rn((float)s_pos[token], s_den[i]), &sn, &cs);
+                    s_cs[token * 64 + i] = make_float2(cs, sn);
                 }
             }
         };
@@ -655,9 +642,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
                     asm volatile("bar.sync 1, 128;" ::: "memory");
                     if (et == 0) mark(p, 11);
                 }
-                if (BN > 16 && rope && f.denom != nullptr && c != turned) {
-                    make_turns(c * 16, t_cnt);
-                    turned = c;
+                if (BN > 16 && rope && f.denom != nullptr) {
+                    // the cosines and sines of these 16 rows (s_seq and s_pos were filled when the tile was taken)
+                    const int half = f.rot >> 1;
+                    for (int idx = et; idx < t_cnt * half; idx += 128) {
+                        const int t = idx / half, i = idx - t * half;
+                        float sn = 0.f, cs = 1.f;
+                        if (s_seq[c * 16 + t] >= 0) sincosf(__fdiv_rn((float)s_pos[c * 16 + t], s_den[i]), &sn, &cs);
+                        s_cs[t * 64 + i] = make_float2(cs, sn);
+                    }
                     asm volatile("bar.sync 1, 128;" ::: "memory");
                 }
                 finish_rows(p_blk, q_blk, c * 16, t_cnt);
@@ -709,8 +702,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
             const bool staged = can_stage && (p_blk + 1) * TILE_P <= p.p_rows;
             load_scale(p.swapped ? q_blk : p_blk);
             const bool quarters = BN == 16 && p.shared_finish && item.nseg > 1;      // this CTA finishes a share of the rows
-            if (staged) prefetch_tile(p_blk, q_blk, quarters ? 4 * (item.part - tile * p.splits) : 0, quarters ? 4 : bn,
-                                      p.shared_finish && item.nseg > 1 ? item.part - tile * p.splits : 0);
+            if (staged) prefetch_tile(p_blk, q_blk, quarters ? 4 * (item.part - tile * p.splits) : 0, quarters ? 4 : bn);
             float ss_row = 0.f;                            // rows-on-M with a norm begun: this row's sum of squares over the tile
             if (norm_rows) {
                 asm volatile("bar.sync 1, 128;" ::: "memory");
