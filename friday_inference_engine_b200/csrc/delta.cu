@@ -583,23 +583,31 @@ FR_EXPORT int delta_scan(const float* qkv, const void* a_raw, int ld_a, const vo
     FR_REFUSE("delta scan: unknown dtype %d", raw_dtype);
 }
 
-// Whether delta_scan_chunks takes these sizes (rows in 16-byte pieces, a head's keys within a chunk's tile).
-FR_EXPORT int delta_scan_chunks_supports(const float* qkv, int dk, int dv) {
-    return dk > 0 && dk <= CD && dk % 4 == 0 && dv > 0 && dv % 4 == 0 && ((uintptr_t)qkv & 15) == 0;
+// Bytes of scratch that delta_scan_chunks needs; 0: it does not take these sizes (rows in 16-byte pieces, a head's keys within a
+// chunk's tile).
+FR_EXPORT long long delta_scan_chunks_scratch(const float* qkv, int rows, int n_seqs, int heads, int dk, int dv) {
+    if (dk <= 0 || dk > CD || dk % 4 || dv <= 0 || dv % 4 || ((uintptr_t)qkv & 15) || rows <= 0 || n_seqs <= 0 || n_seqs > 65535 || heads <= 0 || heads > 65535) return 0;
+    return chunk_head_bytes(rows, n_seqs, dv) * chunk_heads(rows, n_seqs, heads, dv);
 }
 
-// delta_scan for prompts: the same arguments and results, sixteen tokens at a time (delta_chunks.cuh).
+// delta_scan for prompts: the same arguments and results, sixteen tokens at a time (delta_chunks.cuh).  rows: of the whole step,
+// whose sequences' rows lie one sequence after another from row 0 on; max_q_len: of the longest sequence; scratch: 16-byte aligned.
 FR_EXPORT int delta_scan_chunks(const float* qkv, const void* a_raw, int ld_a, const void* b_raw, int ld_b, int raw_dtype, const void* a_log,
                                 const void* dt_bias, int vec_dtype, float* out, float* state, long long state_stride, long long s_off,
                                 const int* row_seq, const int* seq_start, const int* seq_qlen, const int* seq_slots, int n_seqs, int heads,
-                                int qk_heads, int dk, int dv, int per_channel, cudaStream_t stream) {
-    if (n_seqs <= 0) return FR_OK;
-    if (heads <= 0 || qk_heads <= 0 || heads % qk_heads || !delta_scan_chunks_supports(qkv, dk, dv))
-        FR_REFUSE("delta chunks: %d heads on %d query/key heads, dk %d, dv %d", heads, qk_heads, dk, dv);
+                                int qk_heads, int dk, int dv, int per_channel, int rows, int max_q_len, void* scratch, long long scratch_bytes,
+                                cudaStream_t stream) {
+    if (n_seqs <= 0 || rows <= 0 || max_q_len <= 0) return FR_OK;
+    if (heads <= 0 || qk_heads <= 0 || heads % qk_heads) FR_REFUSE("delta chunks: %d heads on %d query/key heads", heads, qk_heads);
+    const long long need = delta_scan_chunks_scratch(qkv, rows, n_seqs, heads, dk, dv);
+    if (need == 0 || scratch_bytes < need || ((uintptr_t)scratch & 15))
+        FR_REFUSE("delta chunks: dk %d, dv %d, %lld bytes of scratch for %lld", dk, dv, scratch_bytes, need);
     const ScanArgs p{qkv, a_raw, b_raw, raw_dtype, a_log, dt_bias, vec_dtype, out, state, state_stride, s_off, row_seq, seq_start, seq_qlen,
                      seq_slots, ld_a, ld_b, heads, qk_heads, dk, dv, 0, per_channel ? 1 : 0};
-    if (raw_dtype == FR_F32) return per_channel ? launch_chunks<float, true>(p, n_seqs, stream) : launch_chunks<float, false>(p, n_seqs, stream);
-    if (raw_dtype == FR_BF16) return per_channel ? launch_chunks<bf16, true>(p, n_seqs, stream) : launch_chunks<bf16, false>(p, n_seqs, stream);
+    if (raw_dtype == FR_F32)
+        return per_channel ? launch_chunks<float, true>(p, rows, n_seqs, max_q_len, scratch, stream) : launch_chunks<float, false>(p, rows, n_seqs, max_q_len, scratch, stream);
+    if (raw_dtype == FR_BF16)
+        return per_channel ? launch_chunks<bf16, true>(p, rows, n_seqs, max_q_len, scratch, stream) : launch_chunks<bf16, false>(p, rows, n_seqs, max_q_len, scratch, stream);
     FR_REFUSE("delta chunks: unknown dtype %d", raw_dtype);
 }
 

@@ -13,13 +13,15 @@
 // The walk along a sequence is then three small products per chunk instead of sixteen tokens' chains of sums.  Ratios of decays
 // are running products, never quotients or differences of logarithms.
 //
-// A block owns one head of one sequence and 64 value channels.  Eight warps prepare a chunk (A, B, the triangular solution by
-// forward substitution, a thread per channel; fp32) while four warps, 16 value channels each, walk the chunk before it on the
-// tensor cores (mma.sync.m16n8k16): a warp keeps its channels' transposed state, fp32, in the layout of the instruction's
+// Two kernels.  The first prepares every chunk of every head (A, B, the triangular solution by forward substitution, a thread per
+// channel; fp32), all of them at a time.  The second walks the chunks: a block owns one head of one sequence and 64 value
+// channels; four warps fetch the prepared operands two chunks ahead, four warps, 16 value channels each, multiply on the tensor
+// cores (mma.sync.m16n8k16): a warp keeps its channels' transposed state, fp32, in the layout of the instruction's
 // accumulators, which is also that of its first operand, so that nothing but the prepared operands passes through shared memory.
 // Every operand is three bf16 numbers (hi + mid + lo, all 24 bits) and a product the six partial products that reach
-// 2^-18 of it; hi hi has an accumulator of its own, the state's decay and sum are fp32 multiply-adds, so that the errors stay
-// those of fp32 sums.
+// 2^-18 of it; hi hi has an accumulator of its own, whose sums over 32 key channels are added in fp32 registers, the state's decay and
+// sum are fp32 multiply-adds, so that the errors stay those of fp32 sums.  (Prepared by the walking block itself, a chunk took
+// as long as its preparation, 8,500 cycles.)
 #pragma once
 #include "mma_sync.cuh"
 
@@ -29,24 +31,36 @@ constexpr int CT = 16;               // tokens per chunk
 constexpr int CD = 128;              // key channels (zeros beyond dk)
 constexpr int CV = 64;               // value channels per block
 constexpr int CLD = CD + 8;          // bf16 numbers per row: eight rows' 16-byte pieces lie in different banks
-constexpr int CHAIN_THREADS = 128, PREP_THREADS = 256, CHUNK_THREADS = CHAIN_THREADS + PREP_THREADS;
+constexpr int WALK_THREADS = 128, FETCH_THREADS = 128, PREP_THREADS = 256;
+constexpr int CHUNK_STAGES = 3;      // prepared chunks in a walking block's shared memory
 
-struct ChunkOperands {               // a prepared chunk
+struct ChunkOperands {               // a prepared chunk of one head
     bf16 w[3][CT][CLD], q[3][CT][CLD], k[3][CT][CLD];
     bf16 b[3][CT][CT + 8];
-    float u0[CT][CV + 4];
     float gamma[CD];
 };
-struct ChunkRaw {                    // its rows as they come
-    float q[CT][CD], k[CT][CD], v[CT][CV];
-};
-struct ChunkShared {
-    ChunkOperands ops[2];
-    ChunkRaw raw[2];
-    float g[CT][CD];                 // decays
+typedef float ChunkValues[CT][CV + 4];                       // U0 of 64 value channels
+struct PrepShared {
+    ChunkOperands ops;
+    float q[CT][CD], k[CT][CD];      // its rows as they come
+    float g[CT][CD];                 // decays (one per token in the first row where a head has one)
     float a[CT][CT];
     float beta[CT];
 };
+struct WalkShared {
+    ChunkOperands ops[CHUNK_STAGES];
+    ChunkValues u0[CHUNK_STAGES];
+};
+static_assert(sizeof(ChunkOperands) % 16 == 0 && sizeof(ChunkValues) % 16 == 0, "copied in 16-byte pieces");
+
+struct ChunkArgs {
+    ScanArgs s;
+    ChunkOperands* ops;              // [slots][heads of this call]
+    ChunkValues* u0;                 // [slots][heads of this call][value_blocks]
+    int head0, heads, value_blocks;  // the heads of this call
+};
+// Sequences' chunks lie one after another: a sequence's first row is no multiple of 16, so each may leave one slot empty.
+__device__ __forceinline__ long long chunk_slot(int r0, int seq, int c) { return r0 / CT + seq + c; }
 
 __device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
     hi = pack2(x, y);
@@ -64,174 +78,196 @@ __device__ __forceinline__ void split3(float x, bf16& hi, bf16& mid, bf16& lo) {
     x -= __bfloat162float(mid);
     lo = __float2bfloat16_rn(x);
 }
-// large += a_hi b_hi; small += the five others that count
-__device__ __forceinline__ void mma_split(float (&large)[4], float (&small)[4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][4], int tile) {
-    mma_16816(large, a[0], b[0][2 * tile], b[0][2 * tile + 1]);
-    mma_16816(small, a[0], b[2][2 * tile], b[2][2 * tile + 1]);
-    mma_16816(small, a[2], b[0][2 * tile], b[0][2 * tile + 1]);
-    mma_16816(small, a[1], b[1][2 * tile], b[1][2 * tile + 1]);
-    mma_16816(small, a[0], b[1][2 * tile], b[1][2 * tile + 1]);
-    mma_16816(small, a[1], b[0][2 * tile], b[0][2 * tile + 1]);
+// Tiles' products a b, b of tile i in b[i / 2], columns of place i % 2: large += hi hi; small += the five others that count.  Tile after
+// tile, so that an instruction does not wait for the one before it.
+template <int TILES>
+__device__ __forceinline__ void mma_split(float (&large)[TILES][4], float (&small)[TILES][4], const uint32_t (&a)[3][4], const uint32_t (&b)[TILES / 2][3][4]) {
+    constexpr int PA[6] = {0, 0, 2, 1, 0, 1}, PB[6] = {0, 2, 0, 1, 1, 0};
+#pragma unroll
+    for (int x = 0; x < 6; ++x)
+#pragma unroll
+        for (int i = 0; i < TILES; ++i) {
+            const uint32_t(&bt)[4] = b[i / 2][PB[x]];
+            mma_16816(x == 0 ? large[i] : small[i], a[PA[x]], bt[2 * (i % 2)], bt[2 * (i % 2) + 1]);
+        }
 }
-template <int ID, int THREADS>
-__device__ __forceinline__ void named_sync() { asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(THREADS) : "memory"); }
-__device__ __forceinline__ void chunk_bar_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(CHUNK_THREADS) : "memory"); }
-__device__ __forceinline__ void chunk_bar_arrive(int id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(CHUNK_THREADS) : "memory"); }
-constexpr int BAR_PREP = 1, BAR_FULL = 2, BAR_EMPTY = 4;      // full and empty: one per buffer
+template <int N>
+__device__ __forceinline__ void clear(float (&v)[N][4]) {
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[i][e] = 0.f;
+}
+template <int N>
+__device__ __forceinline__ void add_to(float (&sum)[N][4], const float (&v)[N][4]) {
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sum[i][e] += v[i][e];
+}
+__device__ __forceinline__ void walk_bar_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(WALK_THREADS + FETCH_THREADS) : "memory"); }
+__device__ __forceinline__ void walk_bar_arrive(int id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(WALK_THREADS + FETCH_THREADS) : "memory"); }
+constexpr int BAR_FULL = 1, BAR_EMPTY = 1 + CHUNK_STAGES;     // one of each per stage
 
 template <typename TR, bool PER_CHANNEL>
-__device__ __forceinline__ void prepare_chunks(const ScanArgs& p, ChunkShared& sm, int r0, int n, int head, int col0) {
-    const int who = threadIdx.x - CHAIN_THREADS, warp = who >> 5, lane = who & 31;
+__global__ void __launch_bounds__(PREP_THREADS, 3) delta_prepare_chunks_kernel(const ChunkArgs args) {
+    extern __shared__ __align__(16) unsigned char chunk_smem[];
+    PrepShared& sm = *(PrepShared*)chunk_smem;
+    const ScanArgs& p = args.s;
+    const int c = blockIdx.x, head = args.head0 + blockIdx.y, seq = blockIdx.z;
+    const int who = threadIdx.x, warp = who >> 5, lane = who & 31;
+    const int r0 = p.seq_start[seq], n = p.seq_qlen[seq];
+    fr_pdl_wait();
+    fr_pdl_launch();
+    const int t0 = c * CT, nt = min(CT, n - t0);
+    if (nt <= 0 || p.row_seq[r0] < 0) return;
     const int group = head / (p.heads / p.qk_heads);
     const int qk = p.qk_heads * p.dk, channels = 2 * qk + p.heads * p.dv;
+    const size_t at = (size_t)chunk_slot(r0, seq, c) * args.heads + blockIdx.y;
     const FrVec alog{p.a_log, p.vec_dtype}, dtb{p.dt_bias, p.vec_dtype};
     const float rate = expf(alog.at(head));
-    const int chunks = (n + CT - 1) / CT;
-    constexpr int GZ = PER_CHANNEL ? CT * CD / PREP_THREADS : 1;
-    float gz[GZ], zb = 0.f;
-    // rows of chunk c: q, k, v into shared memory, raw decays and betas into registers
-    auto fetch = [&](int c) {
-        const int t0 = c * CT, nt = min(CT, n - t0);
-        ChunkRaw& raw = sm.raw[c & 1];
-        auto copy = [&](float* dst, const float* src, bool there) {
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(there ? src : p.qkv), "r"(there ? 16 : 0)
-                         : "memory");
-        };
+    ChunkOperands& o = sm.ops;
+    // rows (a token beyond the sequence: no decay, no key, no correction)
 #pragma unroll
-        for (int it = 0; it < CT * CD / 4 / PREP_THREADS; ++it) {
-            const int idx = who + it * PREP_THREADS, t = idx / (CD / 4), i = idx % (CD / 4) * 4;
-            const bool there = t < nt && i < p.dk;
-            const float* row = p.qkv + (size_t)(r0 + t0 + (there ? t : 0)) * channels + group * p.dk + i;
-            copy(&raw.q[t][i], row, there);
-            copy(&raw.k[t][i], row + qk, there);
+    for (int it = 0; it < CT * CD / 4 / PREP_THREADS; ++it) {
+        const int idx = who + it * PREP_THREADS, t = idx / (CD / 4), i = idx % (CD / 4) * 4;
+        float4 q4 = make_float4(0.f, 0.f, 0.f, 0.f), k4 = q4;
+        if (t < nt && i < p.dk) {
+            const float* row = p.qkv + (size_t)(r0 + t0 + t) * channels + group * p.dk + i;
+            q4 = *(const float4*)row;
+            k4 = *(const float4*)(row + qk);
         }
-        static_assert(CT * CV / 4 == PREP_THREADS, "a piece of the values per thread");
-        const int t = who / (CV / 4), j = who % (CV / 4) * 4;
-        const bool there = t < nt && col0 + j < p.dv;
-        copy(&raw.v[t][j], p.qkv + (size_t)(r0 + t0 + (there ? t : 0)) * channels + 2 * qk + head * p.dv + col0 + (there ? j : 0), there);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        if (PER_CHANNEL) {
+        *(float4*)&sm.q[t][i] = q4;
+        *(float4*)&sm.k[t][i] = k4;
+    }
+    if (PER_CHANNEL) {
 #pragma unroll
-            for (int it = 0; it < GZ; ++it) {
-                const int idx = who + it * PREP_THREADS, tt = idx / CD, i = idx % CD;
-                gz[it] = tt < nt && i < p.dk ? raw_at<TR>(p.a_raw, (size_t)(r0 + t0 + tt) * p.ld_a + head * p.dk + i) : 0.f;
-            }
-        } else {
-            gz[0] = who < nt ? raw_at<TR>(p.a_raw, (size_t)(r0 + t0 + who) * p.ld_a + head) : 0.f;
+        for (int it = 0; it < CT * CD / PREP_THREADS; ++it) {
+            const int idx = who + it * PREP_THREADS, t = idx / CD, i = idx % CD;
+            sm.g[t][i] = t < nt && i < p.dk ? expf(-rate * softplus_f(raw_at<TR>(p.a_raw, (size_t)(r0 + t0 + t) * p.ld_a + head * p.dk + i) + dtb.at(head * p.dk + i))) : 1.f;
         }
-        zb = who < nt ? raw_at<TR>(p.b_raw, (size_t)(r0 + t0 + who) * p.ld_b + head) : 0.f;
-    };
-    fetch(0);
-    for (int c = 0; c < chunks; ++c) {
-        const int nt = min(CT, n - c * CT), buf = c & 1;
-        const ChunkRaw& raw = sm.raw[buf];
-        ChunkOperands& o = sm.ops[buf];
-        // decays and betas (a token beyond the sequence: no decay, no key, no correction)
-        if (PER_CHANNEL) {
+    } else if (who < CT) {
+        sm.g[0][who] = who < nt ? expf(-rate * softplus_f(raw_at<TR>(p.a_raw, (size_t)(r0 + t0 + who) * p.ld_a + head) + dtb.at(head))) : 1.f;
+    }
+    if (who < CT) sm.beta[who] = who < nt ? 1.0f / (1.0f + expf(-raw_at<TR>(p.b_raw, (size_t)(r0 + t0 + who) * p.ld_b + head))) : 0.f;
+    __syncthreads();
+    // A and B, a column s per warp and turn: the key of token s as the tokens after it see it
+#pragma unroll 1
+    for (int turn = 0; turn < 2; ++turn) {
+        const int s = turn == 0 ? warp : CT - 1 - warp;
+        float val[32];                                        // A_ts of t = 0 .. 15, then B_ts
+        float4 x = *(const float4*)&sm.k[s][4 * lane];
 #pragma unroll
-            for (int it = 0; it < GZ; ++it) {
-                const int idx = who + it * PREP_THREADS, t = idx / CD, i = idx % CD;
-                sm.g[t][i] = t < nt && i < p.dk ? expf(-rate * softplus_f(gz[it] + dtb.at(head * p.dk + i))) : 1.f;
-            }
-        } else if (who < CT) {
-            sm.g[0][who] = who < nt ? expf(-rate * softplus_f(gz[0] + dtb.at(head))) : 1.f;
-        }
-        if (who < CT) sm.beta[who] = who < nt ? 1.0f / (1.0f + expf(-zb)) : 0.f;
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        named_sync<BAR_PREP, PREP_THREADS>();
-        if (c >= 2) chunk_bar_sync(BAR_EMPTY + buf);
-        if (c + 1 < chunks) fetch(c + 1);                     // (nobody reads that buffer any more: the barrier above)
-        // A and B, a column s per warp and turn: the key of token s as the tokens after it see it
-#pragma unroll
-        for (int turn = 0; turn < 2; ++turn) {
-            const int s = turn == 0 ? warp : CT - 1 - warp;
-            float val[32];                                    // A_ts of t = 0 .. 15, then B_ts
-            float4 x = *(const float4*)&raw.k[s][4 * lane];
-#pragma unroll
-            for (int t = 0; t < CT; ++t) {
-                val[t] = val[CT + t] = 0.f;
-                if (t >= s) {
-                    const float4 qt = *(const float4*)&raw.q[t][4 * lane];
-                    if (t > s) {
-                        const float4 kt = *(const float4*)&raw.k[t][4 * lane];
-                        if (PER_CHANNEL) {
-                            const float4 g = *(const float4*)&sm.g[t][4 * lane];
-                            x.x *= g.x; x.y *= g.y; x.z *= g.z; x.w *= g.w;
-                        } else {
-                            const float g = sm.g[0][t];
-                            x.x *= g; x.y *= g; x.z *= g; x.w *= g;
-                        }
-                        val[t] = fmaf(x.x, kt.x, x.y * kt.y) + fmaf(x.z, kt.z, x.w * kt.w);
+        for (int t = 0; t < CT; ++t) {
+            val[t] = val[CT + t] = 0.f;
+            if (t >= s) {
+                const float4 qt = *(const float4*)&sm.q[t][4 * lane];
+                if (t > s) {
+                    const float4 kt = *(const float4*)&sm.k[t][4 * lane];
+                    if (PER_CHANNEL) {
+                        const float4 g = *(const float4*)&sm.g[t][4 * lane];
+                        x.x *= g.x; x.y *= g.y; x.z *= g.z; x.w *= g.w;
+                    } else {
+                        const float g = sm.g[0][t];
+                        x.x *= g; x.y *= g; x.z *= g; x.w *= g;
                     }
-                    val[CT + t] = fmaf(x.x, qt.x, x.y * qt.y) + fmaf(x.z, qt.z, x.w * qt.w);
+                    val[t] = fmaf(x.x, kt.x, x.y * kt.y) + fmaf(x.z, kt.z, x.w * kt.w);
                 }
+                val[CT + t] = fmaf(x.x, qt.x, x.y * qt.y) + fmaf(x.z, qt.z, x.w * qt.w);
             }
-            // every value summed over the lanes; lane l ends with the l-th
-#pragma unroll
-            for (int half = 16; half > 0; half >>= 1) {
-                const bool upper = (lane & half) != 0;
-#pragma unroll
-                for (int v = 0; v < half; ++v) {
-                    const float give = upper ? val[v] : val[v + half], keep = upper ? val[v + half] : val[v];
-                    val[v] = keep + __shfl_xor_sync(0xffffffffu, give, half);
-                }
-            }
-            const int t = lane & (CT - 1);
-            if (lane < CT) sm.a[t][s] = val[0];
-            else split3(val[0], o.b[0][t][s], o.b[1][t][s], o.b[2][t][s]);
         }
-        named_sync<BAR_PREP, PREP_THREADS>();
-        // the triangular solutions, a thread per channel
-        auto solve = [&](float (&x)[CT]) {                    // x: right hand sides without beta, then the solutions
+        // every value summed over the lanes; lane l ends with the l-th
 #pragma unroll
-            for (int t = 0; t < CT; ++t) {
-                float r0s = 0.f, r1s = 0.f, r2s = 0.f, r3s = 0.f;
+        for (int half = 16; half > 0; half >>= 1) {
+            const bool upper = (lane & half) != 0;
 #pragma unroll
-                for (int s = 0; s < t; s += 4) {
-                    const float4 at = *(const float4*)&sm.a[t][s];
-                    r0s = fmaf(at.x, x[s], r0s);
-                    if (s + 1 < t) r1s = fmaf(at.y, x[s + 1], r1s);
-                    if (s + 2 < t) r2s = fmaf(at.z, x[s + 2], r2s);
-                    if (s + 3 < t) r3s = fmaf(at.w, x[s + 3], r3s);
-                }
-                x[t] = sm.beta[t] * (x[t] - ((r0s + r1s) + (r2s + r3s)));
+            for (int v = 0; v < half; ++v) {
+                const float give = upper ? val[v] : val[v + half], keep = upper ? val[v + half] : val[v];
+                val[v] = keep + __shfl_xor_sync(0xffffffffu, give, half);
             }
-        };
-        float x[CT];
-        if (who < CD) {
-            float gam = 1.f;
+        }
+        const int t = lane & (CT - 1);
+        if (lane < CT) sm.a[t][s] = val[0];
+        else split3(val[0], o.b[0][t][s], o.b[1][t][s], o.b[2][t][s]);
+    }
+    __syncthreads();
+    // the triangular solutions, a thread per channel
+    auto solve = [&](float (&x)[CT]) {                        // x: right hand sides without beta, then the solutions
 #pragma unroll
-            for (int t = 0; t < CT; ++t) {
-                gam *= PER_CHANNEL ? sm.g[t][who] : sm.g[0][t];
-                x[t] = gam * raw.k[t][who];
-                split3(gam * raw.q[t][who], o.q[0][t][who], o.q[1][t][who], o.q[2][t][who]);
+        for (int t = 0; t < CT; ++t) {
+            float r0s = 0.f, r1s = 0.f, r2s = 0.f, r3s = 0.f;
+#pragma unroll
+            for (int s = 0; s < t; s += 4) {
+                const float4 row = *(const float4*)&sm.a[t][s];
+                r0s = fmaf(row.x, x[s], r0s);
+                if (s + 1 < t) r1s = fmaf(row.y, x[s + 1], r1s);
+                if (s + 2 < t) r2s = fmaf(row.z, x[s + 2], r2s);
+                if (s + 3 < t) r3s = fmaf(row.w, x[s + 3], r3s);
             }
-            o.gamma[who] = gam;
+            x[t] = sm.beta[t] * (x[t] - ((r0s + r1s) + (r2s + r3s)));
+        }
+    };
+    float x[CT];
+    if (who < CD) {
+        float gam = 1.f;
+#pragma unroll
+        for (int t = 0; t < CT; ++t) {
+            gam *= PER_CHANNEL ? sm.g[t][who] : sm.g[0][t];
+            x[t] = gam * sm.k[t][who];
+            split3(gam * sm.q[t][who], o.q[0][t][who], o.q[1][t][who], o.q[2][t][who]);
+        }
+        o.gamma[who] = gam;
+        solve(x);
+#pragma unroll
+        for (int t = 0; t < CT; ++t) split3(x[t], o.w[0][t][who], o.w[1][t][who], o.w[2][t][who]);
+    } else {
+        const int i = who - CD;
+        float left = 1.f;
+#pragma unroll
+        for (int t = CT - 1; t >= 0; --t) {
+            split3(left * sm.k[t][i], o.k[0][t][i], o.k[1][t][i], o.k[2][t][i]);
+            left *= PER_CHANNEL ? sm.g[t][i] : sm.g[0][t];
+        }
+        for (int j = i; j < args.value_blocks * CV; j += PREP_THREADS - CD) {
+#pragma unroll
+            for (int t = 0; t < CT; ++t)
+                x[t] = t < nt && j < p.dv ? p.qkv[(size_t)(r0 + t0 + t) * channels + 2 * qk + head * p.dv + j] : 0.f;
             solve(x);
+            float* u = &args.u0[at * args.value_blocks + j / CV][0][j % CV];
 #pragma unroll
-            for (int t = 0; t < CT; ++t) split3(x[t], o.w[0][t][who], o.w[1][t][who], o.w[2][t][who]);
-        } else {
-            const int i = who - CD;
-            float left = 1.f;
-#pragma unroll
-            for (int t = CT - 1; t >= 0; --t) {
-                split3(left * raw.k[t][i], o.k[0][t][i], o.k[1][t][i], o.k[2][t][i]);
-                left *= PER_CHANNEL ? sm.g[t][i] : sm.g[0][t];
-            }
-            if (i < CV) {
-#pragma unroll
-                for (int t = 0; t < CT; ++t) x[t] = raw.v[t][i];
-                solve(x);
-#pragma unroll
-                for (int t = 0; t < CT; ++t) o.u0[t][i] = x[t];
-            }
+            for (int t = 0; t < CT; ++t) u[t * (CV + 4)] = x[t];
         }
-        chunk_bar_arrive(BAR_FULL + buf);
-        if (c + 1 < chunks) named_sync<BAR_PREP, PREP_THREADS>();      // decays, A and rows may be written again
+    }
+    __syncthreads();
+    uint4* dst = (uint4*)(args.ops + at);
+    for (int i = who; i < (int)(sizeof(ChunkOperands) / 16); i += PREP_THREADS) dst[i] = ((const uint4*)&sm.ops)[i];
+}
+
+// the walking block's operands, two chunks ahead of the walk
+__device__ __forceinline__ void fetch_chunks(const ChunkArgs& args, WalkShared& sm, int r0, int seq, int chunks) {
+    const int who = threadIdx.x - WALK_THREADS;
+    auto copy = [&](void* dst, const void* src, int bytes) {
+        for (int i = who * 16; i < bytes; i += FETCH_THREADS * 16)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared((char*)dst + i)), "l"((const char*)src + i) : "memory");
+    };
+    constexpr int AHEAD = CHUNK_STAGES - 1;
+    for (int c = 0; c < chunks + AHEAD; ++c) {
+        if (c < chunks) {
+            const int stage = c % CHUNK_STAGES;
+            if (c >= CHUNK_STAGES) walk_bar_sync(BAR_EMPTY + stage);
+            const size_t at = (size_t)chunk_slot(r0, seq, c) * args.heads + blockIdx.y;
+            copy(&sm.ops[stage], args.ops + at, sizeof(ChunkOperands));
+            copy(&sm.u0[stage], args.u0 + at * args.value_blocks + blockIdx.z, sizeof(ChunkValues));
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (c >= AHEAD) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD) : "memory");
+            walk_bar_arrive(BAR_FULL + (c - AHEAD) % CHUNK_STAGES);
+        }
     }
 }
 
-__device__ __forceinline__ void walk_chunks(const ScanArgs& p, ChunkShared& sm, int r0, int n, int seq, int head, int col0) {
+__device__ __forceinline__ void walk_chunks(const ScanArgs& p, WalkShared& sm, int r0, int n, int seq, int head, int col0) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int c_lo = col0 + warp * 16 + g, c_hi = c_lo + 8, local = warp * 16 + g;
     const int chunks = (n + CT - 1) / CT;
@@ -247,32 +283,39 @@ __device__ __forceinline__ void walk_chunks(const ScanArgs& p, ChunkShared& sm, 
     const int mi = lane >> 3, row_n = (mi >> 1) * 8 + (lane & 7), at_n = (mi & 1) * 8;       // ldmatrix: [n][k] tiles
     const int row_t = (mi & 1) * 8 + (lane & 7), at_t = (mi >> 1) * 8;                       // transposed: [k][n] tiles
     for (int c = 0; c < chunks; ++c) {
-        const int buf = c & 1;
-        const ChunkOperands& o = sm.ops[buf];
-        chunk_bar_sync(BAR_FULL + buf);
-        float ul[2][4] = {}, us[2][4] = {}, ol[2][4] = {}, os[2][4] = {};     // W S0 and (Gamma q) S0, two tiles of 8 tokens each
+        const int stage = c % CHUNK_STAGES;
+        const ChunkOperands& o = sm.ops[stage];
+        walk_bar_sync(BAR_FULL + stage);
+        // W S0 (tiles 0 and 1: tokens 0-7 and 8-15) and (Gamma q) S0 (2 and 3)
+        float sum[4][4], large[4][4], small[4][4];
+        clear(sum);
+        clear(small);
 #pragma unroll
         for (int ks = 0; ks < CD / 16; ++ks) {
-            uint32_t a[3][4], b[3][4];
+            uint32_t a[3][4], b[2][3][4];
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
                 const float* v = s[2 * ks + (r >> 1)] + 2 * (r & 1);
                 split3(v[0], v[1], a[0][r], a[1][r], a[2][r]);
             }
 #pragma unroll
-            for (int pl = 0; pl < 3; ++pl) ldsm4(b[pl], &o.w[pl][row_n][ks * 16 + at_n]);
-            mma_split(ul[0], us[0], a, b, 0);
-            mma_split(ul[1], us[1], a, b, 1);
-#pragma unroll
-            for (int pl = 0; pl < 3; ++pl) ldsm4(b[pl], &o.q[pl][row_n][ks * 16 + at_n]);
-            mma_split(ol[0], os[0], a, b, 0);
-            mma_split(ol[1], os[1], a, b, 1);
+            for (int pl = 0; pl < 3; ++pl) {
+                ldsm4(b[0][pl], &o.w[pl][row_n][ks * 16 + at_n]);
+                ldsm4(b[1][pl], &o.q[pl][row_n][ks * 16 + at_n]);
+            }
+            if (ks % 2 == 0) clear(large);
+            mma_split<4>(large, small, a, b);
+            if (ks % 2 == 1) add_to(sum, large);
         }
-        float u[2][4];
+        add_to(sum, small);
+        float u[2][4], out2[2][4];
 #pragma unroll
         for (int i = 0; i < 2; ++i)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) u[i][e] = o.u0[8 * i + 2 * t + (e & 1)][local + (e < 2 ? 0 : 8)] - (ul[i][e] + us[i][e]);
+            for (int e = 0; e < 4; ++e) {
+                u[i][e] = sm.u0[stage][8 * i + 2 * t + (e & 1)][local + (e < 2 ? 0 : 8)] - sum[i][e];
+                out2[i][e] = sum[2 + i][e];
+            }
         uint32_t ua[3][4];
 #pragma unroll
         for (int r = 0; r < 4; ++r) split3(u[r >> 1][2 * (r & 1)], u[r >> 1][2 * (r & 1) + 1], ua[0][r], ua[1][r], ua[2][r]);
@@ -282,11 +325,15 @@ __device__ __forceinline__ void walk_chunks(const ScanArgs& p, ChunkShared& sm, 
 #pragma unroll
             for (int e = 0; e < 4; ++e) finite = fmaf(0.f, u[i][e], finite);
         if (!__any_sync(0xffffffffu, finite != finite)) {
-            uint32_t b[3][4];
+            uint32_t b[1][3][4];
 #pragma unroll
-            for (int pl = 0; pl < 3; ++pl) ldsm4(b[pl], &o.b[pl][row_n][at_n]);
-            mma_split(ol[0], os[0], ua, b, 0);
-            mma_split(ol[1], os[1], ua, b, 1);
+            for (int pl = 0; pl < 3; ++pl) ldsm4(b[0][pl], &o.b[pl][row_n][at_n]);
+            float bl[2][4], bs[2][4];
+            clear(bl);
+            clear(bs);
+            mma_split<2>(bl, bs, ua, b);
+            add_to(bl, bs);
+            add_to(out2, bl);
         } else {
             // a correction that is not finite reaches its own token and those after it only: no product with a zero of B
 #pragma unroll
@@ -300,8 +347,8 @@ __device__ __forceinline__ void walk_chunks(const ScanArgs& p, ChunkShared& sm, 
                         const int to = 8 * i + 2 * t + e;
                         if (to < src) continue;
                         const float w = __bfloat162float(o.b[0][to][src]) + (__bfloat162float(o.b[1][to][src]) + __bfloat162float(o.b[2][to][src]));
-                        ol[i][e] = fmaf(w, lo, ol[i][e]);
-                        ol[i][2 + e] = fmaf(w, hi, ol[i][2 + e]);
+                        out2[i][e] = fmaf(w, lo, out2[i][e]);
+                        out2[i][2 + e] = fmaf(w, hi, out2[i][2 + e]);
                     }
             }
         }
@@ -312,26 +359,30 @@ __device__ __forceinline__ void walk_chunks(const ScanArgs& p, ChunkShared& sm, 
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int tok = 8 * i + 2 * t + (e & 1), col = e < 2 ? c_lo : c_hi;
-                if (tok < nt && col < p.dv) out[(size_t)tok * p.heads * p.dv + col] = ol[i][e] + os[i][e];
+                if (tok < nt && col < p.dv) out[(size_t)tok * p.heads * p.dv + col] = out2[i][e];
             }
 #pragma unroll
-        for (int jt = 0; jt < CD / 16; ++jt) {
-            uint32_t b[3][4];
+        for (int jt = 0; jt < CD / 16; jt += 2) {             // four tiles of eight key channels at a time
+            uint32_t b[2][3][4];
 #pragma unroll
-            for (int pl = 0; pl < 3; ++pl) ldsm4t(b[pl], &o.k[pl][row_t][jt * 16 + at_t]);
+            for (int pl = 0; pl < 3; ++pl) {
+                ldsm4t(b[0][pl], &o.k[pl][row_t][jt * 16 + at_t]);
+                ldsm4t(b[1][pl], &o.k[pl][row_t][(jt + 1) * 16 + at_t]);
+            }
+            clear(large);
+            clear(small);
+            mma_split<4>(large, small, ua, b);
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
+            for (int i = 0; i < 4; ++i) {
                 const int j = 2 * jt + i;
-                float dl[4] = {}, ds[4] = {};
-                mma_split(dl, ds, ua, b, i);
                 const float2 gam = *(const float2*)&o.gamma[8 * j + 2 * t];
-                s[j][0] = fmaf(gam.x, s[j][0], dl[0] + ds[0]);
-                s[j][1] = fmaf(gam.y, s[j][1], dl[1] + ds[1]);
-                s[j][2] = fmaf(gam.x, s[j][2], dl[2] + ds[2]);
-                s[j][3] = fmaf(gam.y, s[j][3], dl[3] + ds[3]);
+                s[j][0] = fmaf(gam.x, s[j][0], large[i][0] + small[i][0]);
+                s[j][1] = fmaf(gam.y, s[j][1], large[i][1] + small[i][1]);
+                s[j][2] = fmaf(gam.x, s[j][2], large[i][2] + small[i][2]);
+                s[j][3] = fmaf(gam.y, s[j][3], large[i][3] + small[i][3]);
             }
         }
-        if (c + 2 < chunks) chunk_bar_arrive(BAR_EMPTY + buf);
+        if (c + CHUNK_STAGES < chunks) walk_bar_arrive(BAR_EMPTY + stage);
     }
 #pragma unroll
     for (int j = 0; j < CD / 8; ++j)
@@ -342,31 +393,49 @@ __device__ __forceinline__ void walk_chunks(const ScanArgs& p, ChunkShared& sm, 
         }
 }
 
-template <typename TR, bool PER_CHANNEL>
-__global__ void __launch_bounds__(CHUNK_THREADS, 1) delta_chunks_kernel(const ScanArgs p) {
+__global__ void __launch_bounds__(WALK_THREADS + FETCH_THREADS, 1) delta_walk_chunks_kernel(const ChunkArgs args) {
     extern __shared__ __align__(16) unsigned char chunk_smem[];
-    ChunkShared& sm = *(ChunkShared*)chunk_smem;
-    const int seq = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * CV;
+    WalkShared& sm = *(WalkShared*)chunk_smem;
+    const ScanArgs& p = args.s;
+    const int seq = blockIdx.x, head = args.head0 + blockIdx.y;
     const int r0 = p.seq_start[seq], n = p.seq_qlen[seq];
     fr_pdl_wait();
     fr_pdl_launch();
     if (n <= 0 || p.row_seq[r0] < 0) return;
-    if (threadIdx.x < CHAIN_THREADS) walk_chunks(p, sm, r0, n, seq, head, col0);
-    else prepare_chunks<TR, PER_CHANNEL>(p, sm, r0, n, head, col0);
+    if (threadIdx.x < WALK_THREADS) walk_chunks(p, sm, r0, n, seq, head, blockIdx.z * CV);
+    else fetch_chunks(args, sm, r0, seq, (n + CT - 1) / CT);
+}
+
+long long chunk_slots(int rows, int n_seqs) { return (long long)rows / CT + n_seqs + 1; }
+long long chunk_head_bytes(int rows, int n_seqs, int dv) {                 // scratch of one head
+    return chunk_slots(rows, n_seqs) * (long long)(sizeof(ChunkOperands) + (dv + CV - 1) / CV * sizeof(ChunkValues));
+}
+constexpr long long CHUNK_SCRATCH = 128ll << 20;              // heads beyond what this holds go in further rounds (at least one per round)
+int chunk_heads(int rows, int n_seqs, int heads, int dv) {
+    const long long fit = CHUNK_SCRATCH / chunk_head_bytes(rows, n_seqs, dv);
+    return fit < 1 ? 1 : fit < heads ? (int)fit : heads;
 }
 
 template <typename TR, bool PER_CHANNEL>
-int launch_chunks(const ScanArgs& p, int n_seqs, cudaStream_t stream) {
-    static std::atomic<unsigned long long> configured{0};     // devices (as bits) on which the limit has been raised
+int launch_chunks(const ScanArgs& s, int rows, int n_seqs, int max_q_len, void* scratch, cudaStream_t stream) {
+    static std::atomic<unsigned long long> configured{0};     // devices (as bits) on which the limits have been raised
     int device = 0;
     FR_CUDA(cudaGetDevice(&device));
     if (device < 0 || device >= 64) FR_REFUSE("delta chunks: device %d is outside the table of 64", device);
     if (!(configured.load(std::memory_order_acquire) & (1ull << device))) {
-        FR_CUDA(cudaFuncSetAttribute(delta_chunks_kernel<TR, PER_CHANNEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ChunkShared)));
+        FR_CUDA(cudaFuncSetAttribute(delta_prepare_chunks_kernel<TR, PER_CHANNEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PrepShared)));
+        FR_CUDA(cudaFuncSetAttribute(delta_walk_chunks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WalkShared)));
         configured.fetch_or(1ull << device, std::memory_order_release);
     }
-    FR_CUDA(fr_launch(delta_chunks_kernel<TR, PER_CHANNEL>, dim3(n_seqs, p.heads, (p.dv + CV - 1) / CV), dim3(CHUNK_THREADS), sizeof(ChunkShared), stream, p));
-    FR_CHECK_LAUNCH("delta chunks");
+    const int at_once = chunk_heads(rows, n_seqs, s.heads, s.dv), blocks = (s.dv + CV - 1) / CV;
+    for (int h = 0; h < s.heads; h += at_once) {
+        ChunkArgs a{s, (ChunkOperands*)scratch, nullptr, h, s.heads - h < at_once ? s.heads - h : at_once, blocks};
+        a.u0 = (ChunkValues*)(a.ops + chunk_slots(rows, n_seqs) * a.heads);
+        FR_CUDA(fr_launch(delta_prepare_chunks_kernel<TR, PER_CHANNEL>, dim3((max_q_len + CT - 1) / CT, a.heads, n_seqs), dim3(PREP_THREADS), sizeof(PrepShared), stream, a));
+        FR_CHECK_LAUNCH("delta chunks (prepare)");
+        FR_CUDA(fr_launch(delta_walk_chunks_kernel, dim3(n_seqs, a.heads, blocks), dim3(WALK_THREADS + FETCH_THREADS), sizeof(WalkShared), stream, a));
+        FR_CHECK_LAUNCH("delta chunks (walk)");
+    }
     return FR_OK;
 }
 

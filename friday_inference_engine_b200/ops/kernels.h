@@ -136,9 +136,9 @@ struct Delta {
                       int, int, int, cudaStream_t);
     int (*scan)(const float*, const void*, int, const void*, int, int, const void*, const void*, int, float*, float*, long long,
                 long long, const int*, const int*, const int*, const int*, int, int, int, int, int, int, cudaStream_t);
-    int (*chunks_supports)(const float*, int, int);
+    long long (*chunks_scratch)(const float*, int, int, int, int, int);
     int (*chunks)(const float*, const void*, int, const void*, int, int, const void*, const void*, int, float*, float*, long long,
-                  long long, const int*, const int*, const int*, const int*, int, int, int, int, int, int, cudaStream_t);
+                  long long, const int*, const int*, const int*, const int*, int, int, int, int, int, int, int, int, void*, long long, cudaStream_t);
     int (*general_prepare)(const void*, int, int, int, const float*, int, const float*, int, const void*, const void*, int, float*, int, int,
                            int, float, float, int, cudaStream_t);
     int (*general_scan)(const float*, const void*, int, int, float*, float*, long long, long long, const int*, const int*, const int*, int,

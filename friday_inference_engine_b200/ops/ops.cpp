@@ -844,10 +844,21 @@ Tensor Ops::delta_scan(const Tensor& qkv, const Tensor& a_raw, const Tensor& b_r
     Tensor out = alloc(DType::F32, qkv.rows(), (int64_t)s.heads * s.dv);
     const auto& k = kernels::delta();
     Timed t(*this, Attention);
-    const bool chunks = !ctx.decode && ctx.max_q_len >= DELTA_CHUNKS_FROM && k.chunks_supports((const float*)qkv.data, s.dk, s.dv);
-    call(launches_, k, (chunks ? k.chunks : k.scan)((const float*)qkv.data, a_raw.data, (int)a_raw.ld, b_raw.data, (int)b_raw.ld, code(a_raw.dtype),
-                              a_log.data, dt_bias.data, code(a_log.dtype), (float*)out.data, (float*)view.state.data, stride, s_off,
-                              ctx.row_seq, ctx.seq_start, ctx.seq_qlen, view.seq_slots, ctx.n_seqs, s.heads, s.qk_heads, s.dk, s.dv,
+    const int rows = (int)qkv.rows();
+    const long long room = !ctx.decode && ctx.max_q_len >= DELTA_CHUNKS_FROM && ctx.rows == rows
+                               ? k.chunks_scratch((const float*)qkv.data, rows, ctx.n_seqs, s.heads, s.dk, s.dv) : 0;
+    if (room > 0) {
+        float* scratch = scratch_floats((room + 3) / 4);
+        call(launches_, k, k.chunks((const float*)qkv.data, a_raw.data, (int)a_raw.ld, b_raw.data, (int)b_raw.ld, code(a_raw.dtype), a_log.data,
+                                    dt_bias.data, code(a_log.dtype), (float*)out.data, (float*)view.state.data, stride, s_off, ctx.row_seq,
+                                    ctx.seq_start, ctx.seq_qlen, view.seq_slots, ctx.n_seqs, s.heads, s.qk_heads, s.dk, s.dv,
+                                    s.per_channel ? 1 : 0, rows, ctx.max_q_len, scratch, room, stream_), "delta_scan_chunks");
+        ++launches_;                                          // preparing the chunks and walking them
+        return out;
+    }
+    call(launches_, k, k.scan((const float*)qkv.data, a_raw.data, (int)a_raw.ld, b_raw.data, (int)b_raw.ld, code(a_raw.dtype), a_log.data,
+                              dt_bias.data, code(a_log.dtype), (float*)out.data, (float*)view.state.data, stride, s_off, ctx.row_seq,
+                              ctx.seq_start, ctx.seq_qlen, view.seq_slots, ctx.n_seqs, s.heads, s.qk_heads, s.dk, s.dv,
                               s.per_channel ? 1 : 0, stream_), "delta_scan");
     return out;
 }

@@ -29,16 +29,23 @@ def inputs(lens, heads, groups, dk, dv, per_channel, dtype, seed=0):
 
 def run(name, c, over=()):
     fam = lib.family("delta")
-    fam.declare(name, SIGNATURE)
+    chunks = name == "delta_scan_chunks"
+    fam.declare(name, SIGNATURE[:-1] + [I, I, P, L, P] if chunks else SIGNATURE)
     heads, groups, dk, dv, per_channel = c["sizes"]
     n, rows = len(c["lens"]), sum(c["lens"])
     starts = [sum(c["lens"][:i]) for i in range(n)]
     start, count, slots = (torch.tensor(v, dtype=torch.int32, device=DEV) for v in (starts, c["lens"], range(n, 0, -1)))
     row_seq = torch.tensor([-1 if i in over else i for i, m in enumerate(c["lens"]) for _ in range(m)], dtype=torch.int32, device=DEV)
     out, state = torch.full((rows, heads * dv), 7.0, device=DEV), c["state"].clone()
+    more = []
+    if chunks:
+        need = fam.declare("delta_scan_chunks_scratch", [P, I, I, I, I, I], L)(c["qkv"].data_ptr(), rows, n, heads, dk, dv)
+        scratch = torch.full((need,), 255, dtype=torch.uint8, device=DEV)
+        more = [rows, max(c["lens"]), scratch.data_ptr(), need]
     fam.call(name, c["qkv"].data_ptr(), c["a"].data_ptr(), c["a"].stride(0), c["b"].data_ptr(), c["b"].stride(0), 0 if c["a"].dtype == torch.float32 else 1,
              c["a_log"].data_ptr(), c["bias"].data_ptr(), 0, out.data_ptr(), state.data_ptr(), state.stride(0), 5, row_seq.data_ptr(), start.data_ptr(),
-             count.data_ptr(), slots.data_ptr(), n, heads, groups, dk, dv, 1 if per_channel else 0, torch.cuda.current_stream().cuda_stream)
+             count.data_ptr(), slots.data_ptr(), n, heads, groups, dk, dv, 1 if per_channel else 0, *more,
+             torch.cuda.current_stream().cuda_stream)
     torch.cuda.synchronize()
     return out, state
 
