@@ -197,19 +197,10 @@ __device__ __forceinline__ void finish16(const P& p, int gi, int gj0, float (&v)
         } else {
             float* o = (float*)p.out + base;
             const float* r = p.residual ? (const float*)p.residual + base : nullptr;
-            if (whole && (p.ldo % 4 == 0) && ((((uintptr_t)p.out | (uintptr_t)p.residual) & 15) == 0)) {
-                float4 rr[4];
-                if (r)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) rr[j] = ((const float4*)r)[j];
+            if (whole && (p.ldo % 4 == 0) && (((uintptr_t)p.out & 15) == 0) && r == nullptr) {
                 if (p.bias)
 #pragma unroll
                     for (int j = 0; j < 16; ++j) v[j] += bias_at(p, gj0 + j);
-                if (r)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        v[4 * j] += rr[j].x; v[4 * j + 1] += rr[j].y; v[4 * j + 2] += rr[j].z; v[4 * j + 3] += rr[j].w;
-                    }
 #pragma unroll
                 for (int j = 0; j < 4; ++j) ((float4*)o)[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
             } else {
