@@ -715,10 +715,7 @@ post_norm_add_vec_kernel(const float* __restrict__ x, const float* __restrict__ 
     fr_pdl_launch();
     const size_t base = (size_t)blockIdx.x * width;
     const int n4 = width >> 2;
-    // both norms' weights come with the rows (of up to 4,096 columns): behind the sums each would be a trip to memory of its own
-    constexpr bool EARLY = NV <= 4;
     float4 v[NV], r[NV];
-    float wv[EARLY ? NV : 1][4], w2v[EARLY ? NV : 1][4];
     float ss = 0.f;
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
@@ -726,10 +723,6 @@ post_norm_add_vec_kernel(const float* __restrict__ x, const float* __restrict__ 
         if (i < n4) {
             v[k] = ((const float4*)(y + base))[i];
             r[k] = ((const float4*)(x + base))[i];
-            if (EARLY) {
-                w.four(4 * i, wv[EARLY ? k : 0]);
-                if (next != nullptr && w2.p != nullptr) w2.four(4 * i, w2v[EARLY ? k : 0]);
-            }
         }
     }
 #pragma unroll
@@ -745,11 +738,11 @@ post_norm_add_vec_kernel(const float* __restrict__ x, const float* __restrict__ 
         const int i = threadIdx.x + k * 256;
         if (i < n4) {
             const float yv[4] = {v[k].x, v[k].y, v[k].z, v[k].w}, xv[4] = {r[k].x, r[k].y, r[k].z, r[k].w};
-            float o[4], (&wk)[4] = wv[EARLY ? k : 0];
-            if (!EARLY) w.four(4 * i, wk);
+            float o[4], wv[4];
+            w.four(4 * i, wv);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                o[e] = fmaf(mult, yv[e] * inv * wk[e], xv[e]);
+                o[e] = fmaf(mult, yv[e] * inv * wv[e], xv[e]);
                 s2 = fmaf(o[e], o[e], s2);
             }
             store4(out + base + 4 * i, o);
@@ -765,10 +758,10 @@ post_norm_add_vec_kernel(const float* __restrict__ x, const float* __restrict__ 
         const int i = threadIdx.x + k * 256;
         if (i < n4) {
             const float ov[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
-            float o[4], (&wk)[4] = w2v[EARLY ? k : 0];
-            if (!EARLY) w2.four(4 * i, wk);
+            float o[4], wv[4];
+            w2.four(4 * i, wv);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) o[e] = ov[e] * inv2 * wk[e];
+            for (int e = 0; e < 4; ++e) o[e] = ov[e] * inv2 * wv[e];
             store4(next + base + 4 * i, o);
         }
     }
