@@ -257,7 +257,7 @@ __device__ __forceinline__ void fetch_chunks(const ChunkArgs& args, WalkShared& 
             if (c >= CHUNK_STAGES) walk_bar_sync(BAR_EMPTY + stage);
             const size_t at = (size_t)chunk_slot(r0, seq, c) * args.heads + blockIdx.y;
             copy(&sm.ops[stage], args.ops + at, sizeof(ChunkOperands));
-            copy(&sm.u0[stage], args.u0 + at * args.value_blocks + blockIdx.z, sizeof(ChunkValues));
+            copy(&sm.u0[stage], args.u0 + at * args.value_blocks + blockIdx.x, sizeof(ChunkValues));
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
         if (c >= AHEAD) {
@@ -393,16 +393,36 @@ __device__ __forceinline__ void walk_chunks(const ScanArgs& p, WalkShared& sm, i
         }
 }
 
-__global__ void __launch_bounds__(WALK_THREADS + FETCH_THREADS, 1) delta_walk_chunks_kernel(const ChunkArgs args) {
+// RANKED: blocks in order of their sequences' lengths, the longest first, so that an SM's second block is a short one.  Taken where there are
+// more blocks than SMs and sequences are shorter than three quarters of the longest on average (and at most 64 of them, many even out by
+// themselves): 8 prompts of 64 to 512 tokens, 16 heads 177 us, in the order of the sequences 203; but 16 of 300 each,
+// 32 heads, 696 and 661, since the compiler schedules the walk's instructions less well around it.
+constexpr int WALK_RANKED = 64;
+__device__ __forceinline__ int walked_sequence(const ScanArgs& p, int n_seqs, int rank) {
+    __shared__ int lens[WALK_RANKED], found;
+    const int i = threadIdx.x;
+    if (i < n_seqs) lens[i] = p.seq_qlen[i];
+    __syncthreads();
+    if (i < n_seqs) {
+        int before = 0;
+        for (int j = 0; j < n_seqs; ++j) before += lens[j] > lens[i] || (lens[j] == lens[i] && j < i);
+        if (before == rank) found = i;
+    }
+    __syncthreads();
+    return found;
+}
+
+template <bool RANKED>
+__global__ void __launch_bounds__(WALK_THREADS + FETCH_THREADS, 1) delta_walk_chunks_kernel(const ChunkArgs args, int n_seqs) {
     extern __shared__ __align__(16) unsigned char chunk_smem[];
     WalkShared& sm = *(WalkShared*)chunk_smem;
     const ScanArgs& p = args.s;
-    const int seq = blockIdx.x, head = args.head0 + blockIdx.y;
+    const int seq = RANKED ? walked_sequence(p, n_seqs, blockIdx.z) : blockIdx.z, head = args.head0 + blockIdx.y;
     const int r0 = p.seq_start[seq], n = p.seq_qlen[seq];
     fr_pdl_wait();
     fr_pdl_launch();
     if (n <= 0 || p.row_seq[r0] < 0) return;
-    if (threadIdx.x < WALK_THREADS) walk_chunks(p, sm, r0, n, seq, head, blockIdx.z * CV);
+    if (threadIdx.x < WALK_THREADS) walk_chunks(p, sm, r0, n, seq, head, blockIdx.x * CV);
     else fetch_chunks(args, sm, r0, seq, (n + CT - 1) / CT);
 }
 
@@ -410,10 +430,13 @@ long long chunk_slots(int rows, int n_seqs) { return (long long)rows / CT + n_se
 long long chunk_head_bytes(int rows, int n_seqs, int dv) {                 // scratch of one head
     return chunk_slots(rows, n_seqs) * (long long)(sizeof(ChunkOperands) + (dv + CV - 1) / CV * sizeof(ChunkValues));
 }
-constexpr long long CHUNK_SCRATCH = 128ll << 20;              // heads beyond what this holds go in further rounds (at least one per round)
+// Heads go in equal rounds of what this holds (at least one per round).
+constexpr long long CHUNK_SCRATCH = 256ll << 20;
 int chunk_heads(int rows, int n_seqs, int heads, int dv) {
     const long long fit = CHUNK_SCRATCH / chunk_head_bytes(rows, n_seqs, dv);
-    return fit < 1 ? 1 : fit < heads ? (int)fit : heads;
+    if (fit < 1) return 1;
+    const long long rounds = (heads + fit - 1) / fit;
+    return (int)((heads + rounds - 1) / rounds);
 }
 
 template <typename TR, bool PER_CHANNEL>
@@ -424,16 +447,19 @@ int launch_chunks(const ScanArgs& s, int rows, int n_seqs, int max_q_len, void* 
     if (device < 0 || device >= 64) FR_REFUSE("delta chunks: device %d is outside the table of 64", device);
     if (!(configured.load(std::memory_order_acquire) & (1ull << device))) {
         FR_CUDA(cudaFuncSetAttribute(delta_prepare_chunks_kernel<TR, PER_CHANNEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PrepShared)));
-        FR_CUDA(cudaFuncSetAttribute(delta_walk_chunks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WalkShared)));
+        FR_CUDA(cudaFuncSetAttribute(delta_walk_chunks_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WalkShared)));
+        FR_CUDA(cudaFuncSetAttribute(delta_walk_chunks_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WalkShared)));
         configured.fetch_or(1ull << device, std::memory_order_release);
     }
-    const int at_once = chunk_heads(rows, n_seqs, s.heads, s.dv), blocks = (s.dv + CV - 1) / CV;
+    const int sms = fr_sm_count() > 0 ? fr_sm_count() : 148, at_once = chunk_heads(rows, n_seqs, s.heads, s.dv), blocks = (s.dv + CV - 1) / CV;
     for (int h = 0; h < s.heads; h += at_once) {
         ChunkArgs a{s, (ChunkOperands*)scratch, nullptr, h, s.heads - h < at_once ? s.heads - h : at_once, blocks};
         a.u0 = (ChunkValues*)(a.ops + chunk_slots(rows, n_seqs) * a.heads);
         FR_CUDA(fr_launch(delta_prepare_chunks_kernel<TR, PER_CHANNEL>, dim3((max_q_len + CT - 1) / CT, a.heads, n_seqs), dim3(PREP_THREADS), sizeof(PrepShared), stream, a));
         FR_CHECK_LAUNCH("delta chunks (prepare)");
-        FR_CUDA(fr_launch(delta_walk_chunks_kernel, dim3(n_seqs, a.heads, blocks), dim3(WALK_THREADS + FETCH_THREADS), sizeof(WalkShared), stream, a));
+        const bool ranked = n_seqs > 1 && n_seqs <= WALK_RANKED && (long long)blocks * a.heads * n_seqs > sms && 4ll * rows < 3ll * max_q_len * n_seqs;
+        FR_CUDA(fr_launch(ranked ? delta_walk_chunks_kernel<true> : delta_walk_chunks_kernel<false>, dim3(blocks, a.heads, n_seqs),
+                          dim3(WALK_THREADS + FETCH_THREADS), sizeof(WalkShared), stream, a, n_seqs));
         FR_CHECK_LAUNCH("delta chunks (walk)");
     }
     return FR_OK;

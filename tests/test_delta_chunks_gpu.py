@@ -72,7 +72,8 @@ def exact(c):
 
 
 @pytest.mark.parametrize("lens,heads,groups,dk,dv", [([16], 1, 1, 128, 64), ([1, 37, 100, 17], 4, 2, 128, 128), ([65, 3, 32], 3, 3, 20, 24),
-                                                     ([200], 2, 1, 64, 132), ([33, 15], 2, 2, 4, 4)])
+                                                     ([200], 2, 1, 64, 132), ([33, 15], 2, 2, 4, 4),
+                                                     ([20, 50, 20, 50, 1, 90], 26, 13, 16, 8), ([1] * 62 + [17, 3], 4, 1, 8, 4)])
 @pytest.mark.parametrize("per_channel", [False, True])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_delta_chunks(lens, heads, groups, dk, dv, per_channel, dtype):
