@@ -720,7 +720,6 @@ FR_API int friday_ops_linear_norm(void* h, const FridayTensor* x, const FridayTe
         auto r = o.begin().linear_norm(rows_of(x, in_ssq, in_eps), *T(weight), *T(norm_weight), eps, bias ? T(bias) : nullptr,
                                        residual ? T(residual) : nullptr);
         o.copy_out(r.first, out);
-        if (r.second.deferred && !r.second.ssq.defined()) r.second = Rows(o.ops->materialize(r.second));     // (nothing of it has begun)
         o.copy_out(r.second.t, normed);
         *deferred = r.second.deferred ? 1 : 0;
         if (r.second.deferred) {

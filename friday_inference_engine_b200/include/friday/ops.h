@@ -101,6 +101,7 @@ public:
     cudaStream_t stream() const { return stream_; }
     int sm_count() const { return sms_; }
     Arena* arena = nullptr;                                   // where results come from
+    bool leave_norms = false;                                 // linear_norm may return deferred rows without `ssq` (the engine's step does)
     Tensor alloc(DType dtype, int64_t rows, int64_t cols);
     float* scratch_floats(int64_t n);                         // from the arena
 

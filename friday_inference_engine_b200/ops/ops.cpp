@@ -1426,7 +1426,7 @@ std::pair<Tensor, Rows> Ops::linear_norm(const Rows& x, const Tensor& weight, co
         }
     }
     Tensor out = linear(x, weight, bias, residual);
-    if (out.dtype == DType::F32 && rows <= 16 && norm_weight.numel() == n && fusion_enabled()) {
+    if (leave_norms && out.dtype == DType::F32 && rows <= 16 && norm_weight.numel() == n && fusion_enabled()) {
         Rows r(out);                                          // few 32-bit rows: the products that read them do their norm
         r.deferred = true;
         r.eps = eps;
