@@ -23,10 +23,10 @@
 // sum are fp32 multiply-adds, so that the errors stay those of fp32 sums.  (Prepared by the walking block itself, a chunk took
 // as long as its preparation, 8,500 cycles.)
 //
-// The walk is bound by the rate of mma.sync (four fifths of it on a busy SM) and by its longest sequence.  Measured on B200, heads
-// of 128, us token by token and so, with a decay per head and per channel: 16 heads, 8 prompts of 64 to 512 tokens 313 -> 177 and 479 -> 203, one of 2,048 551 -> 367
-// and 693 -> 389, 8 of 64 63 -> 45 and 107 -> 49; 32 heads, 16 of 300 858 -> 650 and 1,618 -> 749.  Errors against 64 bits are no larger in any of them
-// (outputs of the first 1.8e-7 and 1.6e-7, of the second 1.3e-7 both).
+// The walk is bound by the rate of mma.sync (four fifths of it on a busy SM) and by its longest sequence.  Measured on B200, heads of 128, us token
+// by token and so, with a decay per head and per channel: 16 heads, 8 prompts of 64 to 512 tokens 313 -> 177 and 479 -> 203, one of
+// 2,048 551 -> 367 and 693 -> 389, 8 of 64 63 -> 45 and 107 -> 49; 32 heads, 16 of 300 858 -> 650 and 1,618 -> 749.  Errors against
+// 64 bits: of outputs never larger (1.8e-7 and 1.6e-7 in the first, 1.3e-7 both in the second), of states 0.75 to 1.06 times.
 #pragma once
 #include "mma_sync.cuh"
 
