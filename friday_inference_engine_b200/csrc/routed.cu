@@ -22,7 +22,6 @@
 #include <atomic>
 
 #include "common.cuh"
-#include "mma_sync.cuh"
 
 FR_EXPORT const char* routed_last_error() { return fr_error_text; }
 
@@ -188,17 +187,31 @@ gate_up_kernel(const T* __restrict__ h, const int* __restrict__ ids, const T* __
 }
 
 // Few rows: the weights of the experts that were chosen stream through once for all the (row, choice) pairs that chose them.
-// A unit is eight weight rows of one expert: four channels' gate and up rows, or eight columns of the down matrix.  The units of
-// all chosen experts, one expert after another, are dealt out over three blocks per SM; a block's warps share k, and their sums
-// meet in shared memory.  A lane fetches 16 bytes of a weight row (eight consecutive k) eight times before it uses the first, the next
-// unit's before it sums the present one's, and multiplies with mma.sync.m16n8k16: the weights on its M side (half of it), up to 8
-// pairs' activations on its N side.  Bound by reading the weights: 8 rows, 2 of 8 experts of 2048 x 2048 each, 117 MB in 33.7 us and 59 MB
-// in 19.6, where fp32 multiply-adds of the unpacked weights took 37.3 and 24.7.
+// A unit is two weight rows of one expert: a channel's gate and up rows, or two columns of the down matrix.  The units of all
+// chosen experts, one expert after another, are dealt out over the warps of two blocks per SM.  A warp keeps the next
+// RING - 1 pieces of its units on their way into shared memory (every lane reads back what it copied itself, so nothing is
+// synchronised between threads) and takes its lanes' share of the pairs' activations from L1.  Bound by reading the weights: at
+// width 2048, inner 2048, 8 experts, 16 pairs on a B200 the gate/up and down products of a decoding step take 35 to 39 and 21 to 27
+// us for some 117 and 59 MB (63 to 73 and 44 to 51 us when a block of one expert staged the rows first and then read its weights
+// in a few rounds).
 constexpr int SHARE = 16;                      // pairs of one expert that are finished together; more take the expert again
+constexpr int RING = 4, PIECE = 512;           // pieces of a warp's ring; elements of a weight row in one piece
 constexpr int MAX_FEW = 16;                    // rows of a call that runs here
 constexpr int MAX_FEW_PAIRS = MAX_FEW * 32;
-constexpr int STREAM_WARPS = 8, STREAM_ROWS = 8, STREAM_STEPS = 8;      // weight rows of a unit; pieces of 32 k that a warp has in flight
-constexpr int STREAM_K = STREAM_STEPS * 32;
+constexpr int STREAM_WARPS = 8;
+constexpr int STREAM_SMEM = STREAM_WARPS * RING * 2 * PIECE * 2;
+
+template <int N>
+struct Number {
+    static constexpr int value = N;
+};
+
+typedef unsigned long long Two;                // two floats
+__device__ __forceinline__ Two two_of(uint32_t bf16_pair) {
+    return (Two)(bf16_pair << 16) | ((Two)(bf16_pair & 0xffff0000u) << 32);
+}
+__device__ __forceinline__ void fma_two(Two& acc, Two x, Two y) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(x), "l"(y)); }
+__device__ __forceinline__ float sum_two(Two v) { return __uint_as_float((uint32_t)v) + __uint_as_float((uint32_t)(v >> 32)); }
 
 struct StreamArgs {
     const bf16* x;            // activations: row pair / x_share for pair
@@ -211,10 +224,73 @@ struct StreamArgs {
     float limit, slope;
 };
 
+// One piece of a unit: its lanes' products with `n` (at most NB) pairs' activations into acc[2 r], acc[2 r + 1].
+template <int NB>
+__device__ __forceinline__ void stream_piece(const uint4* slot, const bf16* x, int ldx, const int* rows, int n, int q0, int q_end, int lane, Two* acc) {
+#pragma unroll
+    for (int i = 0; i < PIECE / 256; ++i) {
+        const int q = q0 + lane + 32 * i;
+        if (q >= q_end) break;
+        const uint4 g = slot[lane + 32 * i], u = slot[PIECE / 8 + lane + 32 * i];
+        const Two gw[4] = {two_of(g.x), two_of(g.y), two_of(g.z), two_of(g.w)}, uw[4] = {two_of(u.x), two_of(u.y), two_of(u.z), two_of(u.w)};
+#pragma unroll
+        for (int r = 0; r < NB; ++r) {
+            if (NB > 4 && r >= n) break;
+            const uint4 xv = ((const uint4*)(x + (size_t)rows[NB > 4 ? r : min(r, n - 1)] * ldx))[q];
+            const Two xw[4] = {two_of(xv.x), two_of(xv.y), two_of(xv.z), two_of(xv.w)};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                fma_two(acc[2 * r], xw[j], gw[j]);
+                fma_two(acc[2 * r + 1], xw[j], uw[j]);
+            }
+        }
+    }
+}
+
+// The sums over the lanes of 2 NB values; lane (v * 16 / NB) ends with value v.
+template <int NB>
+__device__ __forceinline__ float lane_sums(const Two* acc, int lane) {
+    float s[2 * NB];
+#pragma unroll
+    for (int v = 0; v < 2 * NB; ++v) s[v] = sum_two(acc[v]);
+    int half = NB;
+#pragma unroll
+    for (int bit = 16; bit > 0; bit >>= 1) {
+        if (half > 0) {
+            const bool upper = (lane & bit) != 0;
+#pragma unroll
+            for (int v = 0; v < NB; ++v)
+                if (v < half) {
+                    const float give = upper ? s[v] : s[v + half], keep = upper ? s[v + half] : s[v];
+                    s[v] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+                }
+            half >>= 1;
+        } else {
+            s[0] += __shfl_xor_sync(0xffffffffu, s[0], bit);
+        }
+    }
+    return s[0];
+}
+
+template <int NB, bool DOWN>
+__device__ __forceinline__ void stream_store(const StreamArgs& p, const Two* acc, const int* pairs, int n, int unit, int lane) {
+    const float v = lane_sums<NB>(acc, lane);
+    constexpr int EACH = 16 / NB;                        // lanes that hold the same value
+    const float up = __shfl_down_sync(0xffffffffu, v, EACH);
+    const int value = lane / EACH, r = value >> 1;
+    if (lane % EACH != 0 || r >= n) return;
+    if (DOWN) {
+        const int c = 2 * unit + (value & 1);
+        if (c < p.width) ((float*)p.out)[(size_t)pairs[r] * p.width + c] = v;
+    } else if ((value & 1) == 0) {
+        fr_store((bf16*)p.out + (size_t)pairs[r] * p.units + unit, fr_gated(p.kind, v, up, p.limit, p.slope));
+    }
+}
+
 template <bool DOWN>
-__global__ void __launch_bounds__(32 * STREAM_WARPS, 3)
+__global__ void __launch_bounds__(32 * STREAM_WARPS, 2)
 expert_stream_kernel(const StreamArgs p) {
-    __shared__ float red[2][STREAM_WARPS][SHARE][STREAM_ROWS + 1];
+    extern __shared__ __align__(16) unsigned char raw[];
     __shared__ int count[256], group_expert[256 + MAX_FEW_PAIRS / SHARE], group_at[256 + MAX_FEW_PAIRS / SHARE], group_n[256 + MAX_FEW_PAIRS / SHARE];
     __shared__ int pair_of[MAX_FEW_PAIRS], row_of[MAX_FEW_PAIRS], id_of[MAX_FEW_PAIRS], place_of[MAX_FEW_PAIRS], n_groups;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -260,77 +336,53 @@ expert_stream_kernel(const StreamArgs p) {
         row_of[count[e] + place_of[i]] = i / p.x_share;
     }
     __syncthreads();
-    const int weight_rows = DOWN ? p.width : 2 * p.units, units = (weight_rows + STREAM_ROWS - 1) / STREAM_ROWS, total = n_groups * units;
-    const int g = lane >> 2, t = lane & 3;
-    uint4 w[STREAM_STEPS];
-    auto fetch = [&](int item, int k0) {
-        const int group = item / units, row = min((item - group * units) * STREAM_ROWS + g, weight_rows - 1);
-        const bf16* src = p.w + (size_t)group_expert[group] * p.w_expert + (size_t)row * p.ld + t * 8;
+    const int total = n_groups * p.units, step = gridDim.x * STREAM_WARPS;
+    const int pieces = (p.k + PIECE - 1) / PIECE, q_end = p.k / 8;
+    uint4* ring = (uint4*)raw + warp * (RING * 2 * PIECE / 8);
+    // the next piece to fetch: piece `fetch_piece` of item `fetch`; an item is (group, unit)
+    int fetch = blockIdx.x * STREAM_WARPS + warp, fetch_piece = 0, fetch_slot = 0;
+    auto fetch_next = [&]() {
+        if (fetch < total) {
+            const int g = fetch / p.units, unit = fetch - g * p.units;
+            const bf16* w0 = p.w + (size_t)group_expert[g] * p.w_expert + (size_t)(2 * unit) * p.ld;
+            const bf16* w1 = DOWN && 2 * unit + 1 >= p.width ? w0 : w0 + p.ld;
+            uint4* slot = ring + fetch_slot * (2 * PIECE / 8);
 #pragma unroll
-        for (int s = 0; s < STREAM_STEPS; ++s) {
-            const int k = k0 + s * 32;
-            w[s] = make_uint4(0, 0, 0, 0);
-            if (k + t * 8 < p.k)
-                asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w[s].x), "=r"(w[s].y), "=r"(w[s].z), "=r"(w[s].w) : "l"(src + k));
+            for (int i = 0; i < PIECE / 256; ++i) {
+                const int q = fetch_piece * (PIECE / 8) + lane + 32 * i;
+                if (q < q_end) {
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(slot + lane + 32 * i)), "l"((const uint4*)w0 + q) : "memory");
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(slot + PIECE / 8 + lane + 32 * i)), "l"((const uint4*)w1 + q) : "memory");
+                }
+            }
+            if (++fetch_piece == pieces) { fetch_piece = 0; fetch += step; }
+            if (++fetch_slot == RING) fetch_slot = 0;
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    int item = blockIdx.x, buf = 0;
-    if (item < total) fetch(item, warp * STREAM_K);
-    while (item < total) {
-        const int group = item / units, first = (item - group * units) * STREAM_ROWS, n = group_n[group];
-        const int* pairs = pair_of + group_at[group];
-        const int* rows = row_of + group_at[group];
-        const bf16* x0 = p.x + (size_t)rows[min(g, n - 1)] * p.k + t * 8;
-        const bf16* x1 = p.x + (size_t)rows[min(g + 8, n - 1)] * p.k + t * 8;
-        float acc[2][4] = {};
-        for (int k0 = warp * STREAM_K;;) {
 #pragma unroll
-            for (int s = 0; s < STREAM_STEPS; ++s) {
-                const int k = k0 + s * 32;
-                if (k >= p.k) break;
-                const bool there = k + t * 8 < p.k;
-                uint4 b = there ? *(const uint4*)(x0 + k) : make_uint4(0, 0, 0, 0);
-                const uint32_t lo[4] = {w[s].x, 0u, w[s].y, 0u}, hi[4] = {w[s].z, 0u, w[s].w, 0u};
-                mma_16816(acc[0], lo, b.x, b.y);
-                mma_16816(acc[0], hi, b.z, b.w);
-                if (n > 8) {
-                    b = there ? *(const uint4*)(x1 + k) : make_uint4(0, 0, 0, 0);
-                    mma_16816(acc[1], lo, b.x, b.y);
-                    mma_16816(acc[1], hi, b.z, b.w);
-                }
-            }
-            k0 += STREAM_WARPS * STREAM_K;
-            if (k0 >= p.k) break;
-            fetch(item, k0);
+    for (int i = 0; i < RING - 1; ++i) fetch_next();
+    int slot = 0;
+    auto unit_of = [&](auto nb, int g, int unit, int n) {
+        constexpr int NB = decltype(nb)::value;
+        Two acc[2 * NB];
+#pragma unroll
+        for (int v = 0; v < 2 * NB; ++v) acc[v] = 0ull;
+        for (int piece = 0; piece < pieces; ++piece) {
+            fetch_next();                                // into the slot that was read last
+            asm volatile("cp.async.wait_group %0;" ::"n"(RING - 1) : "memory");
+            stream_piece<NB>(ring + slot * (2 * PIECE / 8), p.x, p.k, row_of + group_at[g], n, piece * (PIECE / 8), q_end, lane, acc);
+            if (++slot == RING) slot = 0;
         }
-        item += gridDim.x;
-        if (item < total) fetch(item, warp * STREAM_K);      // on their way while this unit's sums meet
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = 0; j < 2; ++j) red[buf][warp][8 * i + 2 * t + j][g] = acc[i][j];
-        __syncthreads();                                     // (the other buffer's sums have been taken: everyone is past them)
-        if (DOWN) {
-            const int r = threadIdx.x >> 3, c = threadIdx.x & 7;
-            if (r < n && first + c < p.width) {
-                float v = 0.f;
-#pragma unroll
-                for (int j = 0; j < STREAM_WARPS; ++j) v += red[buf][j][r][c];
-                ((float*)p.out)[(size_t)pairs[r] * p.width + first + c] = v;
-            }
-        } else {
-            const int r = threadIdx.x >> 2, c = threadIdx.x & 3, unit = (first >> 1) + c;
-            if (r < n && unit < p.units) {
-                float v = 0.f, u = 0.f;
-#pragma unroll
-                for (int j = 0; j < STREAM_WARPS; ++j) {
-                    v += red[buf][j][r][2 * c];
-                    u += red[buf][j][r][2 * c + 1];
-                }
-                fr_store((bf16*)p.out + (size_t)pairs[r] * p.units + unit, fr_gated(p.kind, v, u, p.limit, p.slope));
-            }
-        }
-        buf ^= 1;
+        stream_store<NB, DOWN>(p, acc, pair_of + group_at[g], n, unit, lane);
+    };
+    for (int item = blockIdx.x * STREAM_WARPS + warp; item < total; item += step) {
+        const int g = item / p.units, unit = item - g * p.units, n = group_n[g];
+        if (n == 1) unit_of(Number<1>{}, g, unit, n);
+        else if (n == 2) unit_of(Number<2>{}, g, unit, n);
+        else if (n <= 4) unit_of(Number<4>{}, g, unit, n);
+        else if (n <= 8) unit_of(Number<8>{}, g, unit, n);
+        else unit_of(Number<16>{}, g, unit, n);
     }
 }
 
@@ -478,9 +530,17 @@ inline bool few_pairs_stream(int rows, int top, int experts, int k, int ld) {
 
 template <bool DOWN>
 int launch_stream(const StreamArgs& p, cudaStream_t stream) {
-    const int sms = fr_sm_count() > 0 ? fr_sm_count() : 148, rows = DOWN ? p.width : 2 * p.units;
-    const long long most = (long long)p.pairs * ((rows + STREAM_ROWS - 1) / STREAM_ROWS);          // blocks that can find a unit
-    FR_CUDA(fr_launch(expert_stream_kernel<DOWN>, dim3((unsigned)(most < 3 * sms ? most : 3 * sms)), dim3(32 * STREAM_WARPS), 0, stream, p));
+    static std::atomic<unsigned long long> configured{0};          // devices (as bits) on which the limit has been raised
+    int device = 0;
+    FR_CUDA(cudaGetDevice(&device));
+    if (device < 0 || device >= 64) FR_REFUSE("experts: device %d is outside the table of 64", device);
+    if (!(configured.load(std::memory_order_acquire) & (1ull << device))) {
+        FR_CUDA(cudaFuncSetAttribute(expert_stream_kernel<DOWN>, cudaFuncAttributeMaxDynamicSharedMemorySize, STREAM_SMEM));
+        configured.fetch_or(1ull << device, std::memory_order_release);
+    }
+    const int sms = fr_sm_count() > 0 ? fr_sm_count() : 148;
+    const long long most = ((long long)p.pairs * p.units + STREAM_WARPS - 1) / STREAM_WARPS;      // blocks that can find a unit
+    FR_CUDA(fr_launch(expert_stream_kernel<DOWN>, dim3((unsigned)(most < 2 * sms ? most : 2 * sms)), dim3(32 * STREAM_WARPS), STREAM_SMEM, stream, p));
     FR_CHECK_LAUNCH("experts (streamed)");
     return FR_OK;
 }

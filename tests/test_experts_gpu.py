@@ -126,3 +126,22 @@ def test_grouped_product_of_planes(groups, size, n, k):
     for e in range(groups):
         a, b = x[:, e * k:(e + 1) * k].double(), w[:, e * k:(e + 1) * k].double()
         assert bool(((out[e * size:(e + 1) * size].double() - a @ b.T).abs() <= k * 2.0 ** -23 * (a.abs() @ b.abs().T)).all())
+
+
+# The down product's sums are fp32 multiply-adds that round: a lane adds k / 64 terms in each of two sums, whose partial sums grow like
+# the square root of their number, each addition off by 2^-24 / sqrt(3) (root mean square) of the sum so far at most; over all sums that is
+# 2^-24 / sqrt(3) * sqrt(k / 128) of the result's norm.  (An accumulator that drops bits is two to five times as far off.)
+@pytest.mark.parametrize("rows,top", [(1, 8), (8, 2), (16, 3)])
+@pytest.mark.parametrize("inner", [1024, 2048, 4096])
+def test_streamed_experts_sums_round(rows, top, inner):
+    r = lib.family("routed")
+    r.declare("routed_down_combine", [P, P, P, P, I, P, P, I, I, I, I, I, I, P, I, P])
+    width, experts = 512, 8
+    ids = torch.stack([torch.randperm(experts, generator=torch.Generator().manual_seed(i))[:top] for i in range(rows)]).int().to(DEV)
+    act, down = rnd((rows * top, inner), 5), rnd((width, experts * inner), 6)
+    weights, scratch, out = torch.ones((rows, top), device=DEV), torch.empty(rows * top * width, device=DEV), torch.empty((rows, width), device=DEV)
+    r.call("routed_down_combine", ptr(act), ptr(ids), ptr(weights), ptr(down), experts * inner, None, ptr(out), 0, rows, top, experts, width, inner,
+           ptr(scratch), 1, stream())
+    want = torch.stack([down[:, e * inner:(e + 1) * inner].double() @ act[pair].double() for pair, e in enumerate(ids.flatten().tolist())])
+    error = (scratch.view(rows * top, width).double() - want).norm() / want.norm()
+    assert float(error) <= 2.0 ** -24 / 3 ** 0.5 * (inner / 128) ** 0.5
