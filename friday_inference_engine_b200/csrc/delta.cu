@@ -22,7 +22,8 @@
 //   step           all of it and the heads' gated norm for one token per sequence (below)
 //
 // State of a sequence: [taps-1][channels] history (channel order of the stacked projection: q, k, v), then the heads'
-// matrices [heads][dk][dv], all fp32.  Everything here is fp32 arithmetic; only the projection's rows may be bf16.
+// matrices [heads][dk][dv], all fp32.  Everything here is fp32 arithmetic (scan_chunks: also 64-bit, and products of fp32 numbers on the
+// tensor cores as sums of three bf16); only the projection's rows may be bf16.
 #include <math.h>
 
 #include <atomic>

@@ -10,23 +10,25 @@
 //
 //     U = U0 - W S0,    o_t = S0^T (Gamma_t q_t) + sum_(s <= t) B_ts u_s,    S = Gamma_16 S0 + sum_s (Gamma_16 / Gamma_s k_s) u_s^T.
 //
-// The walk along a sequence is then three small products per chunk instead of sixteen tokens' chains of sums.  Ratios of decays
-// are running products, never quotients or differences of logarithms.
+// (the blocked form of the rule by its triangular system: Yang et al., "Parallelizing linear transformers with the delta rule over
+// sequence length", 2024).  The walk along a sequence is then three small products per chunk instead of sixteen tokens' chains of sums.
+// Ratios of decays are running products, never quotients or differences of logarithms.
 //
 // Two kernels.  The first prepares every chunk of every head (A, B, the triangular solution by forward substitution, a thread per
-// channel; fp32), all of them at a time.  The second walks the chunks: a block owns one head of one sequence and 64 value
-// channels; four warps fetch the prepared operands two chunks ahead, four warps, 16 value channels each, multiply on the tensor
-// cores (mma.sync.m16n8k16): a warp keeps its channels' transposed state, fp32, in the layout of the instruction's
-// accumulators, which is also that of its first operand, so that nothing but the prepared operands passes through shared memory.
-// Every operand is three bf16 numbers (hi + mid + lo, all 24 bits) and a product the six partial products that reach
-// 2^-18 of it; hi hi has an accumulator of its own, whose sums over 32 key channels are added in fp32 registers, the state's decay and
-// sum are fp32 multiply-adds, so that the errors stay those of fp32 sums.  (Prepared by the walking block itself, a chunk took
-// as long as its preparation, 8,500 cycles.)
+// channel), all of them at a time, in 64 bits: its results round once, when they are stored.  The second walks the chunks: a block owns
+// one head of one sequence and 64 value channels; four warps fetch the prepared operands two chunks ahead, four warps, 16 value channels
+// each, walk.  W S0 and S0^T (Gamma q) run on the tensor cores (mma.sync.m16n8k16): a warp keeps its channels' transposed state, fp32,
+// in the layout of the instruction's accumulators, which is also that of its first operand.  Their operands are three bf16 numbers (hi +
+// mid + lo: all 24 bits of magnitudes above 2^-110, fewer below) and a product the six partial products that reach 2^-18 of it; hi hi has an
+// accumulator of its own, whose sums over 16 key channels are added in fp32 registers.  What goes into a result as it is, the sum over B
+// and the state's decay and sum, are fp32 multiply-adds, which round: on the tensor cores, whose accumulators drop bits, the state's
+// error was up to 1.2 times that of the walk token by token.
 //
-// The walk is bound by the rate of mma.sync (four fifths of it on a busy SM) and by its longest sequence.  Measured on B200, heads of 128, us token
-// by token and so, with a decay per head and per channel: 16 heads, 8 prompts of 64 to 512 tokens 313 -> 177 and 479 -> 203, one of
-// 2,048 551 -> 367 and 693 -> 389, 8 of 64 63 -> 45 and 107 -> 49; 32 heads, 16 of 300 858 -> 650 and 1,618 -> 749.  Errors against
-// 64 bits: of outputs never larger (1.8e-7 and 1.6e-7 in the first, 1.3e-7 both in the second), of states 0.75 to 1.06 times.
+// Errors against 64 bits, in units of those token by token (norms, three sequences of up to 400 tokens, decays of exp(-0.03) to exp(-2) a
+// token, keys with something or nothing in common): outputs 0.69 to 0.97, states 0.91 to 1.00 (nearly parallel keys 1.02).  Measured on B200, heads of 128, us token by token and so, with
+// a decay per head and per channel: 16 heads, 8 prompts of 64 to 512 tokens 300 -> 202 and 618 -> 241, one of 2,048 552 -> 480 and 913 -> 516;
+// 32 heads, 16 of 300 857 -> 880 and 2,990 -> 1,032 (with both products of the state on the tensor cores and the preparation in fp32: 155 and 181, 365 and
+// 387, 640 and 737).
 #pragma once
 #include "mma_sync.cuh"
 
@@ -40,17 +42,18 @@ constexpr int WALK_THREADS = 128, FETCH_THREADS = 128, PREP_THREADS = 256;
 constexpr int CHUNK_STAGES = 3;      // prepared chunks in a walking block's shared memory
 
 struct ChunkOperands {               // a prepared chunk of one head
-    bf16 w[3][CT][CLD], q[3][CT][CLD], k[3][CT][CLD];
-    bf16 b[3][CT][CT + 8];
+    bf16 w[3][CT][CLD], q[3][CT][CLD];
+    float k[CT][CD];                 // Gamma_16 / Gamma_s k_s
+    float b[CT][CT];                 // B_ts at [s][t]
     float gamma[CD];
 };
 typedef float ChunkValues[CT][CV + 4];                       // U0 of 64 value channels
 struct PrepShared {
     ChunkOperands ops;
-    float q[CT][CD], k[CT][CD];      // its rows as they come
-    float g[CT][CD];                 // decays (one per token in the first row where a head has one)
-    float a[CT][CT];
-    float beta[CT];
+    double q[CT][CD], k[CT][CD];     // its rows as they come
+    double g[CT][CD];                // decays (one per token in the first row where a head has one)
+    double a[CT][CT];
+    double beta[CT];
 };
 struct WalkShared {
     ChunkOperands ops[CHUNK_STAGES];
@@ -110,12 +113,15 @@ __device__ __forceinline__ void add_to(float (&sum)[N][4], const float (&v)[N][4
 #pragma unroll
         for (int e = 0; e < 4; ++e) sum[i][e] += v[i][e];
 }
+typedef unsigned long long Pair2;    // two floats
+__device__ __forceinline__ Pair2 pair_of(float lo, float hi) { return (Pair2)__float_as_uint(lo) | (Pair2)__float_as_uint(hi) << 32; }
+__device__ __forceinline__ void fma_pair2(Pair2& acc, Pair2 x, Pair2 y) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(x), "l"(y)); }
 __device__ __forceinline__ void walk_bar_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(WALK_THREADS + FETCH_THREADS) : "memory"); }
 __device__ __forceinline__ void walk_bar_arrive(int id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(WALK_THREADS + FETCH_THREADS) : "memory"); }
 constexpr int BAR_FULL = 1, BAR_EMPTY = 1 + CHUNK_STAGES;     // one of each per stage
 
 template <typename TR, bool PER_CHANNEL>
-__global__ void __launch_bounds__(PREP_THREADS, 3) delta_prepare_chunks_kernel(const ChunkArgs args) {
+__global__ void __launch_bounds__(PREP_THREADS, 2) delta_prepare_chunks_kernel(const ChunkArgs args) {
     extern __shared__ __align__(16) unsigned char chunk_smem[];
     PrepShared& sm = *(PrepShared*)chunk_smem;
     const ScanArgs& p = args.s;
@@ -142,8 +148,10 @@ __global__ void __launch_bounds__(PREP_THREADS, 3) delta_prepare_chunks_kernel(c
             q4 = *(const float4*)row;
             k4 = *(const float4*)(row + qk);
         }
-        *(float4*)&sm.q[t][i] = q4;
-        *(float4*)&sm.k[t][i] = k4;
+        *(double2*)&sm.q[t][i] = make_double2(q4.x, q4.y);
+        *(double2*)&sm.q[t][i + 2] = make_double2(q4.z, q4.w);
+        *(double2*)&sm.k[t][i] = make_double2(k4.x, k4.y);
+        *(double2*)&sm.k[t][i + 2] = make_double2(k4.z, k4.w);
     }
     if (PER_CHANNEL) {
 #pragma unroll
@@ -160,25 +168,25 @@ __global__ void __launch_bounds__(PREP_THREADS, 3) delta_prepare_chunks_kernel(c
 #pragma unroll 1
     for (int turn = 0; turn < 2; ++turn) {
         const int s = turn == 0 ? warp : CT - 1 - warp;
-        float val[32];                                        // A_ts of t = 0 .. 15, then B_ts
-        float4 x = *(const float4*)&sm.k[s][4 * lane];
+        double val[32];                                       // A_ts of t = 0 .. 15, then B_ts
+        double2 x = *(const double2*)&sm.k[s][2 * lane], y = *(const double2*)&sm.k[s][64 + 2 * lane];
 #pragma unroll
         for (int t = 0; t < CT; ++t) {
-            val[t] = val[CT + t] = 0.f;
+            val[t] = val[CT + t] = 0.0;
             if (t >= s) {
-                const float4 qt = *(const float4*)&sm.q[t][4 * lane];
+                const double2 q0 = *(const double2*)&sm.q[t][2 * lane], q1 = *(const double2*)&sm.q[t][64 + 2 * lane];
                 if (t > s) {
-                    const float4 kt = *(const float4*)&sm.k[t][4 * lane];
+                    const double2 k0 = *(const double2*)&sm.k[t][2 * lane], k1 = *(const double2*)&sm.k[t][64 + 2 * lane];
                     if (PER_CHANNEL) {
-                        const float4 g = *(const float4*)&sm.g[t][4 * lane];
-                        x.x *= g.x; x.y *= g.y; x.z *= g.z; x.w *= g.w;
+                        const double2 g0 = *(const double2*)&sm.g[t][2 * lane], g1 = *(const double2*)&sm.g[t][64 + 2 * lane];
+                        x.x *= g0.x; x.y *= g0.y; y.x *= g1.x; y.y *= g1.y;
                     } else {
-                        const float g = sm.g[0][t];
-                        x.x *= g; x.y *= g; x.z *= g; x.w *= g;
+                        const double g = sm.g[0][t];
+                        x.x *= g; x.y *= g; y.x *= g; y.y *= g;
                     }
-                    val[t] = fmaf(x.x, kt.x, x.y * kt.y) + fmaf(x.z, kt.z, x.w * kt.w);
+                    val[t] = fma(x.x, k0.x, x.y * k0.y) + fma(y.x, k1.x, y.y * k1.y);
                 }
-                val[CT + t] = fmaf(x.x, qt.x, x.y * qt.y) + fmaf(x.z, qt.z, x.w * qt.w);
+                val[CT + t] = fma(x.x, q0.x, x.y * q0.y) + fma(y.x, q1.x, y.y * q1.y);
             }
         }
         // every value summed over the lanes; lane l ends with the l-th
@@ -187,50 +195,48 @@ __global__ void __launch_bounds__(PREP_THREADS, 3) delta_prepare_chunks_kernel(c
             const bool upper = (lane & half) != 0;
 #pragma unroll
             for (int v = 0; v < half; ++v) {
-                const float give = upper ? val[v] : val[v + half], keep = upper ? val[v + half] : val[v];
+                const double give = upper ? val[v] : val[v + half], keep = upper ? val[v + half] : val[v];
                 val[v] = keep + __shfl_xor_sync(0xffffffffu, give, half);
             }
         }
         const int t = lane & (CT - 1);
         if (lane < CT) sm.a[t][s] = val[0];
-        else split3(val[0], o.b[0][t][s], o.b[1][t][s], o.b[2][t][s]);
+        else o.b[s][t] = (float)val[0];
     }
     __syncthreads();
     // the triangular solutions, a thread per channel
-    auto solve = [&](float (&x)[CT]) {                        // x: right hand sides without beta, then the solutions
+    auto solve = [&](double (&x)[CT]) {                       // x: right hand sides without beta, then the solutions
 #pragma unroll
         for (int t = 0; t < CT; ++t) {
-            float r0s = 0.f, r1s = 0.f, r2s = 0.f, r3s = 0.f;
+            double r0s = 0.0, r1s = 0.0;
 #pragma unroll
-            for (int s = 0; s < t; s += 4) {
-                const float4 row = *(const float4*)&sm.a[t][s];
-                r0s = fmaf(row.x, x[s], r0s);
-                if (s + 1 < t) r1s = fmaf(row.y, x[s + 1], r1s);
-                if (s + 2 < t) r2s = fmaf(row.z, x[s + 2], r2s);
-                if (s + 3 < t) r3s = fmaf(row.w, x[s + 3], r3s);
+            for (int s = 0; s < t; s += 2) {
+                const double2 row = *(const double2*)&sm.a[t][s];
+                r0s = fma(row.x, x[s], r0s);
+                if (s + 1 < t) r1s = fma(row.y, x[s + 1], r1s);
             }
-            x[t] = sm.beta[t] * (x[t] - ((r0s + r1s) + (r2s + r3s)));
+            x[t] = sm.beta[t] * (x[t] - (r0s + r1s));
         }
     };
-    float x[CT];
+    double x[CT];
     if (who < CD) {
-        float gam = 1.f;
+        double gam = 1.0;
 #pragma unroll
         for (int t = 0; t < CT; ++t) {
             gam *= PER_CHANNEL ? sm.g[t][who] : sm.g[0][t];
             x[t] = gam * sm.k[t][who];
-            split3(gam * sm.q[t][who], o.q[0][t][who], o.q[1][t][who], o.q[2][t][who]);
+            split3((float)(gam * sm.q[t][who]), o.q[0][t][who], o.q[1][t][who], o.q[2][t][who]);
         }
-        o.gamma[who] = gam;
+        o.gamma[who] = (float)gam;
         solve(x);
 #pragma unroll
-        for (int t = 0; t < CT; ++t) split3(x[t], o.w[0][t][who], o.w[1][t][who], o.w[2][t][who]);
+        for (int t = 0; t < CT; ++t) split3((float)x[t], o.w[0][t][who], o.w[1][t][who], o.w[2][t][who]);
     } else {
         const int i = who - CD;
-        float left = 1.f;
+        double left = 1.0;
 #pragma unroll
         for (int t = CT - 1; t >= 0; --t) {
-            split3(left * sm.k[t][i], o.k[0][t][i], o.k[1][t][i], o.k[2][t][i]);
+            o.k[t][i] = (float)(left * sm.k[t][i]);
             left *= PER_CHANNEL ? sm.g[t][i] : sm.g[0][t];
         }
         for (int j = i; j < args.value_blocks * CV; j += PREP_THREADS - CD) {
@@ -240,7 +246,7 @@ __global__ void __launch_bounds__(PREP_THREADS, 3) delta_prepare_chunks_kernel(c
             solve(x);
             float* u = &args.u0[at * args.value_blocks + j / CV][0][j % CV];
 #pragma unroll
-            for (int t = 0; t < CT; ++t) u[t * (CV + 4)] = x[t];
+            for (int t = 0; t < CT; ++t) u[t * (CV + 4)] = (float)x[t];
         }
     }
     __syncthreads();
@@ -286,7 +292,6 @@ __device__ __forceinline__ void walk_chunks(const ScanArgs& p, WalkShared& sm, i
             s[j][e] = i < p.dk && col < p.dv ? S[(size_t)i * p.dv + col] : 0.f;
         }
     const int mi = lane >> 3, row_n = (mi >> 1) * 8 + (lane & 7), at_n = (mi & 1) * 8;       // ldmatrix: [n][k] tiles
-    const int row_t = (mi & 1) * 8 + (lane & 7), at_t = (mi >> 1) * 8;                       // transposed: [k][n] tiles
     for (int c = 0; c < chunks; ++c) {
         const int stage = c % CHUNK_STAGES;
         const ChunkOperands& o = sm.ops[stage];
@@ -308,9 +313,9 @@ __device__ __forceinline__ void walk_chunks(const ScanArgs& p, WalkShared& sm, i
                 ldsm4(b[0][pl], &o.w[pl][row_n][ks * 16 + at_n]);
                 ldsm4(b[1][pl], &o.q[pl][row_n][ks * 16 + at_n]);
             }
-            if (ks % 2 == 0) clear(large);
+            clear(large);
             mma_split<4>(large, small, a, b);
-            if (ks % 2 == 1) add_to(sum, large);
+            add_to(sum, large);
         }
         add_to(sum, small);
         float u[2][4], out2[2][4];
@@ -321,42 +326,29 @@ __device__ __forceinline__ void walk_chunks(const ScanArgs& p, WalkShared& sm, i
                 u[i][e] = sm.u0[stage][8 * i + 2 * t + (e & 1)][local + (e < 2 ? 0 : 8)] - sum[i][e];
                 out2[i][e] = sum[2 + i][e];
             }
-        uint32_t ua[3][4];
+        // every token's correction of this lane's two columns
+        float ul[CT], uh[CT];
 #pragma unroll
-        for (int r = 0; r < 4; ++r) split3(u[r >> 1][2 * (r & 1)], u[r >> 1][2 * (r & 1) + 1], ua[0][r], ua[1][r], ua[2][r]);
-        float finite = 0.f;
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) finite = fmaf(0.f, u[i][e], finite);
-        if (!__any_sync(0xffffffffu, finite != finite)) {
-            uint32_t b[1][3][4];
-#pragma unroll
-            for (int pl = 0; pl < 3; ++pl) ldsm4(b[0][pl], &o.b[pl][row_n][at_n]);
-            float bl[2][4], bs[2][4];
-            clear(bl);
-            clear(bs);
-            mma_split<2>(bl, bs, ua, b);
-            add_to(bl, bs);
-            add_to(out2, bl);
-        } else {
-            // a correction that is not finite reaches its own token and those after it only: no product with a zero of B
-#pragma unroll
-            for (int src = 0; src < CT; ++src) {
-                const int from = (lane & ~3) | ((src & 7) >> 1);
-                const float lo = __shfl_sync(0xffffffffu, u[src >> 3][src & 1], from), hi = __shfl_sync(0xffffffffu, u[src >> 3][2 + (src & 1)], from);
-#pragma unroll
-                for (int i = 0; i < 2; ++i)
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const int to = 8 * i + 2 * t + e;
-                        if (to < src) continue;
-                        const float w = __bfloat162float(o.b[0][to][src]) + (__bfloat162float(o.b[1][to][src]) + __bfloat162float(o.b[2][to][src]));
-                        out2[i][e] = fmaf(w, lo, out2[i][e]);
-                        out2[i][2 + e] = fmaf(w, hi, out2[i][2 + e]);
-                    }
-            }
+        for (int src = 0; src < CT; ++src) {
+            const int from = (lane & ~3) | ((src & 7) >> 1);
+            ul[src] = __shfl_sync(0xffffffffu, u[src >> 3][src & 1], from);
+            uh[src] = __shfl_sync(0xffffffffu, u[src >> 3][2 + (src & 1)], from);
         }
+        // (a token's correction reaches itself and those after it only, whatever its value is)
+#pragma unroll
+        for (int src = 0; src < CT; ++src)
+#pragma unroll
+            for (int i = src >> 3; i < 2; ++i) {
+                const float2 w = *(const float2*)&o.b[src][8 * i + 2 * t];
+                if (8 * i + 2 * t >= src) {
+                    out2[i][0] = fmaf(w.x, ul[src], out2[i][0]);
+                    out2[i][2] = fmaf(w.x, uh[src], out2[i][2]);
+                }
+                if (8 * i + 2 * t + 1 >= src) {
+                    out2[i][1] = fmaf(w.y, ul[src], out2[i][1]);
+                    out2[i][3] = fmaf(w.y, uh[src], out2[i][3]);
+                }
+            }
         float* out = p.out + (size_t)(r0 + c * CT) * ((size_t)p.heads * p.dv) + (size_t)head * p.dv;
         const int nt = min(CT, n - c * CT);
 #pragma unroll
@@ -366,25 +358,36 @@ __device__ __forceinline__ void walk_chunks(const ScanArgs& p, WalkShared& sm, i
                 const int tok = 8 * i + 2 * t + (e & 1), col = e < 2 ? c_lo : c_hi;
                 if (tok < nt && col < p.dv) out[(size_t)tok * p.heads * p.dv + col] = out2[i][e];
             }
+        // two channels of a column per instruction
+        Pair2 pl[CT], ph[CT];
 #pragma unroll
-        for (int jt = 0; jt < CD / 16; jt += 2) {             // four tiles of eight key channels at a time
-            uint32_t b[2][3][4];
+        for (int src = 0; src < CT; ++src) {
+            pl[src] = pair_of(ul[src], ul[src]);
+            ph[src] = pair_of(uh[src], uh[src]);
+        }
 #pragma unroll
-            for (int pl = 0; pl < 3; ++pl) {
-                ldsm4t(b[0][pl], &o.k[pl][row_t][jt * 16 + at_t]);
-                ldsm4t(b[1][pl], &o.k[pl][row_t][(jt + 1) * 16 + at_t]);
+        for (int j0 = 0; j0 < CD / 8; j0 += 4) {              // four tiles of eight key channels at a time
+            Pair2 lo[4], hi[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float2 gam = *(const float2*)&o.gamma[8 * (j0 + j) + 2 * t];
+                float(&v)[4] = s[j0 + j];
+                lo[j] = pair_of(gam.x * v[0], gam.y * v[1]);
+                hi[j] = pair_of(gam.x * v[2], gam.y * v[3]);
             }
-            clear(large);
-            clear(small);
-            mma_split<4>(large, small, ua, b);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int j = 2 * jt + i;
-                const float2 gam = *(const float2*)&o.gamma[8 * j + 2 * t];
-                s[j][0] = fmaf(gam.x, s[j][0], large[i][0] + small[i][0]);
-                s[j][1] = fmaf(gam.y, s[j][1], large[i][1] + small[i][1]);
-                s[j][2] = fmaf(gam.x, s[j][2], large[i][2] + small[i][2]);
-                s[j][3] = fmaf(gam.y, s[j][3], large[i][3] + small[i][3]);
+            for (int src = 0; src < CT; ++src)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const Pair2 k2 = *(const Pair2*)&o.k[src][8 * (j0 + j) + 2 * t];
+                    fma_pair2(lo[j], k2, pl[src]);
+                    fma_pair2(hi[j], k2, ph[src]);
+                }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                float(&v)[4] = s[j0 + j];
+                v[0] = __uint_as_float((uint32_t)lo[j]); v[1] = __uint_as_float((uint32_t)(lo[j] >> 32));
+                v[2] = __uint_as_float((uint32_t)hi[j]); v[3] = __uint_as_float((uint32_t)(hi[j] >> 32));
             }
         }
         if (c + CHUNK_STAGES < chunks) walk_bar_arrive(BAR_EMPTY + stage);
