@@ -585,6 +585,23 @@ FR_EXPORT int delta_scan(const float* qkv, const void* a_raw, int ld_a, const vo
     FR_REFUSE("delta scan: unknown dtype %d", raw_dtype);
 }
 
+// Whether a prompt goes in chunks: where that was the faster of the two.  Measured on B200, us token by token and in chunks:
+//   up to 64 key channels, or few value channels: a chunk costs the same for any head size up to 128 and for 64 value channels at a time, a
+//   token does not (16 heads of 64, one of 2,048 tokens 433 and 480, 64 of 33 68 and 190): token by token.
+//   A decay per channel, 128 channels: from 32 tokens on (16 heads, one of 32 20 and 19, one of 2,048 913 and 516, 64 of 33 633 and 327).
+//   A decay per head, 128 value channels and more (of 64 it is behind: 4 of 1,000 287 and 352): a token costs 0.27 us along the longest
+//   sequence, a chunk 3.7, so chunks are ahead where the longest sequence is the bound (one of 64 23 and 24, of 256 74 and 64, of 2,048 552
+//   and 480, 16 heads) and where lengths differ (their walks start with the longest: 8 of 64 to 512 300 and 202); where equal sequences
+//   keep all SMs busy both take as long (16 of 300 441 and 439, 32 heads 857 and 880), and a chunk that is not full costs as much as a full
+//   one (64 of 33 255 and 291, one of 96 and 20 of 33 on 32 heads 199 and 212).
+FR_EXPORT int delta_scan_chunks_pays(int rows, int n_seqs, int max_q_len, int heads, int dk, int dv, int per_channel) {
+    if (dk <= 64 || dv < 64 || max_q_len < 32) return 0;
+    if (per_channel) return 1;
+    const bool longest_is_the_bound = (long long)rows * heads <= 128ll * max_q_len && rows >= 16ll * n_seqs;
+    const bool unequal = 4ll * rows < 3ll * max_q_len * n_seqs && rows >= 64ll * n_seqs;
+    return dv >= 128 && max_q_len >= 96 && (longest_is_the_bound || unequal);
+}
+
 // Bytes of scratch that delta_scan_chunks needs; 0: it does not take these sizes (rows in 16-byte pieces, a head's keys within a
 // chunk's tile).
 FR_EXPORT long long delta_scan_chunks_scratch(const float* qkv, int rows, int n_seqs, int heads, int dk, int dv) {

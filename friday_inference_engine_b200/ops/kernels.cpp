@@ -137,7 +137,7 @@ FAMILY(Ssd, ssd, "ssd", resolve(h, fam, "ssd_scratch_floats", t.scratch_floats);
        resolve(h, fam, "ssd_gate_group_norm", t.gate_group_norm);)
 FAMILY(Delta, delta, "delta", resolve(h, fam, "delta_conv_prepare", t.conv_prepare);
        resolve(h, fam, "delta_conv_state", t.conv_state); resolve(h, fam, "delta_scan", t.scan);
-       resolve(h, fam, "delta_scan_chunks_scratch", t.chunks_scratch); resolve(h, fam, "delta_scan_chunks", t.chunks);
+       resolve(h, fam, "delta_scan_chunks_pays", t.chunks_pays); resolve(h, fam, "delta_scan_chunks_scratch", t.chunks_scratch); resolve(h, fam, "delta_scan_chunks", t.chunks);
        resolve(h, fam, "delta_general_prepare", t.general_prepare); resolve(h, fam, "delta_general_scan", t.general_scan);
        resolve(h, fam, "delta_step_supports", t.step_supports); resolve(h, fam, "delta_step", t.step);)
 FAMILY(AttentionLatent, attention_latent, "attention_latent", resolve(h, fam, "attention_latent_rotate_pairs", t.rotate_pairs);

@@ -136,6 +136,7 @@ struct Delta {
                       int, int, int, cudaStream_t);
     int (*scan)(const float*, const void*, int, const void*, int, int, const void*, const void*, int, float*, float*, long long,
                 long long, const int*, const int*, const int*, const int*, int, int, int, int, int, int, cudaStream_t);
+    int (*chunks_pays)(int, int, int, int, int, int, int);
     long long (*chunks_scratch)(const float*, int, int, int, int, int);
     int (*chunks)(const float*, const void*, int, const void*, int, int, const void*, const void*, int, float*, float*, long long,
                   long long, const int*, const int*, const int*, const int*, int, int, int, int, int, int, int, int, void*, long long, cudaStream_t);

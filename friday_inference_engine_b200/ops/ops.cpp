@@ -830,11 +830,6 @@ Tensor Ops::conv_silu_unit(const Tensor& proj, const Tensor& taps, const DeltaSp
     return out;
 }
 
-// Tokens of the longest sequence from which on the delta rule goes in chunks of sixteen tokens.  Heads of 128, token by token and in chunks, us
-// (decay per head / per channel): 8 sequences of 17 tokens 25 and 29 / 46 and 32, one of 32 15 and 16 / 18 and 18, 8 of 40 42 and 35 / 75 and 37,
-// one of 64 (8 heads) 23 and 21 / 27 and 23.
-static constexpr int DELTA_CHUNKS_FROM = 32;
-
 Tensor Ops::delta_scan(const Tensor& qkv, const Tensor& a_raw, const Tensor& b_raw, const Tensor& a_log, const Tensor& dt_bias,
                        const DeltaSpec& s, const CacheView& view, const StepContext& ctx) {
     if (view.kind != CacheRequest::State || !view.state.defined() || view.state.dtype != DType::F32)
@@ -849,7 +844,7 @@ Tensor Ops::delta_scan(const Tensor& qkv, const Tensor& a_raw, const Tensor& b_r
     const auto& k = kernels::delta();
     Timed t(*this, Attention);
     const int rows = (int)qkv.rows();
-    const long long room = !ctx.decode && ctx.max_q_len >= DELTA_CHUNKS_FROM && ctx.rows == rows
+    const long long room = !ctx.decode && ctx.rows == rows && k.chunks_pays(rows, ctx.n_seqs, ctx.max_q_len, s.heads, s.dk, s.dv, s.per_channel ? 1 : 0)
                                ? k.chunks_scratch((const float*)qkv.data, rows, ctx.n_seqs, s.heads, s.dk, s.dv) : 0;
     if (room > 0) {
         float* scratch = scratch_floats((room + 3) / 4);

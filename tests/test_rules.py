@@ -1,0 +1,27 @@
+"""Which kernel a call goes to, asked of the built libraries on the host: on both sides of each line, at sizes that were timed."""
+import pytest
+
+from friday_inference_engine_b200.ops import lib
+
+
+def ask(family, name, *args):
+    try:
+        fam = lib.family(family)
+    except Exception as e:           # no compiler, or no CUDA runtime library to load against
+        pytest.skip("the %s library is not available here: %s" % (family, e))
+    fn = getattr(fam.cdll, name)
+    fn.argtypes = [lib.P if a is None else lib.c_longlong if abs(a) >= 1 << 31 else lib.I for a in args]
+    return fn(*args)
+
+
+# (lengths, heads, dk, dv), a decay per head, a decay per channel: whether chunks of sixteen tokens were the faster way
+@pytest.mark.parametrize("lens,heads,dk,dv,per_head,per_channel", [
+    ([2048], 16, 128, 128, 1, 1), ([256], 4, 128, 128, 1, 1), ([64], 16, 128, 128, 0, 1), ([32], 16, 128, 128, 0, 1), ([31], 16, 128, 128, 0, 0),
+    ([64, 512, 300, 128, 400, 90, 230, 480], 16, 128, 128, 1, 1), ([64, 512, 300, 128, 400, 90, 230, 480], 32, 128, 128, 1, 1),
+    ([300] * 16, 32, 128, 128, 0, 1), ([300] * 16, 4, 128, 128, 1, 1), ([33] * 64, 16, 128, 128, 0, 1), ([128] + [1] * 63, 16, 128, 128, 0, 1),
+    ([512] + [17] * 31, 16, 128, 128, 1, 1), ([2048], 16, 64, 64, 0, 0), ([2048], 16, 16, 128, 0, 0), ([300] * 8, 16, 128, 16, 0, 0),
+    ([1000] * 4, 16, 128, 64, 0, 1), ([96] + [33] * 20, 32, 128, 128, 0, 1),
+])
+def test_delta_rule_in_chunks(lens, heads, dk, dv, per_head, per_channel):
+    for flag, want in ((0, per_head), (1, per_channel)):
+        assert ask("delta", "delta_scan_chunks_pays", sum(lens), len(lens), max(lens), heads, dk, dv, flag) == want
