@@ -602,8 +602,8 @@ FR_EXPORT int delta_scan_chunks_pays(int rows, int n_seqs, int max_q_len, int he
     return dv >= 128 && max_q_len >= 96 && (longest_is_the_bound || unequal);
 }
 
-// Bytes of scratch that delta_scan_chunks needs; 0: it does not take these sizes (rows in 16-byte pieces, a head's keys within a
-// chunk's tile).
+// Bytes of scratch that delta_scan_chunks needs, CHUNK_SCRATCH at most; 0: it does not take these sizes (rows in 16-byte pieces, a head's
+// keys within a chunk's tile, a head's chunks within the scratch).
 FR_EXPORT long long delta_scan_chunks_scratch(const float* qkv, int rows, int n_seqs, int heads, int dk, int dv) {
     if (dk <= 0 || dk > CD || dk % 4 || dv <= 0 || dv % 4 || ((uintptr_t)qkv & 15) || rows <= 0 || n_seqs <= 0 || n_seqs > 65535 || heads <= 0 || heads > 65535) return 0;
     return chunk_head_bytes(rows, n_seqs, dv) * chunk_heads(rows, n_seqs, heads, dv);

@@ -438,11 +438,12 @@ long long chunk_slots(int rows, int n_seqs) { return (long long)rows / CT + n_se
 long long chunk_head_bytes(int rows, int n_seqs, int dv) {                 // scratch of one head
     return chunk_slots(rows, n_seqs) * (long long)(sizeof(ChunkOperands) + (dv + CV - 1) / CV * sizeof(ChunkValues));
 }
-// Heads go in equal rounds of what this holds (at least one per round).
-constexpr long long CHUNK_SCRATCH = 256ll << 20;
+// Heads go in equal rounds of what this holds (0: not even one head fits).  Twice what 16 heads of 128 with 2,048 tokens take; half of it
+// would cost them a second round.
+constexpr long long CHUNK_SCRATCH = 128ll << 20;
 int chunk_heads(int rows, int n_seqs, int heads, int dv) {
     const long long fit = CHUNK_SCRATCH / chunk_head_bytes(rows, n_seqs, dv);
-    if (fit < 1) return 1;
+    if (fit < 1) return 0;
     const long long rounds = (heads + fit - 1) / fit;
     return (int)((heads + rounds - 1) / rounds);
 }

@@ -457,7 +457,9 @@ private:
     void fusion_in(const Rows& x, GemmFusion& f) const;
     int device_, sms_;
     cudaStream_t stream_;
+    void* chunk_room(size_t bytes);                           // null: no memory for them now
     DeviceBuffer tc_scratch_, tc_counters_, status_, attn_counters_;
+    DeviceBuffer chunks_;                                     // prepared chunks of the delta rule's prompts (one stream uses them in turn)
     std::map<std::tuple<int64_t, int64_t, int64_t>, std::tuple<bool, int, int>> plans_;
     std::map<std::pair<int, int>, int> cluster_fit_;
     bool attn_tc_, profile_ = false;

@@ -830,6 +830,22 @@ Tensor Ops::conv_silu_unit(const Tensor& proj, const Tensor& taps, const DeltaSp
     return out;
 }
 
+// The chunks are dead when the call's kernels have run: one buffer, grown when a prompt needs more, serves every layer.  Where the device has
+// no memory for it (or a graph is being captured), the caller walks token by token, which needs none.
+void* Ops::chunk_room(size_t bytes) {
+    if (chunks_.bytes() >= bytes) return chunks_.get();
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream_, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return nullptr;
+    chunks_ = DeviceBuffer();
+    try {
+        chunks_ = DeviceBuffer(bytes);
+    } catch (const KernelError&) {
+        cudaGetLastError();                                   // (the failed allocation is dealt with)
+        return nullptr;
+    }
+    return chunks_.get();
+}
+
 Tensor Ops::delta_scan(const Tensor& qkv, const Tensor& a_raw, const Tensor& b_raw, const Tensor& a_log, const Tensor& dt_bias,
                        const DeltaSpec& s, const CacheView& view, const StepContext& ctx) {
     if (view.kind != CacheRequest::State || !view.state.defined() || view.state.dtype != DType::F32)
@@ -846,8 +862,7 @@ Tensor Ops::delta_scan(const Tensor& qkv, const Tensor& a_raw, const Tensor& b_r
     const int rows = (int)qkv.rows();
     const long long room = !ctx.decode && ctx.rows == rows && k.chunks_pays(rows, ctx.n_seqs, ctx.max_q_len, s.heads, s.dk, s.dv, s.per_channel ? 1 : 0)
                                ? k.chunks_scratch((const float*)qkv.data, rows, ctx.n_seqs, s.heads, s.dk, s.dv) : 0;
-    if (room > 0) {
-        float* scratch = scratch_floats((room + 3) / 4);
+    if (void* scratch = room > 0 ? chunk_room((size_t)room) : nullptr) {
         call(launches_, k, k.chunks((const float*)qkv.data, a_raw.data, (int)a_raw.ld, b_raw.data, (int)b_raw.ld, code(a_raw.dtype), a_log.data,
                                     dt_bias.data, code(a_log.dtype), (float*)out.data, (float*)view.state.data, stride, s_off, ctx.row_seq,
                                     ctx.seq_start, ctx.seq_qlen, view.seq_slots, ctx.n_seqs, s.heads, s.qk_heads, s.dk, s.dv,

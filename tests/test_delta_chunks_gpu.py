@@ -121,3 +121,15 @@ def test_errors_are_those_of_rounded_sums(rate, common, dk, dv, per_channel):
     for i in (0, 1):
         assert errors["delta_scan_chunks"][i] <= (1.1 if common else 1.02) * errors["delta_scan"][i]
         assert errors["delta_scan_chunks"][i] / 3 <= 1e-6             # losing a third bf16 number of any operand is 1.5e-6 and more
+
+
+# more heads than the scratch holds at a time: two rounds of 34 and 33, whose chunks lie at other places of it
+@pytest.mark.parametrize("per_channel", [False, True])
+def test_heads_in_uneven_rounds(per_channel):
+    c = inputs([700, 33, 267], 67, 1, 8, 4, per_channel, torch.float32)
+    need = lib.family("delta").declare("delta_scan_chunks_scratch", [P, I, I, I, I, I], L)(c["qkv"].data_ptr(), 1000, 3, 67, 8, 4)
+    one = lib.family("delta").declare("delta_scan_chunks_scratch", [P, I, I, I, I, I], L)(c["qkv"].data_ptr(), 1000, 3, 1, 8, 4)
+    assert need == 34 * one
+    out, state = run("delta_scan_chunks", c)
+    ref, ref_state = exact(c)
+    assert (out.double() - ref).norm() <= 1e-6 * ref.norm() and (state.double() - ref_state).norm() <= 1e-6 * ref_state.norm()
