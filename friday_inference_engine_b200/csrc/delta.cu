@@ -609,6 +609,12 @@ FR_EXPORT long long delta_scan_chunks_scratch(const float* qkv, int rows, int n_
     return chunk_head_bytes(rows, n_seqs, dv) * chunk_heads(rows, n_seqs, heads, dv);
 }
 
+// Kernels that delta_scan_chunks launches: two per round of heads.
+FR_EXPORT int delta_scan_chunks_launches(int rows, int n_seqs, int heads, int dv) {
+    const int at_once = rows > 0 && n_seqs > 0 && heads > 0 && dv > 0 ? chunk_heads(rows, n_seqs, heads, dv) : 0;
+    return at_once > 0 ? 2 * ((heads + at_once - 1) / at_once) : 0;
+}
+
 // delta_scan for prompts: the same arguments and results, sixteen tokens at a time (delta_chunks.cuh).  rows: of the whole step,
 // whose sequences' rows lie one sequence after another from row 0 on; max_q_len: of the longest sequence; scratch: 16-byte aligned.
 FR_EXPORT int delta_scan_chunks(const float* qkv, const void* a_raw, int ld_a, const void* b_raw, int ld_b, int raw_dtype, const void* a_log,

@@ -588,6 +588,12 @@ FR_EXPORT int gemm_simt_split_pays(const void* a, const void* w, int m, int n, i
     return weights >= 2ll << 20 ? m >= 48 || weights >= 6ll << 20 : weights >= 1ll << 20 && m > 64;
 }
 
+// Kernels that gemm_simt_split launches: two per portion of rows.
+FR_EXPORT int gemm_simt_split_launches(int m, int k, long long scratch_bytes) {
+    const int rows = m > 0 && k > 0 ? split_rows_at_once(m, k, scratch_bytes) : 0;
+    return rows > 0 ? 2 * ((m + rows - 1) / rows) : 0;
+}
+
 // scratch: 16-byte aligned, used by the kernels of this call only; status: a word that a wait that gave up is noted in.
 FR_EXPORT int gemm_simt_split(const float* a, const float* w, float* out, const void* bias, int bias_dtype, const float* residual, int m, int n,
                               int k, int lda, int ldw, int ldo, int fixed_weights, void* scratch, long long scratch_bytes, int* status,

@@ -97,6 +97,7 @@ FAMILY(Rowwise, rowwise, "rowwise",
        resolve(h, fam, "rowwise_random_normal", t.random_normal);)
 FAMILY(GemmSimt, gemm_simt, "gemm_simt", resolve(h, fam, "gemm_simt_weights", t.gemm);
        resolve(h, fam, "gemm_simt_split_pays", t.split_pays); resolve(h, fam, "gemm_simt_split", t.split);
+       resolve(h, fam, "gemm_simt_split_launches", t.split_launches);
        resolve(h, fam, "gemm_simt_few_supports", t.few_supports); resolve(h, fam, "gemm_simt_few", t.few);)
 FAMILY(GemmTc, gemm_tc, "gemm_tc", resolve(h, fam, "gemm_tc_fused", t.fused); resolve(h, fam, "gemm_tc_plan", t.plan);
        resolve(h, fam, "gemm_tc_grouped", t.grouped);)
@@ -138,6 +139,7 @@ FAMILY(Ssd, ssd, "ssd", resolve(h, fam, "ssd_scratch_floats", t.scratch_floats);
 FAMILY(Delta, delta, "delta", resolve(h, fam, "delta_conv_prepare", t.conv_prepare);
        resolve(h, fam, "delta_conv_state", t.conv_state); resolve(h, fam, "delta_scan", t.scan);
        resolve(h, fam, "delta_scan_chunks_pays", t.chunks_pays); resolve(h, fam, "delta_scan_chunks_scratch", t.chunks_scratch); resolve(h, fam, "delta_scan_chunks", t.chunks);
+       resolve(h, fam, "delta_scan_chunks_launches", t.chunks_launches);
        resolve(h, fam, "delta_general_prepare", t.general_prepare); resolve(h, fam, "delta_general_scan", t.general_scan);
        resolve(h, fam, "delta_step_supports", t.step_supports); resolve(h, fam, "delta_step", t.step);)
 FAMILY(AttentionLatent, attention_latent, "attention_latent", resolve(h, fam, "attention_latent_rotate_pairs", t.rotate_pairs);

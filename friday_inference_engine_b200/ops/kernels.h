@@ -37,6 +37,7 @@ struct GemmSimt {
     int (*gemm)(const void*, int, const void*, int, void*, int, const void*, int, const void*, int, int, int, int, int, int,
                 int, cudaStream_t);
     int (*split_pays)(const void*, const void*, int, int, int, int, int, long long);
+    int (*split_launches)(int, int, long long);
     int (*split)(const float*, const float*, float*, const void*, int, const float*, int, int, int, int, int, int, int, void*, long long, int*,
                  cudaStream_t);
     int (*few_supports)(const float*, const float*, int, int, int, int, int);
@@ -138,6 +139,7 @@ struct Delta {
                 long long, const int*, const int*, const int*, const int*, int, int, int, int, int, int, cudaStream_t);
     int (*chunks_pays)(int, int, int, int, int, int, int);
     long long (*chunks_scratch)(const float*, int, int, int, int, int);
+    int (*chunks_launches)(int, int, int, int);
     int (*chunks)(const float*, const void*, int, const void*, int, int, const void*, const void*, int, float*, float*, long long,
                   long long, const int*, const int*, const int*, const int*, int, int, int, int, int, int, int, int, void*, long long, cudaStream_t);
     int (*general_prepare)(const void*, int, int, int, const float*, int, const float*, int, const void*, const void*, int, float*, int, int,

@@ -867,7 +867,7 @@ Tensor Ops::delta_scan(const Tensor& qkv, const Tensor& a_raw, const Tensor& b_r
                                     dt_bias.data, code(a_log.dtype), (float*)out.data, (float*)view.state.data, stride, s_off, ctx.row_seq,
                                     ctx.seq_start, ctx.seq_qlen, view.seq_slots, ctx.n_seqs, s.heads, s.qk_heads, s.dk, s.dv,
                                     s.per_channel ? 1 : 0, rows, ctx.max_q_len, scratch, room, stream_), "delta_scan_chunks");
-        ++launches_;                                          // preparing the chunks and walking them
+        launches_ += k.chunks_launches(rows, ctx.n_seqs, s.heads, s.dv) - 1;      // (call counts one)
         return out;
     }
     call(launches_, k, k.scan((const float*)qkv.data, a_raw.data, (int)a_raw.ld, b_raw.data, (int)b_raw.ld, code(a_raw.dtype), a_log.data,
@@ -1305,7 +1305,7 @@ Tensor Ops::linear_simt(const Tensor& x, const Tensor& weight, const Tensor* bia
                      residual ? (const float*)residual->data : nullptr, m, n, k, (int)x.ld, (int)weight.ld, (int)out.ld, fixed(weight) ? 1 : 0,
                      tc_scratch_.get(), room, (int*)status_.get(), stream_),
              "gemm_simt_split");
-        ++launches_;                                          // the rows' split and the product
+        launches_ += g.split_launches(m, k, room) - 1;        // (call counts one)
         return out;
     }
     call(launches_, g,

@@ -3,6 +3,8 @@ import pytest
 
 from friday_inference_engine_b200.ops import lib
 
+SCRATCH = lib.c_longlong(2 * 148 * 128 * 256 * 4)          # what Ops gives a product
+
 
 def ask(family, name, *args):
     try:
@@ -10,7 +12,7 @@ def ask(family, name, *args):
     except Exception as e:           # no compiler, or no CUDA runtime library to load against
         pytest.skip("the %s library is not available here: %s" % (family, e))
     fn = getattr(fam.cdll, name)
-    fn.argtypes = [lib.P if a is None else lib.c_longlong if abs(a) >= 1 << 31 else lib.I for a in args]
+    fn.argtypes = [lib.P if a is None else type(a) if isinstance(a, lib.c_longlong) else lib.I for a in args]
     return fn(*args)
 
 
@@ -25,3 +27,10 @@ def ask(family, name, *args):
 def test_delta_rule_in_chunks(lens, heads, dk, dv, per_head, per_channel):
     for flag, want in ((0, per_head), (1, per_channel)):
         assert ask("delta", "delta_scan_chunks_pays", sum(lens), len(lens), max(lens), heads, dk, dv, flag) == want
+
+
+# two kernels per round of heads (50 heads' chunks fit at a time), per portion of rows (341 rows of 18,944 fit, and go 176 at a time then)
+def test_launches_of_calls_that_go_in_parts():
+    assert [ask("delta", "delta_scan_chunks_launches", 1000, 3, heads, 64) for heads in (1, 50, 51, 101)] == [2, 2, 4, 6]
+    assert ask("delta", "delta_scan_chunks_launches", 100000, 1, 4, 64) == 0
+    assert [ask("gemm_simt", "gemm_simt_split_launches", m, 18944, SCRATCH) for m in (17, 341, 342, 600)] == [2, 2, 4, 8]
