@@ -617,6 +617,22 @@ FR_EXPORT int gemm_simt_few_supports(const float* a, const float* w, int m, int 
     return k > 0 && n > 0 && !((k | lda | ldw) & 3) && !(((uintptr_t)a | (uintptr_t)w) & 15) && m <= (n < 8192 ? FEW_ROWS : FEW_ROWS_WIDE);
 }
 
+// Whether gemm_simt_few is the faster way: `end` 0 a product alone, 1 a gated unit, 2 rotary columns; `norm`: with the norm of its input.  It saves
+// the launches of its neighbours, 1 to 2 us each, and pays for them in the product itself: a third more registers, so fewer loads in flight, and
+// the norm's multiplications in every warp.  Measured on B200 with the norm, us, the kernels one after another and this one:
+//   one row: always ahead (4608 x 3584 rotary 42 and 21, 160 x 96 plain 3.0 and 1.8; 32768 x 96 plain 4.6 and 4.7)
+//   two rows: up to 9472 columns (more do not fit the SMs at once: 9728 x 896 plain 10.7 and 13.4) and, if not rotary, k below 4096 (4608 x 3584
+//   plain 27 and 22; 1024 x 4096 plain 22.7 and 24.1)
+//   three and four: rotary up to 6144 columns (4608 x 3584 32 and 27; 8192 x 1024 14 and 19), gated up to 8192 columns of k up to 1024 (4864 x 896
+//   10.1 and 8.8; 2048 x 2048 15 and 19), plain of k up to 128 (1000 x 96 3.2 and 2.6; 512 x 256 3.4 and 3.7)
+//   five to sixteen: gated and rotary up to 1024 x 512, with a norm (512 x 96 gated 4.3 and 3.4; 8 x 4608 x 3584 rotary 37 and 53, 16 rows 56 and 143)
+FR_EXPORT int gemm_simt_few_pays(int m, int n, int k, int end, int norm) {
+    if (m <= 1) return 1;
+    if (m == 2) return n <= 9472 && (end == FEW_ROTARY || k < 4096);
+    if (m <= 4) return end == FEW_ROTARY ? n <= 6144 : end == FEW_GATED ? n <= 8192 && k <= 1024 : n <= 8192 && k <= 128;
+    return end != FEW_PLAIN && norm && n <= 1024 && k <= 512;
+}
+
 // gemm_simt for few rows with the work that `fusion` asks for; out is [m][n], of a gated unit [m][n / 2].
 FR_EXPORT int gemm_simt_few(const float* a, const float* w, float* out, const void* bias, int bias_dtype, const float* residual, int m, int n,
                             int k, int lda, int ldw, int ldo, const GemmFewFusion* fusion, cudaStream_t stream) {

@@ -422,7 +422,7 @@ public:
     Tensor linear_tc(const Tensor& x, const Tensor& weight, const Tensor* bias, const Tensor* residual, Tensor& out,
                      int swap = -1, int bn = -1, int splits = -1, int act = 0, GemmFusion* fusion = nullptr);
     Tensor linear_simt(const Tensor& x, const Tensor& weight, const Tensor* bias, const Tensor* residual, Tensor& out);
-    bool few_in(const Rows& x, const Tensor& weight, DType out, GemmFewFusion& f) const;
+    bool few_in(const Rows& x, const Tensor& weight, DType out, int end, GemmFewFusion& f) const;
     Tensor linear_few(const Rows& x, const Tensor& weight, const Tensor* bias, const Tensor* residual, Tensor& out, const GemmFewFusion& f);
     bool tensor_core_ok(const Tensor& x, const Tensor& weight, const Tensor& out, const Tensor* residual) const;
     void plan(int64_t rows, int64_t n, int64_t k, bool* swapped, int* bn, int* splits = nullptr);

@@ -98,7 +98,7 @@ FAMILY(Rowwise, rowwise, "rowwise",
 FAMILY(GemmSimt, gemm_simt, "gemm_simt", resolve(h, fam, "gemm_simt_weights", t.gemm);
        resolve(h, fam, "gemm_simt_split_pays", t.split_pays); resolve(h, fam, "gemm_simt_split", t.split);
        resolve(h, fam, "gemm_simt_split_launches", t.split_launches);
-       resolve(h, fam, "gemm_simt_few_supports", t.few_supports); resolve(h, fam, "gemm_simt_few", t.few);)
+       resolve(h, fam, "gemm_simt_few_supports", t.few_supports); resolve(h, fam, "gemm_simt_few_pays", t.few_pays); resolve(h, fam, "gemm_simt_few", t.few);)
 FAMILY(GemmTc, gemm_tc, "gemm_tc", resolve(h, fam, "gemm_tc_fused", t.fused); resolve(h, fam, "gemm_tc_plan", t.plan);
        resolve(h, fam, "gemm_tc_grouped", t.grouped);)
 FAMILY(AttentionSimt, attention_simt, "attention_simt", resolve(h, fam, "attention_simt", t.run);

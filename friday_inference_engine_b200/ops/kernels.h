@@ -41,6 +41,7 @@ struct GemmSimt {
     int (*split)(const float*, const float*, float*, const void*, int, const float*, int, int, int, int, int, int, int, void*, long long, int*,
                  cudaStream_t);
     int (*few_supports)(const float*, const float*, int, int, int, int, int);
+    int (*few_pays)(int, int, int, int, int);
     int (*few)(const float*, const float*, float*, const void*, int, const float*, int, int, int, int, int, int, const GemmFewFusion*,
                cudaStream_t);
 };

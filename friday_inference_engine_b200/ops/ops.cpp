@@ -1338,16 +1338,19 @@ Tensor Ops::linear(const Rows& x, const Tensor& weight, const Tensor* bias, cons
         return linear_tc(xt, weight, bias, residual, o, -1, -1, -1, 0, x.deferred ? &f : nullptr);
     }
     GemmFewFusion f;
-    if (x.deferred && few_in(x, weight, o.dtype, f)) return linear_few(x, weight, bias, residual, o, f);
+    if (x.deferred && few_in(x, weight, o.dtype, 0, f)) return linear_few(x, weight, bias, residual, o, f);
     Tensor xin = x.deferred ? materialize(x) : xt;
     return linear_simt(xin, weight, bias, residual, o);
 }
 
-// Whether the 32-bit product of few rows takes x and weight; if so, f asks it for the norm that x has been promised.
-bool Ops::few_in(const Rows& x, const Tensor& weight, DType out, GemmFewFusion& f) const {
+// Whether the 32-bit product of few rows takes x and weight and is the faster way (end: as gemm_simt_few_pays has it); if so, f asks it for the
+// norm that x has been promised.
+bool Ops::few_in(const Rows& x, const Tensor& weight, DType out, int end, GemmFewFusion& f) const {
     const Tensor& t = x.deferred ? x.source : x.t;
     if (!t.defined() || t.dtype != DType::F32 || weight.dtype != DType::F32 || out != DType::F32 || t.rows() > 16 || !fusion_enabled()) return false;
-    if (!kernels::gemm_simt().few_supports((const float*)t.data, (const float*)weight.data, (int)t.rows(), (int)weight.rows(), (int)t.cols(),
+    const auto& g = kernels::gemm_simt();
+    if (!g.few_pays((int)t.rows(), (int)weight.rows(), (int)t.cols(), end, x.deferred ? 1 : 0) ||
+        !g.few_supports((const float*)t.data, (const float*)weight.data, (int)t.rows(), (int)weight.rows(), (int)t.cols(),
                                            (int)t.ld, (int)weight.ld))
         return false;
     memset(&f, 0, sizeof f);
@@ -1481,7 +1484,7 @@ Tensor Ops::qkv_rope_write(const Rows& x, const Tensor& weight, const Tensor* bi
     }
     GemmFewFusion few;
     if (head_dim % 2 == 0 && rotary_dim % 2 == 0 && n == (int64_t)(n_heads + 2 * n_kv_heads) * head_dim && (denominators || write) &&
-        (!write || view->dtype == DType::F32) && few_in(x, weight, xt.dtype, few)) {
+        (!write || view->dtype == DType::F32) && few_in(x, weight, xt.dtype, 2, few)) {
         Tensor out = alloc(xt.dtype, xt.rows(), n);
         few.row_seq = row_seq;
         few.row_pos = row_pos;
@@ -1519,7 +1522,7 @@ Tensor Ops::linear_swiglu(const Rows& x, const Tensor& weight_pairs, int act, fl
         return linear_tc(xt, weight_pairs, nullptr, nullptr, out, -1, -1, -1, act, x.deferred || act == 3 ? &f : nullptr);
     }
     GemmFewFusion few;
-    if (act > 0 && act <= 3 && few_in(x, weight_pairs, xt.dtype, few)) {
+    if (act > 0 && act <= 3 && few_in(x, weight_pairs, xt.dtype, 1, few)) {
         Tensor out = alloc(xt.dtype, xt.rows(), inner);
         few.act = act;
         few.act_limit = limit;

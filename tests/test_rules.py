@@ -34,3 +34,14 @@ def test_launches_of_calls_that_go_in_parts():
     assert [ask("delta", "delta_scan_chunks_launches", 1000, 3, heads, 64) for heads in (1, 50, 51, 101)] == [2, 2, 4, 6]
     assert ask("delta", "delta_scan_chunks_launches", 100000, 1, 4, 64) == 0
     assert [ask("gemm_simt", "gemm_simt_split_launches", m, 18944, SCRATCH) for m in (17, 341, 342, 600)] == [2, 2, 4, 8]
+
+
+# end: 0 a product alone, 1 a gated unit, 2 rotary columns; with the norm of the input unless said otherwise
+@pytest.mark.parametrize("m,n,k,end,norm,want", [
+    (1, 152064, 896, 0, 1, 1), (1, 37888, 3584, 1, 0, 1), (2, 4608, 3584, 2, 1, 1), (2, 8192, 1024, 0, 1, 1), (2, 9728, 896, 0, 1, 0), (2, 152064, 896, 1, 1, 0),
+    (2, 1024, 4096, 0, 1, 0), (2, 2048, 4096, 2, 1, 1), (3, 1000, 96, 0, 1, 1), (4, 512, 256, 0, 1, 0), (4, 4864, 896, 1, 1, 1), (4, 2048, 2048, 1, 1, 0),
+    (4, 37888, 3584, 1, 1, 0), (4, 6144, 2048, 2, 1, 1), (4, 8192, 1024, 2, 1, 0), (5, 512, 96, 1, 1, 1), (16, 160, 96, 2, 1, 1), (5, 512, 96, 0, 1, 0),
+    (5, 512, 96, 1, 0, 0), (8, 4608, 3584, 2, 1, 0), (16, 3584, 18944, 1, 1, 0),
+])
+def test_few_rows_with_their_neighbours(m, n, k, end, norm, want):
+    assert ask("gemm_simt", "gemm_simt_few_pays", m, n, k, end, norm) == want
