@@ -391,11 +391,13 @@ int launch_prompt_tiles(const PromptArgs& p, int n_seqs, int max_q_len, cudaStre
 }
 
 // Tiles of 64 rows would leave SMs with fewer than two blocks: 32 rows, where the query heads of a kv head fit them.
+bool prompt_tiles_are_few(int group, long long tiles, int sms) { return group <= 32 && tiles < 4ll * sms; }
+
 template <int HD>
 int launch_prompt(const PromptArgs& p, int n_seqs, int max_q_len, cudaStream_t stream) {
     const int sms = fr_sm_count() > 0 ? fr_sm_count() : 148, group = p.nq / p.nkv, tokens = PT_MOST_ROWS / group;
     const long long tiles = (long long)((max_q_len + tokens - 1) / tokens) * p.nkv * n_seqs;
-    if (group <= 32 && tiles < 4ll * sms) return launch_prompt_tiles<HD, 2>(p, n_seqs, max_q_len, stream);
+    if (prompt_tiles_are_few(group, tiles, sms)) return launch_prompt_tiles<HD, 2>(p, n_seqs, max_q_len, stream);
     return launch_prompt_tiles<HD, 4>(p, n_seqs, max_q_len, stream);
 }
 
@@ -466,6 +468,39 @@ FR_EXPORT int attention_simt_prompt_supports(const void* q, int q_stride, const 
                                              int hd, int n_seqs) {
     return hd > 0 && hd <= 128 && hd % 4 == 0 && nkv > 0 && nkv <= 65535 && nq % nkv == 0 && nq / nkv <= PT_MOST_ROWS && q_stride % 4 == 0 && n_seqs <= 65535 &&
            (((uintptr_t)q | (uintptr_t)out | (uintptr_t)k_pool | (uintptr_t)v_pool) & 15) == 0;
+}
+
+// Whether attention_simt_prompt is the faster way for a step (max_kv_len: of the longest sequence, its new rows included; `splits`: of the
+// keys by attention_simt).  Both times are estimated, in us, from what was measured on B200 at 16 to 333 new rows behind 0 to 8,000 keys, heads 28 on 4,
+// 64 on 1, 8 and 16 of their own, 3 on 1:
+//   a warp per row and head: a key costs a warp 0.15 (0.11 up to 64 channels) while few warps run, and the SMs do 6,800 (7,800) keys of a row
+//   and head in a microsecond;
+//   tiles: a block walks its keys whatever the number of its rows, 32 in 3.8 (2.4 and 1.55 up to 64 and 32 channels; of 64 rows 5.2, 3.3 and 2.1), and
+//   never shares them with another block.
+// So few rows behind many keys are the first one's, whose warps split the keys (16 rows behind 8,000 keys: 28 on 4 heads 489 and 945, 8 heads 155 and
+// 939; 64 rows 2,414 and 947, 618 and 942; without keys before them 16 rows 4.5 and 8.2, 64 rows 16 and 12).  Over the 303 steps that were measured
+// the tiles, where taken, were never more than 3 % behind, but for 100 rows beside 64 sequences of one (145 and 167).
+FR_EXPORT int attention_simt_prompt_pays(int rows, int n_seqs, int max_q_len, int max_kv_len, int nq, int nkv, int hd, int window, int splits) {
+    if (rows <= 0 || n_seqs <= 0 || nkv <= 0 || nq < nkv || splits <= 0 || nq / nkv > PT_MOST_ROWS) return 0;
+    const int sms = fr_sm_count() > 0 ? fr_sm_count() : 148, group = nq / nkv, size = hd > 64 ? 2 : hd > 32 ? 1 : 0;
+    const double seen = window > 0 && window < max_kv_len ? window : max_kv_len;
+    double keys = max_kv_len - 0.5 * max_q_len;               // of a row, about
+    if (window > 0 && window < keys) keys = window;
+    const double in_turn = (size == 2 ? 0.15 : 0.11) * ceil(seen / splits), all = (double)rows * keys * nq / (size == 2 ? 6800.0 : 7800.0);
+    const double some = splits > 1 ? all : all + (in_turn < 12.0 ? 0.5 * in_turn : 6.0);        // (the rows that see little end early)
+    const double by_row = (in_turn > some ? in_turn : some) + (splits > 1 ? 8.0 : 3.0);
+
+    const long long tiles = (long long)((max_q_len + PT_MOST_ROWS / group - 1) / (PT_MOST_ROWS / group)) * nkv * n_seqs;
+    const bool few = prompt_tiles_are_few(group, tiles, sms);
+    const double step[2][3] = {{2.1, 3.3, 5.2}, {1.55, 2.4, 3.8}};
+    const int tokens = (few ? 32 : 64) / group;
+    long long blocks = (long long)((max_q_len + tokens - 1) / tokens) * n_seqs;
+    if (rows / tokens + n_seqs < blocks) blocks = rows / tokens + n_seqs;
+    blocks *= nkv;
+    double reach = max_kv_len;
+    if (window > 0 && window + tokens < reach) reach = window + tokens;
+    const double tiled = (few ? 4.4 : 8.0) + ceil(reach / PT_KEYS) * step[few][size] * (double)((blocks + sms - 1) / sms);
+    return tiled <= 0.95 * by_row;
 }
 
 // attention_simt for prompts in fp32: sequence s brings the rows seq_start[s] .. + seq_qlen[s] - 1 at positions from seq_pos0[s] on;

@@ -103,6 +103,7 @@ FAMILY(GemmTc, gemm_tc, "gemm_tc", resolve(h, fam, "gemm_tc_fused", t.fused); re
        resolve(h, fam, "gemm_tc_grouped", t.grouped);)
 FAMILY(AttentionSimt, attention_simt, "attention_simt", resolve(h, fam, "attention_simt", t.run);
        resolve(h, fam, "attention_simt_masked", t.masked);
+       resolve(h, fam, "attention_simt_prompt_pays", t.prompt_pays);
        resolve(h, fam, "attention_simt_prompt_supports", t.prompt_supports); resolve(h, fam, "attention_simt_prompt", t.prompt);)
 FAMILY(AttentionWindow, attention_window, "attention_window", resolve(h, fam, "attention_window_fits", t.fits);
        resolve(h, fam, "attention_window", t.run);)

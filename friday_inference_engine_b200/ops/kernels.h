@@ -59,6 +59,7 @@ struct AttentionSimt {
                int, int, float, int, float*, int, cudaStream_t);
     int (*masked)(const void*, int, void*, const void*, const void*, const int*, int, int, const int*, const int*, int, int, int,
                   int, int, int, int, float, float, int, float*, int, cudaStream_t);
+    int (*prompt_pays)(int, int, int, int, int, int, int, int, int);
     int (*prompt_supports)(const void*, int, const void*, const void*, const void*, int, int, int, int);
     int (*prompt)(const float*, int, float*, const float*, const float*, const int*, int, int, const int*, const int*, const int*, const int*, int,
                   int, int, int, int, int, float, cudaStream_t);

@@ -1690,7 +1690,9 @@ void Ops::attention(const Tensor& q, int64_t q_stride, Tensor& out, const CacheV
         return;
     }
     const auto& k = kernels::attention_simt();
-    if (out.dtype == DType::F32 && geometry && !ctx.decode && ctx.max_q_len >= 16 && view.dtype == DType::F32 &&
+    const int splits = attention_splits(rows, n_heads, ctx.max_kv_len);
+    if (out.dtype == DType::F32 && geometry && !ctx.decode && view.dtype == DType::F32 &&
+        k.prompt_pays(rows, ctx.n_seqs, ctx.max_q_len, ctx.max_kv_len, n_heads, n_kv_heads, head_dim, window, splits) &&
         k.prompt_supports(q.data, (int)q_stride, out.data, view.k_pool, view.v_pool, n_heads, n_kv_heads, head_dim, ctx.n_seqs)) {
         Timed t(*this, Attention);
         call(launches_, k,
@@ -1700,7 +1702,6 @@ void Ops::attention(const Tensor& q, int64_t q_stride, Tensor& out, const CacheV
              "attention_simt_prompt");
         return;
     }
-    const int splits = attention_splits(rows, n_heads, ctx.max_kv_len);
     float* scratch = splits > 1 ? scratch_floats((int64_t)rows * n_heads * splits * (head_dim + 2)) : nullptr;
     Timed t(*this, Attention);
     call(launches_, k,

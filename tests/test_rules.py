@@ -45,3 +45,19 @@ def test_launches_of_calls_that_go_in_parts():
 ])
 def test_few_rows_with_their_neighbours(m, n, k, end, norm, want):
     assert ask("gemm_simt", "gemm_simt_few_pays", m, n, k, end, norm) == want
+
+
+def splits_of(rows, heads, keys):          # of the keys where a warp has a row and head
+    return max(1, min(148 * 16 // (rows * heads), (keys + 63) // 64, 64)) if rows * heads < 148 * 16 and keys > 128 else 1
+
+
+# new tokens, keys before them, heads, kv heads, their size, window: whether the tiles were the faster way
+@pytest.mark.parametrize("lens,before,nq,nkv,hd,window,want", [
+    ([16], 0, 28, 4, 128, 0, 0), ([16], 8000, 28, 4, 128, 0, 0), ([20], 300, 28, 4, 128, 0, 0), ([48], 1000, 28, 4, 128, 0, 1), ([333], 0, 28, 4, 128, 0, 1),
+    ([333], 8000, 28, 4, 128, 0, 1), ([64], 8000, 8, 8, 128, 0, 0), ([200], 8000, 8, 8, 128, 0, 1), ([100], 8000, 3, 1, 32, 0, 0), ([333], 8000, 3, 1, 32, 0, 1),
+    ([16] * 8, 1000, 28, 4, 128, 0, 1), ([16] + [1] * 31, 500, 16, 16, 64, 0, 0), ([300, 33], 0, 28, 4, 128, 0, 1), ([16], 4000, 28, 4, 128, 512, 0),
+    ([300], 4000, 28, 4, 128, 512, 1), ([1] * 64 + [100], 2000, 16, 16, 64, 0, 0), ([256] * 8, 0, 3, 1, 32, 0, 1), ([64] * 16, 2000, 64, 1, 128, 0, 1),
+])
+def test_fp32_attention_of_prompts(lens, before, nq, nkv, hd, window, want):
+    keys = max(lens) + before
+    assert ask("attention_simt", "attention_simt_prompt_pays", sum(lens), len(lens), max(lens), keys, nq, nkv, hd, window, splits_of(sum(lens), nq, keys)) == want
