@@ -579,13 +579,19 @@ FR_EXPORT int gemm_simt(const void* a, int a_dtype, const void* w, int w_dtype, 
 // Products of fp32 operands on the tensor cores (gemm_f32_tc.cuh): whether gemm_simt_split takes this one with `scratch_bytes` of
 // scratch, and is the faster way.  It has two launches and a longer chain from its first load to its last store: below some 2^20
 // weights, or short k, the kernels of one launch are ahead (1024 x 512: 48 rows 10 us against 16; 1024 x 1024: 64 rows level, 128 rows
-// 21 against 16; 2048 x 1024: 48 rows 17 against 14; 200000 x 64: 96 rows 74 against 88).
+// 21 against 16; 2048 x 1024: 48 rows 17 against 14; 200000 x 64: 96 rows 74 against 88).  Fewer than four tiles of columns leave most
+// SMs idle whatever the split of k (128 x 18944: 128 rows 47 against 51, 1,024 rows, in six portions, 214 against 343; 300 x 4096: 65 rows 12.7
+// against 15.2, 333 rows 54 against 20).
+// Rows beyond what the scratch holds go in portions, each of which reads and splits the weights again: with 38.8 MB, 341 rows of k = 18,944 at a
+// time and 1,800 of 3,584 (3584 x 18944: 342 rows 216 us, 353 rows 288; the tiles of one launch take 1,280).
 FR_EXPORT int gemm_simt_split_pays(const void* a, const void* w, int m, int n, int k, int lda, int ldw, long long scratch_bytes) {
-    if (((k | lda | ldw) & 3) || (((uintptr_t)a | (uintptr_t)w) & 15) || k < 1024 || n <= 0) return 0;
+    if (((k | lda | ldw) & 3) || (((uintptr_t)a | (uintptr_t)w) & 15) || k < 1024 || n < 256) return 0;
     const bool few = m <= (n < 8192 ? FEW_ROWS : FEW_ROWS_WIDE);
-    if (few || split_rows_at_once(m, k, scratch_bytes) == 0) return 0;
+    const int at_once = split_rows_at_once(m, k, scratch_bytes);
+    if (few || at_once == 0) return 0;
+    if (n < 512 && (m < 160 || at_once < m)) return 0;
     const long long weights = (long long)n * k;
-    return weights >= 2ll << 20 ? m >= 48 || weights >= 6ll << 20 : weights >= 1ll << 20 && m > 64;
+    return weights >= 2ll << 20 ? m >= 48 || weights >= 6ll << 20 : weights >= 1ll << 20 && m > (n >= 1024 ? 64 : 127);
 }
 
 // Kernels that gemm_simt_split launches: two per portion of rows.

@@ -61,3 +61,12 @@ def splits_of(rows, heads, keys):          # of the keys where a warp has a row 
 def test_fp32_attention_of_prompts(lens, before, nq, nkv, hd, window, want):
     keys = max(lens) + before
     assert ask("attention_simt", "attention_simt_prompt_pays", sum(lens), len(lens), max(lens), keys, nq, nkv, hd, window, splits_of(sum(lens), nq, keys)) == want
+
+
+@pytest.mark.parametrize("m,n,k,want", [
+    (333, 37888, 3584, 1), (333, 3584, 18944, 1), (353, 3584, 18944, 1), (17, 3584, 3584, 1), (16, 3584, 3584, 0), (48, 2048, 1024, 1), (47, 2048, 1024, 0), (65, 1024, 1024, 1),
+    (64, 1024, 1024, 0), (96, 640, 2048, 0), (128, 640, 2048, 1), (1024, 512, 1024, 0), (96, 200000, 64, 0), (128, 128, 18944, 0), (1024, 128, 18944, 0), (96, 300, 4096, 0),
+    (333, 300, 4096, 1), (520, 256, 18944, 0), (48, 512, 8192, 1),
+])
+def test_32_bit_products_on_the_tensor_cores(m, n, k, want):
+    assert ask("gemm_simt", "gemm_simt_split_pays", None, None, m, n, k, k, k, SCRATCH) == want
