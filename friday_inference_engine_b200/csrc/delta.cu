@@ -131,9 +131,18 @@ __global__ void __launch_bounds__(256) conv_prepare_kernel(ConvArgs p) {
 
 // The same for prompts: a warp takes a head, or 128 value channels, along CONV_RUN consecutive rows, four channels per lane, with the
 // taps and the rows before the present one in registers, so that an input is read once instead of once per tap.  2,304 rows of
-// 4,096 channels: 42 us, 110 with a block per row; its bytes take 9.  (The inputs of eight rows fetched together: 45 us, its
-// registers leave half as many warps.)
+// 4,096 channels: 42 us, 110 with a block per row (one call after another, its inputs in L2, 24 and 68); its bytes take 9.  (The inputs of
+// eight rows fetched together: 45 us, its registers leave half as many warps.)
 constexpr int CONV_RUN = 16, CONV_RUN_TAPS = 4;
+// A warp's chain of sixteen rows takes 15 us (heads of up to 64 channels, with taps of half the lanes, 23) however few they are, so it needs as much
+// work as takes a block per row longer.  Measured on B200, us, a block per row and so: heads of 128, 4,096 channels, 64 rows 5.6 and 15.3, 256 rows 14.5 and
+// 15.3, 512 rows 21.9 and 15.3 (512 sequences of one 25.0 and 25.3); 2,048 channels, 512 rows 11.9 and 15.2, 1,024 rows 18.0 and 15.3; 8,192 channels,
+// 256 rows 27.2 and 15.3; heads of 64, 2,048 channels, 1,024 rows 20.4 and 25.1, 2,048 rows 36.8 and 34.0.
+bool conv_runs_pay(int rows, int qk_heads, int dk, int v_channels) {
+    const long long inputs = (long long)rows * (2ll * qk_heads * dk + v_channels);
+    return rows >= 4 * CONV_RUN && inputs >= (dk > 64 ? 2ll << 20 : 4ll << 20);
+}
+
 template <typename T>
 __device__ __forceinline__ void load_four(const T* p, float (&v)[4]);
 template <>
@@ -507,6 +516,9 @@ int fill_conv(ConvArgs& p, const void* x, int ld, int q_off, int k_off, int v_of
 // q, k (qk_heads x dk each) and v (v_channels) of x [rows][ld] -> out [rows][2 qk_heads dk + v_channels] fp32.
 // shift_history: only where every sequence of the step brings exactly one row; the state's history then moves on in this
 // kernel and delta_conv_state is not needed.
+// Whether delta_conv_prepare goes sixteen rows per warp (where the rows' pieces allow it).
+FR_EXPORT int delta_conv_runs_pay(int rows, int qk_heads, int dk, int v_channels) { return conv_runs_pay(rows, qk_heads, dk, v_channels); }
+
 FR_EXPORT int delta_conv_prepare(const void* x, int ld, int q_off, int k_off, int v_off, const void* taps_w, int w_dtype, float* out,
                                  const float* state, long long state_stride, const int* row_seq, const int* seq_start,
                                  const int* seq_slots, int rows, int qk_heads, int dk, int v_channels, int taps, float q_scale,
@@ -519,7 +531,7 @@ FR_EXPORT int delta_conv_prepare(const void* x, int ld, int q_off, int k_off, in
     p.shift = shift_history && taps > 1 ? 1 : 0;
     // prompts whose heads and rows lie in pieces of four channels: 16 rows per warp
     const int piece = dtype == FR_F32 ? 16 : 8;
-    if (!p.shift && rows >= 4 * CONV_RUN && taps <= CONV_RUN_TAPS && dk <= 128 && dk % 4 == 0 && v_channels % 4 == 0 &&
+    if (!p.shift && conv_runs_pay(rows, qk_heads, dk, v_channels) && taps <= CONV_RUN_TAPS && dk <= 128 && dk % 4 == 0 && v_channels % 4 == 0 &&
         ((q_off | k_off | v_off | ld) & 3) == 0 && (uintptr_t)x % piece == 0 && ((uintptr_t)out & 15) == 0 && (dtype == FR_F32 || dtype == FR_BF16)) {
         const dim3 grid((rows + CONV_RUN - 1) / CONV_RUN, (2 * qk_heads + (v_channels + 127) / 128 + 7) / 8);
         if (grid.y <= 65535) {

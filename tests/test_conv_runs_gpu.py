@@ -51,6 +51,15 @@ def test_conv(lens, groups, dk, values, taps, dtype):
         assert (got.double() - ref).abs().max() <= 2.0 ** -18 * max(1.0, float(ref.abs().max()))
 
 
+# as many inputs as make the runs the faster way
+@pytest.mark.parametrize("lens,groups,dk,values,taps", [([1, 2, 300, 3, 17, 200], 8, 128, 2052, 4), ([5500], 16, 20, 132, 3), ([3000, 1, 2, 8000], 3, 64, 4, 2),
+                                                        ([16000, 33], 1, 4, 256, 1)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_conv_in_runs(lens, groups, dk, values, taps, dtype):
+    assert lib.family("delta").declare("delta_conv_runs_pay", [I, I, I, I])(sum(lens), groups, dk, values) == 1
+    test_conv(lens, groups, dk, values, taps, dtype)
+
+
 @pytest.mark.parametrize("rows,heads,dv", [(1, 1, 4), (5, 3, 64), (33, 16, 128), (7, 2, 100)])
 @pytest.mark.parametrize("act,per_head", [(0, 0), (1, 1)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])

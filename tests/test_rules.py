@@ -70,3 +70,11 @@ def test_fp32_attention_of_prompts(lens, before, nq, nkv, hd, window, want):
 ])
 def test_32_bit_products_on_the_tensor_cores(m, n, k, want):
     assert ask("gemm_simt", "gemm_simt_split_pays", None, None, m, n, k, k, k, SCRATCH) == want
+
+
+@pytest.mark.parametrize("rows,qk_heads,dk,values,want", [
+    (64, 8, 128, 2048, 0), (256, 8, 128, 2048, 0), (512, 8, 128, 2048, 1), (2304, 8, 128, 2048, 1), (512, 4, 128, 1024, 0), (1024, 4, 128, 1024, 1),
+    (256, 16, 128, 4096, 1), (100, 32, 128, 8192, 0), (2304, 1, 128, 128, 0), (1024, 8, 64, 1024, 0), (2048, 8, 64, 1024, 1), (2304, 2, 32, 128, 0),
+])
+def test_convolutions_sixteen_rows_per_warp(rows, qk_heads, dk, values, want):
+    assert ask("delta", "delta_conv_runs_pay", rows, qk_heads, dk, values) == want
