@@ -1,19 +1,22 @@
 // The 32-bit product of many rows on the tensor cores.
 //
 // Every fp32 operand is the sum of three bf16 numbers, x = hi + mid + lo, each the rounding of what the ones before it
-// leave: 8 + 8 + 8 significant bits, so nothing of the 24 is lost.  A product is the sum of the six partial products that
-// reach 2^-18 of it (hi hi, hi mid, mid hi, hi lo, mid mid, lo hi; what is left out is below 2^-26), which the tensor
+// leave: 8 + 8 + 8 significant bits, so none of the 24 is lost (the split of a matrix into parts whose products are exact is Ozaki, Ogita, Oishi and
+// Rump's, "Error-free transformations of matrix multiplication", 2012).  A product is the sum of the six partial products that
+// reach 2^-18 of it (hi hi, hi mid, mid hi, hi lo, mid mid, lo hi; what is left out is below 2^-25), which the tensor
 // core forms exactly and adds in fp32.  Its accumulators drop the bits of an addend below the sum's last place instead of
 // rounding, an error that grows with the number of additions.  So hi hi has an accumulator of its own, which sums 128 of k
 // at a time (eight additions); these parts are added in fp32 registers.  The five small products share another accumulator
-// over all of k: its values, and with them what it drops, are 2^-9 of the others.
+// over all of k: its values, and with them what it drops, are 2^-8 of the others.
 //
 // Where all of a tile's weights in a block of k are bf16 numbers already (a bf16 checkpoint run in 32 bits: every block),
 // their mid and lo are zero and the three products with them are not issued: the result is the same.
 //
 // A value that no sum of three bf16 numbers is (not finite, or so near the largest float that hi would round to infinity)
-// marks its row; results of marked rows are computed by one chain of fp32 multiply-adds instead, so that infinities and
-// NaN come out as they do everywhere else.  Magnitudes below 2^-110 lose what lies below bf16's smallest number, 2^-133.
+// marks its row; results of marked rows are computed by fp32 multiply-adds instead, so that infinities and
+// NaN come out as they do everywhere else.  bf16 ends at 2^-133, so magnitudes below 2^-110 have fewer than 24 bits in three of them: rows of x
+// that lie below 2^-63 as a whole are split times 2^64 and their results divided by it, weight rows of that kind (that are no bf16
+// numbers) are marked.  What is left is a value below 2^-110 in a row that reaches 2^-63: off by 2^-134, 2^-71 of the row's largest.
 //
 // Weights lie on the M side (128 columns of the result per tile), rows of x on the N side.  x is split once by a kernel of
 // its own into three planes in memory and comes by TMA.  Weights come by TMA as they are, 32 of k at a time; four converter
@@ -51,13 +54,16 @@ constexpr int SPLIT_STATIC_SMEM = 2048;                        // barriers and f
 constexpr int SPLIT_MAX_SMEM = 227 * 1024 - SPLIT_STATIC_SMEM;
 constexpr int SPLIT_FIXED_SMEM = 1024 + SPLIT_W_STAGES * SPLIT_W_BYTES;    // (1,024 for the alignment)
 
+constexpr int SPLIT_BAD = 1, SPLIT_TINY = 2;
+constexpr uint32_t SPLIT_LARGE_BITS = 0x60000000u;             // some of these are set in magnitudes from 2^-63 on, none in those below
+
 struct SplitArgs {
     const float* x;
     const float* w;
     float* out;
     FrVec bias;
     const float* residual;
-    const int* marked;               // [m] rows of x with a value that is no sum of three bf16
+    const int* marked;               // [m] rows of x: SPLIT_BAD with a value that is no sum of three bf16, SPLIT_TINY times 2^64 in the planes
     int m, n, k, lda, ldw, ldo;
     int bn, tiles_q, x_stages, splits, kb_per, fixed_weights;
     int* status;
@@ -114,9 +120,17 @@ __device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint3
     bad = fmaf(0.f, a + b, bad);
 }
 
+template <bool B>
+struct Scaled {
+    static constexpr bool value = B;
+};
+
 // x [m][k] into planes [3][m][kp] (kp: k up to a multiple of 8, zeros beyond k), a block per row.
 __global__ void __launch_bounds__(256)
 split_rows_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ planes, int* __restrict__ marked, int m, int k, int kp, int lda) {
+    __shared__ uint32_t s_seen;                                // SPLIT_BAD; 2: a magnitude from 2^-63 on; 4: one that is not zero
+    if (threadIdx.x == 0) s_seen = 0u;
+    __syncthreads();
     fr_pdl_wait();
     fr_pdl_launch();
     const int row = blockIdx.x;
@@ -124,28 +138,54 @@ split_rows_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ plane
     const size_t plane = (size_t)m * kp;
     __nv_bfloat16* dst = planes + (size_t)row * kp;
     float bad = 0.f;
-    for (int c = threadIdx.x * 8; c < kp; c += 256 * 8) {
-        const float4 a = *(const float4*)(src + c);
-        const float4 b = c + 4 < k ? *(const float4*)(src + c + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-        uint4 hi, mid, lo;
-        split_pair(a.x, a.y, hi.x, mid.x, lo.x, bad);
-        split_pair(a.z, a.w, hi.y, mid.y, lo.y, bad);
-        split_pair(b.x, b.y, hi.z, mid.z, lo.z, bad);
-        split_pair(b.z, b.w, hi.w, mid.w, lo.w, bad);
-        *(uint4*)(dst + c) = hi;
-        *(uint4*)(dst + plane + c) = mid;
-        *(uint4*)(dst + 2 * plane + c) = lo;
-    }
-    const int any = __syncthreads_or(bad != bad);
-    if (threadIdx.x == 0) marked[row] = any;
+    uint32_t bits = 0u;
+    auto split = [&](auto scaled) {
+        for (int c = threadIdx.x * 8; c < kp; c += 256 * 8) {
+            float4 a = *(const float4*)(src + c);
+            float4 b = c + 4 < k ? *(const float4*)(src + c + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (decltype(scaled)::value) {
+                a.x *= 0x1p64f; a.y *= 0x1p64f; a.z *= 0x1p64f; a.w *= 0x1p64f;
+                b.x *= 0x1p64f; b.y *= 0x1p64f; b.z *= 0x1p64f; b.w *= 0x1p64f;
+            } else {
+                bits |= (__float_as_uint(a.x) | __float_as_uint(a.y)) | (__float_as_uint(a.z) | __float_as_uint(a.w));
+                bits |= (__float_as_uint(b.x) | __float_as_uint(b.y)) | (__float_as_uint(b.z) | __float_as_uint(b.w));
+            }
+            uint4 hi, mid, lo;
+            split_pair(a.x, a.y, hi.x, mid.x, lo.x, bad);
+            split_pair(a.z, a.w, hi.y, mid.y, lo.y, bad);
+            split_pair(b.x, b.y, hi.z, mid.z, lo.z, bad);
+            split_pair(b.z, b.w, hi.w, mid.w, lo.w, bad);
+            *(uint4*)(dst + c) = hi;
+            *(uint4*)(dst + plane + c) = mid;
+            *(uint4*)(dst + 2 * plane + c) = lo;
+        }
+    };
+    split(Scaled<false>{});
+    const uint32_t seen = __reduce_or_sync(0xffffffffu, (bad != bad ? SPLIT_BAD : 0u) | ((bits & SPLIT_LARGE_BITS) ? 2u : 0u) | ((bits & 0x7fffffffu) ? 4u : 0u));
+    if ((threadIdx.x & 31) == 0 && seen != 0u) atomicOr(&s_seen, seen);
+    __syncthreads();
+    const bool tiny = s_seen == 4u;                            // (nothing so small is bad)
+    if (tiny) split(Scaled<true>{});
+    if (threadIdx.x == 0) marked[row] = tiny ? SPLIT_TINY : (s_seen & SPLIT_BAD);
 }
 
+// (rows lie in pieces of four; a part of 256 at a time, so that the error stays near that of the sums on the tensor cores)
 __device__ __forceinline__ float split_plain_dot(const SplitArgs& p, int row, int col) {
     const float* a = p.x + (size_t)row * p.lda;
     const float* b = p.w + (size_t)col * p.ldw;
-    float s = 0.f;
-    for (int i = 0; i < p.k; ++i) s = fmaf(a[i], b[i], s);
-    return s;
+    float total = 0.f;
+    for (int k0 = 0; k0 < p.k; k0 += 256) {
+        float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+        for (int i = k0; i < min(k0 + 256, p.k); i += 4) {
+            const float4 u = *(const float4*)(a + i), v = *(const float4*)(b + i);
+            s0 = fmaf(u.x, v.x, s0);
+            s1 = fmaf(u.y, v.y, s1);
+            s2 = fmaf(u.z, v.z, s2);
+            s3 = fmaf(u.w, v.w, s3);
+        }
+        total += (s0 + s1) + (s2 + s3);
+    }
+    return total;
 }
 
 __global__ void __launch_bounds__(SPLIT_THREADS, 1)
@@ -155,7 +195,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     __shared__ uint32_t tmem_slot;
     __shared__ int s_wide[SPLIT_A_STAGES][4];                  // a quarter of the stage's weights has mid or lo parts
     __shared__ float s_bad[TILE_P];                            // weight rows that cannot be split
-    __shared__ float s_any;                                    // such a row, of weights or of x, is among the tile's
+    __shared__ float s_any;                                    // such a row, or a marked one of x, is among the tile's
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* x_ring = smem + SPLIT_W_STAGES * SPLIT_W_BYTES;
     const int bn = p.bn, XS = p.x_stages;
@@ -204,6 +244,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const int quarter = warp & 3, row = quarter * 32 + lane, blocks = kb1 - kb0;
         const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16) + SPLIT_A0;
         float bad4[4] = {0.f, 0.f, 0.f, 0.f};
+        uint32_t bits = 0u;                                    // all of the row's
         for (int i = 0; i < blocks; ++i) {
             const int ws = i % SPLIT_W_STAGES, as = i % SPLIT_A_STAGES;
             if (!mbar_wait(wfull + 8 * ws, (i / SPLIT_W_STAGES) & 1, p.status, 11)) break;
@@ -217,7 +258,9 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             uint32_t low[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
             for (int j = 0; j < 32; ++j) low[j & 3] |= __float_as_uint(v[j]);
-            const bool wide = __any_sync(0xffffffffu, (((low[0] | low[1]) | (low[2] | low[3])) & 0xffffu) != 0);
+            low[0] = (low[0] | low[1]) | (low[2] | low[3]);
+            bits |= low[0];
+            const bool wide = __any_sync(0xffffffffu, (low[0] & 0xffffu) != 0);
             if (lane == 0) mbar_arrive(wempty + 8 * ws);       // (the vote has seen every lane's loads)
             if (!mbar_wait(aempty + 8 * as, ((i / SPLIT_A_STAGES) & 1) ^ 1, p.status, 12)) break;
             tc_fence_after();
@@ -251,7 +294,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             }
         }
         const float bad = (bad4[0] + bad4[1]) + (bad4[2] + bad4[3]);
-        if (bad != bad) {
+        const bool tiny = (bits & SPLIT_LARGE_BITS) == 0u && ((bits & 0xffffu) != 0u || ((bits & 0x7f800000u) == 0u && (bits & 0x7fffffu) != 0u));
+        if (bad != bad || tiny) {
             s_bad[row] = 1.f;
             s_any = 1.f;
         }
@@ -404,11 +448,12 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         if (gm >= p.m || gn >= p.n) continue;
         const int cols = min(4, p.n - gn);
         if (any != 0.f) {
-            const bool row_bad = p.marked[gm] != 0;
+            const int mark = p.marked[gm];
             for (int j = 0; j < cols; ++j) {
                 float b = s_bad[c + j];
                 for (int s = 0; s < p.splits && p.splits > 1; ++s) b += fr_cluster_load(s_bad + c + j, s);
-                if (row_bad || b != 0.f) v[j] = split_plain_dot(p, gm, gn + j);
+                if (mark == SPLIT_BAD || b != 0.f) v[j] = split_plain_dot(p, gm, gn + j);
+                else if (mark == SPLIT_TINY) v[j] *= 0x1p-64f;
             }
         }
         const size_t at = (size_t)gm * p.ldo + gn;

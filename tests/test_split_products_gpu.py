@@ -74,3 +74,33 @@ def test_values_that_cannot_be_split(k):
     assert torch.equal(got[rows][:, 140], ref[rows][:, 140].float())
     fits = ref[5][cols].abs() < 0.99 * torch.finfo(torch.float32).max
     assert fits.any() and ((got[5][cols][fits].double() - ref[5][cols][fits]).abs() <= 1e-4 * ref[5][cols][fits].abs() + 1e32).all()
+
+
+# Values so small that three bf16 numbers do not hold their 24 bits: rows of x as a whole (and beside ordinary ones), and weight rows, bf16 numbers or
+# not.  2^-21 of a row's norm is three times what k = 4,096 was measured at for ordinary values, and above what sums of 64 rounded terms come to
+# (sqrt(64 / 2) 2^-24 / sqrt(3), a fifth more for adding 64 of them); without care it is 2^-13 here.
+@pytest.mark.parametrize("m,n,k", [(20, 150, 64), (40, 130, 4096), (300, 128, 1028)])
+@pytest.mark.parametrize("exponent", [-120, -100, -140])
+def test_rows_of_very_small_values(m, n, k, exponent):
+    g = torch.Generator(device=DEV).manual_seed(m)
+    x, w = torch.randn(m, k, device=DEV, generator=g), torch.randn(n, k, device=DEV, generator=g)
+
+    def small(rows):
+        return torch.ldexp(rows.double(), torch.tensor(exponent, device=DEV)).float()
+
+    def rows_close(out, a, b):
+        ref = a.double() @ b.double().T
+        assert ((out.double() - ref).norm(dim=1) <= 2.0 ** -21 * ref.norm(dim=1)).all()
+    for some in (slice(None), slice(3, None, 2)):
+        tiny = x.clone()
+        tiny[some] = small(tiny[some])
+        big = w * 2.0 ** 60                                      # (results well within the normal numbers)
+        rows_close(product(tiny, big), tiny, big)
+    for weights in (w, w.bfloat16().float()):
+        tiny = weights.clone()
+        tiny[1::3] = small(tiny[1::3])
+        big = x * 2.0 ** 60
+        rows_close(product(big, tiny).T, tiny, big)
+    zero = x.clone()
+    zero[2] = 0.0
+    assert (product(zero, w)[2] == 0).all()
