@@ -262,7 +262,6 @@ Engine::Engine(const EngineOptions& opt) : impl_(new Impl) {
     cuda_check(cudaSetDevice(e.device), "cudaSetDevice");
     cuda_check(cudaStreamCreateWithFlags(&e.stream, cudaStreamNonBlocking), "cudaStreamCreate");
     e.ops.reset(new Ops(e.device, e.stream));
-    e.ops->leave_norms = true;
     if (opt.profile) e.ops->set_profile(true);
     if (!source) source = random_weights(e.model->named_params(), opt.seed, "BF16", opt.random_on_device);
     e.model->load(*source, *e.ops);

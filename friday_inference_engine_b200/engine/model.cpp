@@ -46,6 +46,10 @@ DecoderModel::DecoderModel(const ModelSpec& s, DType dtype) : spec(s) {
     if (s.vocab_size <= 0 || s.width <= 0) throw ConfigError("a model needs a vocabulary and a width");
     owners = spec.cache_entries();
     for (const auto& ls : spec.layers) layers.emplace_back(build<Block>("block", ls, env));
+    // a norm between two layers may be left to the second one if that takes it (the head does), whoever follows the first
+    for (size_t i = 0; i < spec.program.size(); ++i) layers[(size_t)spec.program[i].layer]->leave_last_norm(true);
+    for (size_t i = 0; i + 1 < spec.program.size(); ++i)
+        if (!layers[(size_t)spec.program[i + 1].layer]->takes_left_norms()) layers[(size_t)spec.program[i].layer]->leave_last_norm(false);
     final_norm.reset(build<Norm>("norm", spec.final_norm, env));
     if (!spec.embed_norm.kind.empty()) embed_norm.reset(build<Norm>("norm", spec.embed_norm, env));
     for (const auto& c : spec.program)

@@ -69,9 +69,10 @@ private:
 // Rows on their way from one product to the next.  Plain rows are a tensor.  Deferred rows are rows whose
 // RMSNorm the product that made them has begun: `t` holds weight (*) x rounded to bf16, `ssq` [parts, rows]
 // each part's share of the rows' sums of squares; the product that takes them finishes the norm by scaling
-// its own rows with 1 / sqrt(sum / width + eps).  Deferred rows without `ssq` (few 32-bit rows) are `source` itself with
-// nothing of the norm begun: the product that takes them does all of it.  Anything else asks Ops::materialize, which runs
-// the norm's kernel on `source`.
+// its own rows with 1 / sqrt(sum / width + eps).  Left rows (deferred without `ssq`; few 32-bit rows) are `source` itself with
+// nothing of the norm begun: the product that takes them does all of it.  Only a part that says so (takes_left_norms) is given
+// left rows, and only a part whose owner says so (leave_norm) returns them.  Anything else asks Ops::materialize, which runs the
+// norm's kernel on `source`.
 struct Rows {
     Tensor t;
     bool deferred = false;
@@ -79,6 +80,7 @@ struct Rows {
     float eps = 0;
     Rows() {}
     Rows(const Tensor& x) : t(x) {}
+    bool left() const { return deferred && !ssq.defined(); }
 };
 
 struct PartOut {
@@ -101,7 +103,6 @@ public:
     cudaStream_t stream() const { return stream_; }
     int sm_count() const { return sms_; }
     Arena* arena = nullptr;                                   // where results come from
-    bool leave_norms = false;                                 // linear_norm may return deferred rows without `ssq` (the engine's step does)
     Tensor alloc(DType dtype, int64_t rows, int64_t cols);
     float* scratch_floats(int64_t n);                         // from the arena
 
@@ -370,9 +371,10 @@ public:
     // no multiple of 128.)
     Tensor linear_alone(const Rows& x, const Tensor& weight, const Tensor* bias = nullptr);
     // linear(...) and the RMSNorm of its result.  For bf16 rows whose sizes allow it the norm is begun in the
-    // product's epilogue and the second result is deferred; otherwise the norm's kernel runs.
+    // product's epilogue and the second result is deferred; otherwise the norm's kernel runs, or, with `leave`, up to 16 32-bit
+    // rows are returned as left rows.
     std::pair<Tensor, Rows> linear_norm(const Rows& x, const Tensor& weight, const Tensor& norm_weight, float eps,
-                                        const Tensor* bias = nullptr, const Tensor* residual = nullptr);
+                                        const Tensor* bias = nullptr, const Tensor* residual = nullptr, bool leave = false);
     // linear(x, weight, bias) followed by rope_kv_write on its result; for up to 64 bf16 rows and a head size that
     // divides 128 both happen in the product's epilogue.
     Tensor qkv_rope_write(const Rows& x, const Tensor& weight, const Tensor* bias, const int* row_seq,

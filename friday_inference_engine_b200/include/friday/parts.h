@@ -299,6 +299,8 @@ public:
     using Part::Part;
     // forward returns residual + out_scale * mix(h); a mixer that runs others side by side sets its members' scales.
     float out_scale = 1.0f;
+    bool leave_norm = false;             // set by an owner whose next part takes left rows (ops.h): the norm `then` may be left to it
+    virtual bool takes_left_norms() const { return false; }        // every product that reads `h` is one of Ops'
     virtual CacheRequest cache_request() const { return CacheRequest(); }
     virtual PartOut forward(Ops& ops, const Rows& h, const Tensor& residual, const StepContext& ctx,
                             const CacheView& view, Norm* then) = 0;
@@ -307,6 +309,8 @@ public:
 class FeedForward : public Part {
 public:
     using Part::Part;
+    bool leave_norm = false;                                       // as a mixer's
+    virtual bool takes_left_norms() const { return false; }
     virtual PartOut forward(Ops& ops, const Rows& h, const Tensor& residual, const StepContext& ctx, Norm* then) = 0;
 };
 
@@ -322,6 +326,8 @@ public:
     using Part::Part;
     virtual CacheRequest cache_request() const { return CacheRequest(); }
     virtual Norm* first_norm() { return nullptr; }       // the norm the block begins with, if the block before may apply it
+    virtual bool takes_left_norms() const { return false; }        // `normed` may be left rows (ops.h)
+    virtual void leave_last_norm(bool) {}                          // whether what follows the block takes them
     // normed: first_norm of x if the caller has it already (else null); then: the norm that follows this block.
     virtual PartOut forward(Ops& ops, const Tensor& x, const Rows* normed, const StepContext& ctx,
                             const CacheView& view, Norm* then) = 0;

@@ -1388,7 +1388,7 @@ Tensor Ops::materialize(const Rows& h) {
 }
 
 std::pair<Tensor, Rows> Ops::linear_norm(const Rows& x, const Tensor& weight, const Tensor& norm_weight, float eps,
-                                         const Tensor* bias, const Tensor* residual) {
+                                         const Tensor* bias, const Tensor* residual, bool leave) {
     const Tensor& xt = x.t;
     check_product(xt, weight);
     const int64_t rows = xt.rows(), n = weight.rows();
@@ -1439,7 +1439,7 @@ std::pair<Tensor, Rows> Ops::linear_norm(const Rows& x, const Tensor& weight, co
         }
     }
     Tensor out = linear(x, weight, bias, residual);
-    if (leave_norms && out.dtype == DType::F32 && rows <= 16 && norm_weight.numel() == n && fusion_enabled()) {
+    if (leave && out.dtype == DType::F32 && rows <= 16 && norm_weight.numel() == n && fusion_enabled()) {
         Rows r(out);                                          // few 32-bit rows: the products that read them do their norm
         r.deferred = true;
         r.eps = eps;

@@ -464,6 +464,7 @@ public:
         if (talking_ && keep_first_ > 0) throw ConfigError("gqa_attention: kept first keys with talking heads are not built");
     }
     CacheRequest cache_request() const override { return CacheRequest::kv(nkv_, hd_, window_, vd_, keep_first_); }
+    bool takes_left_norms() const override { return true; }
     void finalize(Ops& ops) override {
         Mixer::finalize(ops);
         if (slope_base_ <= 0.0) return;
@@ -509,7 +510,7 @@ public:
         Tensor nw;
         float eps;
         if (then && out_scale == 1.0f && residual.dtype == mixed.dtype && then->as_rmsnorm(&nw, &eps)) {
-            auto r = ops.linear_norm(Rows(mixed), w_o, nw, eps, b_o, &residual);
+            auto r = ops.linear_norm(Rows(mixed), w_o, nw, eps, b_o, &residual, leave_norm);
             return PartOut(r.first, r.second);
         }
         return PartOut(ops.linear_residual(Rows(mixed), w_o, b_o, residual, out_scale));
@@ -603,13 +604,14 @@ public:
         declare(name_of("up", "up_proj.weight"), {inner_, e.width}).stack("w_gate_up", 1, 2);
         declare(down_, {e.width, inner_});
     }
+    bool takes_left_norms() const override { return true; }
     PartOut forward(Ops& ops, const Rows& h, const Tensor& residual, const StepContext&, Norm* then) override {
         Tensor inner = ops.linear_swiglu(h, tensor("w_gate_up"), act_);
         Tensor nw;
         float eps;
         if (!residual.defined()) return PartOut(ops.linear(Rows(inner), tensor(down_), nullptr, nullptr, (int)DType::F32));     // the block sums itself
         if (then && residual.dtype == inner.dtype && then->as_rmsnorm(&nw, &eps)) {
-            auto r = ops.linear_norm(Rows(inner), tensor(down_), nw, eps, nullptr, &residual);
+            auto r = ops.linear_norm(Rows(inner), tensor(down_), nw, eps, nullptr, &residual, leave_norm);
             return PartOut(r.first, r.second);
         }
         // a 32-bit stream beside 16-bit activations: the product's result stays 32-bit and is added there
@@ -639,6 +641,7 @@ public:
             const PartSpec& ff = s.part("feed_forward");
             norm2_ = adopt(n2.prefix, build<Norm>("norm", n2, e));
             ffn_ = adopt(ff.prefix, build<FeedForward>("feed_forward", ff, e));
+            mixer_->leave_norm = ffn_->takes_left_norms();
         }
         if (s.parts.count("token_input")) {
             const PartSpec& ti = s.part("token_input");
@@ -668,6 +671,11 @@ public:
         return CacheRequest::flat(all);
     }
     Norm* first_norm() override { return taps_ ? nullptr : norm1_; }        // with a convolution the norm runs inside this block
+    bool takes_left_norms() const override { return taps_ == 0 && mixer_->takes_left_norms(); }
+    void leave_last_norm(bool on) override {
+        if (ffn_) ffn_->leave_norm = on;
+        else mixer_->leave_norm = on;
+    }
 
     PartOut forward(Ops& ops, const Tensor& x, const Rows* normed, const StepContext& ctx, const CacheView& view,
                     Norm* then) override {
