@@ -2,7 +2,8 @@
 //
 // The choices follow what was measured on a B200: a bf16 product goes to the tcgen05
 // kernel whenever its operands' rows start on 16-byte boundaries and to the CUDA-core
-// kernel otherwise (and always in float32: the true 32-bit path uses no tensor cores);
+// kernel otherwise (the true 32-bit path rounds nothing to 16 bits: its products of many rows and its delta rule use the
+// tensor cores on operands split into three bf16 numbers each);
 // one-token steps let norms, rotation and the cache write ride in the products'
 // epilogues; prompts' attention runs both products on tcgen05, one-token steps split
 // the keys over the CTAs of a cluster.
@@ -835,7 +836,11 @@ Tensor Ops::conv_silu_unit(const Tensor& proj, const Tensor& taps, const DeltaSp
 void* Ops::chunk_room(size_t bytes) {
     if (chunks_.bytes() >= bytes) return chunks_.get();
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream_, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return nullptr;
+    if (cudaStreamIsCapturing(stream_, &capturing) != cudaSuccess) {
+        cudaGetLastError();                                    // (the default stream, while another one is captured)
+        return nullptr;
+    }
+    if (capturing != cudaStreamCaptureStatusNone) return nullptr;
     chunks_ = DeviceBuffer();
     try {
         chunks_ = DeviceBuffer(bytes);
