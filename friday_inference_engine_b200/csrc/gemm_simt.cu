@@ -1,8 +1,8 @@
 // out[m][n] = sum_k a[m][k] * w[n][k]  (+ bias[n]) (+ residual[m][n])
 //
 // Matrix product with fp32 multiply-adds: the true 32-bit path of the model (no
-// reduced-precision mode; many rows go to gemm_f32_tc.cuh, which drops no bit of the
-// operands either), and the fallback of the bf16 path for sizes that the tensor-core
+// reduced-precision mode; many rows go to gemm_f32_tc.cuh, which keeps the operands'
+// 24 bits), and the fallback of the bf16 path for sizes that the tensor-core
 // kernel refuses.  Both operands are row-major with k
 // innermost, which is how activations [rows][k] and projection weights [out][in] are
 // stored, so nothing is transposed.  Any m, n, k.  Four kernels:
