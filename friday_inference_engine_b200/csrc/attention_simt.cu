@@ -481,7 +481,8 @@ FR_EXPORT int attention_simt_prompt_supports(const void* q, int q_stride, const 
 // 939; 64 rows 2,414 and 947, 618 and 942; without keys before them 16 rows 4.5 and 8.2, 64 rows 16 and 12).  Over the 303 steps that were measured
 // the tiles, where taken, were never more than 3 % behind, but for 100 rows beside 64 sequences of one (145 and 167).
 FR_EXPORT int attention_simt_prompt_pays(int rows, int n_seqs, int max_q_len, int max_kv_len, int nq, int nkv, int hd, int window, int splits) {
-    if (rows <= 0 || n_seqs <= 0 || nkv <= 0 || nq < nkv || splits <= 0 || nq / nkv > PT_MOST_ROWS) return 0;
+    // (fewer new tokens than were measured stay where they are)
+    if (rows <= 0 || n_seqs <= 0 || max_q_len < 16 || nkv <= 0 || nq < nkv || splits <= 0 || nq / nkv > PT_MOST_ROWS) return 0;
     const int sms = fr_sm_count() > 0 ? fr_sm_count() : 148, group = nq / nkv, size = hd > 64 ? 2 : hd > 32 ? 1 : 0;
     const double seen = window > 0 && window < max_kv_len ? window : max_kv_len;
     double keys = max_kv_len - 0.5 * max_q_len;               // of a row, about

@@ -56,7 +56,8 @@ def splits_of(rows, heads, keys):          # of the keys where a warp has a row 
     ([16], 0, 28, 4, 128, 0, 0), ([16], 8000, 28, 4, 128, 0, 0), ([20], 300, 28, 4, 128, 0, 0), ([48], 1000, 28, 4, 128, 0, 1), ([333], 0, 28, 4, 128, 0, 1),
     ([333], 8000, 28, 4, 128, 0, 1), ([64], 8000, 8, 8, 128, 0, 0), ([200], 8000, 8, 8, 128, 0, 1), ([100], 8000, 3, 1, 32, 0, 0), ([333], 8000, 3, 1, 32, 0, 1),
     ([16] * 8, 1000, 28, 4, 128, 0, 1), ([16] + [1] * 31, 500, 16, 16, 64, 0, 0), ([300, 33], 0, 28, 4, 128, 0, 1), ([16], 4000, 28, 4, 128, 512, 0),
-    ([300], 4000, 28, 4, 128, 512, 1), ([1] * 64 + [100], 2000, 16, 16, 64, 0, 0), ([256] * 8, 0, 3, 1, 32, 0, 1), ([64] * 16, 2000, 64, 1, 128, 0, 1),
+    ([300], 4000, 28, 4, 128, 512, 1), ([1] * 64 + [100], 2000, 16, 16, 64, 0, 0), ([256] * 8, 0, 3, 1, 32, 0, 1), ([64] * 16, 2000, 64, 1, 128, 0, 1), ([15] * 64, 2000, 28, 4, 128, 0, 0),
+    ([16] * 64, 2000, 28, 4, 128, 0, 1),
 ])
 def test_fp32_attention_of_prompts(lens, before, nq, nkv, hd, window, want):
     keys = max(lens) + before
